@@ -9,12 +9,12 @@
 // therefore what lv_create + lv_run (and the CPU oracle) give for that graph
 // alone.
 //
-// Execution.  One CTA runs one graph from start to finish; CTAs take graphs
-// from a device queue ordered by decreasing entry count, so one launch covers
-// the whole batch and the large graphs start first.  A graph's state lives in
-// slices of batch-wide arrays at the graph's own vertex and entry offsets, and
-// the steps of the level loop are separated by CTA barriers instead of kernel
-// launches and host round trips.  Vertex ids stay global at every level: the
+// Execution.  One CTA, or a thread-block cluster of up to 16 for a large
+// graph, runs one graph from start to finish; graphs start in decreasing
+// entry count.  A graph's state lives in slices of batch-wide arrays at the
+// graph's own vertex and entry offsets, and the steps of the level loop are
+// separated by CTA or cluster barriers instead of kernel launches and host
+// round trips.  Vertex ids stay global at every level: the
 // level-L vertices of a graph whose first vertex is v0 are v0 .. v0 + V_L - 1.
 //
 // Tables.  A vertex of degree <= DW (or a merged row of at most DW entries)
@@ -23,9 +23,9 @@
 // slots fit, else with the graph's own global table of 2^ceil(log2(2 V0))
 // slots.  Every table is empty between uses.
 //
-// Coherence.  Rows of aggregated levels and the community state are written
-// inside the launch, so they are read with ordinary (coherent) loads; only the
-// caller's level-0 CSR goes through the read-only cache.
+// Coherence.  Rows of aggregated levels, the fixed-point weights and the
+// community state are written inside the launch, so they are read with
+// ordinary (coherent) loads.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -33,32 +33,48 @@
 #include <string>
 #include <vector>
 
+// one kernel holds the whole level loop: near-tie comparisons stay out of line
+#define LV_EXACT_CALL 1
 #include "../../include/louvain_b200.h"
 #include "lv_internal.h"
 
 namespace lv {
 namespace {
 
-// 512 threads and 2 CTAs per SM (64 registers): 16 warps per graph shorten
-// the largest graphs' latency, which bounds the launch, and 32 resident warps
-// per SM raise throughput; measured against 256 x 3 (80 registers) on the
-// 4096-graph batch: 469 ms vs 713 ms per launch.
-#ifndef LV_BATCH_THREADS
-#define LV_BATCH_THREADS 512
-#endif
-#ifndef LV_BATCH_MINB
-#define LV_BATCH_MINB 2
-#endif
-constexpr int BT = LV_BATCH_THREADS;   // threads per CTA
-constexpr int BW = BT / 32;            // warps per CTA
+// 512 threads and 2 CTAs per SM (64 registers).  Smaller CTAs were measured
+// for small graphs (8 CTAs of 128 threads per SM): 2048 planted graphs of 100
+// to 1500 vertices took 7.7 ms against 5.8 ms, since eight graphs at different
+// points of the level loop do not share the instruction cache.
+constexpr int BT = 512;             // threads per CTA
+constexpr int BW = BT / 32;         // warps per CTA
 constexpr int WTAB = 256;           // slots of one warp's table
 constexpr int DW = WTAB / 2;        // degree / merged-row bound served by a warp table
 constexpr int CTAB = BW * WTAB;     // slots of the CTA table (the warp tables together)
+constexpr int WIDE_CLAIMS = 160;    // distinct communities a warp accepts in a longer row
+// Work split of a launch (plan_launch): a team's CTA takes TEAM_PART of the
+// entries that one resident CTA would have if the batch were spread evenly
+// over the GPU.  256 planted graphs of 100 to 50,000 vertices took 27.0 /
+// 25.9 / 24.8 / 25.4 / 34.3 ms with 0.3 / 0.5 / 0.7 / 1 / 2 (152 ms with one
+// CTA per graph, the largest graph's time), 2048 of 100 to 1500 vertices 7.1 /
+// 6.0 / 5.8 / 5.8 / 5.8 ms.  A lone graph is split down to 2048 entries per CTA.
+constexpr double TEAM_PART = 0.7, TEAM_MIN_PART = 2048.0;
 // Iteration caps that keep a launch bounded; a graph that reaches one stops
 // with LV_ERR_DEVICE (the rule itself has no cap: with min_gain <= 0 a sweep
 // loop that keeps moving at zero gain would not end).
 constexpr int SWEEP_CAP = 4096;
 constexpr int LEVEL_CAP = 256;
+
+// CTAs of the largest team (a thread-block cluster) that one graph runs on.
+constexpr int TEAM_MAX = 16;
+
+// Exchange area of a team in global memory (zero before the first launch,
+// counters returned to zero after each use).
+struct TeamScratch {
+    u64 red[2][TEAM_MAX][6];   // per-CTA parts of a team reduction, double-buffered
+    u64 drift;                 // drift of the level so far (GState::drift_of)
+    int32_t cnt[16], cur[16];  // bucket sizes and cursors
+    int32_t nbig;
+};
 
 struct BatchParams {
     // the caller's block-diagonal CSR (read-only during the launch)
@@ -68,19 +84,20 @@ struct BatchParams {
     const int32_t *gptr;       // [G + 1] first vertex of each graph
     const int32_t *order;      // [G] graphs by decreasing entry count
     const int64_t *tbl_off;    // [G + 1] first slot of each graph's global table
-    int32_t G;
+    int32_t lo;                // the launch's first graph in order
     int32_t max_sweeps;
     double min_gain;
     // per vertex (V entries; mstart / roff: V + G, the slice of graph g starts at v0 + g)
     int32_t *comm, *newc, *size, *blist, *newid, *members, *o2c, *mstart, *roff;
     int32_t *rs[2], *re[2];    // aggregated levels: row v = [rs[v], re[v])
     u64 *k, *S;
+    u64 *lim;                  // a vertex keeps its community while the level's drift is below lim
     // per entry (E entries): aggregated rows, ping-pong
     int32_t *colb[2];
     u64 *wb[2];
     int32_t *tkeys;            // global tables (-1 / 0 between uses)
     u64 *tvals;
-    int32_t *next;             // queue head
+    TeamScratch *scratch;      // one per graph that runs on a team, in order
     // results
     int32_t *out_comm;         // [V] community of each vertex, numbered within its graph
     double *q;
@@ -89,19 +106,7 @@ struct BatchParams {
     u64 *t_start, *t_end;      // %globaltimer (ns) around each graph
 };
 
-struct BatchSmem {
-    u64 vals[CTAB];
-    int32_t keys[CTAB];
-    u64 red[2 * BW];
-    double bgd[BW];
-    u64 be[BW], bS[BW], beo[BW];
-    int32_t bc[BW];
-    int32_t scan[BW];
-    int32_t bcnt[16], boff[16], bcur[16];   // bucket b: [2b] degree <= DW, [2b + 1] larger
-    int32_t gi, err, nbig, cnt;
-};
-
-// A graph's current level and totals (the same in every thread of the CTA).
+// A graph's current level and totals (the same in every thread of the team).
 struct GState {
     int32_t g, v0, V0, V;
     int64_t e0;     // first entry of the graph in the caller's CSR
@@ -110,6 +115,12 @@ struct GState {
     u64 T;
     double scale;
     int cur;        // -1: level 0 (the caller's CSR), else the buffer of the level's rows
+    int dsh;        // drift is counted in units of 2^dsh
+    float dunit;    // 2^-dsh
+    bool narrow;    // level-0 weights fit 32 bits
+    bool sym;       // every entry has its mirror entry (same weight): vertices may be skipped
+    // what one move of a vertex of weight k adds to the drift: an upper bound of 2 k
+    __device__ __forceinline__ u64 drift_of(u64 k) const { return ((2 * k) >> dsh) + 1; }
 };
 
 struct Acc {
@@ -119,30 +130,21 @@ struct Acc {
     double q;
 };
 
-// Level views: row bounds, column and fixed-point weight of an entry.
-template <typename WT>
-struct Lv;
-template <>
-struct Lv<float> {
-    const int32_t *rp;
-    const int32_t *col;
-    const float *w;
-    double scale;
-    __device__ __forceinline__ int32_t r0(int32_t v) const { return __ldg(rp + v); }
-    __device__ __forceinline__ int32_t r1(int32_t v) const { return __ldg(rp + v + 1); }
-    __device__ __forceinline__ int32_t c(int64_t e) const { return __ldg(col + e); }
-    __device__ __forceinline__ u64 x(int64_t e) const { return wfix(w, e, scale); }
-};
-template <>
-struct Lv<u64> {
+// A level's rows: [rs[v], re[v]) in col and in w32 (level 0, when its
+// fixed-point weights fit 32 bits) or w64.  Level 0 reads the fixed-point
+// weights that level_setup wrote, so that one code path serves every level
+// (the kernel's code has to fit the instruction cache) and no sweep converts
+// floats.
+struct Rows {
     const int32_t *rs;
     const int32_t *re;
     const int32_t *col;
-    const u64 *w;
+    const uint32_t *w32;
+    const u64 *w64;
     __device__ __forceinline__ int32_t r0(int32_t v) const { return rs[v]; }
     __device__ __forceinline__ int32_t r1(int32_t v) const { return re[v]; }
     __device__ __forceinline__ int32_t c(int64_t e) const { return col[e]; }
-    __device__ __forceinline__ u64 x(int64_t e) const { return w[e]; }
+    __device__ __forceinline__ u64 x(int64_t e) const { return w32 ? (u64)w32[e] : w64[e]; }
 };
 
 // Update-order bucket of a degree (modularity_optimisation.cuh:7-8).
@@ -168,31 +170,224 @@ __device__ __forceinline__ int table_lg(int32_t bound) {
     return lg < 1 ? 1 : lg;
 }
 
-// ---- CTA-wide reductions and scan (every thread gets the result) ----
-__device__ __forceinline__ u64 block_sum_u64(u64 x, BatchSmem &sm) {
-    x = warp_sum_u64(x);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sm.red[threadIdx.x >> 5] = x;
-    __syncthreads();
-    u64 t = 0;
-    for (int i = 0; i < BW; ++i) t += sm.red[i];
-    return t;
+// ---- reductions and scan (every thread gets the result) ----
+struct Totals5 {
+    u64 a, b;      // wrapping sums
+    u128 s2;       // exact sum
+    u64 err;       // OR
+};
+
+// ---- which vertices need a decision ----
+// A vertex v that was evaluated and stayed, with slack = T e_own - max(0, max_C
+// G(C)) >= 0, stays as long as no neighbour changes community and Sigma_tot
+// moves little: then every e_C is unchanged and G(C) = T e_C + k (S_own - k -
+// S_C) grows by at most k times the total change of Sigma_tot, to which a move
+// of a vertex of weight k' adds 2 k'.  The level's drift sums an upper bound
+// of 2 k' over its moves, and v is skipped while drift < lim[v] =
+// drift at evaluation + floor(slack / k) + 1 (in drift units).  A move sets
+// lim to 0 (evaluate next time) for the mover and for its neighbours; a vertex
+// that was alone in its community when evaluated is never skipped, since the
+// singleton guard may have hidden candidates from its slack.  Decisions are
+// therefore exactly those of evaluating every vertex; the batch of 256 planted
+// graphs of 100 to 50,000 vertices takes 30.7 ms with skipping and 40.9 ms
+// without.
+__device__ __forceinline__ u64 skip_limit(const MoveCtx &m, const Best &b, u64 drift, float dunit) {
+    constexpr u64 FAR = (u64)1 << 62;
+    if (m.kv == 0) return FAR;
+    // a lower bound of slack / k in drift units: gain_err bounds the estimate
+    // gd, and 2^-20 covers the roundings of the remaining operations
+    const double g = b.c == m.own ? 0.0 : fmax(0.0, b.gd + gain_err(m, b));
+    const double slack = fmax(0.0, m.Td * (double)b.eo * (1.0 - 0x1p-48) - g);
+    const float d = __fdividef((float)slack, (float)m.kvd) * dunit * (1.0f - 0x1p-20f);
+    return d < 0x1p61f ? drift + (u64)d + 1 : FAR;
 }
 
-__device__ __forceinline__ u128 block_sum_u128(u128 x, BatchSmem &sm) {
-    x = warp_sum_u128(x);
+// calculateModularity (modularity_optimisation.cu:395-401) from exact totals.
+__device__ __forceinline__ double modularity_from(const GState &gs, u64 e_own, u128 s2) {
+    return q_from_parts_dev(gs.T, e_own, (u64)(s2 >> 64), (u64)s2);
+}
+
+// One entry's share of the symmetry check: the sum over all entries of
+// mix(row, col, w) - mix(col, row, w) is zero when the entries and their
+// mirror images are the same multiset (and otherwise zero by a chance of
+// 2^-64 only).
+__device__ __forceinline__ u64 sym_mix(uint32_t a, uint32_t b, uint32_t w) {
+    u64 x = ((u64)a << 32 | b) * 0x9E3779B97F4A7C15ull + w;
+    x ^= x >> 29;
+    x *= 0xD6E8FEB86659FD93ull;
+    return x ^ (x >> 32);
+}
+
+// Group tables: the sum of a slot is kept in three 32-bit counters of 22-bit
+// pieces, so that an add is two or three shared atomics without a returned
+// value or a carry; exact for up to 1024 adds per slot (rows of at most DW
+// entries) and weights up to 2^62 (T <= 2^62).
+struct PieceSlots {
+    int32_t *keys;
+    uint32_t *lo, *mid, *hi;
+    // adds w to key's sum; the slot when it was newly claimed, else -1
+    __device__ __forceinline__ int32_t insert(int lg, int32_t key, u64 w, int *err) const {
+        const uint32_t mask = (1u << lg) - 1u;
+        uint32_t s = hash_slot(key, lg);
+        int32_t claimed = -1;
+        for (uint32_t p = 0;; ++p) {
+            const int32_t k = ((volatile int32_t *)keys)[s];
+            if (k == key) break;
+            if (k < 0) {
+                const int32_t prev = atomicCAS(keys + s, -1, key);
+                if (prev < 0) claimed = (int32_t)s;
+                if (prev < 0 || prev == key) break;
+            }
+            if (p == mask) {
+                atomicOr(err, DEVERR_HASH_FULL);
+                return -1;
+            }
+            s = (s + 1u) & mask;
+        }
+        atomicAdd(lo + s, (uint32_t)w & 0x3FFFFFu);
+        const uint32_t b = (uint32_t)(w >> 22) & 0x3FFFFFu, c = (uint32_t)(w >> 44);
+        if (b) atomicAdd(mid + s, b);
+        if (c) atomicAdd(hi + s, c);
+        return claimed;
+    }
+    // the sum of slot s, which is emptied
+    __device__ __forceinline__ u64 take(int s) const {
+        const u64 x = (u64)lo[s] + ((u64)mid[s] << 22) + ((u64)hi[s] << 44);
+        keys[s] = -1;
+        lo[s] = 0;
+        mid[s] = 0;
+        hi[s] = 0;
+        return x;
+    }
+};
+static_assert(DW <= 1024, "pieces of 22 bits in 32-bit counters");
+
+// The level loop of one graph.
+struct Loop {
+struct BatchSmem {
+    u64 vals[CTAB];            // 64-bit sums, or two counters of PieceSlots per slot
+    uint32_t hi[CTAB];         // the third counter
+    int32_t keys[CTAB];
+    u64 red[BW][5];
+    u64 tot[5];
+    u64 drift;
+    double bgd[BW];
+    u64 be[BW], bS[BW], beo[BW];
+    int32_t bc[BW];
+    int32_t scan[BW];
+    int32_t bcnt[16], boff[16], bcur[16];   // bucket b: [2b] degree <= DW, [2b + 1] larger
+    int32_t err, nbig, cnt;
+    uint8_t ord[BW][32];       // a warp's chunk: lanes holding vertices to decide, in order
+    uint8_t occ[BW][DW];       // claimed slots of the warp's group tables
+};
+
+// The CTAs that run one graph together: this CTA alone (nc == 1), or every
+// CTA of its cluster.  Steps of the level loop are separated by sync(): the
+// cluster barrier orders the team's accesses to the graph's global arrays
+// (release on arrival, acquire on the wait).  Every branch around a sync()
+// depends only on values that all threads of the team agree on (the graph's
+// sizes and reduced totals), so the team's CTAs pass the same barriers.
+struct Team {
+    int32_t rank, nc;
+    int par;                   // which half of scratch->red the next reduction uses
+    TeamScratch *scr;
+    __device__ __forceinline__ void sync() const {
+        if (nc == 1) {
+            __syncthreads();
+        } else {
+            asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::
+                             : "memory");
+        }
+    }
+    __device__ __forceinline__ int32_t tid() const { return rank * BT + (int32_t)threadIdx.x; }
+    __device__ __forceinline__ int32_t threads() const { return nc * BT; }
+    __device__ __forceinline__ int32_t warp() const { return rank * BW + (int32_t)(threadIdx.x >> 5); }
+    __device__ __forceinline__ int32_t warps() const { return nc * BW; }
+};
+
+// Sums over the CTA (warp 0 combines the warps' parts); contains barriers.
+static __device__ __forceinline__ Totals5 block_totals(Totals5 x, BatchSmem &sm) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    x.a = warp_sum_u64(x.a);
+    x.b = warp_sum_u64(x.b);
+    x.s2 = warp_sum_u128(x.s2);
+    x.err = __reduce_or_sync(FULL, (unsigned)x.err);
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) {
-        sm.red[2 * (threadIdx.x >> 5)] = (u64)(x >> 64);
-        sm.red[2 * (threadIdx.x >> 5) + 1] = (u64)x;
+    if (lane == 0) {
+        sm.red[warp][0] = x.a;
+        sm.red[warp][1] = x.b;
+        sm.red[warp][2] = (u64)(x.s2 >> 64);
+        sm.red[warp][3] = (u64)x.s2;
+        sm.red[warp][4] = x.err;
     }
     __syncthreads();
-    u128 t = 0;
-    for (int i = 0; i < BW; ++i) t += ((u128)sm.red[2 * i] << 64) | (u128)sm.red[2 * i + 1];
+    if (warp == 0) {
+        Totals5 y{};
+        if (lane < BW) {
+            y.a = sm.red[lane][0];
+            y.b = sm.red[lane][1];
+            y.s2 = ((u128)sm.red[lane][2] << 64) | (u128)sm.red[lane][3];
+            y.err = sm.red[lane][4];
+        }
+        y.a = warp_sum_u64(y.a);
+        y.b = warp_sum_u64(y.b);
+        y.s2 = warp_sum_u128(y.s2);
+        y.err = __reduce_or_sync(FULL, (unsigned)y.err);
+        if (lane == 0) {
+            sm.tot[0] = y.a;
+            sm.tot[1] = y.b;
+            sm.tot[2] = (u64)(y.s2 >> 64);
+            sm.tot[3] = (u64)y.s2;
+            sm.tot[4] = y.err;
+        }
+    }
+    __syncthreads();
+    Totals5 t;
+    t.a = sm.tot[0];
+    t.b = sm.tot[1];
+    t.s2 = ((u128)sm.tot[2] << 64) | (u128)sm.tot[3];
+    t.err = sm.tot[4];
     return t;
 }
 
-__device__ __forceinline__ int block_max_i32(int x, BatchSmem &sm) {
+// Sums over the team.  Each CTA writes its part to the scratch area and reads
+// all parts after the barrier; the next reduction uses the other half, and
+// the one after that is separated from this one's reads by a barrier.
+static __device__ __forceinline__ Totals5 team_totals(Totals5 x, Team &t, BatchSmem &sm) {
+    x = block_totals(x, sm);
+    if (t.nc == 1) return x;
+    u64(*red)[6] = t.scr->red[t.par];
+    t.par ^= 1;
+    if (threadIdx.x == 0) {
+        red[t.rank][0] = x.a;
+        red[t.rank][1] = x.b;
+        red[t.rank][2] = (u64)(x.s2 >> 64);
+        red[t.rank][3] = (u64)x.s2;
+        red[t.rank][4] = x.err;
+    }
+    t.sync();
+    const int lane = threadIdx.x & 31;
+    Totals5 y{};
+    if (lane < t.nc) {
+        y.a = __ldcg(&red[lane][0]);
+        y.b = __ldcg(&red[lane][1]);
+        y.s2 = ((u128)__ldcg(&red[lane][2]) << 64) | (u128)__ldcg(&red[lane][3]);
+        y.err = __ldcg(&red[lane][4]);
+    }
+    y.a = warp_sum_u64(y.a);
+    y.b = warp_sum_u64(y.b);
+    y.s2 = warp_sum_u128(y.s2);
+    y.err = __reduce_or_sync(FULL, (unsigned)y.err);
+    return y;
+}
+
+static __device__ __forceinline__ u64 block_sum_u64(u64 x, BatchSmem &sm) {
+    Totals5 t{};
+    t.a = x;
+    return block_totals(t, sm).a;
+}
+
+static __device__ __forceinline__ int block_max_i32(int x, BatchSmem &sm) {
     for (int off = 16; off > 0; off >>= 1) x = max(x, __shfl_xor_sync(FULL, x, off));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) sm.scan[threadIdx.x >> 5] = x;
@@ -203,14 +398,33 @@ __device__ __forceinline__ int block_max_i32(int x, BatchSmem &sm) {
 }
 
 // Exclusive scan of get(0 .. n-1); put(i, prefix, value) for each i; returns
-// the total.  Each index is read and written by the same thread.
+// the total.  Each index is read and written by the same thread, and each CTA
+// of a team scans its own range after the ranges' totals were exchanged.
 template <class Get, class Put>
-__device__ int32_t block_scan(int32_t n, Get get, Put put, BatchSmem &sm) {
+static __device__ int32_t team_scan(int32_t n, Get get, Put put, Team &t, BatchSmem &sm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int32_t carry = 0;
-    for (int32_t base = 0; base < n; base += BT) {
+    int32_t lo = 0, hi = n, carry = 0, all = -1;
+    if (t.nc > 1) {
+        const int32_t part = (n + t.nc - 1) / t.nc;
+        lo = min(n, t.rank * part);
+        hi = min(n, lo + part);
+        u64 s = 0;
+        for (int32_t i = lo + threadIdx.x; i < hi; i += BT) s += (u64)get(i);
+        s = block_sum_u64(s, sm);
+        u64(*red)[6] = t.scr->red[t.par];
+        t.par ^= 1;
+        if (threadIdx.x == 0) red[t.rank][0] = s;
+        t.sync();
+        all = 0;
+        for (int r = 0; r < t.nc; ++r) {
+            const int32_t x = (int32_t)__ldcg(&red[r][0]);
+            carry += r < t.rank ? x : 0;
+            all += x;
+        }
+    }
+    for (int32_t base = lo; base < hi; base += BT) {
         const int32_t i = base + threadIdx.x;
-        const int32_t x = i < n ? get(i) : 0;
+        const int32_t x = i < hi ? get(i) : 0;
         int32_t inc = x;
         for (int off = 1; off < 32; off <<= 1) {
             const int32_t y = __shfl_up_sync(FULL, inc, off);
@@ -221,134 +435,142 @@ __device__ int32_t block_scan(int32_t n, Get get, Put put, BatchSmem &sm) {
         __syncthreads();
         int32_t pre = 0, tot = 0;
         for (int j = 0; j < BW; ++j) {
-            const int32_t t = sm.scan[j];
-            pre += j < warp ? t : 0;
-            tot += t;
+            const int32_t y = sm.scan[j];
+            pre += j < warp ? y : 0;
+            tot += y;
         }
-        if (i < n) put(i, carry + pre + inc - x, x);
+        if (i < hi) put(i, carry + pre + inc - x, x);
         carry += tot;
     }
-    __syncthreads();
-    return carry;
+    t.sync();
+    return t.nc > 1 ? all : carry;
+}
+
+// List entries per chunk when nw warps share n of them: at most 32, the same
+// number of chunks for every warp, as nearly as multiples of g allow.
+static __device__ __forceinline__ int32_t chunk_of(int32_t n, int32_t nw, int32_t g) {
+    const int32_t rounds = max(1, (n + nw * 32 - 1) / (nw * 32));
+    return min(32, ((n + nw * rounds - 1) / (nw * rounds) + g - 1) / g * g);
 }
 
 // ---- move phase ----
-// Vertices of one bucket with degree <= 2^(LG-1): a group of W lanes per
-// vertex (32/W vertices per warp at a time) and a table of 2^LG slots per
-// group inside the warp's table.  U entries per lane are in flight at a
-// time (U column loads, then U community gathers), and the next vertex's
-// row bounds and community are loaded while the current one is evaluated.
-template <typename WT, int W, int LG, int U>
-__device__ void decide_groups(const Lv<WT> &L, const BatchParams &P, const GState &gs,
-                              const int32_t *list, int32_t n, BatchSmem &sm) {
+// Vertices of one bucket with degree <= 2^(lg-1): a warp takes chunks of the
+// list (32 vertices, or fewer when the list is short for the team's warps),
+// loads the headers of the vertices that need a decision (one per lane) and
+// decides them with W lanes each (32/W at a time) and a table of 2^lg slots
+// per group inside the warp's table.  U entries per lane are in flight at a
+// time (U column loads, then U community gathers).
+template <int W, int U>
+static __device__ void decide_groups(const Rows &L, const BatchParams &P, const GState &gs, const Team &t,
+                              const int32_t *list, int32_t n, int lg, u64 drift, BatchSmem &sm) {
     constexpr int GPW = 32 / W;
-    constexpr int NSLOT = 1 << LG;
-    constexpr int EU = (NSLOT / W) < 4 ? (NSLOT / W) : 4;   // table slots per lane in flight
-    constexpr int32_t STRIDE = BW * GPW;
-    static_assert(GPW * NSLOT <= WTAB, "group tables fit the warp's table");
+    constexpr int GTAB = WTAB / GPW;   // slots of one group's table, of which 2^lg are used
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int grp = lane / W, gl = lane % W;
-    int32_t *keys = sm.keys + warp * WTAB + grp * NSLOT;
-    u64 *vals = sm.vals + warp * WTAB + grp * NSLOT;
-    int32_t i = warp * GPW + grp;
-    int32_t v = -1, own = -1, r0 = 0, r1 = 0;
-    u64 kv = 0;
-    if (i < n) {
-        v = list[i];
-        r0 = L.r0(v);
-        r1 = L.r1(v);
-        own = P.comm[v];
-        kv = P.k[v];
-    }
-    for (int32_t i0 = warp * GPW; i0 < n; i0 += STRIDE) {
-        const int32_t inext = i + STRIDE;
-        const int32_t vnext = inext < n ? list[inext] : -1;
-        u64 sown = 0;
-        bool single = false;
-        if (v >= 0) {
-            sown = P.S[own];
-            single = P.size[own] == 1;
+    const unsigned gmask = W == 32 ? FULL : (((1u << (W & 31)) - 1u) << (grp * W));
+    PieceSlots tb;
+    tb.keys = sm.keys + warp * WTAB + grp * GTAB;
+    tb.lo = reinterpret_cast<uint32_t *>(sm.vals + warp * WTAB) + grp * GTAB;
+    tb.mid = tb.lo + WTAB;
+    tb.hi = sm.hi + warp * WTAB + grp * GTAB;
+    uint8_t *occ = sm.occ[warp] + grp * (DW / GPW);
+    uint8_t *ord = sm.ord[warp];
+    const int32_t nw = t.warps();
+    const int32_t cs = chunk_of(n, nw, GPW);
+    for (int32_t c0 = t.warp() * cs; c0 < n; c0 += nw * cs) {
+        const int32_t idx = c0 + lane;
+        int32_t lv = -1, lr0 = 0, lr1 = 0, lown = -1;
+        u64 lkv = 0, lsown = 0;
+        bool need = false, lsingle = false;
+        if (lane < cs && idx < n) {
+            lv = list[idx];
+            need = drift >= P.lim[lv];
         }
-        u64 eo = 0;
-        for (int32_t base = r0 + gl; base < r1; base += U * W) {
-            int32_t jj[U];
-            u64 xx[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int32_t e = base + u * W;
-                jj[u] = -1;
-                xx[u] = 0;
-                if (e < r1) {
-                    jj[u] = L.c(e);
-                    xx[u] = L.x(e);
-                }
-            }
-            int32_t cc[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) cc[u] = (jj[u] >= 0 && jj[u] != v) ? P.comm[jj[u]] : -1;
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (cc[u] < 0) continue;
-                if (cc[u] == own) eo += xx[u];
-                else table_insert<0>(keys, vals, LG, cc[u], xx[u], &sm.err);
-            }
-        }
-        // the next vertex's row bounds, community and weight (its id has arrived)
-        int32_t nr0 = 0, nr1 = 0, nown = -1;
-        u64 nkv = 0;
-        if (vnext >= 0) {
-            nr0 = L.r0(vnext);
-            nr1 = L.r1(vnext);
-            nown = P.comm[vnext];
-            nkv = P.k[vnext];
+        const unsigned mask = __ballot_sync(FULL, need);
+        if (!mask) continue;
+        if (need) {
+            lr0 = L.r0(lv);
+            lr1 = L.r1(lv);
+            lown = P.comm[lv];
+            lkv = P.k[lv];
+            lsown = P.S[lown];
+            lsingle = P.size[lown] == 1;
+            ord[__popc(mask & ((1u << lane) - 1u))] = (uint8_t)lane;
         }
         __syncwarp();
-        const MoveCtx m = move_ctx(own, single, gs.T, kv, sown);
-        Best b = best_init(own);
-        b.eo = eo;
-        for (int s0 = gl; s0 < NSLOT; s0 += EU * W) {
-            int32_t cc[EU];
-            u64 ee[EU];
+        const int cnt = __popc(mask);
+        for (int q0 = 0; q0 < cnt; q0 += GPW) {
+            const bool have = q0 + grp < cnt;
+            const int src = have ? ord[q0 + grp] : 0;
+            int32_t v = __shfl_sync(FULL, lv, src), own = __shfl_sync(FULL, lown, src);
+            int32_t r0 = __shfl_sync(FULL, lr0, src), r1 = __shfl_sync(FULL, lr1, src);
+            const u64 kv = __shfl_sync(FULL, lkv, src), sown = __shfl_sync(FULL, lsown, src);
+            const bool single = __shfl_sync(FULL, (int)lsingle, src) != 0;
+            if (!have) {
+                v = -1;
+                own = -1;
+                r0 = r1 = 0;
+            }
+            u64 eo = 0;
+            int nocc = 0;
+            // every lane of the warp takes the same number of steps
+            const int steps = (int)__reduce_max_sync(FULL, (unsigned)((r1 - r0 + U * W - 1) / (U * W)));
+            for (int st = 0; st < steps; ++st) {
+                const int32_t base = r0 + gl + st * U * W;
+                int32_t jj[U];
+                u64 xx[U];
 #pragma unroll
-            for (int u = 0; u < EU; ++u) {
-                const int s = s0 + u * W;
-                cc[u] = keys[s];
-                ee[u] = 0;
-                if (cc[u] >= 0) {
-                    ee[u] = vals[s];
-                    keys[s] = -1;
-                    vals[s] = 0;
+                for (int u = 0; u < U; ++u) {
+                    const int32_t e = base + u * W;
+                    jj[u] = -1;
+                    xx[u] = 0;
+                    if (e < r1) {
+                        jj[u] = L.c(e);
+                        xx[u] = L.x(e);
+                    }
+                }
+                int32_t cc[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) cc[u] = (jj[u] >= 0 && jj[u] != v) ? P.comm[jj[u]] : -1;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    int32_t claimed = -1;
+                    if (cc[u] >= 0) {
+                        if (cc[u] == own) eo += xx[u];
+                        else claimed = tb.insert(lg, cc[u], xx[u], &sm.err);
+                    }
+                    // the group's claimed slots are listed, so that only they are evaluated and emptied
+                    const unsigned bal = __ballot_sync(FULL, claimed >= 0) & gmask;
+                    if (claimed >= 0) occ[nocc + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)claimed;
+                    nocc += __popc(bal);
                 }
             }
-            u64 SS[EU];
-            int32_t zz[EU];
-#pragma unroll
-            for (int u = 0; u < EU; ++u) {
-                SS[u] = cc[u] >= 0 ? P.S[cc[u]] : 0;
-                zz[u] = (cc[u] >= 0 && guard_needs_size(m, cc[u])) ? P.size[cc[u]] : 0;
+            __syncwarp();
+            const MoveCtx m = move_ctx(own, single, gs.T, kv, sown);
+            Best b = best_init(own);
+            b.eo = eo;
+            for (int i = gl; i < nocc; i += W) {
+                const int s = occ[i];
+                const int32_t c = tb.keys[s];
+                const u64 Sc = P.S[c];
+                const int32_t szc = guard_needs_size(m, c) ? P.size[c] : 0;
+                eval_loaded(c, tb.take(s), Sc, szc, m, b);
             }
-#pragma unroll
-            for (int u = 0; u < EU; ++u)
-                if (cc[u] >= 0) eval_loaded(cc[u], ee[u], SS[u], zz[u], m, b);
+            __syncwarp();
+            group_reduce_best(m, b, W);
+            if (v >= 0 && gl == 0) {
+                u64 d;
+                const int32_t nc = move_decision(m, b, &d);
+                P.newc[v] = nc;
+                P.lim[v] = (nc == own && gs.sym && !single) ? skip_limit(m, b, drift, gs.dunit) : 0;
+            }
         }
         __syncwarp();
-        group_reduce_best(m, b, W);
-        if (v >= 0 && gl == 0) {
-            u64 d;
-            P.newc[v] = move_decision(m, b, &d);
-        }
-        i = inext;
-        v = vnext;
-        r0 = nr0;
-        r1 = nr1;
-        own = nown;
-        kv = nkv;
     }
 }
 
 // One vertex of degree > DW by the whole CTA.
-template <typename WT>
-__device__ void decide_cta(const Lv<WT> &L, const BatchParams &P, const GState &gs, int32_t v,
+static __device__ void decide_cta(const Rows &L, const BatchParams &P, const GState &gs, int32_t v, u64 drift,
                            BatchSmem &sm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int32_t r0 = L.r0(v), r1 = L.r1(v);
@@ -404,10 +626,109 @@ __device__ void decide_cta(const Lv<WT> &L, const BatchParams &P, const GState &
         group_reduce_best(m, x, 32);
         if (lane == 0) {
             u64 d;
-            P.newc[v] = move_decision(m, x, &d);
+            const int32_t nc = move_decision(m, x, &d);
+            P.newc[v] = nc;
+            P.lim[v] = (nc == own && gs.sym && !single) ? skip_limit(m, x, drift, gs.dunit) : 0;
         }
     }
     __syncthreads();
+}
+
+// The vertices of degree > DW of a bucket: a warp each, with the warp's table
+// while the row shows at most WIDE_CLAIMS distinct communities (most rows of
+// an aggregated level after its first sweeps), else a whole CTA afterwards
+// (the vertices are listed in members, free during sweeps).  A vertex whose
+// table needs the graph's one global table is left to the first CTA.
+static __device__ void decide_wide(const Rows &L, const BatchParams &P, const GState &gs, const Team &t,
+                            const int32_t *list, int32_t n, u64 drift, BatchSmem &sm) {
+    constexpr int U = 2;
+    constexpr int LG = ilog2_c(WTAB);
+    static_assert(WIDE_CLAIMS + 32 * U < WTAB, "a step's claims fit the warp's table");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t *keys = sm.keys + warp * WTAB;
+    u64 *vals = sm.vals + warp * WTAB;
+    int32_t *ovf = P.members + gs.v0;
+    int32_t *novf = t.nc == 1 ? &sm.nbig : &t.scr->nbig;   // zero here (level_setup, sweep)
+    __syncwarp();
+    for (int32_t i = t.warp(); i < n; i += t.warps()) {
+        const int32_t v = list[i];
+        if (drift < P.lim[v]) continue;
+        const int32_t r0 = L.r0(v), r1 = L.r1(v);
+        const int32_t own = P.comm[v];
+        const u64 kv = P.k[v], sown = P.S[own];
+        const bool single = P.size[own] == 1;
+        u64 eo = 0;
+        int32_t claims = 0;
+        bool over = false;
+        for (int32_t b0 = r0; b0 < r1 && !over; b0 += 32 * U) {
+            int32_t jj[U];
+            u64 xx[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int32_t e = b0 + lane + 32 * u;
+                jj[u] = -1;
+                xx[u] = 0;
+                if (e < r1) {
+                    jj[u] = L.c(e);
+                    xx[u] = L.x(e);
+                }
+            }
+            int32_t cc[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) cc[u] = (jj[u] >= 0 && jj[u] != v) ? P.comm[jj[u]] : -1;
+            unsigned mine = 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (cc[u] < 0) continue;
+                if (cc[u] == own) eo += xx[u];
+                else mine += table_insert_claim<0>(keys, vals, LG, cc[u], xx[u], &sm.err) >= 0 ? 1u : 0u;
+            }
+            claims += (int32_t)__reduce_add_sync(FULL, mine);
+            over = claims > WIDE_CLAIMS;
+        }
+        __syncwarp();
+        if (over) {
+            for (int s = lane; s < WTAB; s += 32) {
+                keys[s] = -1;
+                vals[s] = 0;
+            }
+            if (lane == 0) ovf[atomicAdd(novf, 1)] = v;
+            __syncwarp();
+            continue;
+        }
+        const MoveCtx m = move_ctx(own, single, gs.T, kv, sown);
+        Best b = best_init(own);
+        b.eo = eo;
+        for (int s = lane; s < WTAB; s += 32) {
+            const int32_t c = keys[s];
+            if (c < 0) continue;
+            const u64 ec = vals[s];
+            keys[s] = -1;
+            vals[s] = 0;
+            eval_loaded(c, ec, P.S[c], guard_needs_size(m, c) ? P.size[c] : 0, m, b);
+        }
+        __syncwarp();
+        group_reduce_best(m, b, 32);
+        if (lane == 0) {
+            u64 d;
+            const int32_t nc = move_decision(m, b, &d);
+            P.newc[v] = nc;
+            P.lim[v] = (nc == own && gs.sym && !single) ? skip_limit(m, b, drift, gs.dunit) : 0;
+        }
+    }
+    t.sync();
+    const int32_t no = *(volatile int32_t *)novf;
+    for (int pass = 0; pass < (t.nc > 1 ? 2 : 1); ++pass) {
+        if (pass == 1 && t.rank != 0) break;
+        for (int32_t i = pass ? 0 : t.rank; i < no; i += pass ? 1 : t.nc) {
+            const int32_t v = ovf[i];
+            if (t.nc > 1) {
+                const bool global = (1 << table_lg(min(L.r1(v) - L.r0(v), gs.V))) > CTAB;
+                if (global != (pass == 1)) continue;
+            }
+            decide_cta(L, P, gs, v, drift, sm);
+        }
+    }
 }
 
 // Exact change of sum_i e_{i->C(i)} when one sub-round's decisions commit.
@@ -415,41 +736,70 @@ __device__ void decide_cta(const Lv<WT> &L, const BatchParams &P, const GState &
 // w ([n == C'(x)] - [o == C(x)]): counted twice from v's row when x stays
 // (the entry in x's row is not visited), once from each row when x moves
 // too.  Between sub-rounds newc == comm, so newc[x] != comm[x] marks a mover
-// of this sub-round.  Lane groups of 8 per vertex; wrapping uint64 sum.
-template <typename WT>
-__device__ __forceinline__ u64 commit_delta(const Lv<WT> &L, const BatchParams &P, const int32_t *list,
-                                            int32_t n) {
+// of this sub-round.  The neighbours need a new evaluation (lim = 0).  A warp
+// takes chunks of the list as in decide_groups and spreads the movers of a
+// chunk over lane groups of 8; wrapping uint64 sum.
+static __device__ __forceinline__ u64 commit_delta(const Rows &L, const BatchParams &P, const Team &t,
+                                            const int32_t *list, int32_t n, BatchSmem &sm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int grp = lane >> 3, gl = lane & 7;
+    uint8_t *ord = sm.ord[warp];
+    const int32_t nw = t.warps();
+    const int32_t cs = chunk_of(n, nw, 4);
     u64 d = 0;
-    for (int32_t i0 = warp * 4; i0 < n; i0 += BW * 4) {
-        const int32_t i = i0 + (lane >> 3);
-        if (i >= n) continue;
-        const int32_t v = list[i];
-        const int32_t nv = P.newc[v], ov = P.comm[v];
-        if (nv == ov) continue;
-        const int32_t r1 = L.r1(v);
-        for (int32_t e = L.r0(v) + (lane & 7); e < r1; e += 8) {
-            const int32_t x = L.c(e);
-            if (x == v) continue;
-            const u64 w = L.x(e);
-            const int32_t cx = P.comm[x], nx = P.newc[x];
-            if (nx != cx) {
-                if (nv == nx) d += w;
-                if (ov == cx) d -= w;
-            } else {
-                if (nv == cx) d += 2 * w;
-                if (ov == cx) d -= 2 * w;
-            }
+    for (int32_t c0 = t.warp() * cs; c0 < n; c0 += nw * cs) {
+        int32_t lv = -1, ln = 0, lo = 0;
+        if (lane < cs && c0 + lane < n) {
+            lv = list[c0 + lane];
+            ln = P.newc[lv];
+            lo = P.comm[lv];
         }
+        const bool mover = ln != lo;
+        const unsigned mask = __ballot_sync(FULL, mover);
+        if (!mask) continue;
+        int32_t lr0 = 0, lr1 = 0;
+        if (mover) {
+            lr0 = L.r0(lv);
+            lr1 = L.r1(lv);
+            ord[__popc(mask & ((1u << lane) - 1u))] = (uint8_t)lane;
+        }
+        __syncwarp();
+        const int cnt = __popc(mask);
+        for (int q0 = 0; q0 < cnt; q0 += 4) {
+            const int src = q0 + grp < cnt ? ord[q0 + grp] : -1;
+            const int at = src < 0 ? 0 : src;
+            const int32_t v = __shfl_sync(FULL, lv, at), nv = __shfl_sync(FULL, ln, at), ov = __shfl_sync(FULL, lo, at);
+            const int32_t r0 = __shfl_sync(FULL, lr0, at);
+            const int32_t r1s = __shfl_sync(FULL, lr1, at), r1 = src < 0 ? 0 : r1s;
+            for (int32_t e = r0 + gl; e < r1; e += 8) {
+                const int32_t x = L.c(e);
+                if (x == v) continue;
+                const u64 w = L.x(e);
+                const int32_t cx = P.comm[x], nx = P.newc[x];
+                P.lim[x] = 0;
+                if (nx != cx) {
+                    if (nv == nx) d += w;
+                    if (ov == cx) d -= w;
+                } else {
+                    if (nv == cx) d += 2 * w;
+                    if (ov == cx) d -= 2 * w;
+                }
+            }
+            __syncwarp();
+        }
+        __syncwarp();
     }
     return d;
 }
 
 // updateVertexCommunity (modularity_optimisation.cu:237-249) for one
-// sub-round's vertices, with exact Sigma_tot and size updates.
-__device__ __forceinline__ int32_t commit_list(const BatchParams &P, const int32_t *list, int32_t n) {
+// sub-round's vertices, with exact Sigma_tot and size updates; *drift gets
+// the thread's share of the drift.
+static __device__ __forceinline__ int32_t commit_list(const BatchParams &P, const GState &gs, const Team &t,
+                                               const int32_t *list, int32_t n, u64 *drift) {
     int32_t moved = 0;
-    for (int32_t i = threadIdx.x; i < n; i += BT) {
+    u64 dd = 0;
+    for (int32_t i = t.tid(); i < n; i += t.threads()) {
         const int32_t v = list[i];
         const int32_t nc = P.newc[v], oc = P.comm[v];
         if (nc == oc) continue;
@@ -459,50 +809,53 @@ __device__ __forceinline__ int32_t commit_list(const BatchParams &P, const int32
         const u64 kv = P.k[v];
         atomicAdd(P.S + oc, (u64)0 - kv);
         atomicAdd(P.S + nc, kv);
+        dd += gs.drift_of(kv);
         ++moved;
     }
+    *drift = dd;
     return moved;
 }
 
 // One sweep: the seven sub-rounds, each deciding against the state committed
-// before it.  Returns the number of moves; *de receives the exact change of
-// sum_i e_{i->C(i)}.
-template <typename WT>
-__device__ int64_t sweep(const Lv<WT> &L, const BatchParams &P, const GState &gs, BatchSmem &sm, u64 *de) {
-    int32_t moved = 0;
-    u64 d = 0;
+// before it.  Returns this thread's moves; *de receives its share of the exact
+// change of sum_i e_{i->C(i)}.
+static __device__ u64 sweep(const Rows &L, const BatchParams &P, const GState &gs, Team &t, BatchSmem &sm, u64 *de) {
+    u64 moved = 0, d = 0;
     const int32_t *bl = P.blist + gs.v0;
+    volatile u64 *drift_at = t.nc == 1 ? &sm.drift : &t.scr->drift;
     for (int b = 0; b < NBUCKETS; ++b) {
         const int32_t o = sm.boff[2 * b], ns = sm.bcnt[2 * b], nb = sm.bcnt[2 * b + 1];
         if (ns + nb == 0) continue;
-        switch (b) {
-        case 0: decide_groups<WT, 4, 3, 1>(L, P, gs, bl + o, ns, sm); break;
-        case 1: decide_groups<WT, 4, 4, 2>(L, P, gs, bl + o, ns, sm); break;
-        case 2: decide_groups<WT, 8, 5, 2>(L, P, gs, bl + o, ns, sm); break;
-        case 3: decide_groups<WT, 8, 6, 4>(L, P, gs, bl + o, ns, sm); break;
-        default: decide_groups<WT, 32, 8, 4>(L, P, gs, bl + o, ns, sm); break;
+        const u64 drift = *drift_at;
+        // one code path for the short buckets and one for the longer rows: the
+        // kernel's code would not fit the instruction cache with one per bucket
+        if (b < 3) decide_groups<4, 4>(L, P, gs, t, bl + o, ns, 3 + b, drift, sm);
+        else if (b == 3) decide_groups<8, 4>(L, P, gs, t, bl + o, ns, 6, drift, sm);
+        else if (ns) decide_groups<32, 4>(L, P, gs, t, bl + o, ns, 8, drift, sm);
+        if (nb) decide_wide(L, P, gs, t, bl + o + ns, nb, drift, sm);
+        t.sync();
+        if (nb && t.tid() == 0) *(t.nc == 1 ? &sm.nbig : &t.scr->nbig) = 0;   // used again after the barriers below
+        d += commit_delta(L, P, t, bl + o, ns + nb, sm);
+        t.sync();
+        u64 dd = 0;
+        const int32_t mv = commit_list(P, gs, t, bl + o, ns + nb, &dd);
+        moved += (u64)mv;
+        if (__any_sync(FULL, mv != 0)) {
+            dd = warp_sum_u64(dd);
+            if ((threadIdx.x & 31) == 0) atomicAdd((u64 *)drift_at, dd);
         }
-        if (nb) {
-            __syncthreads();
-            for (int32_t i = 0; i < nb; ++i) decide_cta(L, P, gs, bl[o + ns + i], sm);
-        }
-        __syncthreads();
-        d += commit_delta(L, P, bl + o, ns + nb);
-        __syncthreads();
-        moved += commit_list(P, bl + o, ns + nb);
-        __syncthreads();
+        t.sync();
     }
-    *de = block_sum_u64(d, sm);
-    return (int64_t)block_sum_u64((u64)moved, sm);
+    *de = d;
+    return moved;
 }
 
-// sum_i e_{i->C(i)} over whole rows, self-loops included
+// This thread's share of sum_i e_{i->C(i)} over whole rows, self-loops included
 // (calculateToOwnCommunity, modularity_optimisation.cu:365-393).
-template <typename WT>
-__device__ u64 own_weight(const Lv<WT> &L, const BatchParams &P, const GState &gs, BatchSmem &sm) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+static __device__ u64 own_weight(const Rows &L, const BatchParams &P, const GState &gs, const Team &t) {
+    const int lane = threadIdx.x & 31;
     u64 eo = 0;
-    for (int32_t i0 = warp * 4; i0 < gs.V; i0 += BW * 4) {
+    for (int32_t i0 = t.warp() * 4; i0 < gs.V; i0 += t.warps() * 4) {
         const int32_t i = i0 + (lane >> 3);
         if (i >= gs.V) continue;
         const int32_t v = gs.v0 + i;
@@ -511,60 +864,87 @@ __device__ u64 own_weight(const Lv<WT> &L, const BatchParams &P, const GState &g
         for (int32_t e = L.r0(v) + (lane & 7); e < r1; e += 8)
             if (P.comm[L.c(e)] == cv) eo += L.x(e);
     }
-    return block_sum_u64(eo, sm);
+    return eo;
 }
 
-// calculateModularity (modularity_optimisation.cu:395-401) from the exact
-// sum_i e_{i->C(i)} and a pass over Sigma_tot.
-__device__ double modularity_from(u64 e_own, const BatchParams &P, const GState &gs, BatchSmem &sm) {
+// This thread's share of sum_C Sigma_tot^2.
+static __device__ __forceinline__ u128 s2_part(const BatchParams &P, const GState &gs, const Team &t) {
     u128 s2 = 0;
-    for (int32_t i = threadIdx.x; i < gs.V; i += BT) {
+    for (int32_t i = t.tid(); i < gs.V; i += t.threads()) {
         const u64 s = P.S[gs.v0 + i];
         s2 += (u128)s * (u128)s;
     }
-    const u128 ts = block_sum_u128(s2, sm);
-    return q_from_parts_dev(gs.T, e_own, (u64)(ts >> 64), (u64)ts);
+    return s2;
 }
 
 // Level set-up: k_i (level 0; aggregation writes it for later levels),
 // singleton communities, Sigma_tot = k, and the bucket lists.
-template <typename WT>
-__device__ void level_setup(const Lv<WT> &L, const BatchParams &P, GState &gs, BatchSmem &sm,
-                            bool level0) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+static __device__ void level_setup(const Rows &L, const BatchParams &P, GState &gs, Team &t, BatchSmem &sm) {
+    const int lane = threadIdx.x & 31;
     const int32_t v0 = gs.v0, V = gs.V;
-    if (level0) {
-        u64 tot = 0;
-        for (int32_t i0 = warp * 4; i0 < V; i0 += BW * 4) {
+    if (gs.cur < 0) {
+        Totals5 tt{};
+        for (int32_t i0 = t.warp() * 4; i0 < V; i0 += t.warps() * 4) {
             const int32_t i = i0 + (lane >> 3);
             u64 s = 0;
             if (i < V) {
                 const int32_t r1 = L.r1(v0 + i);
-                for (int32_t e = L.r0(v0 + i) + (lane & 7); e < r1; e += 8) s += L.x(e);
+                for (int32_t e = L.r0(v0 + i) + (lane & 7); e < r1; e += 8) {
+                    const u64 x = wfix(P.w, e, gs.scale);
+                    if (gs.narrow) const_cast<uint32_t *>(L.w32)[e] = (uint32_t)x;
+                    else const_cast<u64 *>(L.w64)[e] = x;
+                    const int32_t j = L.c(e);
+                    s += x;
+                    const uint32_t xw = (uint32_t)x ^ (uint32_t)(x >> 32) * 0x85EBCA6Bu;
+                    tt.b += sym_mix((uint32_t)(v0 + i), (uint32_t)j, xw) - sym_mix((uint32_t)j, (uint32_t)(v0 + i), xw);
+                }
             }
             for (int off = 4; off > 0; off >>= 1) s += __shfl_xor_sync(FULL, s, off);
             if (i < V && (lane & 7) == 0) {
                 P.k[v0 + i] = s;
-                tot += s;
+                tt.a += s;
             }
         }
-        gs.T = block_sum_u64(tot, sm);
+        tt = team_totals(tt, t, sm);
+        gs.T = tt.a;
+        gs.sym = tt.b == 0;
+        // T in at most 2^40 drift units: the drift of a level stays far below 2^62
+        gs.dsh = max(0, 64 - __clzll((long long)gs.T) - 40);
+        gs.dunit = ldexpf(1.0f, -gs.dsh);
     }
-    for (int32_t i = threadIdx.x; i < V; i += BT) {
+    if (threadIdx.x < 16) sm.bcnt[threadIdx.x] = 0;
+    if (threadIdx.x == 0) {
+        sm.drift = 0;
+        sm.nbig = 0;
+        if (t.nc > 1 && t.rank == 0) {
+            t.scr->drift = 0;
+            t.scr->nbig = 0;
+        }
+    }
+    __syncthreads();
+    // k of an aggregated level, and the rows, were written before the last barrier
+    for (int32_t i = t.tid(); i < V; i += t.threads()) {
         const int32_t v = v0 + i;
         P.comm[v] = v;
         P.newc[v] = v;
         P.size[v] = 1;
         P.S[v] = P.k[v];
-    }
-    if (threadIdx.x < 16) sm.bcnt[threadIdx.x] = 0;
-    __syncthreads();
-    for (int32_t i = threadIdx.x; i < V; i += BT) {
-        const int32_t d = L.r1(v0 + i) - L.r0(v0 + i);
+        P.lim[v] = 0;
+        const int32_t d = L.r1(v) - L.r0(v);
         const int b = bucket_of(d);
         if (b >= 0) atomicAdd(&sm.bcnt[2 * b + (d > DW ? 1 : 0)], 1);
     }
     __syncthreads();
+    int32_t mine = 0;
+    if (t.nc > 1) {
+        if (threadIdx.x < 16) {
+            mine = sm.bcnt[threadIdx.x];
+            if (mine) atomicAdd(&t.scr->cnt[threadIdx.x], mine);
+        }
+        t.sync();
+        if (threadIdx.x < 16) sm.bcnt[threadIdx.x] = __ldcg(&t.scr->cnt[threadIdx.x]);
+        __syncthreads();
+    }
     if (threadIdx.x == 0) {
         int32_t o = 0;
         for (int j = 0; j < 2 * NBUCKETS; ++j) {
@@ -574,23 +954,35 @@ __device__ void level_setup(const Lv<WT> &L, const BatchParams &P, GState &gs, B
         }
     }
     __syncthreads();
-    for (int32_t i = threadIdx.x; i < V; i += BT) {
+    if (t.nc > 1) {
+        // this CTA's part of each bucket's range
+        if (threadIdx.x < 2 * NBUCKETS && mine) sm.bcur[threadIdx.x] += atomicAdd(&t.scr->cur[threadIdx.x], mine);
+        __syncthreads();
+    }
+    for (int32_t i = t.tid(); i < V; i += t.threads()) {
         const int32_t d = L.r1(v0 + i) - L.r0(v0 + i);
         const int b = bucket_of(d);
         if (b >= 0) P.blist[v0 + atomicAdd(&sm.bcur[2 * b + (d > DW ? 1 : 0)], 1)] = v0 + i;
     }
-    __syncthreads();
+    t.sync();
+    if (t.nc > 1 && t.rank == 0 && threadIdx.x < 16) {
+        t.scr->cnt[threadIdx.x] = 0;   // read again only after this level's barriers
+        t.scr->cur[threadIdx.x] = 0;
+    }
 }
 
 // optimiseModularity (modularity_optimisation.cu:284-363): sweeps while the
 // sweep's gain >= min_gain (the first always runs), stopping after a sweep
 // without moves; changed = some sweep gained (> 0).  Then
 // originalToCommunity <- C(originalToCommunity) (:251-257, :361).
-template <typename WT>
-__device__ int optimise_level(const Lv<WT> &L, const BatchParams &P, const GState &gs, BatchSmem &sm,
+static __device__ int optimise_level(const Rows &L, const BatchParams &P, const GState &gs, Team &t, BatchSmem &sm,
                               Acc &acc) {
-    u64 e_own = own_weight(L, P, gs, sm);
-    double q_before = modularity_from(e_own, P, gs, sm);
+    Totals5 tt{};
+    tt.a = own_weight(L, P, gs, t);
+    tt.s2 = s2_part(P, gs, t);
+    tt = team_totals(tt, t, sm);
+    u64 e_own = tt.a;
+    double q_before = modularity_from(gs, e_own, tt.s2);
     double gain = P.min_gain;
     int changed = 0, sw = 0;
     while (gain >= P.min_gain) {
@@ -599,16 +991,20 @@ __device__ int optimise_level(const Lv<WT> &L, const BatchParams &P, const GStat
             acc.status = LV_ERR_DEVICE;
             break;
         }
-        u64 de = 0;
-        const int64_t moves = sweep(L, P, gs, sm, &de);
+        tt = Totals5{};
+        tt.b = sweep(L, P, gs, t, sm, &tt.a);
+        tt.s2 = s2_part(P, gs, t);
+        tt.err = (u64)(unsigned)sm.err;
+        tt = team_totals(tt, t, sm);
+        const int64_t moves = (int64_t)tt.b;
         ++sw;
         acc.moves += moves;
-        if (sm.err) {
+        if (tt.err) {
             acc.status = LV_ERR_DEVICE;
             break;
         }
-        e_own += de;
-        const double q_after = modularity_from(e_own, P, gs, sm);
+        e_own += tt.a;
+        const double q_after = modularity_from(gs, e_own, tt.s2);
         gain = __dsub_rn(q_after, q_before);
         if (gain > 0) changed = 1;
         q_before = q_after;
@@ -618,11 +1014,11 @@ __device__ int optimise_level(const Lv<WT> &L, const BatchParams &P, const GStat
     acc.edge_sweeps += (int64_t)sw * gs.E;
     acc.vertex_sweeps += (int64_t)sw * gs.V;
     acc.q = q_before;
-    for (int32_t u = threadIdx.x; u < gs.V0; u += BT) {
+    for (int32_t u = t.tid(); u < gs.V0; u += t.threads()) {
         const int32_t x = P.o2c[gs.v0 + u];
         P.o2c[gs.v0 + u] = P.comm[x];
     }
-    __syncthreads();
+    t.sync();
     return changed;
 }
 
@@ -632,61 +1028,76 @@ __device__ int optimise_level(const Lv<WT> &L, const BatchParams &P, const GStat
 // entries become one self-loop); new k = row sum; originalToCommunity <-
 // newID (:222-228).  Rows are written at the offset of their bound (the sum of
 // the members' degrees) inside the graph's entry range and stay there.
-template <typename WT>
-__device__ void aggregate(const Lv<WT> &L, const BatchParams &P, GState &gs, BatchSmem &sm) {
+// Returns whether a device check failed.
+static __device__ bool aggregate(const Rows &L, const BatchParams &P, GState &gs, Team &t, BatchSmem &sm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = gs.cur < 0 ? 0 : 1 - gs.cur;
     const int32_t v0 = gs.v0, V = gs.V;
+    const int32_t tid = t.tid(), tn = t.threads();
+    int32_t *nbig_at = t.nc == 1 ? &sm.nbig : &t.scr->nbig;
     int32_t *ms = P.mstart + v0 + gs.g;
     int32_t *ro = P.roff + v0 + gs.g;
     int32_t *nid = P.newid;
-    const int32_t nv = block_scan(
+    const int32_t nv = team_scan(
         V, [&](int32_t i) { return P.size[v0 + i] > 0 ? 1 : 0; },
-        [&](int32_t i, int32_t pre, int32_t x) { nid[v0 + i] = x ? pre : -1; }, sm);
-    for (int32_t i = threadIdx.x; i <= nv; i += BT) {
+        [&](int32_t i, int32_t pre, int32_t x) { nid[v0 + i] = x ? pre : -1; }, t, sm);
+    for (int32_t i = tid; i <= nv; i += tn) {
         ms[i] = 0;
         ro[i] = 0;
     }
-    __syncthreads();
-    for (int32_t i = threadIdx.x; i < V; i += BT) {
+    t.sync();
+    for (int32_t i = tid; i < V; i += tn) {
         const int32_t v = v0 + i;
         const int32_t c = nid[P.comm[v]];
         atomicAdd(ms + c, 1);
         atomicAdd(ro + c, L.r1(v) - L.r0(v));
     }
-    __syncthreads();
-    block_scan(nv + 1, [&](int32_t i) { return ms[i]; }, [&](int32_t i, int32_t pre, int32_t) { ms[i] = pre; }, sm);
-    block_scan(nv + 1, [&](int32_t i) { return ro[i]; }, [&](int32_t i, int32_t pre, int32_t) { ro[i] = pre; }, sm);
-    for (int32_t i = threadIdx.x; i < nv; i += BT) P.newc[v0 + i] = ms[i];
-    __syncthreads();
-    for (int32_t i = threadIdx.x; i < V; i += BT) {
+    t.sync();
+    team_scan(nv + 1, [&](int32_t i) { return ms[i]; },
+              [&](int32_t i, int32_t pre, int32_t) {
+                  ms[i] = pre;
+                  if (i < nv) P.newc[v0 + i] = pre;
+              }, t, sm);
+    team_scan(nv + 1, [&](int32_t i) { return ro[i]; }, [&](int32_t i, int32_t pre, int32_t) { ro[i] = pre; }, t,
+              sm);
+    if (tid == 0) *nbig_at = 0;
+    for (int32_t i = tid; i < V; i += tn) {
         const int32_t v = v0 + i;
         const int32_t pos = atomicAdd(P.newc + v0 + nid[P.comm[v]], 1);
         P.members[v0 + pos] = v;
     }
-    if (threadIdx.x == 0) sm.nbig = 0;
-    __syncthreads();
+    t.sync();
 
     int32_t *ocol = P.colb[nb];
     u64 *ow = P.wb[nb];
     int32_t *ors = P.rs[nb], *ore = P.re[nb];
     u64 enew = 0;
     // merged rows of bound <= DW: one warp each, table in the warp's slots
-    for (int32_t c = warp; c < nv; c += BW) {
+    for (int32_t c = t.warp(); c < nv; c += t.warps()) {
         const int32_t bound = ro[c + 1] - ro[c];
         if (bound > DW) {
-            if (lane == 0) P.blist[v0 + atomicAdd(&sm.nbig, 1)] = c;
+            if (lane == 0) P.blist[v0 + atomicAdd(nbig_at, 1)] = c;
             continue;
         }
         const int lg = table_lg(min(bound, nv));
         int32_t *keys = sm.keys + warp * WTAB;
         u64 *vals = sm.vals + warp * WTAB;
+        u64 self = 0;   // weight inside the community (its self-loop), summed in registers
+        bool any = false;
         for (int32_t j = ms[c]; j < ms[c + 1]; ++j) {
             const int32_t m = P.members[v0 + j];
             const int32_t r1 = L.r1(m);
-            for (int32_t e = L.r0(m) + lane; e < r1; e += 32)
-                table_insert<1>(keys, vals, lg, nid[P.comm[L.c(e)]], L.x(e), &sm.err);
+            for (int32_t e = L.r0(m) + lane; e < r1; e += 32) {
+                const int32_t key = nid[P.comm[L.c(e)]];
+                if (key == c) {
+                    self += L.x(e);
+                    any = true;
+                } else {
+                    table_insert<1>(keys, vals, lg, key, L.x(e), &sm.err);
+                }
+            }
         }
+        if (any) table_insert<1>(keys, vals, lg, c, self, &sm.err);
         __syncwarp();
         const int64_t base = gs.e0 + ro[c];
         int32_t cnt = 0;
@@ -719,73 +1130,92 @@ __device__ void aggregate(const Lv<WT> &L, const BatchParams &P, GState &gs, Bat
             enew += (u64)cnt;
         }
     }
-    __syncthreads();
-    // larger merged rows: the whole CTA, one at a time
-    const int32_t nbig = sm.nbig;
-    for (int32_t t = 0; t < nbig; ++t) {
-        const int32_t c = P.blist[v0 + t];
-        const int32_t bound = ro[c + 1] - ro[c];
-        const int lg = table_lg(min(bound, nv));
-        int32_t *keys = sm.keys;
-        u64 *vals = sm.vals;
-        if ((1 << lg) > CTAB) {
-            keys = P.tkeys + gs.tbl;
-            vals = P.tvals + gs.tbl;
-        }
-        for (int32_t j = ms[c] + warp; j < ms[c + 1]; j += BW) {
-            const int32_t m = P.members[v0 + j];
-            const int32_t r1 = L.r1(m);
-            for (int32_t e = L.r0(m) + lane; e < r1; e += 32)
-                table_insert<1>(keys, vals, lg, nid[P.comm[L.c(e)]], L.x(e), &sm.err);
-        }
-        if (threadIdx.x == 0) sm.cnt = 0;
-        __syncthreads();
-        const int64_t base = gs.e0 + ro[c];
-        u64 ks = 0;
-        for (int32_t s0 = 0; s0 < (1 << lg); s0 += BT) {
-            const int32_t s = s0 + threadIdx.x;
-            const int32_t key = s < (1 << lg) ? keys[s] : -1;
-            const unsigned bal = __ballot_sync(FULL, key >= 0);
-            int32_t wbase = 0;
-            if (lane == 0 && bal) wbase = atomicAdd(&sm.cnt, __popc(bal));
-            wbase = __shfl_sync(FULL, wbase, 0);
-            if (key >= 0) {
-                const int32_t pos = wbase + __popc(bal & ((1u << lane) - 1u));
-                const u64 x = vals[s];
-                if (pos < bound) {
-                    ocol[base + pos] = v0 + key;
-                    ow[base + pos] = x;
-                } else {
-                    atomicOr(&sm.err, DEVERR_BAD_STATE);
-                }
-                ks += x;
-                keys[s] = -1;
-                vals[s] = 0;
+    t.sync();
+    // larger merged rows: a whole CTA each (the first CTA for those that need
+    // the graph's one global table)
+    const int32_t nbig = *(volatile int32_t *)nbig_at;
+    for (int pass = 0; pass < (t.nc > 1 ? 2 : 1); ++pass) {
+        if (pass == 1 && t.rank != 0) break;
+        for (int32_t b = pass ? 0 : t.rank; b < nbig; b += pass ? 1 : t.nc) {
+            const int32_t c = P.blist[v0 + b];
+            const int32_t bound = ro[c + 1] - ro[c];
+            const int lg = table_lg(min(bound, nv));
+            if (t.nc > 1 && ((1 << lg) > CTAB) != (pass == 1)) continue;
+            int32_t *keys = sm.keys;
+            u64 *vals = sm.vals;
+            if ((1 << lg) > CTAB) {
+                keys = P.tkeys + gs.tbl;
+                vals = P.tvals + gs.tbl;
             }
+            u64 self = 0;
+            bool any = false;
+            for (int32_t j = ms[c] + warp; j < ms[c + 1]; j += BW) {
+                const int32_t m = P.members[v0 + j];
+                const int32_t r1 = L.r1(m);
+                for (int32_t e = L.r0(m) + lane; e < r1; e += 32) {
+                    const int32_t key = nid[P.comm[L.c(e)]];
+                    if (key == c) {
+                        self += L.x(e);
+                        any = true;
+                    } else {
+                        table_insert<1>(keys, vals, lg, key, L.x(e), &sm.err);
+                    }
+                }
+            }
+            if (any) table_insert<1>(keys, vals, lg, c, self, &sm.err);
+            if (threadIdx.x == 0) sm.cnt = 0;
+            __syncthreads();
+            const int64_t base = gs.e0 + ro[c];
+            u64 ks = 0;
+            for (int32_t s0 = 0; s0 < (1 << lg); s0 += BT) {
+                const int32_t s = s0 + threadIdx.x;
+                const int32_t key = s < (1 << lg) ? keys[s] : -1;
+                const unsigned bal = __ballot_sync(FULL, key >= 0);
+                int32_t wbase = 0;
+                if (lane == 0 && bal) wbase = atomicAdd(&sm.cnt, __popc(bal));
+                wbase = __shfl_sync(FULL, wbase, 0);
+                if (key >= 0) {
+                    const int32_t pos = wbase + __popc(bal & ((1u << lane) - 1u));
+                    const u64 x = vals[s];
+                    if (pos < bound) {
+                        ocol[base + pos] = v0 + key;
+                        ow[base + pos] = x;
+                    } else {
+                        atomicOr(&sm.err, DEVERR_BAD_STATE);
+                    }
+                    ks += x;
+                    keys[s] = -1;
+                    vals[s] = 0;
+                }
+            }
+            const u64 ktot = block_sum_u64(ks, sm);
+            if (threadIdx.x == 0) {
+                const int32_t cnt = sm.cnt;
+                ors[v0 + c] = (int32_t)base;
+                ore[v0 + c] = (int32_t)(base + cnt);
+                P.k[v0 + c] = ktot;
+                enew += (u64)cnt;
+            }
+            __syncthreads();
         }
-        const u64 ktot = block_sum_u64(ks, sm);
-        if (threadIdx.x == 0) {
-            const int32_t cnt = sm.cnt;
-            ors[v0 + c] = (int32_t)base;
-            ore[v0 + c] = (int32_t)(base + cnt);
-            P.k[v0 + c] = ktot;
-            enew += (u64)cnt;
-        }
-        __syncthreads();
     }
-    const u64 etot = block_sum_u64(enew, sm);
-    for (int32_t u = threadIdx.x; u < gs.V0; u += BT) {
+    for (int32_t u = tid; u < gs.V0; u += tn) {
         const int32_t x = P.o2c[v0 + u];
         P.o2c[v0 + u] = v0 + nid[x];
     }
-    gs.V = nv;
-    gs.E = (int64_t)etot;
-    gs.cur = nb;
     __syncthreads();
+    Totals5 tt{};
+    tt.a = enew;
+    tt.err = (u64)(unsigned)sm.err;
+    tt = team_totals(tt, t, sm);
+    gs.V = nv;
+    gs.E = (int64_t)tt.a;
+    gs.cur = nb;
+    return tt.err != 0;
 }
 
 // The whole level loop of one graph (gpulouvain.cu:30-37).
-__device__ void run_graph(const BatchParams &P, int32_t g, BatchSmem &sm) {
+static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, BatchSmem &sm) {
     GState gs;
     gs.g = g;
     gs.v0 = P.gptr[g];
@@ -797,28 +1227,46 @@ __device__ void run_graph(const BatchParams &P, int32_t g, BatchSmem &sm) {
     gs.T = 0;
     gs.scale = 1.0;
     gs.cur = -1;
-    if (threadIdx.x == 0) {
-        sm.err = 0;
-        P.t_start[g] = globaltimer();
-    }
+    gs.dsh = 0;
+    gs.dunit = 1.0f;
+    gs.narrow = false;
+    gs.sym = false;
+    if (threadIdx.x == 0) sm.err = 0;
+    if (t.tid() == 0) P.t_start[g] = globaltimer();
     for (int s = threadIdx.x; s < CTAB; s += BT) {
         sm.keys[s] = -1;
         sm.vals[s] = 0;
+        sm.hi[s] = 0;
     }
     // column range of the graph and the fixed-point scale (orc_choose_scale)
     int need = 0, top = 0, bad = 0;
-    for (int64_t e = gs.e0 + threadIdx.x; e < gs.e0 + gs.E; e += BT) {
+    for (int64_t e = gs.e0 + t.tid(); e < gs.e0 + gs.E; e += t.threads()) {
         const int32_t j = __ldg(P.col + e);
         if (j < gs.v0 || j >= gs.v0 + gs.V0) bad = 1;
-        int n, t, b;
-        weight_bits_dev(__ldg(P.w + e), n, t, b);
+        int n, tp, b;
+        weight_bits_dev(__ldg(P.w + e), n, tp, b);
         need = max(need, n);
-        top = max(top, t);
+        top = max(top, tp);
         bad |= b;
     }
     need = block_max_i32(need, sm);
     top = block_max_i32(top, sm);
     bad = block_max_i32(bad, sm);
+    if (t.nc > 1) {
+        u64(*red)[6] = t.scr->red[t.par];
+        t.par ^= 1;
+        if (threadIdx.x == 0) {
+            red[t.rank][0] = (u64)need;
+            red[t.rank][1] = (u64)top;
+            red[t.rank][2] = (u64)bad;
+        }
+        t.sync();
+        for (int r = 0; r < t.nc; ++r) {
+            need = max(need, (int)__ldcg(&red[r][0]));
+            top = max(top, (int)__ldcg(&red[r][1]));
+            bad = max(bad, (int)__ldcg(&red[r][2]));
+        }
+    }
     Acc acc{};
     acc.status = LV_OK;
     acc.q = 0.0;
@@ -830,41 +1278,48 @@ __device__ void run_graph(const BatchParams &P, int32_t g, BatchSmem &sm) {
         const int sc = need < cap ? need : cap;
         if (sc < 0) acc.status = LV_ERR_TOO_LARGE;
         else gs.scale = ldexp(1.0, sc);
+        gs.narrow = !top || tp + 1 + sc <= 31;   // every weight is at most 2^(tp + 1 + sc)
     }
     if (acc.status == LV_OK) {
-        for (int32_t u = threadIdx.x; u < gs.V0; u += BT) P.o2c[gs.v0 + u] = gs.v0 + u;
-        const Lv<float> L0{P.rowptr, P.col, P.w, gs.scale};
-        level_setup(L0, P, gs, sm, true);
-        int changed = optimise_level(L0, P, gs, sm, acc);
-        acc.levels = 1;
-        if (changed && acc.status == LV_OK) aggregate(L0, P, gs, sm);
-        while (changed && acc.status == LV_OK) {
-            if (sm.err) {
-                acc.status = LV_ERR_DEVICE;
-                break;
+        for (int32_t u = t.tid(); u < gs.V0; u += t.threads()) P.o2c[gs.v0 + u] = gs.v0 + u;
+        for (;;) {
+            Rows L;
+            if (gs.cur < 0) {
+                // level 0's fixed-point weights use the graph's part of the second
+                // weight buffer, which the first aggregation does not write
+                L.rs = P.rowptr;
+                L.re = P.rowptr + 1;
+                L.col = P.col;
+                L.w64 = P.wb[1];
+                L.w32 = gs.narrow ? reinterpret_cast<const uint32_t *>(P.wb[1] + gs.e0) - gs.e0 : nullptr;
+            } else {
+                L.rs = P.rs[gs.cur];
+                L.re = P.re[gs.cur];
+                L.col = P.colb[gs.cur];
+                L.w64 = P.wb[gs.cur];
+                L.w32 = nullptr;
             }
-            if (acc.levels >= LEVEL_CAP) {
-                acc.status = LV_ERR_DEVICE;
-                break;
-            }
-            const Lv<u64> L{P.rs[gs.cur], P.re[gs.cur], P.colb[gs.cur], P.wb[gs.cur]};
-            level_setup(L, P, gs, sm, false);
-            changed = optimise_level(L, P, gs, sm, acc);
+            level_setup(L, P, gs, t, sm);
+            const int changed = optimise_level(L, P, gs, t, sm, acc);
             acc.levels += 1;
-            if (changed && acc.status == LV_OK) aggregate(L, P, gs, sm);
+            if (!changed || acc.status != LV_OK) break;
+            if (aggregate(L, P, gs, t, sm) || acc.levels >= LEVEL_CAP) {
+                acc.status = LV_ERR_DEVICE;
+                break;
+            }
         }
     }
     if (acc.status != LV_OK) {
         // leave the graph's global table empty for the next run
         const int64_t n = P.tbl_off[g + 1] - gs.tbl;
-        for (int64_t s = threadIdx.x; s < n; s += BT) {
+        for (int64_t s = t.tid(); s < n; s += t.threads()) {
             P.tkeys[gs.tbl + s] = -1;
             P.tvals[gs.tbl + s] = 0;
         }
     }
-    for (int32_t u = threadIdx.x; u < gs.V0; u += BT)
+    for (int32_t u = t.tid(); u < gs.V0; u += t.threads())
         P.out_comm[gs.v0 + u] = acc.status == LV_OK ? P.o2c[gs.v0 + u] - gs.v0 : -1;
-    if (threadIdx.x == 0) {
+    if (t.tid() == 0) {
         P.q[g] = acc.q;
         P.nc[g] = acc.status == LV_OK ? gs.V : 0;
         P.status[g] = acc.status;
@@ -875,20 +1330,33 @@ __device__ void run_graph(const BatchParams &P, int32_t g, BatchSmem &sm) {
         P.moves[g] = acc.moves;
         P.t_end[g] = globaltimer();
     }
-    __syncthreads();
+    t.sync();
 }
 
-__global__ void __launch_bounds__(BT, LV_BATCH_MINB) batch_kernel(const __grid_constant__ BatchParams P) {
+};
+
+__device__ __forceinline__ int32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int32_t)r;
+}
+__device__ __forceinline__ int32_t cluster_ctas() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return (int32_t)r;
+}
+
+// Cluster i of a launch runs graph order[lo + i].
+__global__ void __launch_bounds__(BT, 1024 / BT) batch_kernel(const __grid_constant__ BatchParams P) {
     extern __shared__ __align__(16) unsigned char batch_smem[];
-    BatchSmem &sm = *reinterpret_cast<BatchSmem *>(batch_smem);
-    for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) sm.gi = atomicAdd(P.next, 1);
-        __syncthreads();
-        const int32_t gi = sm.gi;
-        if (gi >= P.G) break;
-        run_graph(P, P.order[gi], sm);
-    }
+    Loop::BatchSmem &sm = *reinterpret_cast<Loop::BatchSmem *>(batch_smem);
+    Loop::Team t;
+    t.nc = cluster_ctas();
+    t.rank = t.nc > 1 ? cluster_rank() : 0;
+    t.par = 0;
+    const int32_t i = P.lo + (int32_t)blockIdx.x / t.nc;
+    t.scr = P.scratch + i;
+    Loop::run_graph(P, P.order[i], t, sm);
 }
 
 // first entry of each graph: out[g] = rowptr[gptr[g]]
@@ -925,7 +1393,10 @@ struct lv_batch {
     BatchParams P{};
     int64_t tbl_total = 0;
     std::vector<void *> allocs;
-    int grid = 1;
+    struct Tier { int nc; int32_t lo, hi; };   // CTAs per graph, graphs order[lo .. hi)
+    std::vector<Tier> tiers;
+    std::vector<cudaStream_t> side;            // streams of the launches after the first
+    std::vector<cudaEvent_t> side_ev;
     bool ran = false;
     bool tables_dirty = false;
     float last_ms = 0;
@@ -1017,6 +1488,54 @@ int batch_begin(const int32_t *graph_ptr, int32_t G, int32_t V, int64_t E, const
     return LV_OK;
 }
 
+void launch_config(cudaStream_t s, int ctas, int cluster, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at) {
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(BT);
+    cfg.dynamicSmemBytes = sizeof(Loop::BatchSmem);
+    cfg.stream = s;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)cluster;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
+}
+
+// Launches by graph size (the order is by decreasing entries): the larger the
+// graph, the more CTAs run it, entries / (TEAM_PART * even share) of them,
+// rounded up to a power of two and at most 16 (the largest cluster).
+int plan_launch(lv_batch *b, const std::vector<int32_t> &order) {
+    constexpr size_t SM = sizeof(Loop::BatchSmem);
+    LVB_CUDA(b, cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM));
+    int sms = 148, widest = 1;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+    cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (int cl = TEAM_MAX; cl > 1; cl /= 2) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        launch_config(b->stream, cl, cl, cfg, at);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, batch_kernel, &cfg) == cudaSuccess && n > 0) {
+            widest = cl;
+            break;
+        }
+    }
+    cudaGetLastError();
+    int64_t total = 0;
+    for (int64_t e : b->entries_h) total += e;
+    const double part = std::max(TEAM_MIN_PART, TEAM_PART * (double)total / (2.0 * (sms > 0 ? sms : 148)));
+    b->tiers.clear();
+    for (int32_t i = 0; i < b->G; ++i) {
+        const double e = (double)b->entries_h[order[i]];
+        int nc = 1;
+        while (nc < widest && e > part * nc) nc *= 2;
+        if (b->tiers.empty() || b->tiers.back().nc != nc) b->tiers.push_back({nc, i, i});
+        b->tiers.back().hi = i + 1;
+    }
+    return LV_OK;
+}
+
 int batch_finish(lv_batch *b) {
     const int32_t G = b->G, V = b->V;
     const int64_t E = b->E;
@@ -1074,7 +1593,6 @@ int batch_finish(lv_batch *b) {
     P.gptr = gptr_d;
     P.order = order_d;
     P.tbl_off = toff_d;
-    P.G = G;
     P.max_sweeps = b->opts.max_sweeps;
     LVB_TRY(balloc(b, &P.comm, nv));
     LVB_TRY(balloc(b, &P.newc, nv));
@@ -1093,9 +1611,9 @@ int batch_finish(lv_batch *b) {
     }
     LVB_TRY(balloc(b, &P.k, nv));
     LVB_TRY(balloc(b, &P.S, nv));
+    LVB_TRY(balloc(b, &P.lim, nv));
     LVB_TRY(balloc(b, &P.tkeys, (size_t)b->tbl_total));
     LVB_TRY(balloc(b, &P.tvals, (size_t)b->tbl_total));
-    LVB_TRY(balloc(b, &P.next, 4));
     LVB_TRY(balloc(b, &P.out_comm, nv));
     LVB_TRY(balloc(b, &P.q, (size_t)G + 1));
     LVB_TRY(balloc(b, &P.nc, (size_t)G + 1));
@@ -1111,13 +1629,20 @@ int batch_finish(lv_batch *b) {
         fill_tables_kernel<<<148 * 8, 256, 0, b->stream>>>(P.tkeys, P.tvals, b->tbl_total);
         note_launches(1);
     }
-    int occ = 1, sms = 148;
-    cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BatchSmem));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel, BT, sizeof(BatchSmem));
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-    cudaGetLastError();
-    const int64_t slots = (int64_t)(occ > 0 ? occ : 1) * (sms > 0 ? sms : 148);
-    b->grid = (int)std::max<int64_t>(1, std::min<int64_t>(slots, G));
+    LVB_TRY(plan_launch(b, order));
+    size_t teams = 0;
+    for (const auto &t : b->tiers)
+        if (t.nc > 1) teams = (size_t)t.hi;   // the team launches come first in order
+    LVB_TRY(balloc(b, &P.scratch, teams + 1));
+    LVB_CUDA(b, cudaMemsetAsync(P.scratch, 0, sizeof(TeamScratch) * (teams + 1), b->stream));
+    for (size_t i = 1; i < b->tiers.size(); ++i) {
+        cudaStream_t s = nullptr;
+        cudaEvent_t ev = nullptr;
+        LVB_CUDA(b, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        b->side.push_back(s);
+        LVB_CUDA(b, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        b->side_ev.push_back(ev);
+    }
     return batch_sync(b);
 }
 
@@ -1135,6 +1660,11 @@ int lv_batch_destroy(lv_batch *b) {
         pool_free(b->device, (void *)b->w, b->stream);
     }
     for (void *p : b->allocs) pool_free(b->device, p, b->stream);
+    for (cudaStream_t s : b->side) {
+        cudaStreamSynchronize(s);
+        cudaStreamDestroy(s);
+    }
+    for (cudaEvent_t e : b->side_ev) cudaEventDestroy(e);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->stream) {
@@ -1213,12 +1743,22 @@ int lv_batch_run(lv_batch *b, float min_gain) {
         b->tables_dirty = false;
     }
     b->P.min_gain = (double)min_gain;
-    LVB_CUDA(b, cudaMemsetAsync(b->P.next, 0, sizeof(int32_t), b->stream));
     cudaEventRecord(b->ev0, b->stream);
-    if (b->G > 0) {
-        batch_kernel<<<b->grid, BT, sizeof(BatchSmem), b->stream>>>(b->P);
+    // the launches run side by side: the smaller graphs fill what the larger leave
+    for (size_t i = 0; i < b->tiers.size(); ++i) {
+        const lv_batch::Tier &t = b->tiers[i];
+        const cudaStream_t s = i ? b->side[i - 1] : b->stream;
+        if (i) LVB_CUDA(b, cudaStreamWaitEvent(s, b->ev0, 0));
+        BatchParams P = b->P;
+        P.lo = t.lo;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        launch_config(s, (t.hi - t.lo) * t.nc, t.nc, cfg, at);
+        LVB_CUDA(b, cudaLaunchKernelEx(&cfg, batch_kernel, P));
         note_launches(1);
+        if (i) LVB_CUDA(b, cudaEventRecord(b->side_ev[i - 1], s));
     }
+    for (cudaEvent_t e : b->side_ev) LVB_CUDA(b, cudaStreamWaitEvent(b->stream, e, 0));
     cudaEventRecord(b->ev1, b->stream);
     LVB_TRY(batch_sync(b));
     cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1);
@@ -1309,7 +1849,10 @@ int lv_batch_get_stats(lv_batch *b, double *device_ms, int64_t *edge_sweeps, int
     if (device_ms) *device_ms = b->last_ms;
     if (edge_sweeps) *edge_sweeps = b->last_edge_sweeps;
     if (vertex_sweeps) *vertex_sweeps = b->last_vertex_sweeps;
-    if (ctas) *ctas = b->grid;
+    if (ctas) {
+        *ctas = 0;
+        for (const auto &t : b->tiers) *ctas += (t.hi - t.lo) * t.nc;
+    }
     return LV_OK;
 }
 

@@ -754,11 +754,33 @@ __device__ __forceinline__ double gain_err(const MoveCtx &m, const Best &b) {
     return (m.Td * (double)b.e + m.kvd * fabs(dd)) * 0x1p-50;
 }
 
+// LV_EXACT_CALL (set by a translation unit before this header): the exact
+// comparison of near-ties is a call instead of being expanded at every use,
+// for kernels whose code would otherwise not fit the instruction cache.
+#ifndef LV_EXACT_CALL
+#define LV_EXACT_CALL 0
+#endif
+#if LV_EXACT_CALL
+static __device__ __noinline__ bool better_exact(u64 T, u64 kv, u64 sown, int32_t own, u64 ae, u64 aS, int32_t ac,
+                                                 u64 be, u64 bS, int32_t bc) {
+    MoveCtx m;
+    m.T = T;
+    m.kv = kv;
+    m.sown = sown;
+    const i128 ga = ac == own ? (i128)0 : exact_gain(m, ae, aS);
+    const i128 gb = bc == own ? (i128)0 : exact_gain(m, be, bS);
+    return ga > gb || (ga == gb && ac < bc);
+}
+#endif
+
 // true iff candidate a is strictly better than b (exact order).
 __device__ __forceinline__ bool better(const MoveCtx &m, const Best &a, const Best &b) {
     const double ea = gain_err(m, a), eb = gain_err(m, b);
     if (a.gd - ea > b.gd + eb) return true;
     if (b.gd - eb > a.gd + ea) return false;
+#if LV_EXACT_CALL
+    return better_exact(m.T, m.kv, m.sown, m.own, a.e, a.S, a.c, b.e, b.S, b.c);
+#endif
     const i128 ga = a.c == m.own ? (i128)0 : exact_gain(m, a.e, a.S);
     const i128 gb = b.c == m.own ? (i128)0 : exact_gain(m, b.e, b.S);
     return ga > gb || (ga == gb && a.c < b.c);

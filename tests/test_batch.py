@@ -114,6 +114,39 @@ def test_batch_upper_bounds_match_oracle(lvb, orc):
     _check_against_oracle(lvb, orc, graphs, 1e-6)
 
 
+def _fine_weights(lvb, g):
+    """g with symmetric float32 weights that use the whole mantissa (64-bit sums)."""
+    row = np.repeat(np.arange(g.V, dtype=np.int64), np.diff(g.rowptr))
+    a, b = np.minimum(row, g.col), np.maximum(row, g.col)
+    x = (a * 0x9E3779B1 + b * 0x85EBCA77) & 0xFFFFFFFF
+    x ^= x >> 15
+    w = -np.log(((x * 0x2C1B3C6D) % (1 << 31) + 0.5) / (1 << 31))
+    return lvb.Graph(g.rowptr, g.col, w.astype(np.float32))
+
+
+TEAM_GRAPHS = {
+    # a batch's only graph runs on a cluster of as many CTAs as it has 2048-entry parts
+    "one_cta": lambda lvb, gnp: [lvb.gen_planted(90, 6, 12.0, 2.0, 4)],
+    "two_ctas": lambda lvb, gnp: [lvb.gen_planted(200, 8, 14.0, 2.0, 4, "uniform")],
+    "sixteen_ctas": lambda lvb, gnp: [lvb.gen_planted(20011, 100, 18.0, 3.0, 8, "uniform")],
+    # rows longer than a warp's table, hubs and merged rows in the graph's global table
+    "rmat_hubs": lambda lvb, gnp: [lvb.gen_rmat(13, seed=6, weights="unit")],
+    "star_pairs": lambda lvb, gnp: [_star_pairs(lvb, gnp, 5000, 3000)],
+    "clique": lambda lvb, gnp: [_edges_graph(lvb, gnp, 300, [(i, j, 1.0) for i in range(300) for j in range(i)])],
+    # 64-bit weights at level 0
+    "fine_weights": lambda lvb, gnp: [_fine_weights(lvb, lvb.gen_planted(6000, 40, 16.0, 2.0, 3)),
+                                      _fine_weights(lvb, lvb.gen_rmat(11, seed=3))],
+    # teams of every size beside single CTAs
+    "mixed": lambda lvb, gnp: [lvb.gen_planted(40 << i, 4 + i, 14.0, 2.0, i) for i in range(10) for _ in range(3)],
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(TEAM_GRAPHS))
+def test_batch_teams_match_oracle(lvb, orc, gnp, name):
+    _check_against_oracle(lvb, orc, TEAM_GRAPHS[name](lvb, gnp), 1e-6)
+
+
 @pytest.mark.gpu
 def test_batch_max_sweeps_matches_oracle(lvb, orc, gnp):
     graphs = _mixed_batch(lvb, gnp)[:12]
