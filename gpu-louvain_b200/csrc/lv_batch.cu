@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -77,10 +78,18 @@ struct TeamScratch {
 };
 
 struct BatchParams {
-    // the caller's block-diagonal CSR (read-only during the launch)
-    const int32_t *rowptr;
+    // the caller's block-diagonal CSR (read-only during the launch); w is null
+    // when the start rows carry fixed-point sums (s_w64, job only)
+    const int32_t *rowptr, *rowend;
     const int32_t *col;
     const float *w;
+    const u64 *s_w64;
+    TeamResult *job;           // set: one graph of V, E (checked by the caller), results here
+    int32_t job_V;
+    int64_t job_E;
+    double job_scale;
+    int job_narrow;
+    int32_t sweep_cap, level_cap;
     const int32_t *gptr;       // [G + 1] first vertex of each graph
     const int32_t *order;      // [G] graphs by decreasing entry count
     const int64_t *tbl_off;    // [G + 1] first slot of each graph's global table
@@ -890,9 +899,9 @@ static __device__ void level_setup(const Rows &L, const BatchParams &P, GState &
             if (i < V) {
                 const int32_t r1 = L.r1(v0 + i);
                 for (int32_t e = L.r0(v0 + i) + (lane & 7); e < r1; e += 8) {
-                    const u64 x = wfix(P.w, e, gs.scale);
+                    const u64 x = P.w ? wfix(P.w, e, gs.scale) : L.w64[e];
                     if (gs.narrow) const_cast<uint32_t *>(L.w32)[e] = (uint32_t)x;
-                    else const_cast<u64 *>(L.w64)[e] = x;
+                    else if (P.w) const_cast<u64 *>(L.w64)[e] = x;
                     const int32_t j = L.c(e);
                     s += x;
                     const uint32_t xw = (uint32_t)x ^ (uint32_t)(x >> 32) * 0x85EBCA6Bu;
@@ -987,7 +996,7 @@ static __device__ int optimise_level(const Rows &L, const BatchParams &P, const 
     int changed = 0, sw = 0;
     while (gain >= P.min_gain) {
         if (P.max_sweeps > 0 && sw >= P.max_sweeps) break;
-        if (sw >= SWEEP_CAP) {
+        if (sw >= P.sweep_cap) {
             acc.status = LV_ERR_DEVICE;
             break;
         }
@@ -1214,31 +1223,9 @@ static __device__ bool aggregate(const Rows &L, const BatchParams &P, GState &gs
     return tt.err != 0;
 }
 
-// The whole level loop of one graph (gpulouvain.cu:30-37).
-static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, BatchSmem &sm) {
-    GState gs;
-    gs.g = g;
-    gs.v0 = P.gptr[g];
-    gs.V0 = P.gptr[g + 1] - gs.v0;
-    gs.V = gs.V0;
-    gs.e0 = __ldg(P.rowptr + gs.v0);
-    gs.E = (int64_t)__ldg(P.rowptr + gs.v0 + gs.V0) - gs.e0;
-    gs.tbl = P.tbl_off[g];
-    gs.T = 0;
-    gs.scale = 1.0;
-    gs.cur = -1;
-    gs.dsh = 0;
-    gs.dunit = 1.0f;
-    gs.narrow = false;
-    gs.sym = false;
-    if (threadIdx.x == 0) sm.err = 0;
-    if (t.tid() == 0) P.t_start[g] = globaltimer();
-    for (int s = threadIdx.x; s < CTAB; s += BT) {
-        sm.keys[s] = -1;
-        sm.vals[s] = 0;
-        sm.hi[s] = 0;
-    }
-    // column range of the graph and the fixed-point scale (orc_choose_scale)
+// Range check and fixed-point scale of a batch's graph (orc_choose_scale):
+// returns its status.
+static __device__ int graph_scale(const BatchParams &P, GState &gs, Team &t, BatchSmem &sm) {
     int need = 0, top = 0, bad = 0;
     for (int64_t e = gs.e0 + t.tid(); e < gs.e0 + gs.E; e += t.threads()) {
         const int32_t j = __ldg(P.col + e);
@@ -1267,18 +1254,57 @@ static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, Batch
             bad = max(bad, (int)__ldcg(&red[r][2]));
         }
     }
+    if (bad) return LV_ERR_INVALID;
+    const int tp = top ? top - 1024 : 0;
+    const int cap = 61 - tp - ceil_log2_i(gs.E > 0 ? gs.E : 1);
+    const int sc = need < cap ? need : cap;
+    if (sc < 0) return LV_ERR_TOO_LARGE;
+    gs.scale = ldexp(1.0, sc);
+    gs.narrow = !top || tp + 1 + sc <= 31;   // every weight is at most 2^(tp + 1 + sc)
+    return LV_OK;
+}
+
+// The whole level loop of one graph (gpulouvain.cu:30-37).
+static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, BatchSmem &sm) {
+    GState gs;
+    gs.g = g;
+    gs.v0 = P.job ? 0 : P.gptr[g];
+    gs.V0 = P.job ? P.job_V : P.gptr[g + 1] - gs.v0;
+    gs.V = gs.V0;
+    gs.e0 = P.job ? 0 : __ldg(P.rowptr + gs.v0);
+    gs.E = P.job ? P.job_E : (int64_t)__ldg(P.rowptr + gs.v0 + gs.V0) - gs.e0;
+    gs.tbl = P.job ? 0 : P.tbl_off[g];
+    gs.T = 0;
+    gs.scale = P.job_scale;
+    gs.cur = -1;
+    gs.dsh = 0;
+    gs.dunit = 1.0f;
+    gs.narrow = P.job_narrow != 0;
+    gs.sym = false;
+    if (threadIdx.x == 0) sm.err = 0;
+    for (int s = threadIdx.x; s < CTAB; s += BT) {
+        sm.keys[s] = -1;
+        sm.vals[s] = 0;
+        sm.hi[s] = 0;
+    }
     Acc acc{};
     acc.status = LV_OK;
     acc.q = 0.0;
-    if (bad) {
-        acc.status = LV_ERR_INVALID;
+    if (P.job) {
+        // the scratch area and the graph's table are this launch's own
+        if (t.tid() == 0) {
+            t.scr->nbig = 0;
+            for (int i = 0; i < 16; ++i) t.scr->cnt[i] = t.scr->cur[i] = 0;
+        }
+        const int32_t n = 1 << ceil_log2_i(2 * (int64_t)gs.V0);
+        for (int32_t s = t.tid(); s < n; s += t.threads()) {
+            P.tkeys[s] = -1;
+            P.tvals[s] = 0;
+        }
+        t.sync();
     } else {
-        const int tp = top ? top - 1024 : 0;
-        const int cap = 61 - tp - ceil_log2_i(gs.E > 0 ? gs.E : 1);
-        const int sc = need < cap ? need : cap;
-        if (sc < 0) acc.status = LV_ERR_TOO_LARGE;
-        else gs.scale = ldexp(1.0, sc);
-        gs.narrow = !top || tp + 1 + sc <= 31;   // every weight is at most 2^(tp + 1 + sc)
+        if (t.tid() == 0) P.t_start[g] = globaltimer();
+        acc.status = graph_scale(P, gs, t, sm);
     }
     if (acc.status == LV_OK) {
         for (int32_t u = t.tid(); u < gs.V0; u += t.threads()) P.o2c[gs.v0 + u] = gs.v0 + u;
@@ -1288,9 +1314,9 @@ static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, Batch
                 // level 0's fixed-point weights use the graph's part of the second
                 // weight buffer, which the first aggregation does not write
                 L.rs = P.rowptr;
-                L.re = P.rowptr + 1;
+                L.re = P.rowend;
                 L.col = P.col;
-                L.w64 = P.wb[1];
+                L.w64 = P.w ? P.wb[1] : P.s_w64;
                 L.w32 = gs.narrow ? reinterpret_cast<const uint32_t *>(P.wb[1] + gs.e0) - gs.e0 : nullptr;
             } else {
                 L.rs = P.rs[gs.cur];
@@ -1303,11 +1329,26 @@ static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, Batch
             const int changed = optimise_level(L, P, gs, t, sm, acc);
             acc.levels += 1;
             if (!changed || acc.status != LV_OK) break;
-            if (aggregate(L, P, gs, t, sm) || acc.levels >= LEVEL_CAP) {
+            if (aggregate(L, P, gs, t, sm) || acc.levels >= P.level_cap) {
                 acc.status = LV_ERR_DEVICE;
                 break;
             }
         }
+    }
+    if (P.job) {
+        if (t.tid() == 0) {
+            P.job->q = acc.q;
+            P.job->status = acc.status;
+            P.job->V = gs.V;
+            P.job->levels = acc.levels;
+            P.job->cur = gs.cur;
+            P.job->E = gs.E;
+            P.job->sweeps = acc.sweeps;
+            P.job->edge_sweeps = acc.edge_sweeps;
+            P.job->vertex_sweeps = acc.vertex_sweeps;
+            P.job->moves = acc.moves;
+        }
+        return;
     }
     if (acc.status != LV_OK) {
         // leave the graph's global table empty for the next run
@@ -1356,7 +1397,7 @@ __global__ void __launch_bounds__(BT, 1024 / BT) batch_kernel(const __grid_const
     t.par = 0;
     const int32_t i = P.lo + (int32_t)blockIdx.x / t.nc;
     t.scr = P.scratch + i;
-    Loop::run_graph(P, P.order[i], t, sm);
+    Loop::run_graph(P, P.job ? 0 : P.order[i], t, sm);
 }
 
 // first entry of each graph: out[g] = rowptr[gptr[g]]
@@ -1373,10 +1414,138 @@ __global__ void fill_tables_kernel(int32_t *keys, u64 *vals, int64_t n) {
     }
 }
 
+void launch_config(cudaStream_t s, int ctas, int cluster, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at) {
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(BT);
+    cfg.dynamicSmemBytes = sizeof(Loop::BatchSmem);
+    cfg.stream = s;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)cluster;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
+}
+
+// Dynamic shared memory and cluster attributes of batch_kernel (once per
+// device and process); the widest cluster the device takes.
+int widest_team(int device) {
+    static std::mutex mu;
+    static int widest[64] = {};
+    std::lock_guard<std::mutex> lock(mu);
+    if (device >= 0 && device < 64 && widest[device]) return widest[device];
+    if (cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(Loop::BatchSmem)) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    int cl = TEAM_MAX;
+    for (; cl > 1; cl /= 2) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        launch_config(0, cl, cl, cfg, at);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, batch_kernel, &cfg) == cudaSuccess && n > 0) break;
+    }
+    cudaGetLastError();
+    if (device >= 0 && device < 64) widest[device] = cl;
+    return cl;
+}
+
 }  // namespace
 }  // namespace lv
 
 using namespace lv;
+
+namespace {
+// Layout of a team run's arena for V vertices and E entries.
+struct TeamArena {
+    size_t at = 0;
+    template <typename T>
+    T *take(unsigned char *base, size_t n) {
+        at = (at + 255) / 256 * 256;
+        T *p = reinterpret_cast<T *>(base + at);
+        at += n * sizeof(T);
+        return p;
+    }
+    BatchParams lay(unsigned char *base, int32_t V, int64_t E) {
+        BatchParams P{};
+        at = 0;
+        const size_t v = (size_t)V + 1, e = (size_t)E + 1;
+        P.job = take<TeamResult>(base, 1);
+        P.scratch = take<TeamScratch>(base, 1);
+        P.o2c = take<int32_t>(base, v);
+        P.blist = take<int32_t>(base, v);
+        P.newid = take<int32_t>(base, v);
+        P.members = take<int32_t>(base, v);
+        P.mstart = take<int32_t>(base, v);
+        P.roff = take<int32_t>(base, v);
+        P.lim = take<u64>(base, v);
+        for (int i = 0; i < 2; ++i) {
+            P.rs[i] = take<int32_t>(base, v);
+            P.re[i] = take<int32_t>(base, v);
+            P.colb[i] = take<int32_t>(base, e);
+            P.wb[i] = take<u64>(base, e);
+        }
+        const size_t slots = (size_t)1 << ceil_log2_i(2 * (int64_t)V);
+        P.tkeys = take<int32_t>(base, slots);
+        P.tvals = take<u64>(base, slots);
+        return P;
+    }
+};
+}  // namespace
+
+size_t lv::team_arena_bytes(int32_t V, int64_t E) {
+    TeamArena a;
+    a.lay(nullptr, V, E);
+    return a.at;
+}
+
+int lv::team_run(const TeamJob &j, void *arena, int device, cudaStream_t s, TeamRows *rows) {
+    TeamArena a;
+    BatchParams P = a.lay((unsigned char *)arena, j.V, j.E);
+    P.rowptr = j.rs;
+    P.rowend = j.re;
+    P.col = j.col;
+    P.w = j.w;
+    P.s_w64 = j.w64;
+    P.job_V = j.V;
+    P.job_E = j.E;
+    P.job_scale = j.scale;
+    P.job_narrow = j.w && j.narrow;
+    P.sweep_cap = TEAM_RUN_SWEEP_CAP;
+    P.level_cap = 1 << 20;
+    P.max_sweeps = j.max_sweeps;
+    P.min_gain = j.min_gain;
+    P.comm = j.comm;
+    P.newc = j.newc;
+    P.size = j.size;
+    P.k = j.k;
+    P.S = j.S;
+    const int widest = widest_team(device);
+    if (!widest) return 0;
+    int nc = 1;
+    while (nc < widest && (double)j.E > TEAM_MIN_PART * nc) nc *= 2;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    launch_config(s, nc, nc, cfg, at);
+    if (cudaLaunchKernelEx(&cfg, batch_kernel, P) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    note_launches(1);
+    rows->result = P.job;
+    rows->o2c = P.o2c;
+    for (int i = 0; i < 2; ++i) {
+        rows->rs[i] = P.rs[i];
+        rows->re[i] = P.re[i];
+        rows->col[i] = P.colb[i];
+        rows->w64[i] = P.wb[i];
+    }
+    return 1;
+}
 
 struct lv_batch {
     int device = 0;
@@ -1488,40 +1657,14 @@ int batch_begin(const int32_t *graph_ptr, int32_t G, int32_t V, int64_t E, const
     return LV_OK;
 }
 
-void launch_config(cudaStream_t s, int ctas, int cluster, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at) {
-    cfg = cudaLaunchConfig_t{};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(BT);
-    cfg.dynamicSmemBytes = sizeof(Loop::BatchSmem);
-    cfg.stream = s;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)cluster;
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = cluster > 1 ? 1 : 0;
-}
-
 // Launches by graph size (the order is by decreasing entries): the larger the
 // graph, the more CTAs run it, entries / (TEAM_PART * even share) of them,
 // rounded up to a power of two and at most 16 (the largest cluster).
 int plan_launch(lv_batch *b, const std::vector<int32_t> &order) {
-    constexpr size_t SM = sizeof(Loop::BatchSmem);
-    LVB_CUDA(b, cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM));
-    int sms = 148, widest = 1;
+    int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-    cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    for (int cl = TEAM_MAX; cl > 1; cl /= 2) {
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute at;
-        launch_config(b->stream, cl, cl, cfg, at);
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, batch_kernel, &cfg) == cudaSuccess && n > 0) {
-            widest = cl;
-            break;
-        }
-    }
-    cudaGetLastError();
+    const int widest = widest_team(b->device);
+    if (!widest) return bfail(b, LV_ERR_CUDA, "batch kernel attributes");
     int64_t total = 0;
     for (int64_t e : b->entries_h) total += e;
     const double part = std::max(TEAM_MIN_PART, TEAM_PART * (double)total / (2.0 * (sms > 0 ? sms : 148)));
@@ -1588,6 +1731,10 @@ int batch_finish(lv_batch *b) {
     }
     const size_t nv = (size_t)V + 1, nvg = (size_t)V + G + 1, ne = (size_t)E + 1;
     P.rowptr = b->rowptr;
+    P.rowend = b->rowptr + 1;
+    P.sweep_cap = SWEEP_CAP;
+    P.level_cap = LEVEL_CAP;
+    P.job_scale = 1.0;
     P.col = b->col;
     P.w = b->w;
     P.gptr = gptr_d;

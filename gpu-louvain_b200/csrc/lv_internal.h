@@ -219,6 +219,48 @@ void launch_row_reduce(int cls, int mode, const GraphView<WT> &g, const int32_t 
                        cudaStream_t s);
 void launch_s2(const u64 *S, int32_t V, u64 *total_hi_lo, cudaStream_t s);
 
+// ---- small graphs: the rest of the level loop in one launch (lv_batch.cu) ----
+// One graph of at most TEAM_RUN_MAX_V vertices and TEAM_RUN_MAX_E entries, its
+// current level's communities singletons: a thread-block cluster runs the
+// level loop of lv_run to its end.  rows / w64 are the level's rows, w (level
+// 0) the float weights instead of w64.  comm, newc, size, k and S are the
+// caller's arrays and hold the last level's state afterwards.
+struct TeamJob {
+    const int32_t *rs, *re, *col;
+    const float *w;
+    const u64 *w64;
+    int32_t V;
+    int64_t E;
+    double scale;
+    bool narrow;           // level-0 weights fit 32 bits
+    double min_gain;
+    int32_t max_sweeps;
+    int32_t *comm, *newc, *size;
+    u64 *k, *S;
+};
+struct TeamResult {
+    double q;
+    int32_t status, V, levels, cur;   // cur: row buffer of the last level, -1 = the start rows
+    int64_t E, sweeps, edge_sweeps, vertex_sweeps, moves;
+};
+struct TeamRows {
+    TeamResult *result;    // in the arena
+    int32_t *o2c;          // start level's vertex -> last level's community
+    int32_t *rs[2], *re[2], *col[2];
+    u64 *w64[2];
+};
+// Where the line lies: see team_fits (lv_engine.cu).
+constexpr int32_t TEAM_RUN_MAX_V = 8192;
+constexpr int64_t TEAM_RUN_MAX_E = 65536;
+// Every sweep of a level but its last gains at least min_gain, and modularity
+// stays within [-1, 1]: with min_gain >= TEAM_RUN_MIN_GAIN no level reaches
+// the cap.
+constexpr double TEAM_RUN_MIN_GAIN = 5e-7;
+constexpr int32_t TEAM_RUN_SWEEP_CAP = 1 << 23;
+size_t team_arena_bytes(int32_t V, int64_t E);
+// Returns 1 when the launch was made, 0 when the device cannot run it.
+int team_run(const TeamJob &j, void *arena, int device, cudaStream_t s, TeamRows *rows);
+
 // ---- primitives (lv_prims.cu) ----
 // Exclusive scan of n int32 values (out may alias in); writes the total to
 // *total_dev.  tmp must hold scan_tmp_elems(n) int32.

@@ -451,3 +451,48 @@ def test_work_mapping_knobs_are_checked(lvb):
         with pytest.raises(lvb.LouvainError) as ex:
             lvb.Louvain(g, **kw)
         assert ex.value.status == lvb.LV_ERR_INVALID
+
+
+SMALL_RUNS = {
+    # sizes on both sides of the one-launch path's limits, and its level-0 weight widths
+    "two_vertices": lambda lvb: lvb.Graph(np.array([0, 1, 2], np.int32), np.array([1, 0], np.int32),
+                                          np.ones(2, np.float32)),
+    "small": lambda lvb: lvb.gen_planted(700, 12, 12.0, 2.0, 3),
+    "at_vertex_limit": lambda lvb: lvb.gen_planted(8192, 300, 5.0, 1.0, 4, "uniform"),
+    "over_vertex_limit": lambda lvb: lvb.gen_planted(8193, 300, 5.0, 1.0, 4, "uniform"),
+    "over_entry_limit": lambda lvb: lvb.gen_planted(5000, 32, 16.0, 2.0, 5, "uniform"),
+    "hubs": lambda lvb: lvb.gen_rmat(11, 16, 5, weights="unit"),
+}
+
+
+@pytest.mark.parametrize("name", sorted(SMALL_RUNS))
+def test_small_graph_runs_match_oracle(lvb, orc, name):
+    """lv_run on graphs small enough for the one-launch path: the result, and
+    the handle's state afterwards (communities, level, CSR, further sweeps,
+    aggregation and a reset) as on the level-by-level path."""
+    g = SMALL_RUNS[name](lvb)
+    o = orc.Oracle(g.rowptr, g.col, g.w)
+    q_ref, info = o.run(1e-6)
+    with lvb.Louvain(g) as e:
+        for again in range(2):
+            assert e.run(1e-6) == q_ref
+            assert np.array_equal(e.original_to_community()[0], o.original_to_community())
+            assert e.level_info()[:2] == (o.V, o.E)
+            assert np.array_equal(e.communities(), o.communities())
+            assert canon(*e.csr()) == canon(*o.csr())
+            st = e.stats()
+            assert (st["levels"], st["sweeps"], st["edge_sweeps"]) == (info["levels"], info["sweeps"],
+                                                                      info["edge_sweeps"])
+            assert e.calculate_modularity() == q_ref
+            if not again:
+                e.reset()
+                e.clear_stats()
+        assert e.sweep() == o.sweep()
+        assert np.array_equal(e.communities(), o.communities())
+        e.aggregate_communities()
+        o.aggregate_communities()
+        assert e.level_info()[:2] == (o.V, o.E)
+        e.reset()
+        assert np.array_equal(e.communities(), np.arange(g.V))
+        assert int(e.level_classes()[0].sum()) == int((np.diff(g.rowptr) > 0).sum())
+    o.close()
