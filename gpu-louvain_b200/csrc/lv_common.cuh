@@ -303,9 +303,16 @@ struct StateView {
     float *feat;   // learned active set: 2 features per vertex, written when set
     const uint8_t *wrow;   // rows with a weight of 2^32 or more (nullptr: none); such a
                            // vertex is decided by the large fallback queue (64-bit sums)
+    // the sub-round's movers: mv_cnt holds their count (low half) and their row
+    // units of 32 entries (high half), mv_off[i] the units before mover i
+    u64 *mv_cnt;
+    int32_t *mv_list;
+    uint32_t *mv_off;
     int dedup;             // aggregated level: the narrow insert loops combine a warp's
                            // equal keys before their shared atomics (key_peers)
 };
+
+__device__ __forceinline__ uint32_t mover_units(int32_t d) { return (uint32_t)(d + 31) >> 5; }
 
 // Exact 64-bit add to a table value.  In shared memory a 64-bit atomicAdd
 // is a compare-and-swap loop that spins when many lanes hit one slot, so it

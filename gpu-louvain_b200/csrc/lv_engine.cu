@@ -74,6 +74,17 @@ struct Totals {
     int pad;
 };
 
+// Counters of one sweep, cleared together with the totals by one memset: the
+// sub-rounds' mover counts, and a set of fallback-queue counters (count, next
+// per queue, then the warp cursor) for each launch of the wide kernels.
+constexpr int FB_SETS = 4;
+constexpr int FB_CTR = 2 * (NFBQ + 1) + 2;
+struct SweepBlock {
+    u64 movers[NBUCKETS];
+    int32_t fb[FB_SETS][FB_CTR];
+    Totals tot;
+};
+
 struct Pending {
     int kind;   // 0..NCLS-1 class, 100 move phase, 101 modularity, 102 aggregate, 103 setup
     cudaEvent_t a, b;
@@ -131,6 +142,8 @@ struct lv_handle {
     int cur_buf = -1;
 
     int32_t *comm = nullptr, *newc = nullptr, *size = nullptr, *orig2comm = nullptr;
+    int32_t *mv_list = nullptr;    // movers of a sub-round
+    uint32_t *mv_off = nullptr;
     u64 *k = nullptr, *S = nullptr;
     int32_t *list = nullptr;
     int32_t *cls_scratch = nullptr;   // class counts, cursors, then V0 entries of scratch
@@ -175,7 +188,8 @@ struct lv_handle {
 
     FallbackSet fb;
 
-    Totals *tot_d = nullptr;
+    SweepBlock *blk_d = nullptr;   // sweep counters and totals
+    Totals *tot_d = nullptr;       // = &blk_d->tot
     Totals *tot_h = nullptr;
     int32_t *small_h = nullptr;   // pinned scratch for counts
 
@@ -514,6 +528,7 @@ bool narrow_weights(const lv_handle *h) {
 StateView state_of(lv_handle *h) {
     return StateView{h->comm, h->newc, h->size, h->k, h->S, h->T, &h->tot_d->err, h->feat,
                      (LV_NARROW_ESCAPES == 1 && h->cur_w32 && h->wrows_any) ? h->wrow : nullptr,
+                     h->blk_d->movers, h->mv_list, h->mv_off,
                      (LV_DEDUP == 2 || (LV_DEDUP == 1 && h->level > 0)) ? 1 : 0};
 }
 
@@ -813,6 +828,18 @@ int ensure_setup(lv_handle *h) {
 // ---------------------------------------------------------------------------
 // Profile slots of the move phase: 0..3 the group kernels of buckets 0..3,
 // 4, 5, 6 the warp + fallback kernels of buckets 4, 5 and 6.
+// The fallback queues on counter set i of the sweep.
+FallbackSet queues_on(const lv_handle *h, int i) {
+    FallbackSet fs = h->fb;
+    int32_t *c = h->blk_d->fb[i];
+    for (int q = 0; q <= NFBQ; ++q) {
+        fs.q[q].count = c + 2 * q;
+        fs.q[q].next = fs.q[q].count + 1;
+    }
+    fs.warp_next = c + 2 * (NFBQ + 1);
+    return fs;
+}
+
 template <typename WT>
 void enqueue_sweep(lv_handle *h) {
     GraphView<WT> g = view_of<WT>(h);
@@ -826,6 +853,8 @@ void enqueue_sweep(lv_handle *h) {
         const int32_t lo = h->cls_off[c0], hi = h->cls_off[c1];
         if (hi == lo) continue;
         const int32_t hg0 = (b == 6) ? h->cls_off[CLS_HG] : hi;   // bucket 6: giants after
+        const FallbackSet fs = queues_on(h, b >= 4 ? b - 4 : 3);
+        st.mv_cnt = h->blk_d->movers + b;
         int64_t edges = 0;
         for (int c = c0; c < c1; ++c)
             if (c != CLS_HG) edges += h->cls_edges[c];
@@ -839,10 +868,11 @@ void enqueue_sweep(lv_handle *h) {
         }
         if (b < 4)
             launch_move_class<WT>(b, g, st, h->list + lo, hi - lo, h->di, dE, h->stream, narrow_weights<WT>(h),
-                                  h->fb);
+                                  fs);
         else if (hg0 > lo)
-            launch_move_wide<WT>(g, st, h->list + lo, hg0 - lo, h->fb, h->di, dE, h->stream,
-                                 b == 6 ? h->giant_degree : (b == 4 ? 84 : 319), narrow_weights<WT>(h));
+            launch_move_wide<WT>(g, st, h->list + lo, hg0 - lo, fs, h->di, dE, h->stream,
+                                 b == 6 ? h->giant_degree : (b == 4 ? 84 : 319), narrow_weights<WT>(h),
+                                 hi > hg0);
         if (tc) {
             tc->stop();
             delete tc;
@@ -856,17 +886,14 @@ void enqueue_sweep(lv_handle *h) {
                 tc->bytes = 12.0 * (double)tc->edges + 20.0 * (double)tc->verts;
                 tc->sbytes = (8.0 + wbytes) * (double)tc->edges + 20.0 * (double)tc->verts;
             }
-            launch_move_giants<WT>(g, st, h->hub_move.view, h->fb, h->di, dE, h->stream, narrow_weights<WT>(h));
+            launch_move_giants<WT>(g, st, h->hub_move.view, fs, h->di, dE, h->stream, narrow_weights<WT>(h));
             if (tc) {
                 tc->stop();
                 delete tc;
             }
         }
-        // exact modularity bookkeeping for neighbours that moved together
-        for (int c = c0; c < c1; ++c)
-            launch_correction<WT>(c, g, st, h->list + h->cls_off[c], h->cls_off[c + 1] - h->cls_off[c],
-                                  h->di, dE, h->stream);
-        launch_commit(st, h->list + lo, hi - lo, &h->tot_d->moves, h->stream);
+        if (b >= 4) launch_collect_movers<WT>(g, st, h->list + lo, hi - lo, h->stream);
+        launch_movers<WT>(g, st, hi - lo, h->di, dE, &h->tot_d->moves, h->stream);
         sweep_verts += hi - lo;
     }
     tm.bytes = 12.0 * (double)h->E + 20.0 * (double)sweep_verts;
@@ -896,8 +923,9 @@ double q_from_totals(u64 T, const Totals &t) {
     return a - b;
 }
 
+// Clears the sweep counters and the totals, keeping the device error word.
 int reset_totals(lv_handle *h) {
-    LV_CUDA(h, cudaMemsetAsync(h->tot_d, 0, offsetof(Totals, err), h->stream));
+    LV_CUDA(h, cudaMemsetAsync(h->blk_d, 0, offsetof(SweepBlock, tot) + offsetof(Totals, err), h->stream));
     return LV_OK;
 }
 
@@ -928,6 +956,7 @@ int sweep_and_q(lv_handle *h, int64_t *moves, double *q) {
         LV_TRY(modularity(h, &q0));
     }
     LV_TRY(reset_totals(h));
+    clear_move_state(h->fb, h->hub_move.view, h->stream);
     LV_BY_WEIGHT(h, enqueue_sweep, h);
     {
         Timer tm(h, 101);
@@ -1020,6 +1049,7 @@ int sweep_loop_graph(lv_handle *h, float min_gain, double q_start, int *ch, int 
     ls.q_last = q_start;
     ls.max_sweeps = h->opts.max_sweeps;
     LV_CUDA(h, cudaMemcpyAsync(ld, &ls, sizeof(ls), cudaMemcpyHostToDevice, h->stream));
+    clear_move_state(h->fb, h->hub_move.view, h->stream);
     LV_TRY(sync(h));
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -1043,7 +1073,7 @@ int sweep_loop_graph(lv_handle *h, float min_gain, double q_start, int *ch, int 
                                            cudaStreamCaptureModeRelaxed) == cudaSuccess;
         if (ok) {
             h->capturing = true;
-            cudaMemsetAsync(h->tot_d, 0, offsetof(Totals, err), h->stream);
+            reset_totals(h);
             LV_BY_WEIGHT(h, enqueue_sweep, h);
             launch_s2(h->S, h->V, h->tot_d->s2, h->stream);
             sweep_end_kernel<<<1, 32, 0, h->stream>>>(cond, h->tot_d, ld);
@@ -1139,21 +1169,25 @@ void enqueue_sweep_active(lv_handle *h, const int32_t *cnt) {
         int64_t any = 0;
         for (int c = c0; c < c1; ++c) any += cnt[c];
         if (!any) continue;
+        st.mv_cnt = h->blk_d->movers + b;
         if (b < 4) {
             launch_move_class<WT>(b, g, st, h->alist + h->cls_off[b], cnt[b], h->di, dE, h->stream,
-                                  narrow_weights<WT>(h), h->fb);
+                                  narrow_weights<WT>(h), queues_on(h, 3));
         } else {
             for (int c = c0; c < c1; ++c) {
                 if (c == CLS_HG || !cnt[c]) continue;
                 const int32_t maxdeg = c == CLS_B4 ? 84 : (c == CLS_B5 ? 319 : (c == CLS_H1 ? 1024 : h->giant_degree));
-                launch_move_wide<WT>(g, st, h->alist + h->cls_off[c], cnt[c], h->fb, h->di, dE, h->stream, maxdeg,
-                                     narrow_weights<WT>(h));
+                // sets 0..3: classes B4, B5, H1, H2 (H2 shares its large queue with the giants)
+                launch_move_wide<WT>(g, st, h->alist + h->cls_off[c], cnt[c], queues_on(h, c - CLS_B4), h->di, dE,
+                                     h->stream, maxdeg, narrow_weights<WT>(h), c == CLS_H2 && cnt[CLS_HG] > 0);
             }
-            if (b == 6 && cnt[CLS_HG]) launch_move_giants<WT>(g, st, h->hub_move.view, h->fb, h->di, dE, h->stream, narrow_weights<WT>(h));
+            if (b == 6 && cnt[CLS_HG])
+                launch_move_giants<WT>(g, st, h->hub_move.view, queues_on(h, CLS_H2 - CLS_B4), h->di, dE, h->stream,
+                                       narrow_weights<WT>(h));
         }
         for (int c = c0; c < c1; ++c)
-            launch_correction<WT>(c, g, st, h->alist + h->cls_off[c], cnt[c], h->di, dE, h->stream);
-        for (int c = c0; c < c1; ++c) launch_commit(st, h->alist + h->cls_off[c], cnt[c], &h->tot_d->moves, h->stream);
+            if (b >= 4) launch_collect_movers<WT>(g, st, h->alist + h->cls_off[c], cnt[c], h->stream);
+        launch_movers<WT>(g, st, (int32_t)any, h->di, dE, &h->tot_d->moves, h->stream);
         verts += any;
     }
     tm.bytes = 20.0 * (double)verts;
@@ -1166,6 +1200,7 @@ void enqueue_sweep_active(lv_handle *h, const int32_t *cnt) {
 int sweep_learned(lv_handle *h, bool full, bool predict, int64_t *moves, double *q, int64_t *movers,
                   int64_t *hits, int64_t *fresh_movers) {
     LV_TRY(reset_totals(h));
+    clear_move_state(h->fb, h->hub_move.view, h->stream);
     LV_CUDA(h, cudaMemsetAsync(h->actr, 0, 2 * sizeof(u64), h->stream));
     LV_CUDA(h, cudaMemsetAsync(h->actr + 3, 0, sizeof(u64), h->stream));
     const int32_t n = h->cls_off[NCLS];
@@ -1564,6 +1599,8 @@ int ensure_move(lv_handle *h) {
     if (h->move_ready) return LV_OK;
     const size_t V = (size_t)h->V0;
     LV_TRY(dalloc(h, &h->list, V + 1));
+    LV_TRY(dalloc(h, &h->mv_list, V + 1));
+    LV_TRY(dalloc(h, &h->mv_off, V + 1));
     LV_TRY(dalloc(h, &h->sort_buf, 3 * V + 16));
     h->sort_temp_bytes = sort_by_degree_temp_bytes((int32_t)V, HG_MIN_DEG_HI) + 256;
     {
@@ -1577,17 +1614,12 @@ int ensure_move(lv_handle *h) {
         // level); a large item covers FB_KEYS edges of a vertex of degree
         // > FBQ_MAXDEG(NFBQ - 1), or as many staged pairs of a giant.
         FallbackSet &fs = h->fb;
-        int32_t *counters = nullptr;
-        LV_TRY(dalloc(h, &counters, 2 * (NFBQ + 1) + 2));
-        fs.warp_next = counters + 2 * (NFBQ + 1);
         LV_TRY(dalloc(h, &fs.hint, V + 1));
         LV_CUDA(h, cudaMemsetAsync(fs.hint, 0, V + 1, h->stream));
         const size_t cap_row = (size_t)(h->E0 / fs.warp_limit) + 64;
         const size_t cap_large = (size_t)(2 * (h->E0 / FBQ_MAXDEG(NFBQ - 1) + h->E0 / FB_KEYS)) + 64;
         for (int q = 0; q <= NFBQ; ++q) {
             Fallback &f = fs.q[q];
-            f.count = counters + 2 * q;
-            f.next = f.count + 1;
             const size_t cap = q < NFBQ ? cap_row : cap_large;
             f.cap = (int32_t)cap;
             LV_TRY(dalloc(h, &f.v, cap));
@@ -1622,8 +1654,9 @@ int finish_create(lv_handle *h) {
     LV_TRY(dalloc(h, &h->k, V + 1));
     LV_TRY(dalloc(h, &h->S, V + 1));
     LV_TRY(dalloc(h, &h->cls_scratch, V + SCRATCH_OFF + 16));
-    LV_TRY(dalloc(h, &h->tot_d, 1));
-    LV_CUDA(h, cudaMemsetAsync(h->tot_d, 0, sizeof(Totals), h->stream));
+    LV_TRY(dalloc(h, &h->blk_d, 1));
+    h->tot_d = &h->blk_d->tot;
+    LV_CUDA(h, cudaMemsetAsync(h->blk_d, 0, sizeof(SweepBlock), h->stream));
     LV_TRY(pinned_take(h));
     // CSR validation
     launch_validate_csr(h->in_rowptr, h->in_col, h->V0, h->E0, &h->tot_d->err, h->stream);
@@ -1773,7 +1806,7 @@ int lv_destroy(lv_handle *h) {
     }
     {
         FallbackSet &fs = h->fb;
-        dfree(h, fs.q[0].count); dfree(h, fs.hint);
+        dfree(h, fs.hint);
         for (int q = 0; q <= NFBQ; ++q) {
             Fallback &f = fs.q[q];
             dfree(h, f.v); dfree(h, f.p); dfree(h, f.P); dfree(h, f.first); dfree(h, f.done); dfree(h, f.src);
@@ -1810,7 +1843,8 @@ int lv_destroy(lv_handle *h) {
         dfree(h, t);
         h->team_arena = nullptr;
     }
-    dfree(h, h->tot_d);
+    dfree(h, h->blk_d);
+    dfree(h, h->mv_list); dfree(h, h->mv_off);
     dfree(h, h->feat); dfree(h, h->moved); dfree(h, h->nmoved); dfree(h, h->pred); dfree(h, h->fresh);
     dfree(h, h->comm_prev); dfree(h, h->alist);
     dfree(h, h->acnt); dfree(h, h->actr); dfree(h, h->model); dfree(h, h->tr_x); dfree(h, h->tr_v);

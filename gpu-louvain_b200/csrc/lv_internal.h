@@ -196,21 +196,32 @@ void launch_move_class(int cls, const GraphView<WT> &g, const StateView &st, con
                        int32_t n, const DeviceInfo &di, u64 *dE, cudaStream_t s, bool narrow,
                        const FallbackSet &fb);
 // 32 < degree <= 8192 (the vertices of one update bucket): warp kernel +
-// fallback.  Degree > 8192: staged chunks + merge (hg describes the giants).
+// fallback (large_later: the large queue's items are left to a following
+// launch_move_giants on the same queue counters).  Degree > 8192: staged chunks + merge (hg describes the giants).
 // narrow: every weight the kernels read is below 2^32 (piece-counter tables).
 template <typename WT>
 void launch_move_wide(const GraphView<WT> &g, const StateView &st, const int32_t *list, int32_t n,
                       const FallbackSet &fb, const DeviceInfo &di, u64 *dE, cudaStream_t s,
-                      int32_t max_degree, bool narrow);
+                      int32_t max_degree, bool narrow, bool large_later = false);
 template <typename WT>
 void launch_move_giants(const GraphView<WT> &g, const StateView &st, const HubGlobal &hg,
                         const FallbackSet &fb, const DeviceInfo &di, u64 *dE, cudaStream_t s, bool narrow);
-// Exact correction of dE for neighbours that moved in the same sub-round.
+// Lists the movers among list[0 .. n) (the kernels of buckets 0..3 list their
+// own).
 template <typename WT>
-void launch_correction(int cls, const GraphView<WT> &g, const StateView &st, const int32_t *list,
-                       int32_t n, const DeviceInfo &di, u64 *dE, cudaStream_t s);
-void launch_commit(const StateView &st, const int32_t *list, int32_t n, u64 *moves,
+void launch_collect_movers(const GraphView<WT> &g, const StateView &st, const int32_t *list, int32_t n,
+                           cudaStream_t s);
+// The sub-round's listed movers: exact correction of dE for neighbours that
+// moved together, then the commit.  n bounds their number.
+template <typename WT>
+void launch_movers(const GraphView<WT> &g, const StateView &st, int32_t n, const DeviceInfo &di, u64 *dE, u64 *moves,
                    cudaStream_t s);
+// The staging counters, own-community sums and partition done counters of the
+// giant and large-queue paths are returned to zero by the kernel that consumes
+// them; cleared before a level's sweeps as well, so that a sweep that ended
+// early (a device error, an item the full large queue could not take) cannot
+// leave a count that makes a later staging pass append beyond a giant's area.
+void clear_move_state(const FallbackSet &fs, const HubGlobal &hg, cudaStream_t s);
 
 // k_i = row sums (mode 0) or e_own total (mode 1) over the vertices of one class.
 template <typename WT>

@@ -35,6 +35,41 @@ __device__ __forceinline__ void block_add_total(u64 x, u64 *total) {
     __syncthreads();
 }
 
+// Lists the CTA's movers (v >= 0 in the threads that hold one, with the units
+// of their rows) with one global atomic: count and unit total share it, so a
+// mover's index and unit offset rise together.  Every thread calls it.
+template <int THREADS>
+__device__ __forceinline__ void block_note_movers(const StateView &st, int32_t v, uint32_t units) {
+    constexpr int NW = THREADS / 32;
+    __shared__ u64 wsum[NW];
+    __shared__ u64 at0;
+    if (!__syncthreads_or(v >= 0)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const u64 own = v >= 0 ? ((u64)units << 32) | 1ull : 0ull;
+    u64 inc = own;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const u64 y = __shfl_up_sync(FULL, inc, off);
+        if (lane >= off) inc += y;
+    }
+    if (lane == 31) wsum[w] = inc;
+    __syncthreads();
+    u64 pre = 0, tot = 0;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+        const u64 y = wsum[i];
+        pre += i < w ? y : 0;
+        tot += y;
+    }
+    if (threadIdx.x == 0) at0 = atomicAdd(st.mv_cnt, tot);
+    __syncthreads();
+    if (v >= 0) {
+        const u64 at = at0 + pre + inc - own;
+        st.mv_list[(uint32_t)at] = v;
+        st.mv_off[(uint32_t)at] = (uint32_t)(at >> 32);
+    }
+}
+
 // Queue vertex v (degree d) for the large queue only (64-bit sums, any row):
 // the vertices of a 32-bit-view level whose row holds a sum of 2^32 or more.
 // One lane calls it.
@@ -91,11 +126,15 @@ __global__ void __launch_bounds__(256) move_group_kernel(GraphView<WT> g, StateV
     if (active) eval_slots<(CAP / G > 1 ? (LV_U_EVAL < 2 ? LV_U_EVAL : 2) : 1), false, false>(keys, vals, nullptr, CAP, lane, G, m, st.S, st.size, b);
     group_reduce_best(m, b, G);
     u64 delta = 0;
+    int32_t mover = -1;
     if (active && lane == 0) {
-        st.newc[v] = move_decision(m, b, &delta);
+        const int32_t nc = move_decision(m, b, &delta);
+        st.newc[v] = nc;
+        if (nc != own) mover = v;
         record_features(st, v, m, b);
     }
     block_add_total<256>(delta, dE);
+    block_note_movers<256>(st, mover, 1u);
 }
 
 // move_group_kernel for weights below 2^32: the group's table keeps its sums
@@ -156,11 +195,15 @@ __global__ void __launch_bounds__(256) move_group_narrow_kernel(GraphView<WT> g,
     }
     group_reduce_best(m, b, G);
     u64 delta = 0;
+    int32_t mover = -1;
     if (active && lane == 0) {
-        st.newc[v] = move_decision(m, b, &delta);
+        const int32_t nc = move_decision(m, b, &delta);
+        st.newc[v] = nc;
+        if (nc != own) mover = v;
         record_features(st, v, m, b);
     }
     block_add_total<256>(delta, dE);
+    block_note_movers<256>(st, mover, 1u);
 }
 
 // CTA-wide reduction of a Best; the result is valid in thread 0.
@@ -1326,102 +1369,121 @@ __device__ __forceinline__ u64 pair_correction(int32_t cu, int32_t nu, int32_t c
     return (u64)(i64)t * w;
 }
 
-template <int G, typename WT>
-__global__ void __launch_bounds__(256) corr_group_kernel(GraphView<WT> g, const int32_t *__restrict__ comm,
-                                                         const int32_t *__restrict__ newc,
-                                                         const int32_t *__restrict__ list, int32_t n,
-                                                         u64 *dE) {
-    const int grp = threadIdx.x / G, lane = threadIdx.x % G;
-    const int32_t idx = blockIdx.x * (256 / G) + grp;
+// The movers' rows, cut into units of 32 entries, are shared evenly by the
+// grid's warps (the movers' unit offsets are the list's prefix sums), so that
+// neither a hub among the movers nor many short rows leave warps idle, and a
+// sub-round without movers costs one read.  Bound by the latency of the
+// column -> community chain; four units are in flight per warp.
+constexpr int CORR_U = 4;
+
+// The movers of buckets 4 to 6, found after the sub-round's decisions: noting
+// them in the warp kernels cost the 64-bit one 12 % (119 against 107 ms for
+// degrees 320 to 8192 of an R-MAT-24 run).
+template <typename WT>
+__global__ void __launch_bounds__(256) collect_movers_kernel(GraphView<WT> g, StateView st,
+                                                             const int32_t *__restrict__ list, int32_t n) {
+    const int32_t i = blockIdx.x * 256 + threadIdx.x;
+    int32_t v = -1;
+    uint32_t units = 0;
+    if (i < n) {
+        const int32_t x = list[i];
+        if (st.newc[x] != st.comm[x]) {
+            v = x;
+            units = mover_units(g.rowend[x] - g.rowptr[x]);
+        }
+    }
+    block_note_movers<256>(st, v, units);
+}
+
+template <typename WT>
+__global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, StateView st, u64 *dE) {
+    const u64 cu64 = *st.mv_cnt;
+    const uint32_t n = (uint32_t)cu64, units = (uint32_t)(cu64 >> 32);
+    const int lane = threadIdx.x & 31;
+    const uint32_t nw = gridDim.x * 8, w = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const uint32_t per = (units + nw - 1) / nw;
+    if ((u64)blockIdx.x * 8 * per >= units) return;   // the whole CTA is past the end
+    u64 u0 = (u64)w * per, u1 = u0 + per;
+    if (u1 > units) u1 = units;
     u64 acc = 0;
-    if (idx < n) {
-        const int32_t u = list[idx];
-        const int32_t cu = comm[u], nu = newc[u];
-        if (cu != nu) {
-            const int32_t r0 = g.rowptr[u], r1 = g.rowend[u];
-            for (int32_t e = r0 + lane; e < r1; e += G) {
-                const int32_t j = __ldg(g.col + e);
-                if (j == u) continue;
-                const int32_t cj = comm[j], nj = newc[j];
-                if (cj != nj) acc += pair_correction(cu, nu, cj, nj, gw(g, e));
+    if (u0 < u1) {
+        // the last mover whose first unit is at or before u0: 32 probes per step
+        uint32_t lo = 0, hi = n;
+        while (hi - lo > 1) {
+            const uint32_t step = (hi - lo + 31) >> 5;
+            const u64 p = (u64)lo + (u64)lane * step;
+            const bool le = p < hi && st.mv_off[p] <= (uint32_t)u0;
+            const int k = __popc(__ballot_sync(FULL, le)) - 1;   // lane 0 always holds
+            lo += (uint32_t)k * step;
+            hi = (u64)lo + step < hi ? lo + step : hi;
+        }
+        uint32_t u = (uint32_t)u0;
+        const uint32_t ue = (uint32_t)u1;
+        for (uint32_t i0 = lo; u < ue; i0 += 32) {
+            // headers of the next 32 movers, one per lane
+            int32_t lv = 0, lc = 0, ln = 0, lr0 = 0, lr1 = 0;
+            uint32_t lo_u = 0;
+            if (i0 + lane < n) {
+                lv = st.mv_list[i0 + lane];
+                lo_u = st.mv_off[i0 + lane];
+                lc = st.comm[lv];
+                ln = st.newc[lv];
+                lr0 = g.rowptr[lv];
+                lr1 = g.rowend[lv];
+            }
+            for (int k = 0; k < 32 && u < ue; ++k) {
+                const int32_t v = __shfl_sync(FULL, lv, k), cu = __shfl_sync(FULL, lc, k), nu = __shfl_sync(FULL, ln, k);
+                const int32_t r0 = __shfl_sync(FULL, lr0, k), r1 = __shfl_sync(FULL, lr1, k);
+                const uint32_t o = __shfl_sync(FULL, lo_u, k);
+                const uint32_t mu = mover_units(r1 - r0);
+                const uint32_t last = o + mu < ue ? o + mu : ue;   // units [u, last) of this mover
+                const int32_t e1 = last == o + mu ? r1 : r0 + (int32_t)((last - o) << 5);
+                for (int32_t e0 = r0 + (int32_t)((u - o) << 5) + lane; e0 - lane < e1; e0 += 32 * CORR_U) {
+                    int32_t jj[CORR_U];
+#pragma unroll
+                    for (int q = 0; q < CORR_U; ++q) {
+                        const int32_t e = e0 + 32 * q;
+                        jj[q] = e < e1 ? __ldg(g.col + e) : v;
+                    }
+                    int32_t cj[CORR_U], nj[CORR_U];
+#pragma unroll
+                    for (int q = 0; q < CORR_U; ++q) {
+                        cj[q] = nj[q] = 0;
+                        if (jj[q] != v) {
+                            cj[q] = __ldg(st.comm + jj[q]);
+                            nj[q] = __ldg(st.newc + jj[q]);
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < CORR_U; ++q)
+                        if (cj[q] != nj[q]) acc += pair_correction(cu, nu, cj[q], nj[q], gw(g, e0 + 32 * q));
+                }
+                u = last;
             }
         }
     }
     block_add_total<256>(acc, dE);
 }
 
-// Rows of T threads each.  A pass checks CORR_BATCH vertices of the list at
-// once (one per lane of warp 0), gathers the ones that moved in shared
-// memory, and then scans only their rows, so a sub-round with few movers
-// costs one parallel check per CORR_BATCH vertices instead of a serial check
-// per vertex.
-constexpr int CORR_BATCH = 32;
-
-template <int T, typename WT>
-__global__ void __launch_bounds__(T) corr_cta_kernel(GraphView<WT> g, const int32_t *__restrict__ comm,
-                                                     const int32_t *__restrict__ newc,
-                                                     const int32_t *__restrict__ list, int32_t n,
-                                                     u64 *dE) {
-    __shared__ int32_t movers[CORR_BATCH];
-    __shared__ int32_t nm;
-    u64 acc = 0;
-    for (int32_t base = blockIdx.x * CORR_BATCH; base < n; base += gridDim.x * CORR_BATCH) {
-        if (threadIdx.x < 32) {
-            const int32_t idx = base + threadIdx.x;
-            bool moved = false;
-            int32_t u = 0;
-            if (idx < n) {
-                u = list[idx];
-                moved = comm[u] != newc[u];
-            }
-            const unsigned bal = __ballot_sync(FULL, moved);
-            if (moved) movers[__popc(bal & ((1u << threadIdx.x) - 1u))] = u;
-            if (threadIdx.x == 0) nm = __popc(bal);
-        }
-        __syncthreads();
-        const int32_t cnt = nm;
-        for (int32_t k = 0; k < cnt; ++k) {
-            const int32_t u = movers[k];
-            const int32_t cu = comm[u], nu = newc[u];
-            const int32_t r0 = g.rowptr[u], r1 = g.rowend[u];
-            for (int32_t e = r0 + threadIdx.x; e < r1; e += T) {
-                const int32_t j = __ldg(g.col + e);
-                if (j == u) continue;
-                const int32_t cj = comm[j], nj = newc[j];
-                if (cj != nj) acc += pair_correction(cu, nu, cj, nj, gw(g, e));
-            }
-        }
-        __syncthreads();   // movers / nm are rewritten by the next pass
-    }
-    block_add_total<T>(acc, dE);
-}
-
 // ------------------------------------------------------------------------
 // commit of one sub-round (updateVertexCommunity + Sigma_tot update)
 // ------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) commit_kernel(StateView st, const int32_t *__restrict__ list,
-                                                     int32_t n, u64 *moves) {
-    const int32_t i = blockIdx.x * 256 + threadIdx.x;
-    u64 mv = 0;
-    if (i < n) {
-        const int32_t v = list[i];
+// Over the listed movers only (grid-stride; the count is on the device).
+__global__ void __launch_bounds__(256) commit_kernel(StateView st, u64 *moves) {
+    const uint32_t n = (uint32_t)*st.mv_cnt;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(moves, (u64)n);
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        const int32_t v = st.mv_list[i];
         const int32_t nc = st.newc[v], oc = st.comm[v];
-        if (nc != oc) {
-            mv = 1;
-            st.comm[v] = nc;
-            atomicAdd(st.size + nc, 1);
-            atomicSub(st.size + oc, 1);
-            const u64 kv = st.k[v];
-            atomicAdd(st.S + nc, kv);
-            atomicAdd(st.S + oc, (u64)0 - kv);
-        }
+        const u64 kv = st.k[v];
+        st.comm[v] = nc;
+        atomicAdd(st.size + nc, 1);
+        atomicSub(st.size + oc, 1);
+        atomicAdd(st.S + nc, kv);
+        atomicAdd(st.S + oc, (u64)0 - kv);
     }
-    block_add_total<256>(mv, moves);
 }
 
-// ------------------------------------------------------------------------
-// row reductions: k_i (mode 0) and sum_i e_{i->C(i)} (mode 1)
-// ------------------------------------------------------------------------
 template <int G, int MODE, typename WT>
 __global__ void __launch_bounds__(256) row_reduce_group_kernel(GraphView<WT> g,
                                                                const int32_t *__restrict__ comm,
@@ -1688,15 +1750,6 @@ template <typename WT>
 void launch_move_giants(const GraphView<WT> &g, const StateView &st, const HubGlobal &hg,
                         const FallbackSet &fs, const DeviceInfo &di, u64 *dE, cudaStream_t s, bool narrow) {
     if (hg.nhubs <= 0) return;
-    cudaMemsetAsync(fs.q[NFBQ].count, 0, 2 * sizeof(int32_t), s);   // count, next
-    // The staging counters, the own-community sums and the partition done
-    // counters are returned to zero by the kernel that consumes them; they are
-    // cleared here as well, so that a sweep that ended early (a device error,
-    // an item the full large queue could not take) cannot leave a count that
-    // makes the next staging pass append beyond a giant's area.
-    cudaMemsetAsync(hg.nocc, 0, sizeof(int32_t) * (size_t)hg.nhubs, s);
-    cudaMemsetAsync(hg.eown, 0, sizeof(u64) * (size_t)hg.nhubs, s);
-    cudaMemsetAsync(fs.q[NFBQ].done, 0, sizeof(int32_t) * (size_t)fs.q[NFBQ].cap, s);
     if (narrow) {
         giant_stage_narrow_kernel<WT><<<(unsigned)imin64(hg.n_echunks, (int64_t)di.sms * di.occ_stage_narrow),
                                         STAGE_THREADS, STAGE_SMEM, s>>>(g, st, hg);
@@ -1731,16 +1784,19 @@ void launch_move_giants(const GraphView<WT> &g, const StateView &st, const HubGl
     launch_fallback_large<WT>(g, st, hg, fs, di, dE, s);
 }
 
+void clear_move_state(const FallbackSet &fs, const HubGlobal &hg, cudaStream_t s) {
+    cudaMemsetAsync(fs.q[NFBQ].done, 0, sizeof(int32_t) * (size_t)fs.q[NFBQ].cap, s);
+    if (hg.nhubs > 0) {
+        cudaMemsetAsync(hg.nocc, 0, sizeof(int32_t) * (size_t)hg.nhubs, s);
+        cudaMemsetAsync(hg.eown, 0, sizeof(u64) * (size_t)hg.nhubs, s);
+    }
+}
+
 template <typename WT>
 void launch_move_wide(const GraphView<WT> &g, const StateView &st, const int32_t *list, int32_t n,
                       const FallbackSet &fs, const DeviceInfo &di, u64 *dE, cudaStream_t s,
-                      int32_t max_degree, bool narrow) {
+                      int32_t max_degree, bool narrow, bool large_later) {
     if (n <= 0) return;
-    // the queues' (count, next) pairs are contiguous; the large queue's done
-    // counters are cleared as in launch_move_giants
-    cudaMemsetAsync(fs.q[0].count, 0, (2 * (NFBQ + 1) + 1) * sizeof(int32_t), s);   // + the warp cursor
-    if (max_degree > fs.warp_limit || (narrow && st.wrow))
-        cudaMemsetAsync(fs.q[NFBQ].done, 0, sizeof(int32_t) * (size_t)fs.q[NFBQ].cap, s);
     if (narrow) {
         const unsigned grid = (unsigned)imin64((n + 7) / 8, (int64_t)di.sms * di.occ_warp_narrow);
         move_warp_narrow_kernel<WT><<<grid, 256, WARP_NSMEM, s>>>(g, st, list, n, fs, dE);
@@ -1753,7 +1809,7 @@ void launch_move_wide(const GraphView<WT> &g, const StateView &st, const int32_t
         if (narrow && st.wrow) launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
         return;
     }
-    launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
+    if (!large_later) launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
     launch_row_queue<WT, 3>(g, st, fs, di, dE, s, narrow);
     launch_row_queue<WT, 2>(g, st, fs, di, dE, s, narrow);
     launch_row_queue<WT, 1>(g, st, fs, di, dE, s, narrow);
@@ -1761,31 +1817,20 @@ void launch_move_wide(const GraphView<WT> &g, const StateView &st, const int32_t
 }
 
 template <typename WT>
-void launch_correction(int cls, const GraphView<WT> &g, const StateView &st, const int32_t *list,
-                       int32_t n, const DeviceInfo &di, u64 *dE, cudaStream_t s) {
+void launch_collect_movers(const GraphView<WT> &g, const StateView &st, const int32_t *list, int32_t n,
+                           cudaStream_t s) {
     if (n <= 0) return;
-    switch (cls) {
-    case CLS_B0: corr_group_kernel<4, WT><<<nblocks(n, 64), 256, 0, s>>>(g, st.comm, st.newc, list, n, dE); break;
-    case CLS_B1: corr_group_kernel<8, WT><<<nblocks(n, 32), 256, 0, s>>>(g, st.comm, st.newc, list, n, dE); break;
-    case CLS_B2: corr_group_kernel<16, WT><<<nblocks(n, 16), 256, 0, s>>>(g, st.comm, st.newc, list, n, dE); break;
-    case CLS_B3:
-    case CLS_B4: corr_group_kernel<32, WT><<<nblocks(n, 8), 256, 0, s>>>(g, st.comm, st.newc, list, n, dE); break;
-    case CLS_B5:
-        corr_cta_kernel<128, WT><<<(unsigned)imin64(nblocks(n, CORR_BATCH), (int64_t)di.sms * 16), 128, 0, s>>>(g, st.comm, st.newc, list, n, dE);
-        break;
-    case CLS_H1:
-        corr_cta_kernel<256, WT><<<(unsigned)imin64(nblocks(n, CORR_BATCH), (int64_t)di.sms * 8), 256, 0, s>>>(g, st.comm, st.newc, list, n, dE);
-        break;
-    default:
-        corr_cta_kernel<512, WT><<<(unsigned)imin64(nblocks(n, CORR_BATCH), (int64_t)di.sms * 4), 512, 0, s>>>(g, st.comm, st.newc, list, n, dE);
-        break;
-    }
+    collect_movers_kernel<WT><<<nblocks(n, 256), 256, 0, s>>>(g, st, list, n);
     note_launches(1);
 }
 
-void launch_commit(const StateView &st, const int32_t *list, int32_t n, u64 *moves, cudaStream_t s) {
+template <typename WT>
+void launch_movers(const GraphView<WT> &g, const StateView &st, int32_t n, const DeviceInfo &di, u64 *dE, u64 *moves,
+                   cudaStream_t s) {
     if (n <= 0) return;
-    commit_kernel<<<nblocks(n, 256), 256, 0, s>>>(st, list, n, moves); note_launches(1);
+    corr_movers_kernel<WT><<<(unsigned)imin64(nblocks(n, 8), (int64_t)di.sms * 8), 256, 0, s>>>(g, st, dE);
+    commit_kernel<<<(unsigned)imin64(nblocks(n, 256), (int64_t)di.sms * 8), 256, 0, s>>>(st, moves);
+    note_launches(2);
 }
 
 template <typename WT>
@@ -1838,21 +1883,23 @@ template void launch_move_class<u64>(int, const GraphView<u64> &, const StateVie
                                      cudaStream_t, bool, const FallbackSet &);
 template void launch_move_wide<float>(const GraphView<float> &, const StateView &, const int32_t *,
                                       int32_t, const FallbackSet &, const DeviceInfo &, u64 *,
-                                      cudaStream_t, int32_t, bool);
+                                      cudaStream_t, int32_t, bool, bool);
 template void launch_move_wide<u64>(const GraphView<u64> &, const StateView &, const int32_t *,
                                     int32_t, const FallbackSet &, const DeviceInfo &, u64 *,
-                                    cudaStream_t, int32_t, bool);
+                                    cudaStream_t, int32_t, bool, bool);
 template void launch_move_giants<float>(const GraphView<float> &, const StateView &,
                                         const HubGlobal &, const FallbackSet &, const DeviceInfo &,
                                         u64 *, cudaStream_t, bool);
 template void launch_move_giants<u64>(const GraphView<u64> &, const StateView &, const HubGlobal &,
                                       const FallbackSet &, const DeviceInfo &, u64 *, cudaStream_t, bool);
-template void launch_correction<float>(int, const GraphView<float> &, const StateView &,
-                                       const int32_t *, int32_t, const DeviceInfo &, u64 *,
-                                       cudaStream_t);
-template void launch_correction<u64>(int, const GraphView<u64> &, const StateView &,
-                                     const int32_t *, int32_t, const DeviceInfo &, u64 *,
-                                     cudaStream_t);
+template void launch_collect_movers<float>(const GraphView<float> &, const StateView &, const int32_t *, int32_t,
+                                           cudaStream_t);
+template void launch_movers<float>(const GraphView<float> &, const StateView &, int32_t, const DeviceInfo &, u64 *, u64 *,
+                                   cudaStream_t);
+template void launch_collect_movers<u64>(const GraphView<u64> &, const StateView &, const int32_t *, int32_t,
+                                           cudaStream_t);
+template void launch_movers<u64>(const GraphView<u64> &, const StateView &, int32_t, const DeviceInfo &, u64 *, u64 *,
+                                   cudaStream_t);
 template void launch_row_reduce<float>(int, int, const GraphView<float> &, const int32_t *, u64 *,
                                        u64 *, const int32_t *, int32_t, const DeviceInfo &,
                                        cudaStream_t);
@@ -1865,12 +1912,13 @@ template void launch_move_class<uint32_t>(int, const GraphView<uint32_t> &, cons
                                      cudaStream_t, bool, const FallbackSet &);
 template void launch_move_wide<uint32_t>(const GraphView<uint32_t> &, const StateView &, const int32_t *,
                                     int32_t, const FallbackSet &, const DeviceInfo &, u64 *,
-                                    cudaStream_t, int32_t, bool);
+                                    cudaStream_t, int32_t, bool, bool);
 template void launch_move_giants<uint32_t>(const GraphView<uint32_t> &, const StateView &, const HubGlobal &,
                                       const FallbackSet &, const DeviceInfo &, u64 *, cudaStream_t, bool);
-template void launch_correction<uint32_t>(int, const GraphView<uint32_t> &, const StateView &,
-                                     const int32_t *, int32_t, const DeviceInfo &, u64 *,
-                                     cudaStream_t);
+template void launch_collect_movers<uint32_t>(const GraphView<uint32_t> &, const StateView &, const int32_t *, int32_t,
+                                           cudaStream_t);
+template void launch_movers<uint32_t>(const GraphView<uint32_t> &, const StateView &, int32_t, const DeviceInfo &, u64 *, u64 *,
+                                   cudaStream_t);
 template void launch_row_reduce<uint32_t>(int, int, const GraphView<uint32_t> &, const int32_t *, u64 *,
                                      u64 *, const int32_t *, int32_t, const DeviceInfo &,
                                      cudaStream_t);
