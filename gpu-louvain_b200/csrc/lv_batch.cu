@@ -1556,12 +1556,11 @@ struct lv_batch {
     int64_t E = 0;
     std::vector<int32_t> gptr_h;
     std::vector<int64_t> entries_h;   // [G] entries per graph
-    bool owns_input = false;
     const int32_t *rowptr = nullptr, *col = nullptr;
     const float *w = nullptr;
     BatchParams P{};
     int64_t tbl_total = 0;
-    std::vector<void *> allocs;
+    MemSet mem;
     struct Tier { int nc; int32_t lo, hi; };   // CTAs per graph, graphs order[lo .. hi)
     std::vector<Tier> tiers;
     std::vector<cudaStream_t> side;            // streams of the launches after the first
@@ -1583,10 +1582,9 @@ int bfail(lv_batch *b, int code, const std::string &msg) {
 template <typename T>
 int balloc(lv_batch *b, T **p, size_t n) {
     void *q = nullptr;
-    if (pool_alloc(b->device, &q, sizeof(T) * (n ? n : 1), b->stream) != cudaSuccess)
-        return bfail(b, LV_ERR_NOMEM, "device allocation failed");
-    b->allocs.push_back(q);
+    const cudaError_t e = b->mem.alloc(&q, sizeof(T) * n, b->stream);
     *p = (T *)q;
+    if (e != cudaSuccess) return bfail(b, LV_ERR_NOMEM, "device allocation failed");
     return LV_OK;
 }
 
@@ -1642,7 +1640,8 @@ int batch_begin(const int32_t *graph_ptr, int32_t G, int32_t V, int64_t E, const
     }
     b->device = b->opts.device;
     cudaSetDevice(b->device);
-    if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    b->mem.dev = b->device;
+    if (stream_take(b->device, &b->stream) != cudaSuccess) {
         cudaGetLastError();
         delete b;
         return LV_ERR_CUDA;
@@ -1785,7 +1784,7 @@ int batch_finish(lv_batch *b) {
     for (size_t i = 1; i < b->tiers.size(); ++i) {
         cudaStream_t s = nullptr;
         cudaEvent_t ev = nullptr;
-        LVB_CUDA(b, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        LVB_CUDA(b, stream_take(b->device, &s));
         b->side.push_back(s);
         LVB_CUDA(b, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         b->side_ev.push_back(ev);
@@ -1801,23 +1800,12 @@ int lv_batch_destroy(lv_batch *b) {
     if (!b) return LV_OK;
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
-    if (b->owns_input) {
-        pool_free(b->device, (void *)b->rowptr, b->stream);
-        pool_free(b->device, (void *)b->col, b->stream);
-        pool_free(b->device, (void *)b->w, b->stream);
-    }
-    for (void *p : b->allocs) pool_free(b->device, p, b->stream);
-    for (cudaStream_t s : b->side) {
-        cudaStreamSynchronize(s);
-        cudaStreamDestroy(s);
-    }
+    for (cudaStream_t s : b->side) stream_give(b->device, s);
+    b->mem.give_all(b->stream);   // the streams have drained
     for (cudaEvent_t e : b->side_ev) cudaEventDestroy(e);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
-    if (b->stream) {
-        cudaStreamSynchronize(b->stream);
-        cudaStreamDestroy(b->stream);
-    }
+    stream_give(b->device, b->stream);
     delete b;
     return LV_OK;
 }
@@ -1828,18 +1816,14 @@ int lv_batch_create(const int32_t *rowptr, const int32_t *col, const float *w, i
     lv_batch *b = nullptr;
     int rc = batch_begin(graph_ptr, num_graphs, V, E, opts, out, &b);
     if (rc) return rc;
-    b->owns_input = true;
-    void *p = nullptr;
-    rc = pool_alloc(b->device, &p, sizeof(int32_t) * ((size_t)V + 1), b->stream) == cudaSuccess ? 0 : LV_ERR_NOMEM;
-    b->rowptr = (const int32_t *)p;
-    if (!rc) {
-        rc = pool_alloc(b->device, &p, sizeof(int32_t) * (size_t)(E ? E : 1), b->stream) == cudaSuccess ? 0 : LV_ERR_NOMEM;
-        b->col = (const int32_t *)p;
-    }
-    if (!rc) {
-        rc = pool_alloc(b->device, &p, sizeof(float) * (size_t)(E ? E : 1), b->stream) == cudaSuccess ? 0 : LV_ERR_NOMEM;
-        b->w = (const float *)p;
-    }
+    int32_t *rp = nullptr, *cl = nullptr;
+    float *wt = nullptr;
+    rc = balloc(b, &rp, (size_t)V + 1);
+    if (!rc) rc = balloc(b, &cl, (size_t)E);
+    if (!rc) rc = balloc(b, &wt, (size_t)E);
+    b->rowptr = rp;
+    b->col = cl;
+    b->w = wt;
     if (!rc && cudaMemcpyAsync((void *)b->rowptr, rowptr, sizeof(int32_t) * ((size_t)V + 1),
                                cudaMemcpyHostToDevice, b->stream) != cudaSuccess)
         rc = LV_ERR_CUDA;
@@ -1865,7 +1849,6 @@ int lv_batch_create_device(const int32_t *d_rowptr, const int32_t *d_col, const 
     lv_batch *b = nullptr;
     int rc = batch_begin(graph_ptr, num_graphs, V, E, opts, out, &b);
     if (rc) return rc;
-    b->owns_input = false;
     b->rowptr = d_rowptr;
     b->col = d_col;
     b->w = d_w;

@@ -169,8 +169,7 @@ struct lv_handle {
     u64 *eown_buf = nullptr;       // per hub, zero between uses (nocc_cap entries)
     int32_t *ovf_buf = nullptr;    // overflow list (nocc_cap entries) then its count
     bool capturing = false;        // a sweep is being captured into a graph (timers off)
-    bool destroying = false;       // lv_destroy: large buffers go to the per-device cache
-    std::vector<std::pair<void *, size_t>> big;   // live allocations of at least BIG_BYTES
+    MemSet mem;                    // every device buffer of the handle
     void *loop_d = nullptr;        // device state of the graph sweep loop
 
     // level_setup not run yet for the current level: the state arrays are
@@ -246,166 +245,19 @@ int fail(lv_handle *h, int code, const std::string &msg) {
         if (rc__) return rc__;  \
     } while (0)
 
-// Device memory of every handle comes from one stream-ordered pool per
-// device whose release threshold keeps freed memory mapped, so creating a
-// handle after another was destroyed reuses the mapping instead of paying
-// cudaMalloc/cudaFree for the ~20 GB working set of an R-MAT-24 run again.
-// lv_trim_device_memory returns the unused part to the system.
-constexpr int LV_MAX_DEVICES = 64;
-std::mutex g_pool_mu;
-cudaMemPool_t g_pool[LV_MAX_DEVICES] = {};
-
-cudaMemPool_t device_pool(int dev) {
-    if (dev < 0 || dev >= LV_MAX_DEVICES) return nullptr;
-    std::lock_guard<std::mutex> lock(g_pool_mu);
-    if (!g_pool[dev]) {
-        // an error left pending by an earlier asynchronous call would be
-        // reported by the calls below; set-up is retried by the next
-        // allocation if it fails
-        cudaGetLastError();
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t pool = nullptr;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        uint64_t keep = UINT64_MAX;
-        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-            cudaGetLastError();
-            cudaMemPoolDestroy(pool);
-            return nullptr;
-        }
-        g_pool[dev] = pool;
-    }
-    return g_pool[dev];
-}
-
-// Large buffers (at least BIG_BYTES) of destroyed handles are kept per device
-// and handed to the next allocation of exactly the same size: handles of the
-// same graph ask for the same sizes, so a handle created again reuses its
-// predecessor's memory as it is, without the pool having to find or map room
-// for it (which, when its free blocks are fragmented, maps new memory and
-// costs hundreds of milliseconds for the ~20 GB of an R-MAT-24 handle).
-// lv_trim_device_memory releases them.
-constexpr size_t BIG_BYTES = size_t(16) << 20;
-std::mutex g_cache_mu;
-std::vector<std::pair<size_t, void *>> g_cache[LV_MAX_DEVICES];
-
-void *cache_take(int dev, size_t bytes) {
-    if (dev < 0 || dev >= LV_MAX_DEVICES) return nullptr;
-    std::lock_guard<std::mutex> lock(g_cache_mu);
-    auto &c = g_cache[dev];
-    for (size_t i = 0; i < c.size(); ++i)
-        if (c[i].first == bytes) {
-            void *p = c[i].second;
-            c[i] = c.back();
-            c.pop_back();
-            return p;
-        }
-    return nullptr;
-}
-
-// hands every cached buffer of the device back (to the pool, or to the driver
-// when the device has no pool); called by lv_trim_device_memory, by each
-// lv_destroy before it caches its own buffers (so the cache holds one
-// handle's worth at most), and by an allocation that failed
-void cache_release(int dev, cudaMemPool_t pool, cudaStream_t stream) {
-    if (dev < 0 || dev >= LV_MAX_DEVICES) return;
-    std::vector<std::pair<size_t, void *>> cached;
-    {
-        std::lock_guard<std::mutex> lock(g_cache_mu);
-        cached.swap(g_cache[dev]);
-    }
-    for (auto &c : cached) {
-        if (pool) cudaFreeAsync(c.second, stream);
-        else cudaFree(c.second);
-    }
-}
-
-bool cache_put(int dev, size_t bytes, void *p) {
-    if (dev < 0 || dev >= LV_MAX_DEVICES) return false;
-    std::lock_guard<std::mutex> lock(g_cache_mu);
-    g_cache[dev].emplace_back(bytes, p);
-    return true;
-}
-
 template <typename T>
 int dalloc(lv_handle *h, T **p, size_t n) {
-    *p = nullptr;
-    if (n == 0) n = 1;
-    const size_t bytes = n * sizeof(T);
-    if (bytes >= BIG_BYTES) {
-        void *c = cache_take(h->device, bytes);
-        if (c) {
-            *p = (T *)c;
-            h->big.emplace_back(c, bytes);
-            return LV_OK;
-        }
-    }
-    cudaMemPool_t pool = device_pool(h->device);
-    cudaError_t e = pool ? cudaMallocFromPoolAsync((void **)p, bytes, pool, h->stream)
-                         : cudaMalloc((void **)p, bytes);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        cache_release(h->device, pool, h->stream);
-        e = pool ? cudaMallocFromPoolAsync((void **)p, bytes, pool, h->stream)
-                 : cudaMalloc((void **)p, bytes);
-    }
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        *p = nullptr;
-        return fail(h, LV_ERR_NOMEM, std::string("device allocation: ") + cudaGetErrorString(e));
-    }
-    if (bytes >= BIG_BYTES) h->big.emplace_back((void *)*p, bytes);
+    void *q = nullptr;
+    const cudaError_t e = h->mem.alloc(&q, n * sizeof(T), h->stream);
+    *p = (T *)q;
+    if (e != cudaSuccess) return fail(h, LV_ERR_NOMEM, std::string("device allocation: ") + cudaGetErrorString(e));
     return LV_OK;
 }
 
-}  // namespace
-
-// The pool for other handle types of the library (lv_batch).
-cudaError_t lv::pool_alloc(int dev, void **p, size_t bytes, cudaStream_t s) {
-    *p = nullptr;
-    cudaMemPool_t pool = device_pool(dev);
-    const cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s)
-                               : cudaMalloc(p, bytes ? bytes : 1);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        *p = nullptr;
-    }
-    return e;
-}
-
-void lv::pool_free(int dev, void *p, cudaStream_t s) {
-    if (!p) return;
-    if (device_pool(dev)) cudaFreeAsync(p, s);
-    else cudaFree(p);
-}
-
-namespace {
-
-// Stream-ordered free (after the handle's queued work); the memory returns
-// to the device pool.
+// Stream-ordered free (after the handle's queued work).
 template <typename T>
 void dfree(lv_handle *h, T *&p) {
-    if (p) {
-        // a large buffer goes to the per-device cache when the handle is
-        // being destroyed (its stream has drained); otherwise to the pool
-        size_t big = 0;
-        for (size_t i = 0; i < h->big.size(); ++i)
-            if (h->big[i].first == (void *)p) {
-                big = h->big[i].second;
-                h->big[i] = h->big.back();
-                h->big.pop_back();
-                break;
-            }
-        if (!(big && h->destroying && cache_put(h->device, big, (void *)p))) {
-            if (device_pool(h->device)) cudaFreeAsync((void *)p, h->stream);
-            else cudaFree((void *)p);
-        }
-    }
+    if (p) h->mem.free((void *)p, h->stream);
     p = nullptr;
 }
 
@@ -1646,7 +1498,7 @@ int finish_create(lv_handle *h) {
     const size_t V = (size_t)h->V0;
     if (h->opts.trace)
         std::fprintf(stderr, "[lv] device %d memory pool: %s\n", h->device,
-                     device_pool(h->device) ? "on" : "off (cudaMalloc per buffer)");
+                     mem_pooled(h->device) ? "on" : "off (cudaMalloc per buffer)");
     LV_TRY(dalloc(h, &h->comm, V + 1));
     LV_TRY(dalloc(h, &h->newc, V + 1));
     LV_TRY(dalloc(h, &h->size, V + 1));
@@ -1725,7 +1577,9 @@ int begin_create(const lv_opts *opts, int32_t V, int64_t E, lv_handle **out, lv_
     h->fb.hint_set = (h->fb.warp_limit * 3) / 4;
     h->device = h->opts.device;
     cudaSetDevice(h->device);
-    if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    h->mem.dev = h->device;
+    if (stream_take(h->device, &h->stream) != cudaSuccess) {
+        cudaGetLastError();
         delete h;
         return LV_ERR_CUDA;
     }
@@ -1775,20 +1629,8 @@ const char *lv_status_string(int s) {
 }
 
 int lv_trim_device_memory(int32_t device) {
-    if (device < 0 || device >= LV_MAX_DEVICES) return LV_ERR_INVALID;
-    cudaMemPool_t pool = nullptr;
-    {
-        std::lock_guard<std::mutex> lock(g_pool_mu);
-        pool = g_pool[device];
-    }
-    int prev = 0;
-    cudaGetDevice(&prev);
-    cudaSetDevice(device);
-    cache_release(device, pool, 0);
-    cudaDeviceSynchronize();
-    cudaSetDevice(prev);
-    if (!pool) return LV_OK;
-    return cudaMemPoolTrimTo(pool, 0) == cudaSuccess ? LV_OK : LV_ERR_CUDA;
+    if (device < 0 || device >= 64) return LV_ERR_INVALID;
+    return mem_trim(device) == cudaSuccess ? LV_OK : LV_ERR_CUDA;
 }
 
 const char *lv_version(void) { return "louvain_b200 0.1 (sm_100a)"; }
@@ -1797,70 +1639,12 @@ int lv_destroy(lv_handle *h) {
     if (!h) return LV_OK;
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    cache_release(h->device, device_pool(h->device), h->stream);
-    h->destroying = true;
-    if (h->owns_input) {
-        dfree(h, h->in_rowptr);
-        dfree(h, h->in_col);
-        dfree(h, h->in_w);
-    }
-    {
-        FallbackSet &fs = h->fb;
-        dfree(h, fs.hint);
-        for (int q = 0; q <= NFBQ; ++q) {
-            Fallback &f = fs.q[q];
-            dfree(h, f.v); dfree(h, f.p); dfree(h, f.P); dfree(h, f.first); dfree(h, f.done); dfree(h, f.src);
-            dfree(h, f.gd); dfree(h, f.e); dfree(h, f.S); dfree(h, f.eo); dfree(h, f.c); dfree(h, f.cnt);
-        }
-    }
-    dfree(h, h->comm); dfree(h, h->newc); dfree(h, h->size); dfree(h, h->orig2comm);
-    dfree(h, h->k); dfree(h, h->S); dfree(h, h->list); dfree(h, h->cls_scratch); dfree(h, h->sort_buf);
-    {
-        unsigned char *t = (unsigned char *)h->sort_temp;
-        dfree(h, t);
-        h->sort_temp = nullptr;
-    }
-    dfree(h, h->tbl_buf); dfree(h, h->occ_buf); dfree(h, h->nocc_buf);
-    dfree(h, h->stage_key); dfree(h, h->stage_val); dfree(h, h->eown_buf); dfree(h, h->ovf_buf);
-    dfree(h, h->stage2_key); dfree(h, h->stage2_val); dfree(h, h->poff_buf);
-    for (HubLayout *L : {&h->hub_move, &h->hub_agg}) {
-        unsigned char *d = (unsigned char *)L->dev;
-        dfree(h, d);
-        L->dev = nullptr;
-    }
-    AggBuffers &a = h->ab;
-    dfree(h, a.flag); dfree(h, a.cdeg); dfree(h, a.mstart); dfree(h, a.cursor); dfree(h, a.members);
-    dfree(h, a.lab); dfree(h, a.clist); dfree(h, a.newdeg); dfree(h, a.epos_new); dfree(h, a.scan_tmp);
-    dfree(h, a.scalars);
-    dfree(h, h->mslot); dfree(h, h->degm); dfree(h, h->P);
-    for (int b = 0; b < 2; ++b) {
-        dfree(h, h->lvl_start[b]); dfree(h, h->lvl_end[b]); dfree(h, h->lvl_col[b]); dfree(h, h->lvl_w[b]);
-        dfree(h, h->lvl_w32[b]);
-    }
-    dfree(h, h->wrow);
-    {
-        unsigned char *t = (unsigned char *)h->team_arena;
-        dfree(h, t);
-        h->team_arena = nullptr;
-    }
-    dfree(h, h->blk_d);
-    dfree(h, h->mv_list); dfree(h, h->mv_off);
-    dfree(h, h->feat); dfree(h, h->moved); dfree(h, h->nmoved); dfree(h, h->pred); dfree(h, h->fresh);
-    dfree(h, h->comm_prev); dfree(h, h->alist);
-    dfree(h, h->acnt); dfree(h, h->actr); dfree(h, h->model); dfree(h, h->tr_x); dfree(h, h->tr_v);
-    dfree(h, h->tr_y);
-    {
-        LoopState *ld = (LoopState *)h->loop_d;
-        dfree(h, ld);
-        h->loop_d = nullptr;
-    }
+    // every buffer goes back: the stream has drained
+    h->mem.give_all(h->stream);
     pinned_give(h);
     for (const Pending &p : h->pend) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     for (cudaEvent_t e : h->ev_free) cudaEventDestroy(e);
-    if (h->stream) {
-        cudaStreamSynchronize(h->stream);   // the stream-ordered frees above
-        cudaStreamDestroy(h->stream);
-    }
+    stream_give(h->device, h->stream);
     delete h;
     return LV_OK;
 }
@@ -2053,13 +1837,15 @@ int lv_get_csr(lv_handle *h, int32_t *rowptr, int32_t *col, int64_t *wfix) {
             LV_CUDA(h, cudaMemcpyAsync(col, h->cur_col, sizeof(int32_t) * (size_t)h->E,
                                        cudaMemcpyDeviceToHost, h->stream));
         if (wfix && h->E > 0) {
-            int64_t *tmp = nullptr;
-            LV_TRY(dalloc(h, &tmp, (size_t)h->E));
+            MemBlock tb;
+            if (mem_take(h->device, sizeof(int64_t) * (size_t)h->E, h->stream, &tb) != cudaSuccess)
+                return fail(h, LV_ERR_NOMEM, "device allocation");
+            int64_t *tmp = (int64_t *)tb.p;
             launch_weights_to_fixed<float>(h->in_w, h->E, h->scale_d, tmp, h->stream);
             cudaError_t e = cudaMemcpyAsync(wfix, tmp, sizeof(int64_t) * (size_t)h->E,
                                             cudaMemcpyDeviceToHost, h->stream);
             cudaStreamSynchronize(h->stream);
-            dfree(h, tmp);
+            mem_give(h->device, tb, h->stream);
             if (e != cudaSuccess) return fail(h, LV_ERR_CUDA, cudaGetErrorString(e));
         }
         return sync(h);

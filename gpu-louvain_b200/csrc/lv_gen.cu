@@ -5,6 +5,7 @@
 #include <cub/cub.cuh>
 
 #include "../../include/louvain_b200.h"
+#include "lv_internal.h"
 #include "lv_rng.h"
 
 namespace {
@@ -78,7 +79,7 @@ __global__ void swap_kernel(const u64 *in, int64_t nk, int scale, u64 *out) {
 extern "C" {
 
 void lv_free_device(void *p) {
-    if (p) cudaFree(p);
+    if (p && !lv::mem_take_back(p)) cudaFree(p);
 }
 
 int lv_gen_rmat_device(int32_t scale, int32_t edge_factor, uint64_t seed, double a, double b,
@@ -92,6 +93,8 @@ int lv_gen_rmat_device(int32_t scale, int32_t edge_factor, uint64_t seed, double
     const int32_t V = (int32_t)(1u << scale);
     const int bits = 2 * scale;
     const lvrng::RmatParams p = lvrng::rmat_params(scale, a, b, c, seed);
+    lv::MemSet mem;
+    mem.dev = device;
     u64 *k1 = nullptr, *k2 = nullptr;
     void *tmp = nullptr;
     int32_t *dlo = nullptr, *dhi = nullptr, *rp = nullptr, *cl = nullptr;
@@ -107,16 +110,16 @@ int lv_gen_rmat_device(int32_t scale, int32_t edge_factor, uint64_t seed, double
     do {                                              \
         if ((x) != cudaSuccess) { rc = LV_ERR_CUDA; goto done; } \
     } while (0)
-    GEN_CHECK(cudaMalloc(&k1, sizeof(u64) * (size_t)n));
-    GEN_CHECK(cudaMalloc(&k2, sizeof(u64) * (size_t)n));
-    GEN_CHECK(cudaMalloc(&nsel, sizeof(int64_t) * 2));
+    GEN_CHECK(mem.alloc((void **)&k1, sizeof(u64) * (size_t)n, 0));
+    GEN_CHECK(mem.alloc((void **)&k2, sizeof(u64) * (size_t)n, 0));
+    GEN_CHECK(mem.alloc((void **)&nsel, sizeof(int64_t) * 2, 0));
     rmat_draw_kernel<<<grid, 256>>>(p, n, k1);
     cub::DeviceRadixSort::SortKeys(nullptr, t1, k1, k2, (int64_t)n, 0, bits);
     cub::DeviceSelect::Unique(nullptr, t2, k2, k1, nsel, (int64_t)n);
     cub::DeviceScan::ExclusiveSum(nullptr, t3, dlo, rp, V + 1);
     tmp_bytes = t1 > t2 ? t1 : t2;
     tmp_bytes = tmp_bytes > t3 ? tmp_bytes : t3;
-    GEN_CHECK(cudaMalloc(&tmp, tmp_bytes));
+    GEN_CHECK(mem.alloc((void **)&tmp, tmp_bytes, 0));
     GEN_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, k1, k2, (int64_t)n, 0, bits));
     GEN_CHECK(cub::DeviceSelect::Unique(tmp, tmp_bytes, k2, k1, nsel, (int64_t)n));
     GEN_CHECK(cudaMemcpy(&h_nsel, nsel, sizeof(int64_t), cudaMemcpyDeviceToHost));
@@ -130,11 +133,11 @@ int lv_gen_rmat_device(int32_t scale, int32_t edge_factor, uint64_t seed, double
         }
     }
     if (2 * nk > 0x7fffffffLL) { rc = LV_ERR_TOO_LARGE; goto done; }
-    GEN_CHECK(cudaMalloc(&dlo, sizeof(int32_t) * ((size_t)V + 1)));
-    GEN_CHECK(cudaMalloc(&dhi, sizeof(int32_t) * ((size_t)V + 1)));
-    GEN_CHECK(cudaMalloc(&rp, sizeof(int32_t) * ((size_t)V + 1)));
-    GEN_CHECK(cudaMalloc(&cl, sizeof(int32_t) * (size_t)(2 * nk + 1)));
-    GEN_CHECK(cudaMalloc(&wt, sizeof(float) * (size_t)(2 * nk + 1)));
+    GEN_CHECK(mem.alloc((void **)&dlo, sizeof(int32_t) * ((size_t)V + 1), 0));
+    GEN_CHECK(mem.alloc((void **)&dhi, sizeof(int32_t) * ((size_t)V + 1), 0));
+    GEN_CHECK(mem.alloc_own((void **)&rp, sizeof(int32_t) * ((size_t)V + 1), 0));
+    GEN_CHECK(mem.alloc_own((void **)&cl, sizeof(int32_t) * (size_t)(2 * nk + 1), 0));
+    GEN_CHECK(mem.alloc_own((void **)&wt, sizeof(float) * (size_t)(2 * nk + 1), 0));
     GEN_CHECK(cudaMemset(dlo, 0, sizeof(int32_t) * ((size_t)V + 1)));
     GEN_CHECK(cudaMemset(dhi, 0, sizeof(int32_t) * ((size_t)V + 1)));
     degree_kernel<<<grid, 256>>>(k1, nk, scale, dlo, dhi);
@@ -151,18 +154,13 @@ int lv_gen_rmat_device(int32_t scale, int32_t edge_factor, uint64_t seed, double
     GEN_CHECK(cudaGetLastError());
 done:
 #undef GEN_CHECK
-    if (k1) cudaFree(k1);
-    if (k2) cudaFree(k2);
-    if (tmp) cudaFree(tmp);
-    if (dlo) cudaFree(dlo);
-    if (dhi) cudaFree(dhi);
-    if (nsel) cudaFree(nsel);
     if (rc != LV_OK) {
-        if (rp) cudaFree(rp);
-        if (cl) cudaFree(cl);
-        if (wt) cudaFree(wt);
+        cudaDeviceSynchronize();
+        mem.give_all(0);
         return rc;
     }
+    for (void *q : {(void *)rp, (void *)cl, (void *)wt}) mem.hand_over(q);
+    mem.give_all(0);
     *Vout = V;
     *Eout = 2 * nk;
     *d_rowptr = rp;

@@ -10,6 +10,7 @@
 #include <cub/cub.cuh>
 
 #include "../../include/louvain_b200.h"
+#include "lv_internal.h"
 
 namespace {
 
@@ -80,7 +81,9 @@ extern "C" int lv_csr_from_entries_device(int32_t device, int32_t V, int64_t nnz
         return LV_ERR_NO_DEVICE;
     }
     cudaStream_t s = nullptr;
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+    lv::MemSet mem;
+    mem.dev = device;
+    if (lv::stream_take(device, &s) != cudaSuccess) {
         cudaGetLastError();
         return LV_ERR_CUDA;
     }
@@ -104,18 +107,18 @@ extern "C" int lv_csr_from_entries_device(int32_t device, int32_t V, int64_t nnz
             goto done;                                                                       \
         }                                                                                    \
     } while (0)
-    ING_CHECK(cudaMalloc(&rp, sizeof(int32_t) * ((size_t)V + 1)));
-    ING_CHECK(cudaMalloc(&deg, sizeof(int32_t) * ((size_t)V + 1)));
+    ING_CHECK(mem.alloc_own((void **)&rp, sizeof(int32_t) * ((size_t)V + 1), s));
+    ING_CHECK(mem.alloc((void **)&deg, sizeof(int32_t) * ((size_t)V + 1), s));
     ING_CHECK(cudaMemsetAsync(deg, 0, sizeof(int32_t) * ((size_t)V + 1), s));
-    ING_CHECK(cudaMalloc(&err, sizeof(int)));
+    ING_CHECK(mem.alloc((void **)&err, sizeof(int), s));
     ING_CHECK(cudaMemsetAsync(err, 0, sizeof(int), s));
-    ING_CHECK(cudaMalloc(&tot, sizeof(int64_t)));
+    ING_CHECK(mem.alloc((void **)&tot, sizeof(int64_t), s));
     if (nnz > 0) {
-        ING_CHECK(cudaMalloc(&a, sizeof(int32_t) * n));
-        ING_CHECK(cudaMalloc(&b, sizeof(int32_t) * n));
-        ING_CHECK(cudaMalloc(&ww, sizeof(float) * n));
-        ING_CHECK(cudaMalloc(&cnt, sizeof(int32_t) * (n + 1)));   // cnt[n] = 0: pos[n] is the total
-        ING_CHECK(cudaMalloc(&pos, sizeof(int64_t) * (n + 1)));
+        ING_CHECK(mem.alloc((void **)&a, sizeof(int32_t) * n, s));
+        ING_CHECK(mem.alloc((void **)&b, sizeof(int32_t) * n, s));
+        ING_CHECK(mem.alloc((void **)&ww, sizeof(float) * n, s));
+        ING_CHECK(mem.alloc((void **)&cnt, sizeof(int32_t) * (n + 1), s));   // cnt[n] = 0: pos[n] is the total
+        ING_CHECK(mem.alloc((void **)&pos, sizeof(int64_t) * (n + 1), s));
         ING_CHECK(cudaMemcpyAsync(a, v1, sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
         ING_CHECK(cudaMemcpyAsync(b, v2, sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
         ING_CHECK(cudaMemcpyAsync(ww, w, sizeof(float) * n, cudaMemcpyHostToDevice, s));
@@ -126,7 +129,7 @@ extern "C" int lv_csr_from_entries_device(int32_t device, int32_t V, int64_t nnz
         // int32 input type and wrap before the E check below)
         ING_CHECK(cub::DeviceScan::ExclusiveScan(nullptr, tmp_bytes, cnt, pos, ::cuda::std::plus<>{}, (int64_t)0,
                                                  (int64_t)nnz + 1, s));
-        ING_CHECK(cudaMalloc(&tmp, tmp_bytes));
+        ING_CHECK(mem.alloc((void **)&tmp, tmp_bytes, s));
         ING_CHECK(cub::DeviceScan::ExclusiveScan(tmp, tmp_bytes, cnt, pos, ::cuda::std::plus<>{}, (int64_t)0,
                                                  (int64_t)nnz + 1, s));
         ING_CHECK(cudaMemcpyAsync(&E, pos + nnz, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
@@ -137,24 +140,23 @@ extern "C" int lv_csr_from_entries_device(int32_t device, int32_t V, int64_t nnz
     }
     {
         const size_t ne = (size_t)(E > 0 ? E : 1);
-        ING_CHECK(cudaMalloc(&cl, sizeof(int32_t) * ne));
-        ING_CHECK(cudaMalloc(&wt, sizeof(float) * ne));
+        ING_CHECK(mem.alloc_own((void **)&cl, sizeof(int32_t) * ne, s));
+        ING_CHECK(mem.alloc_own((void **)&wt, sizeof(float) * ne, s));
         if (E > 0) {
-            ING_CHECK(cudaMalloc(&row, sizeof(int32_t) * ne));
-            ING_CHECK(cudaMalloc(&idx, sizeof(int32_t) * ne));
-            ING_CHECK(cudaMalloc(&row2, sizeof(int32_t) * ne));
-            ING_CHECK(cudaMalloc(&idx2, sizeof(int32_t) * ne));
-            ING_CHECK(cudaMalloc(&dcol, sizeof(int32_t) * ne));
-            ING_CHECK(cudaMalloc(&dw, sizeof(float) * ne));
+            ING_CHECK(mem.alloc((void **)&row, sizeof(int32_t) * ne, s));
+            ING_CHECK(mem.alloc((void **)&idx, sizeof(int32_t) * ne, s));
+            ING_CHECK(mem.alloc((void **)&row2, sizeof(int32_t) * ne, s));
+            ING_CHECK(mem.alloc((void **)&idx2, sizeof(int32_t) * ne, s));
+            ING_CHECK(mem.alloc((void **)&dcol, sizeof(int32_t) * ne, s));
+            ING_CHECK(mem.alloc((void **)&dw, sizeof(float) * ne, s));
             entry_expand_kernel<<<grid, 256, 0, s>>>(a, b, ww, pos, nnz, V, row, idx, dcol, dw, deg);
             size_t t2 = 0;
             const int bits = bits_for(V);
             ING_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, t2, row, row2, idx, idx2, (int64_t)E, 0, bits, s));
             if (t2 > tmp_bytes) {
-                cudaFree(tmp);
                 tmp = nullptr;
                 tmp_bytes = t2;
-                ING_CHECK(cudaMalloc(&tmp, tmp_bytes));
+                ING_CHECK(mem.alloc((void **)&tmp, tmp_bytes, s));
             }
             // stable: equal rows keep the directed (file) order
             ING_CHECK(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, row, row2, idx, idx2, (int64_t)E, 0, bits, s));
@@ -163,10 +165,9 @@ extern "C" int lv_csr_from_entries_device(int32_t device, int32_t V, int64_t nnz
         size_t t3 = 0;
         ING_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, t3, deg, rp, (int64_t)V + 1, s));
         if (t3 > tmp_bytes) {
-            if (tmp) cudaFree(tmp);
             tmp = nullptr;
             tmp_bytes = t3;
-            ING_CHECK(cudaMalloc(&tmp, tmp_bytes));
+            ING_CHECK(mem.alloc((void **)&tmp, tmp_bytes, s));
         }
         ING_CHECK(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, deg, rp, (int64_t)V + 1, s));
         ING_CHECK(cudaStreamSynchronize(s));
@@ -174,15 +175,13 @@ extern "C" int lv_csr_from_entries_device(int32_t device, int32_t V, int64_t nnz
     }
 done:
 #undef ING_CHECK
-    for (void *p : {(void *)a, (void *)b, (void *)ww, (void *)cnt, (void *)pos, (void *)tot, (void *)err, tmp,
-                    (void *)row, (void *)idx, (void *)row2, (void *)idx2, (void *)dcol, (void *)dw, (void *)deg})
-        if (p) cudaFree(p);
-    cudaStreamDestroy(s);
+    cudaStreamSynchronize(s);
+    if (rc == LV_OK)
+        for (void *p : {(void *)rp, (void *)cl, (void *)wt}) mem.hand_over(p);
+    mem.give_all(s);
+    lv::stream_give(device, s);
     if (rc != LV_OK) {
         cudaGetLastError();
-        if (rp) cudaFree(rp);
-        if (cl) cudaFree(cl);
-        if (wt) cudaFree(wt);
         return rc;
     }
     *Eout = E;

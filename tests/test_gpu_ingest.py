@@ -92,3 +92,29 @@ def test_engine_on_device_built_csr(lvb):
     with lvb.Louvain(lvb.Graph(rp, cl, ww)) as e:
         assert e.run(1e-6) == q_dev
         assert np.array_equal(e.original_to_community()[0], m_dev)
+
+
+@pytest.mark.parametrize("nnz", [0, 1, 1000, 200000])
+def test_kept_memory_is_reused_and_given_back(lvb, nnz):
+    """Graphs built, run and freed in turn with sizes that differ a little (the
+    library keeps blocks between calls): every result equals the first one's,
+    and a trim leaves no more memory in use than before."""
+    import torch
+    V = max(2, nnz // 8)
+    lvb.lib().lv_trim_device_memory(0)
+    free0 = torch.cuda.mem_get_info()[0]
+    first = None
+    for n in (nnz, nnz - nnz // 50, nnz + nnz // 50, nnz):
+        r = np.random.default_rng(7)
+        u, v = r.integers(0, V, n).astype(np.int32), r.integers(0, V, n).astype(np.int32)
+        dg = lvb.csr_from_entries_device(V, u, v, np.ones(n, np.float32))
+        with lvb.Louvain(device_csr=(dg.rowptr, dg.col, dg.w, dg.V, dg.E)) as e:
+            q = e.run(1e-6)
+            m, _ = e.original_to_community()
+        dg.free()
+        if n == nnz:
+            if first is None:
+                first = (q, m)
+            assert np.array_equal(first[1], m) and (q == first[0] or (np.isnan(q) and np.isnan(first[0])))
+    lvb.lib().lv_trim_device_memory(0)
+    assert torch.cuda.mem_get_info()[0] >= free0 - (64 << 20)
