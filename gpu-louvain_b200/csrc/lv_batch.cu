@@ -1686,8 +1686,7 @@ int batch_finish(lv_batch *b) {
     int32_t *chk = nullptr;
     LVB_TRY(balloc(b, &chk, 8 + (size_t)G + 1));
     LVB_CUDA(b, cudaMemsetAsync(chk, 0, sizeof(int32_t) * 8, b->stream));
-    launch_validate_csr(b->rowptr, b->col, V, E, chk, b->stream);
-    launch_weight_scan(b->w, E, chk + 4, b->stream);
+    launch_csr_scan(b->rowptr, b->col, b->w, V, E, chk, chk + 4, nullptr, 0, b->stream);
     int32_t *gptr_d = nullptr;
     LVB_TRY(balloc(b, &gptr_d, (size_t)G + 1));
     if (G > 0) {

@@ -1510,31 +1510,26 @@ int finish_create(lv_handle *h) {
     h->tot_d = &h->blk_d->tot;
     LV_CUDA(h, cudaMemsetAsync(h->blk_d, 0, sizeof(SweepBlock), h->stream));
     LV_TRY(pinned_take(h));
-    // CSR validation
-    launch_validate_csr(h->in_rowptr, h->in_col, h->V0, h->E0, &h->tot_d->err, h->stream);
-    LV_CUDA(h, cudaMemcpyAsync(h->tot_h, h->tot_d, sizeof(Totals), cudaMemcpyDeviceToHost, h->stream));
-    LV_TRY(sync(h));
-    if (h->tot_h->err) return fail(h, LV_ERR_INVALID, "malformed CSR (offsets or column ids)");
-    // fixed-point scale (same rule as the oracle's orc_choose_scale)
+    // CSR checks, fixed-point scale (same rule as the oracle's orc_choose_scale)
+    // and total weight; one read back
     int32_t *ws = h->cls_scratch;
-    launch_weight_scan(h->in_w, h->E0, ws, h->stream);
+    u64 *tw = (u64 *)(h->tot_d);   // reuse e_own slot
+    launch_csr_scan(h->in_rowptr, h->in_col, h->in_w, h->V0, h->E0, &h->tot_d->err, ws, nullptr, 0, h->stream);
+    launch_total_weight(h->in_w, h->E0, &h->tot_d->err, ws, tw, h->stream);
+    LV_CUDA(h, cudaMemcpyAsync(h->tot_h, h->tot_d, sizeof(Totals), cudaMemcpyDeviceToHost, h->stream));
     LV_CUDA(h, cudaMemcpyAsync(h->small_h, ws, sizeof(int32_t) * 3, cudaMemcpyDeviceToHost, h->stream));
     LV_TRY(sync(h));
+    if (h->tot_h->err) return fail(h, LV_ERR_INVALID, "malformed CSR (offsets or column ids)");
     if (h->small_h[2]) return fail(h, LV_ERR_WEIGHT, "negative, NaN or infinite edge weight");
     const int need = h->small_h[0];
     const int top = h->small_h[1] ? h->small_h[1] - 1024 : 0;
-    const int cap = 61 - top - ceil_log2_i(h->E0 > 0 ? h->E0 : 1);
-    const int s = need < cap ? need : cap;
+    const int s = scale_of_scan(h->small_h, h->E0);
     if (s < 0) return fail(h, LV_ERR_TOO_LARGE, "total edge weight exceeds the fixed-point range");
     h->scale = s;
     h->exact = (s == need);
     // every fixed-point weight is at most 2^(top + 1 + scale) (rounding included)
     h->w0_narrow = !h->small_h[1] || top + 1 + s <= 31;
     h->scale_d = std::ldexp(1.0, s);
-    u64 *tw = (u64 *)(h->tot_d);   // reuse e_own slot
-    launch_total_weight(h->in_w, h->E0, h->scale_d, tw, h->stream);
-    LV_CUDA(h, cudaMemcpyAsync(h->tot_h, h->tot_d, sizeof(Totals), cudaMemcpyDeviceToHost, h->stream));
-    LV_TRY(sync(h));
     h->T = h->tot_h->e_own;
     LV_CUDA(h, cudaMemsetAsync(h->tot_d, 0, sizeof(Totals), h->stream));
     return to_level0(h);

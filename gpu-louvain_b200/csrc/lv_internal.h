@@ -336,13 +336,22 @@ void launch_compose_map(int32_t *orig2comm, const int32_t *map, int32_t V0, cuda
 template <typename WT>
 void launch_weights_to_fixed(const WT *w, int64_t E, double scale, int64_t *out, cudaStream_t s);
 
-// Fixed-point scale analysis of float weights: out[0] = max fractional bits,
-// out[1] = max floor(log2 w) + 1024 (0 if no positive weight), out[2] = error flags.
-void launch_weight_scan(const float *w, int64_t E, int32_t *out, cudaStream_t s);
-void launch_total_weight(const float *w, int64_t E, double scale, u64 *total, cudaStream_t s);
-// CSR validation: error bit 1 bad offsets, 2 bad column.
-void launch_validate_csr(const int32_t *rowptr, const int32_t *col, int32_t V, int64_t E,
-                         int *err, cudaStream_t s);
+// One pass over a CSR.  *err (cleared by the caller) gets bit 1 for bad
+// offsets, 2 for a bad column; scan[0] = max fractional bits, scan[1] = max
+// floor(log2 w) + 1024 (0 if no positive weight), scan[2] = 1 for a negative,
+// NaN or infinite weight (scan holds 4 words, cleared here).  clear[0 ..
+// n_clear) is zeroed on the way.
+void launch_csr_scan(const int32_t *rowptr, const int32_t *col, const float *w, int32_t V, int64_t E, int *err,
+                     int32_t *scan, u64 *clear, int64_t n_clear, cudaStream_t s);
+// The fixed-point scale the scan words give for E entries (orc_choose_scale);
+// negative: the total would leave the fixed-point range.
+__host__ __device__ inline int scale_of_scan(const int32_t *scan, int64_t E) {
+    const int top = scan[1] ? scan[1] - 1024 : 0;
+    const int cap = 61 - top - ceil_log2_i(E > 0 ? E : 1);
+    return scan[0] < cap ? scan[0] : cap;
+}
+// *total = the fixed-point total weight (unset when the scan rejects the CSR).
+void launch_total_weight(const float *w, int64_t E, const int *err, const int32_t *scan, u64 *total, cudaStream_t s);
 
 // ---- aggregation (lv_agg.cu) ----
 struct AggBuffers {

@@ -42,53 +42,110 @@ constexpr size_t NOALLOC_BYTES = NOALLOC_HEADER_BYTES + sizeof(u64) * (size_t)LV
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
-__global__ void noalloc_clear_kernel(u64 *words, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
-        words[i] = 0;
-}
-
-// Warp per vertex: k_v (row weight) and the weight to the own community;
-// Sigma_tot[C(v)] += k_v.  Community ids outside [0, V) set error bit 4.
+// Eight lanes per vertex: k_v (row weight) and the weight to the own community;
+// Sigma_tot[C(v)] += k_v, T = sum of k.  Community ids outside [0, V) set error
+// bit 4.  The grid comes from the scan words, and nothing is read beyond the
+// offsets when the scan rejected the CSR.  Each CTA takes a contiguous range of
+// vertices and sums Sigma_tot in a shared table first: an atomic per vertex on
+// the few cache lines of 256 communities took 46 us on 200,003 vertices of
+// about 18 entries, whatever the lanes per vertex; the table takes 18 us (29
+// MB read), now bound by the column -> community gathers.
+constexpr int NA_LG = 10, NA_SLOTS = 1 << NA_LG, NA_PROBES = 8;
 __global__ void __launch_bounds__(256) noalloc_modularity_kernel(const int32_t *__restrict__ rowptr,
                                                                const int32_t *__restrict__ col,
                                                                const float *__restrict__ w,
                                                                const int32_t *__restrict__ comm,
-                                                               int32_t V, double scale, u64 *S,
+                                                               int32_t V, int64_t E, u64 *S,
                                                                NoallocHeader *hdr) {
-    __shared__ u64 part[8];
-    const int lane = threadIdx.x & 31;
-    const int32_t warps = gridDim.x * 8;
-    u64 own_sum = 0;
-    for (int32_t v = blockIdx.x * 8 + (threadIdx.x >> 5); v < V; v += warps) {
-        const int32_t cv = comm[v];
-        if (cv < 0 || cv >= V) {
-            if (lane == 0) atomicOr(&hdr->err, 4);
-            continue;
+    __shared__ u64 part[8], tpart[8], vals[NA_SLOTS];
+    __shared__ int32_t keys[NA_SLOTS];
+    constexpr int U = 4;
+    for (int i = threadIdx.x; i < NA_SLOTS; i += 256) {
+        keys[i] = -1;
+        vals[i] = 0;
+    }
+    __syncthreads();
+    const int sc = scale_of_scan(hdr->scan, E);
+    if ((hdr->err & 3) || hdr->scan[2] || sc < 0) return;
+    const double scale = ldexp(1.0, sc);
+    const int lane = threadIdx.x & 31, gl = lane & 7;
+    u64 own_sum = 0, t_sum = 0;
+    const int32_t chunk = (V + (int32_t)gridDim.x - 1) / (int32_t)gridDim.x;
+    const int32_t lo = min((int64_t)V, (int64_t)blockIdx.x * chunk), hi = min((int64_t)V, (int64_t)lo + chunk);
+    for (int32_t v0 = lo + (int32_t)(threadIdx.x >> 5) * 4; v0 < hi; v0 += 32) {
+        const int32_t v = v0 + (lane >> 3);
+        int32_t cv = -1, r0 = 0, r1 = 0;
+        if (v < hi) {
+            cv = comm[v];
+            r0 = rowptr[v];
+            r1 = rowptr[v + 1];
+            if (cv < 0 || cv >= V) {
+                if (gl == 0) atomicOr(&hdr->err, 4);
+                r1 = r0;
+                cv = -1;
+            }
         }
-        const int32_t r0 = rowptr[v], r1 = rowptr[v + 1];
         u64 k = 0, eo = 0;
-        for (int32_t e = r0 + lane; e < r1; e += 32) {
-            const u64 x = wfix(w, e, scale);
-            k += x;
-            if (comm[__ldg(col + e)] == cv) eo += x;
+        for (int32_t e0 = r0 + gl; e0 < r1; e0 += 8 * U) {
+            int32_t jj[U];
+            u64 xx[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int32_t e = e0 + 8 * u;
+                jj[u] = -1;
+                xx[u] = 0;
+                if (e < r1) {
+                    jj[u] = __ldg(col + e);
+                    xx[u] = wfix(w, e, scale);
+                }
+            }
+            int32_t cc[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) cc[u] = jj[u] >= 0 ? __ldg(comm + jj[u]) : -2;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                k += xx[u];
+                if (cc[u] == cv) eo += xx[u];
+            }
         }
-        k = warp_sum_u64(k);
-        if (lane == 0 && k) atomicAdd(S + cv, k);
+        t_sum += k;
         own_sum += eo;
+        for (int off = 4; off > 0; off >>= 1) k += __shfl_xor_sync(FULL, k, off);
+        if (gl == 0 && k) {
+            uint32_t sl = hash_slot(cv, NA_LG);
+            bool in = false;
+            for (int p = 0; p < NA_PROBES && !in; ++p) {
+                const int32_t prev = atomicCAS(keys + sl, -1, cv);
+                in = prev < 0 || prev == cv;
+                if (!in) sl = (sl + 1) & (NA_SLOTS - 1);
+            }
+            if (in) table_add(vals + sl, k);
+            else atomicAdd(S + cv, k);
+        }
     }
     own_sum = warp_sum_u64(own_sum);
-    if (lane == 0) part[threadIdx.x >> 5] = own_sum;
+    t_sum = warp_sum_u64(t_sum);
+    if (lane == 0) {
+        part[threadIdx.x >> 5] = own_sum;
+        tpart[threadIdx.x >> 5] = t_sum;
+    }
     __syncthreads();
+    for (int i = threadIdx.x; i < NA_SLOTS; i += 256)
+        if (keys[i] >= 0) atomicAdd(S + keys[i], vals[i]);
     if (threadIdx.x == 0) {
-        u64 y = 0;
-        for (int i = 0; i < 8; ++i) y += part[i];
+        u64 y = 0, z = 0;
+        for (int i = 0; i < 8; ++i) {
+            y += part[i];
+            z += tpart[i];
+        }
         if (y) atomicAdd(&hdr->e_own, y);
+        if (z) atomicAdd(&hdr->T, z);
     }
 }
 
 inline unsigned noalloc_grid(int64_t items, int per_block) {
     const int64_t b = (items + per_block - 1) / per_block;
-    return (unsigned)(b < 1 ? 1 : (b > 148 * 16 ? 148 * 16 : b));
+    return (unsigned)(b < 1 ? 1 : (b > 148 * 4 ? 148 * 4 : b));
 }
 
 int noalloc_fail(char *err, int32_t err_len, int code, const char *msg) {
@@ -155,34 +212,28 @@ extern "C" int lv_modularity_noalloc(const int32_t *d_rowptr, const int32_t *d_c
     cudaStream_t s = (cudaStream_t)stream;
     NoallocHeader *dh = (NoallocHeader *)base;
     u64 *S = (u64 *)((unsigned char *)base + NOALLOC_HEADER_BYTES);
-    // the array keeps the previous call's contents: clear the header and
-    // Sigma_tot[0, V)
-    const int64_t words = NOALLOC_HEADER_BYTES / 8 + (int64_t)V;
-    noalloc_clear_kernel<<<noalloc_grid(words, 256), 256, 0, s>>>((u64 *)base, words);
-    note_launches(1);
-    if (V > 0) launch_validate_csr(d_rowptr, d_col, V, E, &dh->err, s);
-    launch_weight_scan(d_w, E, dh->scan, s);
-    NoallocHeader h;
-    rc = noalloc_read(s, dh, &h, err, err_len);
-    if (rc != LV_OK) return rc;
-    if (h.err) return noalloc_fail(err, err_len, LV_ERR_INVALID, "malformed CSR (offsets or column ids)");
-    if (h.scan[2]) return noalloc_fail(err, err_len, LV_ERR_WEIGHT, "negative, NaN or infinite edge weight");
-    // fixed-point scale: the rule of lv_create / lv_create_device
-    const int need = h.scan[0];
-    const int top = h.scan[1] ? h.scan[1] - 1024 : 0;
-    const int cap = 61 - top - ceil_log2_i(E > 0 ? E : 1);
-    const int sc = need < cap ? need : cap;
-    if (sc < 0) return noalloc_fail(err, err_len, LV_ERR_TOO_LARGE, "total edge weight exceeds the fixed-point range");
-    const double scale_d = std::ldexp(1.0, sc);
-    launch_total_weight(d_w, E, scale_d, &dh->T, s);
+    // the array keeps the previous call's contents: the header is cleared here,
+    // Sigma_tot[0, V) by the scan
+    cudaError_t ce = cudaMemsetAsync(dh, 0, NOALLOC_HEADER_BYTES, s);
+    if (ce != cudaSuccess) {
+        if (err && err_len > 0) std::snprintf(err, (size_t)err_len, "CUDA error: %s", cudaGetErrorString(ce));
+        cudaGetLastError();
+        return LV_ERR_CUDA;
+    }
     if (V > 0) {
-        noalloc_modularity_kernel<<<noalloc_grid(V, 8), 256, 0, s>>>(d_rowptr, d_col, d_w, d_comm, V, scale_d,
-                                                                    S, dh);
+        launch_csr_scan(d_rowptr, d_col, d_w, V, E, &dh->err, dh->scan, S, V, s);
+        noalloc_modularity_kernel<<<noalloc_grid(V, 128), 256, 0, s>>>(d_rowptr, d_col, d_w, d_comm, V, E, S, dh);
         note_launches(1);
         launch_s2(S, V, dh->s2, s);
     }
+    NoallocHeader h;
     rc = noalloc_read(s, dh, &h, err, err_len);
     if (rc != LV_OK) return rc;
+    if (h.err & 3) return noalloc_fail(err, err_len, LV_ERR_INVALID, "malformed CSR (offsets or column ids)");
+    if (h.scan[2]) return noalloc_fail(err, err_len, LV_ERR_WEIGHT, "negative, NaN or infinite edge weight");
+    // fixed-point scale: the rule of lv_create / lv_create_device
+    if (scale_of_scan(h.scan, E) < 0)
+        return noalloc_fail(err, err_len, LV_ERR_TOO_LARGE, "total edge weight exceeds the fixed-point range");
     if (h.err) return noalloc_fail(err, err_len, LV_ERR_INVALID, "community id outside [0, V)");
     // the FP64 formula of lv_modularity: e_own / T - sum(S^2) / T^2
     const u128 s2 = ((u128)h.s2[0] << 64) | (u128)h.s2[1];

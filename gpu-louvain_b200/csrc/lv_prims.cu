@@ -208,30 +208,74 @@ __global__ void to_fixed_kernel(const WT *w, int64_t E, double scale, int64_t *o
 
 // Fractional bits / magnitude / validity of float weights; the same rule as
 // the oracle's weight_bits().
-__global__ void weight_scan_kernel(const float *__restrict__ w, int64_t E, int32_t *out) {
-    int need = 0, top = 0, bad = 0;
-    for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < E; e += (int64_t)gridDim.x * 256) {
-        int n, t, b;
-        weight_bits_dev(w[e], n, t, b);
-        need = max(need, n);
-        top = max(top, t);
-        bad |= b;
+// CSR checks and fixed-point scale analysis in one pass over the entries.
+// Bound by reading 8 bytes per entry; one atomic of each kind per CTA, and
+// only when it would change the word (an atomic per warp on the three shared
+// words took 29 us of a 3.6-million-entry scan, 29 MB).
+__global__ void __launch_bounds__(256) csr_scan_kernel(const int32_t *__restrict__ rowptr,
+                                                       const int32_t *__restrict__ col, const float *__restrict__ w,
+                                                       int32_t V, int64_t E, int *err, int32_t *scan, u64 *clear,
+                                                       int64_t n_clear) {
+    __shared__ int sn[8], st[8], sb[8];
+    const int64_t tid = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int64_t stride = (int64_t)gridDim.x * 256;
+    int need = 0, top = 0, bad = 0;   // bad: 1 offsets, 2 column, 4 weight
+    for (int64_t i = tid; i < n_clear; i += stride) clear[i] = 0;
+    if (tid == 0 && (rowptr[0] != 0 || (int64_t)rowptr[V] != E)) bad |= 1;
+    for (int64_t v = tid; v < V; v += stride)
+        if (rowptr[v + 1] < rowptr[v]) bad |= 1;
+    constexpr int U = 4;
+    for (int64_t e0 = tid; e0 < E; e0 += U * stride) {
+        int32_t c[U];
+        float x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t e = e0 + u * stride;
+            c[u] = e < E ? __ldg(col + e) : 0;
+            x[u] = e < E ? __ldg(w + e) : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (c[u] < 0 || c[u] >= V) bad |= e0 + u * stride < E ? 2 : 0;
+            int n, t, b;
+            weight_bits_dev(x[u], n, t, b);
+            need = max(need, n);
+            top = max(top, t);
+            bad |= b ? 4 : 0;
+        }
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        need = max(need, __shfl_xor_sync(FULL, need, off));
-        top = max(top, __shfl_xor_sync(FULL, top, off));
-        bad |= __shfl_xor_sync(FULL, bad, off);
-    }
+    need = (int)__reduce_max_sync(FULL, (unsigned)need);
+    top = (int)__reduce_max_sync(FULL, (unsigned)top);
+    bad = (int)__reduce_or_sync(FULL, (unsigned)bad);
+    const int wid = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
-        if (need) atomicMax(out + 0, need);
-        if (top) atomicMax(out + 1, top);
-        if (bad) atomicOr(out + 2, bad);
+        sn[wid] = need;
+        st[wid] = top;
+        sb[wid] = bad;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; ++i) {
+            need = max(need, sn[i]);
+            top = max(top, st[i]);
+            bad |= sb[i];
+        }
+        if (need > ((volatile int32_t *)scan)[0]) atomicMax(scan + 0, need);
+        if (top > ((volatile int32_t *)scan)[1]) atomicMax(scan + 1, top);
+        if (bad & 4) atomicOr(scan + 2, 1);
+        if (bad & 3) atomicOr(err, bad & 3);
     }
 }
 
-__global__ void total_weight_kernel(const float *__restrict__ w, int64_t E, double scale,
-                                    u64 *total) {
+// Total weight on the grid that the scan words give (left unset for a CSR or
+// weights that the scan rejects).
+__global__ void __launch_bounds__(256) total_weight_kernel(const float *__restrict__ w, int64_t E,
+                                                           const int *__restrict__ err,
+                                                           const int32_t *__restrict__ scan, u64 *total) {
     __shared__ u64 part[8];
+    const int sc = scale_of_scan(scan, E);
+    if (*err || scan[2] || sc < 0) return;
+    const double scale = ldexp(1.0, sc);
     u64 acc = 0;
     for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < E; e += (int64_t)gridDim.x * 256)
         acc += wfix(w, e, scale);
@@ -243,22 +287,6 @@ __global__ void total_weight_kernel(const float *__restrict__ w, int64_t E, doub
         for (int i = 0; i < 8; ++i) y += part[i];
         if (y) atomicAdd(total, y);
     }
-}
-
-__global__ void validate_csr_kernel(const int32_t *__restrict__ rowptr,
-                                    const int32_t *__restrict__ col, int32_t V, int64_t E,
-                                    int *err) {
-    const int64_t tid = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    const int64_t stride = (int64_t)gridDim.x * 256;
-    int bad = 0;
-    if (tid == 0 && (rowptr[0] != 0 || (int64_t)rowptr[V] != E)) bad |= 1;
-    for (int64_t v = tid; v < V; v += stride)
-        if (rowptr[v + 1] < rowptr[v]) bad |= 1;
-    for (int64_t e = tid; e < E; e += stride) {
-        const int32_t c = col[e];
-        if (c < 0 || c >= V) bad |= 2;
-    }
-    if (bad) atomicOr(err, bad);
 }
 
 inline unsigned grid_for(int64_t n, int64_t cap = 148 * 16) {
@@ -377,21 +405,18 @@ void launch_weights_to_fixed(const WT *w, int64_t E, double scale, int64_t *out,
 template void launch_weights_to_fixed<float>(const float *, int64_t, double, int64_t *, cudaStream_t);
 template void launch_weights_to_fixed<u64>(const u64 *, int64_t, double, int64_t *, cudaStream_t);
 
-void launch_weight_scan(const float *w, int64_t E, int32_t *out, cudaStream_t s) {
-    cudaMemsetAsync(out, 0, sizeof(int32_t) * 3, s);
-    if (E <= 0) return;
-    weight_scan_kernel<<<grid_for(E), 256, 0, s>>>(w, E, out); note_launches(1);
+void launch_csr_scan(const int32_t *rowptr, const int32_t *col, const float *w, int32_t V, int64_t E, int *err,
+                     int32_t *scan, u64 *clear, int64_t n_clear, cudaStream_t s) {
+    cudaMemsetAsync(scan, 0, sizeof(int32_t) * 4, s);
+    csr_scan_kernel<<<grid_for(V > E ? V : E, 148 * 8), 256, 0, s>>>(rowptr, col, w, V, E, err, scan, clear, n_clear);
+    note_launches(1);
 }
 
-void launch_total_weight(const float *w, int64_t E, double scale, u64 *total, cudaStream_t s) {
+void launch_total_weight(const float *w, int64_t E, const int *err, const int32_t *scan, u64 *total, cudaStream_t s) {
     cudaMemsetAsync(total, 0, sizeof(u64), s);
     if (E <= 0) return;
-    total_weight_kernel<<<grid_for(E), 256, 0, s>>>(w, E, scale, total); note_launches(1);
-}
-
-void launch_validate_csr(const int32_t *rowptr, const int32_t *col, int32_t V, int64_t E, int *err,
-                         cudaStream_t s) {
-    validate_csr_kernel<<<grid_for(V > E ? V : E), 256, 0, s>>>(rowptr, col, V, E, err); note_launches(1);
+    total_weight_kernel<<<grid_for(E, 148 * 8), 256, 0, s>>>(w, E, err, scan, total);
+    note_launches(1);
 }
 
 }  // namespace lv
