@@ -292,6 +292,32 @@ __device__ __forceinline__ bool mbar_wait_parity(uint64_t *bar, uint32_t parity,
 }
 constexpr uint32_t MBAR_MAX_POLLS = 1u << 22;   // each try_wait may itself suspend for a while
 
+// Programmatic dependent launch of a sweep's short kernels: launched with
+// launch_pdl, they let the next kernel's launch begin once all their CTAs run
+// (pdl_trigger) and touch global memory only after the kernel before them has
+// finished (pdl_wait), so that launches overlap (R-MAT-18 from its entries
+// 22.3 to 21.3 ms, learned sweeps of a 1M-vertex graph 16.9 to 16.1 ms).  The
+// kernels with large shared tables neither trigger nor are launched so: CTAs
+// that wait beside them take the shared memory and L1 that they run on
+// (R-MAT-20 28.6 ms without, 29.8 ms with them).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... K, typename... A>
+inline void launch_pdl(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+}
+
 struct StateView {
     int32_t *comm;
     int32_t *newc;

@@ -869,6 +869,8 @@ struct LoopState {
 };
 
 __global__ void sweep_end_kernel(cudaGraphConditionalHandle cond, const Totals *t, LoopState *ls) {
+    pdl_trigger();
+    pdl_wait();
     if (threadIdx.x != 0) return;
     ls->e_own += t->dE;
     const double q = q_from_parts_dev(ls->T, ls->e_own, t->s2[0], t->s2[1]);
@@ -928,7 +930,7 @@ int sweep_loop_graph(lv_handle *h, float min_gain, double q_start, int *ch, int 
             reset_totals(h);
             LV_BY_WEIGHT(h, enqueue_sweep, h);
             launch_s2(h->S, h->V, h->tot_d->s2, h->stream);
-            sweep_end_kernel<<<1, 32, 0, h->stream>>>(cond, h->tot_d, ld);
+            launch_pdl(sweep_end_kernel, 1, 32, 0, h->stream, cond, h->tot_d, ld);
             note_launches(1);
             h->capturing = false;
             cudaGraph_t captured = nullptr;

@@ -96,6 +96,7 @@ template <int G, int CAP, typename WT>
 __global__ void __launch_bounds__(256) move_group_kernel(GraphView<WT> g, StateView st,
                                                          const int32_t *__restrict__ list,
                                                          int32_t n, u64 *dE) {
+    pdl_trigger();
     constexpr int GPB = 256 / G;
     constexpr int LG = ilog2_c(CAP);
     static_assert((1 << LG) == CAP, "CAP must be a power of two");
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(256) move_group_kernel(GraphView<WT> g, StateV
 #pragma unroll
     for (int s = lane; s < CAP; s += G) { keys[s] = -1; vals[s] = 0; }
     __syncwarp();
+    pdl_wait();
     const bool active = idx < n;
     int32_t v = 0, own = 0;
     u64 e_own = 0;   // weight to the own community: kept out of the table
@@ -143,6 +145,7 @@ template <int G, int CAP, typename WT>
 __global__ void __launch_bounds__(256) move_group_narrow_kernel(GraphView<WT> g, StateView st,
                                                                 const int32_t *__restrict__ list,
                                                                 int32_t n, u64 *dE, Fallback fbl) {
+    pdl_trigger();
     constexpr int GPB = 256 / G;
     constexpr int LG = ilog2_c(CAP);
     static_assert((1 << LG) == CAP, "CAP must be a power of two");
@@ -158,6 +161,7 @@ __global__ void __launch_bounds__(256) move_group_narrow_kernel(GraphView<WT> g,
 #pragma unroll
     for (int s = lane; s < CAP; s += G) { t.keys[s] = -1; t.lo[s] = 0; t.hi[s] = 0; }
     __syncwarp();
+    pdl_wait();
     bool active = idx < n;
     int32_t v = 0, own = 0, r0 = 0, r1 = 0;
     u64 e_own = 0;
@@ -1382,6 +1386,8 @@ constexpr int CORR_U = 4;
 template <typename WT>
 __global__ void __launch_bounds__(256) collect_movers_kernel(GraphView<WT> g, StateView st,
                                                              const int32_t *__restrict__ list, int32_t n) {
+    pdl_trigger();
+    pdl_wait();
     const int32_t i = blockIdx.x * 256 + threadIdx.x;
     int32_t v = -1;
     uint32_t units = 0;
@@ -1397,6 +1403,8 @@ __global__ void __launch_bounds__(256) collect_movers_kernel(GraphView<WT> g, St
 
 template <typename WT>
 __global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, StateView st, u64 *dE) {
+    pdl_trigger();
+    pdl_wait();
     const u64 cu64 = *st.mv_cnt;
     const uint32_t n = (uint32_t)cu64, units = (uint32_t)(cu64 >> 32);
     const int lane = threadIdx.x & 31;
@@ -1470,6 +1478,8 @@ __global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, State
 // ------------------------------------------------------------------------
 // Over the listed movers only (grid-stride; the count is on the device).
 __global__ void __launch_bounds__(256) commit_kernel(StateView st, u64 *moves) {
+    pdl_trigger();
+    pdl_wait();
     const uint32_t n = (uint32_t)*st.mv_cnt;
     if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(moves, (u64)n);
     for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
@@ -1554,6 +1564,8 @@ __global__ void __launch_bounds__(THREADS) row_reduce_cta_kernel(GraphView<WT> g
 
 __global__ void __launch_bounds__(256) s2_kernel(const u64 *__restrict__ S, int32_t V,
                                                  u64 *total_hi_lo) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ u64 plo[8], phi[8];
     u128 acc = 0;
     for (int32_t c = blockIdx.x * 256 + threadIdx.x; c < V; c += gridDim.x * 256) {
@@ -1722,9 +1734,10 @@ void launch_move_class(int cls, const GraphView<WT> &g, const StateView &st, con
 #define LV_GROUP(G, CAP)                                                                              \
     do {                                                                                              \
         if (narrow)                                                                                   \
-            move_group_narrow_kernel<G, CAP, WT><<<nblocks(n, 256 / G), 256, 0, s>>>(g, st, list, n, dE, \
-                                                                                    fs.q[NFBQ]);     \
-        else move_group_kernel<G, CAP, WT><<<nblocks(n, 256 / G), 256, 0, s>>>(g, st, list, n, dE);   \
+            launch_pdl((move_group_narrow_kernel<G, CAP, WT>), nblocks(n, 256 / G), 256, 0, s, g, st, list, n, \
+                       dE, fs.q[NFBQ]);                                                               \
+        else                                                                                          \
+            launch_pdl((move_group_kernel<G, CAP, WT>), nblocks(n, 256 / G), 256, 0, s, g, st, list, n, dE); \
         note_launches(1);                                                                             \
     } while (0)
     switch (cls) {
@@ -1820,7 +1833,7 @@ template <typename WT>
 void launch_collect_movers(const GraphView<WT> &g, const StateView &st, const int32_t *list, int32_t n,
                            cudaStream_t s) {
     if (n <= 0) return;
-    collect_movers_kernel<WT><<<nblocks(n, 256), 256, 0, s>>>(g, st, list, n);
+    launch_pdl(collect_movers_kernel<WT>, nblocks(n, 256), 256, 0, s, g, st, list, n);
     note_launches(1);
 }
 
@@ -1828,8 +1841,8 @@ template <typename WT>
 void launch_movers(const GraphView<WT> &g, const StateView &st, int32_t n, const DeviceInfo &di, u64 *dE, u64 *moves,
                    cudaStream_t s) {
     if (n <= 0) return;
-    corr_movers_kernel<WT><<<(unsigned)imin64(nblocks(n, 8), (int64_t)di.sms * 8), 256, 0, s>>>(g, st, dE);
-    commit_kernel<<<(unsigned)imin64(nblocks(n, 256), (int64_t)di.sms * 8), 256, 0, s>>>(st, moves);
+    launch_pdl(corr_movers_kernel<WT>, (unsigned)imin64(nblocks(n, 8), (int64_t)di.sms * 8), 256, 0, s, g, st, dE);
+    launch_pdl(commit_kernel, (unsigned)imin64(nblocks(n, 256), (int64_t)di.sms * 8), 256, 0, s, st, moves);
     note_launches(2);
 }
 
@@ -1872,7 +1885,8 @@ void launch_row_reduce(int cls, int mode, const GraphView<WT> &g, const int32_t 
 void launch_s2(const u64 *S, int32_t V, u64 *total_hi_lo, cudaStream_t s) {
     if (V <= 0) return;
     unsigned grid = (unsigned)imin64(nblocks(V, 256), 148 * 8);
-    s2_kernel<<<grid, 256, 0, s>>>(S, V, total_hi_lo); note_launches(1);
+    launch_pdl(s2_kernel, grid, 256, 0, s, S, V, total_hi_lo);
+    note_launches(1);
 }
 
 template void launch_move_class<float>(int, const GraphView<float> &, const StateView &,
