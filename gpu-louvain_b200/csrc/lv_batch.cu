@@ -216,17 +216,6 @@ __device__ __forceinline__ double modularity_from(const GState &gs, u64 e_own, u
     return q_from_parts_dev(gs.T, e_own, (u64)(s2 >> 64), (u64)s2);
 }
 
-// One entry's share of the symmetry check: the sum over all entries of
-// mix(row, col, w) - mix(col, row, w) is zero when the entries and their
-// mirror images are the same multiset (and otherwise zero by a chance of
-// 2^-64 only).
-__device__ __forceinline__ u64 sym_mix(uint32_t a, uint32_t b, uint32_t w) {
-    u64 x = ((u64)a << 32 | b) * 0x9E3779B97F4A7C15ull + w;
-    x ^= x >> 29;
-    x *= 0xD6E8FEB86659FD93ull;
-    return x ^ (x >> 32);
-}
-
 // Group tables: the sum of a slot is kept in three 32-bit counters of 22-bit
 // pieces, so that an add is two or three shared atomics without a returned
 // value or a carry; exact for up to 1024 adds per slot (rows of at most DW
@@ -904,8 +893,7 @@ static __device__ void level_setup(const Rows &L, const BatchParams &P, GState &
                     else if (P.w) const_cast<u64 *>(L.w64)[e] = x;
                     const int32_t j = L.c(e);
                     s += x;
-                    const uint32_t xw = (uint32_t)x ^ (uint32_t)(x >> 32) * 0x85EBCA6Bu;
-                    tt.b += sym_mix((uint32_t)(v0 + i), (uint32_t)j, xw) - sym_mix((uint32_t)j, (uint32_t)(v0 + i), xw);
+                    tt.b += sym_share(v0 + i, j, x);
                 }
             }
             for (int off = 4; off > 0; off >>= 1) s += __shfl_xor_sync(FULL, s, off);

@@ -55,6 +55,17 @@ using namespace lv;
 // atomics per add serialise where many lanes add to one community) and
 // 256 ms in mode 2 (the escape test per entry costs more than the 4 bytes
 // per entry it saves).
+// Table sweeps (lv_nct.cuh), see where they are used below; settable so that
+// small graphs can be run through them.
+#ifndef LV_NCT_MIN_ENTRIES
+#define LV_NCT_MIN_ENTRIES (1 << 21)
+#endif
+#ifndef LV_NCT_SWITCH
+#define LV_NCT_SWITCH 0.1
+#endif
+#ifndef LV_NCT_MAX_SLOTS
+#define LV_NCT_MAX_SLOTS 0.3
+#endif
 #ifndef LV_NARROW_ESCAPES
 #define LV_NARROW_ESCAPES 0
 #endif
@@ -81,6 +92,7 @@ constexpr int FB_SETS = 4;
 constexpr int FB_CTR = 2 * (NFBQ + 1) + 2;
 struct SweepBlock {
     u64 movers[NBUCKETS];
+    int32_t nctq[2][2];   // the table build queue's count, next (buckets 5 and 6)
     int32_t fb[FB_SETS][FB_CTR];
     Totals tot;
 };
@@ -171,6 +183,8 @@ struct lv_handle {
     bool capturing = false;        // a sweep is being captured into a graph (timers off)
     MemSet mem;                    // every device buffer of the handle
     void *loop_d = nullptr;        // device state of the graph sweep loop
+    NctView nct;                   // neighbour-community tables (late sweeps)
+    u64 nct_alloc = 0;             // slots allocated in the pool
 
     // level_setup not run yet for the current level: the state arrays are
     // unset (SETUP_ALL) or a team run set them and only the class lists are
@@ -380,7 +394,7 @@ bool narrow_weights(const lv_handle *h) {
 StateView state_of(lv_handle *h) {
     return StateView{h->comm, h->newc, h->size, h->k, h->S, h->T, &h->tot_d->err, h->feat,
                      (LV_NARROW_ESCAPES == 1 && h->cur_w32 && h->wrows_any) ? h->wrow : nullptr,
-                     h->blk_d->movers, h->mv_list, h->mv_off,
+                     h->blk_d->movers, h->mv_list, h->mv_off, nullptr, nullptr,
                      (LV_DEDUP == 2 || (LV_DEDUP == 1 && h->level > 0)) ? 1 : 0};
 }
 
@@ -754,6 +768,46 @@ void enqueue_sweep(lv_handle *h) {
     h->st.move_bytes += tm.bytes;
 }
 
+// A sweep whose vertices of degree > 32 are decided from their tables.
+template <typename WT>
+void enqueue_sweep_tables(lv_handle *h) {
+    GraphView<WT> g = view_of<WT>(h);
+    StateView st = state_of(h);
+    st.tlg = h->nct.lg;
+    st.tnever = h->nct.cursor + 1;
+    const double wbytes = sizeof(WT) == 4 ? 4.0 : 8.0;
+    u64 *dE = &h->tot_d->dE;
+    Timer tm(h, 100);
+    int64_t sweep_verts = 0;
+    for (int b = 0; b < NBUCKETS; ++b) {
+        const int32_t lo = h->cls_off[b], hi = b < 6 ? h->cls_off[b + 1] : h->cls_off[NCLS];
+        if (hi == lo) continue;
+        const FallbackSet fs = queues_on(h, b >= 4 ? b - 4 : 3);
+        st.mv_cnt = h->blk_d->movers + b;
+        if (b < 4) {
+            launch_move_class<WT>(b, g, st, h->list + lo, hi - lo, h->di, dE, h->stream, narrow_weights<WT>(h), fs);
+        } else {
+            // rows of bucket 4 never hold more communities than a warp builds
+            NctView t = h->nct;
+            t.qctr = h->blk_d->nctq[b == 6];
+            launch_nct<WT>(g, st, h->list + lo, hi - lo, t, fs, h->giant_degree, b > 4, h->di, dE, h->stream);
+            if (b == 6) {
+                if (hi > h->cls_off[CLS_HG])
+                    launch_move_giants<WT>(g, st, h->hub_move.view, fs, h->di, dE, h->stream, narrow_weights<WT>(h));
+                else
+                    launch_large<WT>(g, st, fs, h->di, dE, h->stream);
+            }
+            launch_collect_movers<WT>(g, st, h->list + lo, hi - lo, h->stream);
+        }
+        launch_movers<WT>(g, st, hi - lo, h->di, dE, &h->tot_d->moves, h->stream, &h->nct);
+        sweep_verts += hi - lo;
+    }
+    tm.bytes = 12.0 * (double)h->E + 20.0 * (double)sweep_verts;
+    tm.sbytes = (8.0 + wbytes) * (double)h->E + 20.0 * (double)sweep_verts;
+    tm.stop();
+    h->st.move_bytes += tm.bytes;
+}
+
 template <typename WT>
 void enqueue_modularity(lv_handle *h) {
     GraphView<WT> g = view_of<WT>(h);
@@ -862,13 +916,15 @@ struct LoopState {
     u64 T;
     u64 moves_total;
     double q_last;
+    u64 switch_units;   // leave the loop for table sweeps when a sweep's movers have fewer row units
     int32_t max_sweeps;
     int32_t sweeps;
     int32_t changed;
-    int32_t pad;
+    int32_t switched;
 };
 
-__global__ void sweep_end_kernel(cudaGraphConditionalHandle cond, const Totals *t, LoopState *ls) {
+__global__ void sweep_end_kernel(cudaGraphConditionalHandle cond, const SweepBlock *blk, LoopState *ls) {
+    const Totals *t = &blk->tot;
     pdl_trigger();
     pdl_wait();
     if (threadIdx.x != 0) return;
@@ -880,45 +936,103 @@ __global__ void sweep_end_kernel(cudaGraphConditionalHandle cond, const Totals *
     if (gain > 0) ls->changed = 1;
     ls->q_before = q;
     ls->q_last = q;
-    const bool more = gain >= ls->min_gain && t->moves != 0 &&
-                      !(ls->max_sweeps > 0 && ls->sweeps >= ls->max_sweeps) && t->err == 0;
+    bool more = gain >= ls->min_gain && t->moves != 0 &&
+                !(ls->max_sweeps > 0 && ls->sweeps >= ls->max_sweeps) && t->err == 0;
+    if (more && ls->switch_units) {
+        u64 units = 0;
+        for (int b = 0; b < NBUCKETS; ++b) units += blk->movers[b] >> 32;
+        if (units < ls->switch_units) {
+            ls->switched = 1;
+            more = false;
+        }
+    }
     cudaGraphSetConditional(cond, more ? 1u : 0u);
 }
 
-// Returns LV_OK with *done = 1 when the loop ran as a graph; *done = 0 when
-// the graph could not be built (the caller then runs the host loop).
-int sweep_loop_graph(lv_handle *h, float min_gain, double q_start, int *ch, int *done) {
-    *done = 0;
-    if (!h->loop_d) {
-        LoopState *p = nullptr;
-        LV_TRY(dalloc(h, &p, 1));
-        h->loop_d = p;
+// Tables pay off on levels whose sweeps are bound by their rows: below this many
+// entries a table sweep saves less than its graph costs to build (0.3 ms).
+constexpr int64_t NCT_MIN_ENTRIES = LV_NCT_MIN_ENTRIES;
+// ... once the movers' rows, which the table updates visit with random
+// accesses, are a small part of the entries: lv_run of R-MAT-24 takes 240 / 236
+// / 233.4 / 233.4 ms when tables start below 0.02 / 0.05 / 0.1 / 0.2 (273 ms
+// without tables) ...
+constexpr double NCT_SWITCH = LV_NCT_SWITCH;
+// ... and when the tables hold far fewer slots than the rows hold entries
+// (R-MAT-24: 0.12 slots per entry on the second level; over 0.5 on the first,
+// where a table sweep took 51 ms against 18), estimated from sampled rows.
+constexpr double NCT_MAX_SLOTS = LV_NCT_MAX_SLOTS;
+constexpr int32_t NCT_SAMPLES = 4096;
+
+// Prepares table sweeps of the current level; *ok = 0 when its rows do not
+// allow them (an entry without its mirror entry, or of weight zero).
+int nct_begin(lv_handle *h, int *ok) {
+    *ok = 0;
+    LV_TRY(reset_totals(h));
+    u64 *tot = h->tot_d->s2;   // two words
+    launch_nct_sample(h->cur_rowptr, h->cur_rowend, h->cur_col, h->comm, h->list + h->cls_off[CLS_B4],
+                      h->cls_off[CLS_HG] - h->cls_off[CLS_B4], NCT_SAMPLES, tot, h->stream);
+    LV_TRY(read_totals(h));
+    if ((double)h->tot_h->s2[0] > NCT_MAX_SLOTS * (double)h->tot_h->s2[1]) return LV_OK;
+    LV_TRY(reset_totals(h));
+    auto check = [&](auto g) {
+        for (int c = 0; c < NCLS; ++c)
+            launch_row_reduce(c, 2, g, h->comm, nullptr, tot, h->list + h->cls_off[c],
+                              h->cls_off[c + 1] - h->cls_off[c], h->di, h->stream);
+    };
+    if (h->cur_w) check(view_of<u64>(h));
+    else check(view_of<float>(h));
+    LV_TRY(read_totals(h));
+    if (h->tot_h->s2[0] || h->tot_h->s2[1]) return LV_OK;
+    if (!h->nct.lg) {
+        LV_TRY(dalloc(h, &h->nct.lg, (size_t)h->V0 + 1));
+        LV_TRY(dalloc(h, &h->nct.off, (size_t)h->V0 + 1));
+        LV_TRY(dalloc(h, &h->nct.queue, (size_t)h->V0 + 1));
+        LV_TRY(dalloc(h, &h->nct.cursor, 2));
     }
-    LoopState *ld = (LoopState *)h->loop_d;
-    LoopState ls{};
-    ls.q_before = q_start;
-    ls.min_gain = (double)min_gain;
-    ls.e_own = h->e_own_cur;
-    ls.T = h->T;
-    ls.q_last = q_start;
-    ls.max_sweeps = h->opts.max_sweeps;
-    LV_CUDA(h, cudaMemcpyAsync(ld, &ls, sizeof(ls), cudaMemcpyHostToDevice, h->stream));
-    clear_move_state(h->fb, h->hub_move.view, h->stream);
-    LV_TRY(sync(h));
+    // half a slot per entry of the level: rows with many communities that do
+    // not fit go on being summed from the row
+    const u64 want = (u64)h->E / 2 + 1024;
+    if (want > h->nct_alloc) {
+        dfree(h, h->nct.slots);
+        h->nct_alloc = 0;
+        LV_TRY(dalloc(h, &h->nct.slots, (size_t)want));
+        h->nct_alloc = want;
+    }
+    h->nct.cap = want;
+    LV_CUDA(h, cudaMemsetAsync(h->nct.lg, 0, (size_t)h->V, h->stream));
+    LV_CUDA(h, cudaMemsetAsync(h->nct.cursor, 0, 2 * sizeof(u64), h->stream));
+    *ok = 1;
+    return LV_OK;
+}
+
+// A level's sweep loop as one CUDA graph.
+struct LoopGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    long long launches = 0;   // per sweep
+    double bytes = 0;
+    ~LoopGraph() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+    }
+};
+
+// Builds the loop (with table sweeps when `tables`); false when the driver
+// does not take it.
+bool build_loop_graph(lv_handle *h, LoopGraph &lg, bool tables) {
     cudaGraphConditionalHandle cond = 0;
     cudaGraphNode_t node = nullptr;
-    bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess &&
-              cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault) == cudaSuccess;
+    bool ok = cudaGraphCreate(&lg.graph, 0) == cudaSuccess &&
+              cudaGraphConditionalHandleCreate(&cond, lg.graph, 1, cudaGraphCondAssignDefault) == cudaSuccess;
     cudaGraphNodeParams np = {};
     if (ok) {
         np.type = cudaGraphNodeTypeConditional;
         np.conditional.handle = cond;
         np.conditional.type = cudaGraphCondTypeWhile;
         np.conditional.size = 1;
-        ok = cudaGraphAddNode(&node, graph, nullptr, 0, &np) == cudaSuccess;
+        ok = cudaGraphAddNode(&node, lg.graph, nullptr, 0, &np) == cudaSuccess;
     }
+    // the capture's counts are taken back: only sweeps that run are counted
     const long long launches0 = launches_total();
     const double bytes0 = h->st.move_bytes;
     if (ok) {
@@ -928,46 +1042,81 @@ int sweep_loop_graph(lv_handle *h, float min_gain, double q_start, int *ch, int 
         if (ok) {
             h->capturing = true;
             reset_totals(h);
-            LV_BY_WEIGHT(h, enqueue_sweep, h);
+            if (tables) LV_BY_WEIGHT(h, enqueue_sweep_tables, h);
+            else LV_BY_WEIGHT(h, enqueue_sweep, h);
             launch_s2(h->S, h->V, h->tot_d->s2, h->stream);
-            launch_pdl(sweep_end_kernel, 1, 32, 0, h->stream, cond, h->tot_d, ld);
+            launch_pdl(sweep_end_kernel, 1, 32, 0, h->stream, cond, h->blk_d, (LoopState *)h->loop_d);
             note_launches(1);
             h->capturing = false;
             cudaGraph_t captured = nullptr;
             ok = cudaStreamEndCapture(h->stream, &captured) == cudaSuccess;
         }
     }
-    if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
-    const long long per_sweep = launches_total() - launches0;
-    const double bytes_per_sweep = h->st.move_bytes - bytes0;
+    if (ok) ok = cudaGraphInstantiate(&lg.exec, lg.graph, 0) == cudaSuccess;
+    lg.launches = launches_total() - launches0;
+    lg.bytes = h->st.move_bytes - bytes0;
+    note_launches((int)-lg.launches);
+    h->st.move_bytes = bytes0;
     if (!ok) {
         cudaGetLastError();
         h->capturing = false;
-        if (exec) cudaGraphExecDestroy(exec);
-        if (graph) cudaGraphDestroy(graph);
-        note_launches((int)-per_sweep);   // nothing ran
-        h->st.move_bytes = bytes0;
-        return LV_OK;
     }
+    return ok;
+}
+
+// Runs the loop from the state *ls, which is read back.
+int run_loop_graph(lv_handle *h, const LoopGraph &lg, LoopState *ls) {
+    LoopState *ld = (LoopState *)h->loop_d;
+    const int32_t sweeps0 = ls->sweeps;
+    const u64 moves0 = ls->moves_total;
+    LV_CUDA(h, cudaMemcpyAsync(ld, ls, sizeof(*ls), cudaMemcpyHostToDevice, h->stream));
+    clear_move_state(h->fb, h->hub_move.view, h->stream);
     {
         Timer tm(h, 100);
-        LV_CUDA(h, cudaGraphLaunch(exec, h->stream));
+        LV_CUDA(h, cudaGraphLaunch(lg.exec, h->stream));
         tm.stop();
     }
-    LV_CUDA(h, cudaMemcpyAsync(&ls, ld, sizeof(ls), cudaMemcpyDeviceToHost, h->stream));
+    LV_CUDA(h, cudaMemcpyAsync(ls, ld, sizeof(*ls), cudaMemcpyDeviceToHost, h->stream));
     LV_CUDA(h, cudaMemcpyAsync(h->tot_h, h->tot_d, sizeof(Totals), cudaMemcpyDeviceToHost, h->stream));
-    const int rc = sync(h);
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
-    LV_TRY(rc);
+    LV_TRY(sync(h));
     LV_TRY(check_device_error(h, h->tot_h->err));
-    // the captured sweep was counted once; it ran ls.sweeps times
-    note_launches((int)(per_sweep * (ls.sweeps - 1)));
-    h->st.move_bytes = bytes0 + bytes_per_sweep * ls.sweeps;
-    h->e_own_cur = ls.e_own;
-    h->st.sweeps += ls.sweeps;
-    h->st.edge_sweeps += h->E * (int64_t)ls.sweeps;
-    h->st.moves += (int64_t)ls.moves_total;
+    const int32_t ran = ls->sweeps - sweeps0;
+    note_launches((int)(lg.launches * ran));
+    h->st.move_bytes += lg.bytes * ran;
+    h->e_own_cur = ls->e_own;
+    h->st.sweeps += ran;
+    h->st.edge_sweeps += h->E * (int64_t)ran;
+    h->st.moves += (int64_t)(ls->moves_total - moves0);
+    return LV_OK;
+}
+
+// Returns LV_OK with *done = 1 when the loop ran as graphs; *done = 0 when
+// none could be built (the caller then runs the host loop).
+int sweep_loop_graph(lv_handle *h, float min_gain, double q_start, int *ch, int *done) {
+    *done = 0;
+    if (!h->loop_d) {
+        LoopState *p = nullptr;
+        LV_TRY(dalloc(h, &p, 1));
+        h->loop_d = p;
+    }
+    LoopState ls{};
+    ls.q_before = q_start;
+    ls.min_gain = (double)min_gain;
+    ls.e_own = h->e_own_cur;
+    ls.T = h->T;
+    ls.q_last = q_start;
+    ls.max_sweeps = h->opts.max_sweeps;
+    if (h->E >= NCT_MIN_ENTRIES) ls.switch_units = (u64)(NCT_SWITCH * (double)h->E / 32.0);
+    LoopGraph rows, tables;
+    if (!build_loop_graph(h, rows, false)) return LV_OK;
+    LV_TRY(run_loop_graph(h, rows, &ls));
+    if (ls.switched) {
+        ls.switched = 0;
+        ls.switch_units = 0;
+        int ok = 0;
+        LV_TRY(nct_begin(h, &ok));
+        LV_TRY(run_loop_graph(h, ok && build_loop_graph(h, tables, true) ? tables : rows, &ls));
+    }
     *ch = ls.changed;
     *done = 1;
     return LV_OK;

@@ -176,6 +176,18 @@ constexpr int FB_SMEM = FB_CAP * 14;   // table + occupied list
 #endif
 constexpr int WARP_SMEM = 8 * WARP_CAP * 12 + LV_WARP_PAD;   // 8 warp tables per CTA
 
+// Neighbour-community tables of a level's late sweeps (lv_nct.cuh).
+constexpr int NCT_NEVER = 255;
+struct NctView {
+    uint8_t *lg = nullptr;      // [V] log2 of the vertex's slots; 0 = no valid table, NCT_NEVER = none ever
+    uint32_t *off = nullptr;    // [V] first slot
+    GSlot *slots = nullptr;     // the pool: cap slots, *cursor of them taken
+    u64 *cursor = nullptr;      // [0] slots taken, [1] vertices marked NCT_NEVER
+    u64 cap = 0;
+    int32_t *queue = nullptr;   // [V] vertices for the CTA build
+    int32_t *qctr = nullptr;    // its count, next
+};
+
 // A fallback work list (device memory; count and next are adjacent).
 struct Fallback {
     int32_t *count = nullptr;   // items queued
@@ -247,7 +259,21 @@ void launch_collect_movers(const GraphView<WT> &g, const StateView &st, const in
 // moved together, then the commit.  n bounds their number.
 template <typename WT>
 void launch_movers(const GraphView<WT> &g, const StateView &st, int32_t n, const DeviceInfo &di, u64 *dE, u64 *moves,
-                   cudaStream_t s);
+                   cudaStream_t s, const NctView *t = nullptr);   // t: update the tables of the movers' neighbours
+// The vertices list[0 .. n) of degree > 32 of one bucket, from their tables
+// (built on the way); queue_too: some rows may need the CTA build.
+template <typename WT>
+void launch_nct(const GraphView<WT> &g, const StateView &st, const int32_t *list, int32_t n, const NctView &t,
+                const FallbackSet &fs, int32_t giant_degree, bool queue_too, const DeviceInfo &di, u64 *dE,
+                cudaStream_t s);
+// Adds to out[0] / out[1] the table slots / row entries of up to n vertices
+// sampled from list[0 .. m).
+void launch_nct_sample(const int32_t *rowptr, const int32_t *rowend, const int32_t *col, const int32_t *comm,
+                       const int32_t *list, int32_t m, int32_t n, u64 *out, cudaStream_t s);
+// The large queue's items (vertices without tables that launch_nct queued).
+template <typename WT>
+void launch_large(const GraphView<WT> &g, const StateView &st, const FallbackSet &fs, const DeviceInfo &di, u64 *dE,
+                  cudaStream_t s);
 // The staging counters, own-community sums and partition done counters of the
 // giant and large-queue paths are returned to zero by the kernel that consumes
 // them; cleared before a level's sweeps as well, so that a sweep that ended
@@ -255,7 +281,9 @@ void launch_movers(const GraphView<WT> &g, const StateView &st, int32_t n, const
 // leave a count that makes a later staging pass append beyond a giant's area.
 void clear_move_state(const FallbackSet &fs, const HubGlobal &hg, cudaStream_t s);
 
-// k_i = row sums (mode 0) or e_own total (mode 1) over the vertices of one class.
+// Over the vertices of one class: k_i = row sums (mode 0), the e_own total
+// (mode 1), or (mode 2) total[0] += a sum that is zero when every entry has its
+// mirror entry, total[1] += entries of weight zero other than self-loops.
 template <typename WT>
 void launch_row_reduce(int cls, int mode, const GraphView<WT> &g, const int32_t *comm, u64 *k,
                        u64 *total, const int32_t *list, int32_t n, const DeviceInfo &di,

@@ -1145,6 +1145,7 @@ __global__ void __launch_bounds__(THREADS) move_rowq_staged_kernel(GraphView<WT>
 template <typename WT>
 __global__ void __launch_bounds__(STAGE_THREADS) giant_stage_narrow_kernel(GraphView<WT> g, StateView st,
                                                                            HubGlobal hg) {
+    if (st.tnever && *st.tnever == 0) return;   // every giant has its table
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int LCAP = 2 * STAGE_CHUNK;
     constexpr int LLG = ilog2_c(LCAP);
@@ -1165,6 +1166,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) giant_stage_narrow_kernel(Graph
         const int32_t h = hg.echunk_hub[ch];
         const int32_t v = hg.hubs[h];
         if (st.wrow && st.wrow[v]) continue;   // staged by giant_stage_kernel (64-bit sums)
+        if (st.tlg && st.tlg[v] != NCT_NEVER) continue;   // decided from its table
         const int32_t r1 = g.rowend[v];
         const int32_t e0 = g.rowptr[v] + hg.echunk_e0[ch];
         const int32_t e1 = min(e0 + STAGE_CHUNK, r1);
@@ -1199,6 +1201,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) giant_stage_kernel(GraphView<WT
     // the narrow kernel).  Persistent over the chunks, as the narrow kernel:
     // the table is initialised once and after each chunk only its claimed
     // slots are cleared.
+    if (st.tnever && *st.tnever == 0) return;   // every giant has its table
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int LCAP = 2 * STAGE_CHUNK;
     constexpr int LLG = ilog2_c(LCAP);
@@ -1213,6 +1216,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) giant_stage_kernel(GraphView<WT
         const int32_t h = hg.echunk_hub[ch];
         const int32_t v = hg.hubs[h];
         if (only && !only[v]) continue;
+        if (st.tlg && st.tlg[v] != NCT_NEVER) continue;   // decided from its table
         const int32_t r1 = g.rowend[v];
         const int32_t e0 = g.rowptr[v] + hg.echunk_e0[ch];
         const int32_t e1 = min(e0 + STAGE_CHUNK, r1);
@@ -1298,6 +1302,7 @@ template <int THREADS, int CAP>
 __global__ void __launch_bounds__(THREADS) giant_merge_kernel(StateView st, HubGlobal hg, Fallback fb,
                                                               u64 *dE, int32_t n_min) {
     // fb: the large fallback queue
+    if (st.tnever && *st.tnever == 0) return;   // every giant has its table
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64 *vals = reinterpret_cast<u64 *>(smem_raw);
     int32_t *keys = reinterpret_cast<int32_t *>(vals + CAP);
@@ -1308,6 +1313,7 @@ __global__ void __launch_bounds__(THREADS) giant_merge_kernel(StateView st, HubG
     __syncthreads();
     u64 delta_sum = 0;
     for (int32_t h = blockIdx.x; h < hg.nhubs; h += gridDim.x) {
+        if (st.tlg && st.tlg[hg.hubs[h]] != NCT_NEVER) continue;   // decided from its table
         const int32_t n = hg.nocc[h];
         if (2 * (int64_t)n > HG_MERGE_CAP && CAP == HG_MERGE_CAP) {
             // too many staged pairs for one shared table: queue key-space
@@ -1380,6 +1386,8 @@ __device__ __forceinline__ u64 pair_correction(int32_t cu, int32_t nu, int32_t c
 // column -> community chain; four units are in flight per warp.
 constexpr int CORR_U = 4;
 
+#include "lv_nct.cuh"
+
 // The movers of buckets 4 to 6, found after the sub-round's decisions: noting
 // them in the warp kernels cost the 64-bit one 12 % (119 against 107 ms for
 // degrees 320 to 8192 of an R-MAT-24 run).
@@ -1401,8 +1409,9 @@ __global__ void __launch_bounds__(256) collect_movers_kernel(GraphView<WT> g, St
     block_note_movers<256>(st, v, units);
 }
 
-template <typename WT>
-__global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, StateView st, u64 *dE) {
+// TABLES: the neighbours' tables follow the moves as well (lv_nct.cuh).
+template <typename WT, bool TABLES>
+__global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, StateView st, u64 *dE, NctView t) {
     pdl_trigger();
     pdl_wait();
     const u64 cu64 = *st.mv_cnt;
@@ -1463,8 +1472,10 @@ __global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, State
                         }
                     }
 #pragma unroll
-                    for (int q = 0; q < CORR_U; ++q)
+                    for (int q = 0; q < CORR_U; ++q) {
                         if (cj[q] != nj[q]) acc += pair_correction(cu, nu, cj[q], nj[q], gw(g, e0 + 32 * q));
+                        if (TABLES && jj[q] != v) nct_move(t, jj[q], cu, nu, gw(g, e0 + 32 * q));
+                    }
                 }
                 u = last;
             }
@@ -1477,6 +1488,8 @@ __global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, State
 // commit of one sub-round (updateVertexCommunity + Sigma_tot update)
 // ------------------------------------------------------------------------
 // Over the listed movers only (grid-stride; the count is on the device).
+// Summing the changes per community in a shared table first measured no
+// faster (R-MAT-20 28.2 against 27.9 ms).
 __global__ void __launch_bounds__(256) commit_kernel(StateView st, u64 *moves) {
     pdl_trigger();
     pdl_wait();
@@ -1503,14 +1516,19 @@ __global__ void __launch_bounds__(256) row_reduce_group_kernel(GraphView<WT> g,
     const int grp = threadIdx.x / G;
     const int lane = threadIdx.x % G;
     const int32_t idx = blockIdx.x * (256 / G) + grp;
-    u64 acc = 0;
+    u64 acc = 0, zeros = 0;
     int32_t v = 0;
     if (idx < n) {
         v = list[idx];
         const int32_t own = MODE == 1 ? comm[v] : 0;
         const int32_t r0 = g.rowptr[v], r1 = g.rowend[v];
         for (int32_t e = r0 + lane; e < r1; e += G) {
-            if (MODE == 1) {
+            if (MODE == 2) {
+                const int32_t j = __ldg(g.col + e);
+                const u64 x = gw(g, e);
+                acc += sym_share(v, j, x);
+                zeros += x == 0 && j != v ? 1 : 0;
+            } else if (MODE == 1) {
                 if (comm[__ldg(g.col + e)] == own) acc += gw(g, e);
             } else {
                 acc += gw(g, e);
@@ -1522,6 +1540,7 @@ __global__ void __launch_bounds__(256) row_reduce_group_kernel(GraphView<WT> g,
         if (idx < n && lane == 0) k[v] = acc;
     } else {
         block_add_total<256>(acc, total);
+        if (MODE == 2) block_add_total<256>(zeros, total + 1);
     }
 }
 
@@ -1532,14 +1551,19 @@ __global__ void __launch_bounds__(THREADS) row_reduce_cta_kernel(GraphView<WT> g
                                                                  const int32_t *__restrict__ list,
                                                                  int32_t n) {
     __shared__ u64 part[THREADS / 32];
-    u64 grand = 0;
+    u64 grand = 0, zeros = 0;
     for (int32_t idx = blockIdx.x; idx < n; idx += gridDim.x) {
         const int32_t v = list[idx];
         const int32_t own = MODE == 1 ? comm[v] : 0;
         const int32_t r0 = g.rowptr[v], r1 = g.rowend[v];
         u64 acc = 0;
         for (int32_t e = r0 + threadIdx.x; e < r1; e += THREADS) {
-            if (MODE == 1) {
+            if (MODE == 2) {
+                const int32_t j = __ldg(g.col + e);
+                const u64 x = gw(g, e);
+                acc += sym_share(v, j, x);
+                zeros += x == 0 && j != v ? 1 : 0;
+            } else if (MODE == 1) {
                 if (comm[__ldg(g.col + e)] == own) acc += gw(g, e);
             } else {
                 acc += gw(g, e);
@@ -1559,7 +1583,8 @@ __global__ void __launch_bounds__(THREADS) row_reduce_cta_kernel(GraphView<WT> g
             grand += acc;
         }
     }
-    if (MODE == 1) block_add_total<THREADS>(grand, total);
+    if (MODE >= 1) block_add_total<THREADS>(grand, total);
+    if (MODE == 2) block_add_total<THREADS>(zeros, total + 1);
 }
 
 __global__ void __launch_bounds__(256) s2_kernel(const u64 *__restrict__ S, int32_t V,
@@ -1660,6 +1685,7 @@ static void set_attrs_for(DeviceInfo &di) {
     set_row_queue_attrs<WT, 3>(di);
     cudaFuncSetAttribute(move_fallback_kernel<WT, FB_THREADS, FB_CAP, true>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM);
+    cudaFuncSetAttribute(nct_build_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM);
     cudaFuncSetAttribute(giant_stage_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGE_SMEM);
     cudaFuncSetAttribute(giant_stage_narrow_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGE_SMEM);
     {
@@ -1830,6 +1856,33 @@ void launch_move_wide(const GraphView<WT> &g, const StateView &st, const int32_t
 }
 
 template <typename WT>
+void launch_nct(const GraphView<WT> &g, const StateView &st, const int32_t *list, int32_t n, const NctView &t,
+                const FallbackSet &fs, int32_t giant_degree, bool queue_too, const DeviceInfo &di, u64 *dE,
+                cudaStream_t s) {
+    if (n <= 0) return;
+    const unsigned grid = (unsigned)imin64(nblocks(n, 8), (int64_t)di.sms * 6);
+    nct_eval_kernel<WT><<<grid, 256, 0, s>>>(g, st, list, n, t, fs.q[NFBQ], giant_degree, dE);
+    note_launches(1);
+    if (!queue_too) return;
+    nct_build_kernel<WT><<<di.sms, FB_THREADS, FB_SMEM, s>>>(g, st, t, fs.q[NFBQ], giant_degree, dE);
+    note_launches(1);
+}
+
+void launch_nct_sample(const int32_t *rowptr, const int32_t *rowend, const int32_t *col, const int32_t *comm,
+                       const int32_t *list, int32_t m, int32_t n, u64 *out, cudaStream_t s) {
+    if (m <= 0) return;
+    n = n < m ? n : m;
+    nct_sample_kernel<<<nblocks(n, 8), 256, 0, s>>>(rowptr, rowend, col, comm, list, m, n, out);
+    note_launches(1);
+}
+
+template <typename WT>
+void launch_large(const GraphView<WT> &g, const StateView &st, const FallbackSet &fs, const DeviceInfo &di, u64 *dE,
+                  cudaStream_t s) {
+    launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
+}
+
+template <typename WT>
 void launch_collect_movers(const GraphView<WT> &g, const StateView &st, const int32_t *list, int32_t n,
                            cudaStream_t s) {
     if (n <= 0) return;
@@ -1839,9 +1892,11 @@ void launch_collect_movers(const GraphView<WT> &g, const StateView &st, const in
 
 template <typename WT>
 void launch_movers(const GraphView<WT> &g, const StateView &st, int32_t n, const DeviceInfo &di, u64 *dE, u64 *moves,
-                   cudaStream_t s) {
+                   cudaStream_t s, const NctView *t) {
     if (n <= 0) return;
-    launch_pdl(corr_movers_kernel<WT>, (unsigned)imin64(nblocks(n, 8), (int64_t)di.sms * 8), 256, 0, s, g, st, dE);
+    const unsigned grid = (unsigned)imin64(nblocks(n, 8), (int64_t)di.sms * 8);
+    if (t) launch_pdl((corr_movers_kernel<WT, true>), grid, 256, 0, s, g, st, dE, *t);
+    else launch_pdl((corr_movers_kernel<WT, false>), grid, 256, 0, s, g, st, dE, NctView());
     launch_pdl(commit_kernel, (unsigned)imin64(nblocks(n, 256), (int64_t)di.sms * 8), 256, 0, s, st, moves);
     note_launches(2);
 }
@@ -1855,6 +1910,8 @@ void launch_row_reduce(int cls, int mode, const GraphView<WT> &g, const int32_t 
     do {                                                                                     \
         if (mode == 0)                                                                       \
             row_reduce_group_kernel<G, 0, WT><<<nblocks(n, 256 / G), 256, 0, s>>>(g, comm, k, total, list, n); \
+        else if (mode == 2)                                                                  \
+            row_reduce_group_kernel<G, 2, WT><<<nblocks(n, 256 / G), 256, 0, s>>>(g, comm, k, total, list, n); \
         else                                                                                 \
             row_reduce_group_kernel<G, 1, WT><<<nblocks(n, 256 / G), 256, 0, s>>>(g, comm, k, total, list, n); \
         note_launches(1);                                                                    \
@@ -1864,6 +1921,8 @@ void launch_row_reduce(int cls, int mode, const GraphView<WT> &g, const int32_t 
         unsigned grid = (unsigned)imin64(n, (int64_t)di.sms * (2048 / T));            \
         if (mode == 0)                                                                       \
             row_reduce_cta_kernel<T, 0, WT><<<grid, T, 0, s>>>(g, comm, k, total, list, n);  \
+        else if (mode == 2)                                                                  \
+            row_reduce_cta_kernel<T, 2, WT><<<grid, T, 0, s>>>(g, comm, k, total, list, n);  \
         else                                                                                 \
             row_reduce_cta_kernel<T, 1, WT><<<grid, T, 0, s>>>(g, comm, k, total, list, n);  \
         note_launches(1);                                                                    \
@@ -1909,11 +1968,19 @@ template void launch_move_giants<u64>(const GraphView<u64> &, const StateView &,
 template void launch_collect_movers<float>(const GraphView<float> &, const StateView &, const int32_t *, int32_t,
                                            cudaStream_t);
 template void launch_movers<float>(const GraphView<float> &, const StateView &, int32_t, const DeviceInfo &, u64 *, u64 *,
-                                   cudaStream_t);
+                                   cudaStream_t, const NctView *);
+template void launch_nct<float>(const GraphView<float> &, const StateView &, const int32_t *, int32_t, const NctView &,
+                                const FallbackSet &, int32_t, bool, const DeviceInfo &, u64 *, cudaStream_t);
+template void launch_large<float>(const GraphView<float> &, const StateView &, const FallbackSet &, const DeviceInfo &,
+                                  u64 *, cudaStream_t);
 template void launch_collect_movers<u64>(const GraphView<u64> &, const StateView &, const int32_t *, int32_t,
                                            cudaStream_t);
 template void launch_movers<u64>(const GraphView<u64> &, const StateView &, int32_t, const DeviceInfo &, u64 *, u64 *,
-                                   cudaStream_t);
+                                   cudaStream_t, const NctView *);
+template void launch_nct<u64>(const GraphView<u64> &, const StateView &, const int32_t *, int32_t, const NctView &,
+                                const FallbackSet &, int32_t, bool, const DeviceInfo &, u64 *, cudaStream_t);
+template void launch_large<u64>(const GraphView<u64> &, const StateView &, const FallbackSet &, const DeviceInfo &,
+                                  u64 *, cudaStream_t);
 template void launch_row_reduce<float>(int, int, const GraphView<float> &, const int32_t *, u64 *,
                                        u64 *, const int32_t *, int32_t, const DeviceInfo &,
                                        cudaStream_t);
@@ -1932,7 +1999,11 @@ template void launch_move_giants<uint32_t>(const GraphView<uint32_t> &, const St
 template void launch_collect_movers<uint32_t>(const GraphView<uint32_t> &, const StateView &, const int32_t *, int32_t,
                                            cudaStream_t);
 template void launch_movers<uint32_t>(const GraphView<uint32_t> &, const StateView &, int32_t, const DeviceInfo &, u64 *, u64 *,
-                                   cudaStream_t);
+                                   cudaStream_t, const NctView *);
+template void launch_nct<uint32_t>(const GraphView<uint32_t> &, const StateView &, const int32_t *, int32_t, const NctView &,
+                                const FallbackSet &, int32_t, bool, const DeviceInfo &, u64 *, cudaStream_t);
+template void launch_large<uint32_t>(const GraphView<uint32_t> &, const StateView &, const FallbackSet &, const DeviceInfo &,
+                                  u64 *, cudaStream_t);
 template void launch_row_reduce<uint32_t>(int, int, const GraphView<uint32_t> &, const int32_t *, u64 *,
                                      u64 *, const int32_t *, int32_t, const DeviceInfo &,
                                      cudaStream_t);

@@ -124,3 +124,78 @@ def test_rmat20_weight_widths_agree(lvb, rmat20):
     assert out[0][0] == out[1][0]
     assert np.array_equal(out[0][1], out[1][1])
     assert out[0][2] == out[1][2]
+
+
+def _table_graphs(lvb):
+    """Graphs of at least 2^21 entries whose later sweeps run from the
+    neighbour-community tables (rows of more than 32 entries, few movers), or
+    must not: a hub with more communities around it than a table takes, rows on
+    both sides of the giant degree, weights below and above 32 bits, an entry of
+    weight zero, and an entry without its mirror entry."""
+    rng = np.random.default_rng(12)
+    base = lvb.gen_planted(10000, 24, 300.0, 15.0, 3, "uniform")
+    u, v, w = base.edges()
+
+    def build(u, v, w, V):
+        rows = np.concatenate([u, v[u != v]])
+        cols = np.concatenate([v, u[u != v]])
+        ww = np.concatenate([w, w[u != v]]).astype(np.float32)
+        o = np.lexsort((cols, rows))
+        rp = np.zeros(V + 1, np.int32)
+        np.cumsum(np.bincount(rows, minlength=V), out=rp[1:])
+        return lvb.Graph(rp, cols[o].astype(np.int32), ww[o])
+
+    # 9000 heavy pairs, one vertex of each joined to vertex 0 (never merged with
+    # it), and a second hub over all blocks whose row is beyond the giant degree
+    V, n = base.V, 9000
+    pu = V + 2 * np.arange(n)
+    uu = np.concatenate([u, pu + 1, pu, rng.choice(V, 8900, False)])
+    vv = np.concatenate([v, pu, np.zeros(n, np.int64), np.full(8900, V + 2 * n)])
+    ww = np.concatenate([w, np.full(n, 64.0), np.full(n, 2.0 ** -6), np.full(8900, 2.0 ** -6)])
+    keep = uu != vv
+    hubs = build(uu[keep], vv[keep], ww[keep], V + 2 * n + 1)
+    fine = lvb.Graph(base.rowptr, base.col, base.w)
+    row = np.repeat(np.arange(V, dtype=np.int64), np.diff(base.rowptr))
+    x = (np.minimum(row, base.col) * 0x9E3779B1 + np.maximum(row, base.col) * 0x85EBCA77) & 0xFFFFFFFF
+    fine.w = (0.25 - np.log((x + 0.5) / 2.0 ** 32)).astype(np.float32)
+    zero = lvb.Graph(base.rowptr, base.col, np.where((row + base.col) % 1000 == 7, 0.0, base.w))
+    return {"planted": base, "hubs": hubs, "fine": fine, "zero": zero, "rmat18": lvb.gen_rmat(18, 16, 3)}
+
+
+@pytest.fixture(scope="module")
+def table_graphs(lvb):
+    return _table_graphs(lvb)
+
+
+@pytest.mark.parametrize("name", ["planted", "hubs", "fine", "zero", "rmat18"])
+def test_table_sweeps_match_row_sweeps(lvb, table_graphs, name):
+    """The loop that may switch to tables against the host loop, which always
+    sums rows: same map, modularity bits, sweeps and moves."""
+    g = table_graphs[name]
+    assert g.E >= 1 << 21
+    res = []
+    for kw in ({}, {"sweep_graph": False}, {"giant_degree": 1024}):
+        with lvb.Louvain(g, **kw) as e:
+            q = e.run(1e-7)
+            m, n = e.original_to_community()
+            st = e.stats()
+            res.append((q, n, st["levels"], st["sweeps"], st["edge_sweeps"], st["moves"], m))
+    for r in res[1:]:
+        assert r[:6] == res[0][:6]
+        assert np.array_equal(r[6], res[0][6])
+
+
+def test_asymmetric_entries_keep_row_sweeps(lvb, table_graphs):
+    """An entry whose mirror entry has another weight: the tables, which the
+    mirror entries update, are not used, and both loops agree."""
+    g = table_graphs["planted"]
+    w = g.w.copy()
+    w[:: 100] *= 2.0
+    h = lvb.Graph(g.rowptr, g.col, w)
+    res = []
+    for kw in ({}, {"sweep_graph": False}):
+        with lvb.Louvain(h, max_sweeps=40, **kw) as e:
+            e.optimise_modularity(1e-7)
+            res.append((e.communities(), e.stats()["sweeps"], e.stats()["moves"]))
+    assert res[0][1:] == res[1][1:]
+    assert np.array_equal(res[0][0], res[1][0])
