@@ -180,9 +180,9 @@ struct lv_handle {
     size_t poff_cap = 0;
     u64 *eown_buf = nullptr;       // per hub, zero between uses (nocc_cap entries)
     int32_t *ovf_buf = nullptr;    // overflow list (nocc_cap entries) then its count
-    bool capturing = false;        // a sweep is being captured into a graph (timers off)
+    bool in_loop = false;          // sweeps of run_sweeps are being launched (timers off)
     MemSet mem;                    // every device buffer of the handle
-    void *loop_d = nullptr;        // device state of the graph sweep loop
+    void *loop_d = nullptr;        // device state of the sweep loop
     NctView nct;                   // neighbour-community tables (late sweeps)
     u64 nct_alloc = 0;             // slots allocated in the pool
 
@@ -205,6 +205,7 @@ struct lv_handle {
     Totals *tot_d = nullptr;       // = &blk_d->tot
     Totals *tot_h = nullptr;
     int32_t *small_h = nullptr;   // pinned scratch for counts
+    volatile int32_t *flag_h = nullptr;
 
     lv_stats st{};
     lv_class_stats cst{};
@@ -294,7 +295,7 @@ struct Timer {
     double bytes = 0, sbytes = 0;
     int64_t verts = 0, edges = 0;
     Timer(lv_handle *hh, int k) : h(hh), kind(k) {
-        if (h->capturing) return;   // graph bodies hold no event nodes
+        if (h->in_loop) return;   // the sweep loop is one timed region
         a = ev_get(h);
         cudaEventRecord(a, h->stream);
     }
@@ -408,6 +409,7 @@ StateView state_of(lv_handle *h) {
 struct PinnedBlock {
     Totals tot;
     int32_t small[128];
+    volatile int32_t flag[2];   // written by sweep_end_flag_kernel: go on, sweep number
 };
 std::mutex g_pinned_mu;
 std::vector<PinnedBlock *> g_pinned_free;
@@ -424,6 +426,7 @@ int pinned_take(lv_handle *h) {
     if (!b) LV_CUDA(h, cudaMallocHost((void **)&b, sizeof(PinnedBlock)));
     h->tot_h = &b->tot;
     h->small_h = b->small;
+    h->flag_h = b->flag;
     return LV_OK;
 }
 
@@ -899,16 +902,22 @@ int sweep_and_q(lv_handle *h, int64_t *moves, double *q) {
 }
 
 // ---------------------------------------------------------------------------
-// device-side sweep control: a level's sweep loop as one CUDA graph
+// device-side sweep control
 // ---------------------------------------------------------------------------
-// The graph is a while-conditional node whose body is one sweep (totals reset,
-// the seven sub-rounds with corrections and commits, the sum of Sigma_tot^2)
-// followed by sweep_end_kernel, which updates sum_i e_{i->C(i)} by the sweep's
-// exact change, forms Q with the host's FP64 operations (each correctly
-// rounded, so the value is the same bit for bit), and sets the loop condition
-// exactly as the host loop decides: continue while the sweep gained at least
-// min_gain, moved something, the sweep cap is not reached and no device
-// check failed.
+// A level's sweeps (totals reset, the seven sub-rounds with corrections and
+// commits, the sum of Sigma_tot^2) end with sweep_end_kernel, which updates
+// sum_i e_{i->C(i)} by the sweep's exact change, forms Q with the host's FP64
+// operations (each correctly rounded, so the value is the same bit for bit),
+// decides exactly as the host loop does whether another sweep follows (the
+// sweep gained at least min_gain, moved something, the sweep cap is not
+// reached and no device check failed) and writes that to pinned memory, where
+// the host, having launched the sweep's kernels ahead, waits for it.  The
+// same loop as one CUDA graph with a while node saved about 20 us per sweep
+// but took 0.3 ms to build, 0.15 ms to launch and 0.3 ms to destroy per level:
+// planted graph of 10,007 vertices 1.67 ms against 1.53, R-MAT-16 level by
+// level 6.6 against 6.3, R-MAT-20 28.6 against 28.4.  Launching the next sweep
+// before the outcome is known (with a stop word that its kernels test) was
+// slower still (LFR graph of 300,007 vertices 6.46 ms against 6.22 in lv_run).
 struct LoopState {
     double q_before;
     double min_gain;
@@ -923,7 +932,7 @@ struct LoopState {
     int32_t switched;
 };
 
-__global__ void sweep_end_kernel(cudaGraphConditionalHandle cond, const SweepBlock *blk, LoopState *ls) {
+__global__ void sweep_end_kernel(const SweepBlock *blk, LoopState *ls, volatile int32_t *flag, int32_t number) {
     const Totals *t = &blk->tot;
     pdl_trigger();
     pdl_wait();
@@ -946,11 +955,13 @@ __global__ void sweep_end_kernel(cudaGraphConditionalHandle cond, const SweepBlo
             more = false;
         }
     }
-    cudaGraphSetConditional(cond, more ? 1u : 0u);
+    flag[0] = more ? 1 : 0;
+    __threadfence_system();
+    flag[1] = number;
 }
 
 // Tables pay off on levels whose sweeps are bound by their rows: below this many
-// entries a table sweep saves less than its graph costs to build (0.3 ms).
+// entries the tables save less than their checks cost.
 constexpr int64_t NCT_MIN_ENTRIES = LV_NCT_MIN_ENTRIES;
 // ... once the movers' rows, which the table updates visit with random
 // accesses, are a small part of the entries: lv_run of R-MAT-24 takes 240 / 236
@@ -1005,84 +1016,45 @@ int nct_begin(lv_handle *h, int *ok) {
     return LV_OK;
 }
 
-// A level's sweep loop as one CUDA graph.
-struct LoopGraph {
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    long long launches = 0;   // per sweep
-    double bytes = 0;
-    ~LoopGraph() {
-        if (exec) cudaGraphExecDestroy(exec);
-        if (graph) cudaGraphDestroy(graph);
-    }
-};
-
-// Builds the loop (with table sweeps when `tables`); false when the driver
-// does not take it.
-bool build_loop_graph(lv_handle *h, LoopGraph &lg, bool tables) {
-    cudaGraphConditionalHandle cond = 0;
-    cudaGraphNode_t node = nullptr;
-    bool ok = cudaGraphCreate(&lg.graph, 0) == cudaSuccess &&
-              cudaGraphConditionalHandleCreate(&cond, lg.graph, 1, cudaGraphCondAssignDefault) == cudaSuccess;
-    cudaGraphNodeParams np = {};
-    if (ok) {
-        np.type = cudaGraphNodeTypeConditional;
-        np.conditional.handle = cond;
-        np.conditional.type = cudaGraphCondTypeWhile;
-        np.conditional.size = 1;
-        ok = cudaGraphAddNode(&node, lg.graph, nullptr, 0, &np) == cudaSuccess;
-    }
-    // the capture's counts are taken back: only sweeps that run are counted
-    const long long launches0 = launches_total();
-    const double bytes0 = h->st.move_bytes;
-    if (ok) {
-        cudaGraph_t body = np.conditional.phGraph_out[0];
-        ok = cudaStreamBeginCaptureToGraph(h->stream, body, nullptr, nullptr, 0,
-                                           cudaStreamCaptureModeRelaxed) == cudaSuccess;
-        if (ok) {
-            h->capturing = true;
-            reset_totals(h);
-            if (tables) LV_BY_WEIGHT(h, enqueue_sweep_tables, h);
-            else LV_BY_WEIGHT(h, enqueue_sweep, h);
-            launch_s2(h->S, h->V, h->tot_d->s2, h->stream);
-            launch_pdl(sweep_end_kernel, 1, 32, 0, h->stream, cond, h->blk_d, (LoopState *)h->loop_d);
-            note_launches(1);
-            h->capturing = false;
-            cudaGraph_t captured = nullptr;
-            ok = cudaStreamEndCapture(h->stream, &captured) == cudaSuccess;
-        }
-    }
-    if (ok) ok = cudaGraphInstantiate(&lg.exec, lg.graph, 0) == cudaSuccess;
-    lg.launches = launches_total() - launches0;
-    lg.bytes = h->st.move_bytes - bytes0;
-    note_launches((int)-lg.launches);
-    h->st.move_bytes = bytes0;
-    if (!ok) {
-        cudaGetLastError();
-        h->capturing = false;
-    }
-    return ok;
-}
-
-// Runs the loop from the state *ls, which is read back.
-int run_loop_graph(lv_handle *h, const LoopGraph &lg, LoopState *ls) {
+// Runs sweeps (from tables when `tables`) from the state *ls until one ends the
+// loop; *ls is read back.
+int run_sweeps(lv_handle *h, bool tables, LoopState *ls) {
     LoopState *ld = (LoopState *)h->loop_d;
     const int32_t sweeps0 = ls->sweeps;
     const u64 moves0 = ls->moves_total;
     LV_CUDA(h, cudaMemcpyAsync(ld, ls, sizeof(*ls), cudaMemcpyHostToDevice, h->stream));
     clear_move_state(h->fb, h->hub_move.view, h->stream);
-    {
-        Timer tm(h, 100);
-        LV_CUDA(h, cudaGraphLaunch(lg.exec, h->stream));
-        tm.stop();
+    h->flag_h[0] = 0;
+    h->flag_h[1] = 0;
+    Timer tm(h, 100);
+    h->in_loop = true;   // one timed region for the loop, none per sweep
+    int rc = LV_OK;
+    for (int32_t number = 1;; ++number) {
+        rc = reset_totals(h);
+        if (rc) break;
+        if (tables) LV_BY_WEIGHT(h, enqueue_sweep_tables, h);
+        else LV_BY_WEIGHT(h, enqueue_sweep, h);
+        launch_s2(h->S, h->V, h->tot_d->s2, h->stream);
+        launch_pdl(sweep_end_kernel, 1, 32, 0, h->stream, h->blk_d, ld, h->flag_h, number);
+        note_launches(1);
+        // the flag arrives some microseconds before a copy or a synchronisation would return
+        for (uint32_t spin = 1; h->flag_h[1] != number; ++spin) {
+            if ((spin & 0xFFF) != 0) continue;
+            const cudaError_t e = cudaStreamQuery(h->stream);
+            if (e == cudaErrorNotReady || h->flag_h[1] == number) continue;
+            rc = fail(h, LV_ERR_CUDA, std::string("sweep: ") + cudaGetErrorString(e));
+            break;
+        }
+        if (rc || !h->flag_h[0]) break;
     }
+    h->in_loop = false;
+    tm.stop();
+    LV_TRY(rc);
     LV_CUDA(h, cudaMemcpyAsync(ls, ld, sizeof(*ls), cudaMemcpyDeviceToHost, h->stream));
     LV_CUDA(h, cudaMemcpyAsync(h->tot_h, h->tot_d, sizeof(Totals), cudaMemcpyDeviceToHost, h->stream));
     LV_TRY(sync(h));
     LV_TRY(check_device_error(h, h->tot_h->err));
     const int32_t ran = ls->sweeps - sweeps0;
-    note_launches((int)(lg.launches * ran));
-    h->st.move_bytes += lg.bytes * ran;
     h->e_own_cur = ls->e_own;
     h->st.sweeps += ran;
     h->st.edge_sweeps += h->E * (int64_t)ran;
@@ -1090,10 +1062,8 @@ int run_loop_graph(lv_handle *h, const LoopGraph &lg, LoopState *ls) {
     return LV_OK;
 }
 
-// Returns LV_OK with *done = 1 when the loop ran as graphs; *done = 0 when
-// none could be built (the caller then runs the host loop).
-int sweep_loop_graph(lv_handle *h, float min_gain, double q_start, int *ch, int *done) {
-    *done = 0;
+// A level's sweep loop with the decisions taken on the device.
+int sweep_loop_device(lv_handle *h, float min_gain, double q_start, int *ch) {
     if (!h->loop_d) {
         LoopState *p = nullptr;
         LV_TRY(dalloc(h, &p, 1));
@@ -1107,18 +1077,15 @@ int sweep_loop_graph(lv_handle *h, float min_gain, double q_start, int *ch, int 
     ls.q_last = q_start;
     ls.max_sweeps = h->opts.max_sweeps;
     if (h->E >= NCT_MIN_ENTRIES) ls.switch_units = (u64)(NCT_SWITCH * (double)h->E / 32.0);
-    LoopGraph rows, tables;
-    if (!build_loop_graph(h, rows, false)) return LV_OK;
-    LV_TRY(run_loop_graph(h, rows, &ls));
+    LV_TRY(run_sweeps(h, false, &ls));
     if (ls.switched) {
         ls.switched = 0;
         ls.switch_units = 0;
         int ok = 0;
         LV_TRY(nct_begin(h, &ok));
-        LV_TRY(run_loop_graph(h, ok && build_loop_graph(h, tables, true) ? tables : rows, &ls));
+        LV_TRY(run_sweeps(h, ok != 0, &ls));
     }
     *ch = ls.changed;
-    *done = 1;
     return LV_OK;
 }
 
@@ -1345,15 +1312,13 @@ int optimise_level(lv_handle *h, float min_gain, int32_t *changed) {
     double q_before = 0, q_after = 0;
     LV_TRY(modularity(h, &q_before));
     if (h->opts.sweep_graph && !h->opts.profile && !h->opts.verify && !h->opts.trace) {
-        int ch = 0, done = 0;
-        LV_TRY(sweep_loop_graph(h, min_gain, q_before, &ch, &done));
-        if (done) {
-            launch_compose_map(h->orig2comm, h->comm, h->V0, h->stream);
-            h->st.levels += 1;
-            h->st.final_vertices = h->V;
-            if (changed) *changed = ch;
-            return sync(h);
-        }
+        int ch = 0;
+        LV_TRY(sweep_loop_device(h, min_gain, q_before, &ch));
+        launch_compose_map(h->orig2comm, h->comm, h->V0, h->stream);
+        h->st.levels += 1;
+        h->st.final_vertices = h->V;
+        if (changed) *changed = ch;
+        return sync(h);
     }
     double gain = (double)min_gain;
     int ch = 0, sweeps = 0;
@@ -1496,8 +1461,8 @@ int aggregate(lv_handle *h) {
 // ---------------------------------------------------------------------------
 // small levels: the rest of the level loop in one launch
 // ---------------------------------------------------------------------------
-// A level this small spends its time on launches, graph building and host
-// round trips (0.3 to 0.6 ms per level and 0.1 ms per sweep), not on its rows.
+// A level this small spends its time on launches and host round trips (0.3 to
+// 0.6 ms per level and 0.1 ms per sweep), not on its rows.
 // lv_run of planted graphs of 500 / 2000 / 3500 vertices (6 / 27 / 58 thousand
 // entries) takes 0.87 / 0.81 / 0.63 ms in one launch; 2000 vertices took 1.97
 // ms level by level, and at 10,007 vertices (171 thousand entries) the two
@@ -1592,7 +1557,7 @@ int to_level0(lv_handle *h) {
     h->e_own_valid = false;
     launch_iota_i32(h->orig2comm, h->V0, h->stream);
     h->setup_due = SETUP_ALL;
-    // a graph that lv_run hands to one launch needs no class lists
+    // a level that lv_run hands to one launch needs no class lists
     if (team_fits(h)) return LV_OK;
     return ensure_setup(h);
 }

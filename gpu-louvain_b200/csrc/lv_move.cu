@@ -743,6 +743,8 @@ __global__ void __launch_bounds__(THREADS) move_fallback_kernel(GraphView<WT> g,
                                                                 Fallback fb, HubGlobal hg,
                                                                 uint8_t *hint, int32_t hint_set, u64 *dE) {
     constexpr int OCC_CAP = CAP / 2;
+    const int32_t count = min(*fb.count, fb.cap);
+    if ((int32_t)blockIdx.x >= count) return;   // at most one CTA per item
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64 *vals = reinterpret_cast<u64 *>(smem_raw);
     int32_t *keys = reinterpret_cast<int32_t *>(vals + CAP);
@@ -751,7 +753,6 @@ __global__ void __launch_bounds__(THREADS) move_fallback_kernel(GraphView<WT> g,
     for (int s = threadIdx.x; s < CAP; s += THREADS) { keys[s] = -1; vals[s] = 0; }
     if (threadIdx.x == 0) nocc = 0;
     __syncthreads();
-    const int32_t count = min(*fb.count, fb.cap);
     u64 delta_acc = 0;
     for (;;) {
         if (threadIdx.x == 0) item_sh = atomicAdd(fb.next, 1);
@@ -897,6 +898,8 @@ __global__ void __launch_bounds__(THREADS) move_rowq_narrow_kernel(GraphView<WT>
                                                                    uint8_t *hint, int32_t hint_set, u64 *dE) {
     constexpr int OCC_CAP = CAP / 2;
     static_assert(OCC_CAP <= PIECE_MAX_ADDS, "rows of the queue fit the piece counters");
+    const int32_t count = min(*fb.count, fb.cap);
+    if ((int32_t)blockIdx.x >= count) return;   // at most one CTA per item
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PieceTable t;
     t.lo = reinterpret_cast<uint32_t *>(smem_raw);
@@ -907,7 +910,6 @@ __global__ void __launch_bounds__(THREADS) move_rowq_narrow_kernel(GraphView<WT>
     for (int s = threadIdx.x; s < CAP; s += THREADS) { t.keys[s] = -1; t.lo[s] = 0; t.hi[s] = 0; }
     if (threadIdx.x == 0) nocc = 0;
     __syncthreads();
-    const int32_t count = min(*fb.count, fb.cap);
     u64 delta_acc = 0;
     for (;;) {
         if (threadIdx.x == 0) item_sh = atomicAdd(fb.next, 1);

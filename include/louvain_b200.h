@@ -49,11 +49,12 @@ typedef struct lv_opts {
                               maintained modularity against a full pass    */
     int32_t trace;         /* 1: per-level and per-sweep lines on stderr
                               (class sizes, moves, modularity, device ms)  */
-    int32_t sweep_graph;   /* 1 (default): a level's sweep loop runs as one
-                              CUDA graph whose while-node condition is set
-                              on the device after each sweep (no host round
-                              trip per sweep); used when profile, verify and
-                              trace are 0.  0: one host round trip per sweep.
+    int32_t sweep_graph;   /* 1 (default): each sweep's outcome (modularity,
+                              whether another sweep follows) is formed on the
+                              device and the host only launches sweeps;
+                              lv_run finishes small graphs in one launch; used
+                              when profile, verify and trace are 0.  0: the
+                              host reads every sweep's totals and decides.
                               Results are identical.                      */
     int32_t active_set;    /* 1: learned active-set sweeps on levels of at
                               least 65536 vertices (needs a model,
