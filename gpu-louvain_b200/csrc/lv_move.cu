@@ -7,10 +7,12 @@
 //
 // Work mapping (one kernel family per degree class, all classes of one
 // update bucket are decided before that bucket is committed):
-//   - classes B0..B4: a group of G lanes (4/8/16/32) per vertex, the group's
-//     neighbour-community table in shared memory;
-//   - classes B5, H1, H2: one CTA per vertex (persistent grid-stride), table
-//     in shared memory sized to the vertex's degree;
+//   - classes B0..B3 (B4 where it has few rows): a group of G lanes
+//     (4/8/16/32) per vertex, the group's neighbour-community table in shared
+//     memory;
+//   - classes B4..H2: a warp per vertex with a table of fixed size; rows that
+//     do not fit, and all rows of a bucket that has few, get a CTA each, the
+//     table in shared memory sized to the row's degree;
 //   - class HG: many CTAs per hub, table in global memory (insert kernel over
 //     edge chunks, evaluate kernel over slot chunks, final per-hub reduce).
 #include "lv_internal.h"
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(256) move_group_kernel(GraphView<WT> g, StateV
         record_features(st, v, m, b);
     }
     block_add_total<256>(delta, dE);
-    block_note_movers<256>(st, mover, 1u);
+    if constexpr (CAP <= 64) block_note_movers<256>(st, mover, 1u);   // rows of at most 32 entries
 }
 
 // move_group_kernel for weights below 2^32: the group's table keeps its sums
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(256) move_group_narrow_kernel(GraphView<WT> g,
         record_features(st, v, m, b);
     }
     block_add_total<256>(delta, dE);
-    block_note_movers<256>(st, mover, 1u);
+    if constexpr (CAP <= 64) block_note_movers<256>(st, mover, 1u);   // rows of at most 32 entries
 }
 
 // CTA-wide reduction of a Best; the result is valid in thread 0.
@@ -741,9 +743,10 @@ __global__ void __launch_bounds__(256) move_warp_narrow_kernel(GraphView<WT> g, 
 template <typename WT, int THREADS, int CAP, bool PART>
 __global__ void __launch_bounds__(THREADS) move_fallback_kernel(GraphView<WT> g, StateView st,
                                                                 Fallback fb, HubGlobal hg,
-                                                                uint8_t *hint, int32_t hint_set, u64 *dE) {
+                                                                uint8_t *hint, int32_t hint_set, u64 *dE,
+                                                                Fallback large) {
     constexpr int OCC_CAP = CAP / 2;
-    const int32_t count = min(*fb.count, fb.cap);
+    const int32_t count = fb.count ? min(*fb.count, fb.cap) : fb.cap;   // no count: v is a list of cap vertices
     if ((int32_t)blockIdx.x >= count) return;   // at most one CTA per item
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64 *vals = reinterpret_cast<u64 *>(smem_raw);
@@ -767,6 +770,11 @@ __global__ void __launch_bounds__(THREADS) move_fallback_kernel(GraphView<WT> g,
         if (src < 0) {
             // the vertex's row
             const int32_t r0 = g.rowptr[v], r1 = g.rowend[v];
+            if (!PART && r1 - r0 > OCC_CAP) {   // only in a direct list
+                if (threadIdx.x == 0) enqueue_large(large, v, r1 - r0, st.err);
+                __syncthreads();
+                continue;
+            }
             int lg = P > 1 ? ilog2_c(CAP) : ceil_log2_i(2 * (int64_t)(r1 - r0));
             lg = lg < 3 ? 3 : lg;
             if (!PART) {
@@ -895,10 +903,11 @@ __global__ void __launch_bounds__(THREADS) move_fallback_kernel(GraphView<WT> g,
 // claimed-slot list.
 template <typename WT, int THREADS, int CAP>
 __global__ void __launch_bounds__(THREADS) move_rowq_narrow_kernel(GraphView<WT> g, StateView st, Fallback fb,
-                                                                   uint8_t *hint, int32_t hint_set, u64 *dE) {
+                                                                   uint8_t *hint, int32_t hint_set, u64 *dE,
+                                                                   Fallback large) {
     constexpr int OCC_CAP = CAP / 2;
     static_assert(OCC_CAP <= PIECE_MAX_ADDS, "rows of the queue fit the piece counters");
-    const int32_t count = min(*fb.count, fb.cap);
+    const int32_t count = fb.count ? min(*fb.count, fb.cap) : fb.cap;   // no count: v is a list of cap vertices
     if ((int32_t)blockIdx.x >= count) return;   // at most one CTA per item
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PieceTable t;
@@ -919,6 +928,11 @@ __global__ void __launch_bounds__(THREADS) move_rowq_narrow_kernel(GraphView<WT>
         const int32_t v = fb.v[item];
         const int32_t own = __ldg(st.comm + v);
         const int32_t r0 = g.rowptr[v], r1 = g.rowend[v];
+        if (r1 - r0 > OCC_CAP) {   // only in a direct list
+            if (threadIdx.x == 0) enqueue_large(large, v, r1 - r0, st.err);
+            __syncthreads();
+            continue;
+        }
         int lg = ceil_log2_i(2 * (int64_t)(r1 - r0));
         lg = lg < 3 ? 3 : lg;
         u64 e_own = 0;
@@ -1657,13 +1671,19 @@ static void set_row_queue_attrs(DeviceInfo &di) {
 }
 
 template <typename WT, int B>
-static void launch_row_queue(const GraphView<WT> &g, const StateView &st, const FallbackSet &fs,
-                             const DeviceInfo &di, u64 *dE, cudaStream_t s, bool narrow) {
+static void launch_row_queue(const GraphView<WT> &g, const StateView &st, FallbackSet fs,
+                             const DeviceInfo &di, u64 *dE, cudaStream_t s, bool narrow,
+                             const int32_t *list = nullptr, int32_t n = 0) {
+    if (list) {   // the rows of list[0 .. n) instead of the queue's
+        fs.q[B].v = const_cast<int32_t *>(list);
+        fs.q[B].cap = n;
+        fs.q[B].count = nullptr;
+    }
     constexpr int T = FBQ_THREADS(B), CAP = 2 * FBQ_MAXDEG(B), SM = FBQ_SMEM(B);
     if constexpr (sizeof(WT) == 4) {
         // bulk copies need 16-byte aligned arrays
         const bool aligned = (((uintptr_t)g.col | (uintptr_t)g.w) & 15u) == 0;
-        if (LV_ROWQ_STAGE && narrow && aligned) {
+        if (LV_ROWQ_STAGE && narrow && aligned && !list) {
             move_rowq_staged_kernel<WT, T, CAP><<<di.sms * di.occ_fbq_staged[B], T, RowqStage<T, CAP>::BYTES, s>>>(
                 g, st, fs.q[B], fs.hint, fs.hint_set, dE);
             note_launches(1);
@@ -1672,10 +1692,12 @@ static void launch_row_queue(const GraphView<WT> &g, const StateView &st, const 
     }
     if (narrow)
         move_rowq_narrow_kernel<WT, T, CAP><<<di.sms * di.occ_fbq_narrow[B], T, SM, s>>>(g, st, fs.q[B], fs.hint,
-                                                                                        fs.hint_set, dE);
+                                                                                        fs.hint_set, dE,
+                                                                                        fs.q[NFBQ]);
     else
         move_fallback_kernel<WT, T, CAP, false><<<di.sms * di.occ_fbq[B], T, SM, s>>>(g, st, fs.q[B], HubGlobal(),
-                                                                                    fs.hint, fs.hint_set, dE);
+                                                                                    fs.hint, fs.hint_set, dE,
+                                                                                    fs.q[NFBQ]);
     note_launches(1);
 }
 
@@ -1783,7 +1805,7 @@ template <typename WT>
 static void launch_fallback_large(const GraphView<WT> &g, const StateView &st, const HubGlobal &hg,
                                   const FallbackSet &fs, const DeviceInfo &di, u64 *dE, cudaStream_t s) {
     move_fallback_kernel<WT, FB_THREADS, FB_CAP, true><<<di.sms, FB_THREADS, FB_SMEM, s>>>(
-        g, st, fs.q[NFBQ], hg, fs.hint, fs.hint_set, dE);
+        g, st, fs.q[NFBQ], hg, fs.hint, fs.hint_set, dE, Fallback());
     note_launches(1);
 }
 
@@ -1825,6 +1847,14 @@ void launch_move_giants(const GraphView<WT> &g, const StateView &st, const HubGl
     launch_fallback_large<WT>(g, st, hg, fs, di, dE, s);
 }
 
+// Rows per SM up to which a bucket counts as few (launch_move_wide).  Whole
+// runs on one B200, without the rule / with it / with limits four times as
+// high, ms: LFR graph of 300,007 vertices 6.17 / 5.22 / 5.2, of 1,000,003
+// 14.78 / 14.78 / 15.6, R-MAT scale 14 4.74 / 3.47 / 3.5, scale 16 5.90 /
+// 5.08 / 5.1, scale 18 15.0 / 14.8 / 16.3, scale 20 27.3 / 27.2 / 27.3:
+// where every warp has several rows anyway, the warp per row is the cheaper.
+constexpr int32_t SMALL_B4_PER_SM = 192, SMALL_B5_PER_SM = 56, SMALL_B6_PER_SM = 10;
+
 void clear_move_state(const FallbackSet &fs, const HubGlobal &hg, cudaStream_t s) {
     cudaMemsetAsync(fs.q[NFBQ].done, 0, sizeof(int32_t) * (size_t)fs.q[NFBQ].cap, s);
     if (hg.nhubs > 0) {
@@ -1838,6 +1868,30 @@ void launch_move_wide(const GraphView<WT> &g, const StateView &st, const int32_t
                       const FallbackSet &fs, const DeviceInfo &di, u64 *dE, cudaStream_t s,
                       int32_t max_degree, bool narrow, bool large_later) {
     if (n <= 0) return;
+    if (!st.wrow) {
+        // Few rows: a warp per row leaves the GPU to the longest rows' latency
+        // (LFR graph of 300,007 vertices, 655 rows of 320 to 2000 entries: 67
+        // us).  So rows of up to 84 entries go to groups of 32 lanes with a
+        // table of 256 slots (no queue), longer ones to a CTA each.
+        if (max_degree <= 84 && n <= di.sms * SMALL_B4_PER_SM) {
+            if (narrow)
+                launch_pdl((move_group_narrow_kernel<32, 256, WT>), nblocks(n, 8), 256, 0, s, g, st, list, n, dE,
+                           fs.q[NFBQ]);
+            else
+                launch_pdl((move_group_kernel<32, 256, WT>), nblocks(n, 8), 256, 0, s, g, st, list, n, dE);
+            note_launches(1);
+            return;
+        }
+        if (max_degree > 84 && max_degree <= FBQ_MAXDEG(0) && n <= di.sms * SMALL_B5_PER_SM) {
+            launch_row_queue<WT, 0>(g, st, fs, di, dE, s, narrow, list, n);
+            return;
+        }
+        if (max_degree > FBQ_MAXDEG(0) && n <= di.sms * SMALL_B6_PER_SM) {
+            launch_row_queue<WT, NFBQ - 1>(g, st, fs, di, dE, s, narrow, list, n);
+            if (!large_later) launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
+            return;
+        }
+    }
     if (narrow) {
         const unsigned grid = (unsigned)imin64((n + 7) / 8, (int64_t)di.sms * di.occ_warp_narrow);
         move_warp_narrow_kernel<WT><<<grid, 256, WARP_NSMEM, s>>>(g, st, list, n, fs, dE);

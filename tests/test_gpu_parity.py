@@ -496,3 +496,45 @@ def test_small_graph_runs_match_oracle(lvb, orc, name):
         assert np.array_equal(e.communities(), np.arange(g.V))
         assert int(e.level_classes()[0].sum()) == int((np.diff(g.rowptr) > 0).sum())
     o.close()
+
+
+def _rows_of(lvb, degrees, unit, leaves=200003):
+    """One vertex per listed degree, joined to that many of `leaves` vertices
+    (a prime number, so that a stride over them meets each once)."""
+    rng = np.random.default_rng(len(degrees))
+    n = len(degrees)
+    u = np.repeat(np.arange(n, dtype=np.int64), degrees)
+    j = np.arange(len(u)) - np.repeat(np.cumsum(degrees) - degrees, degrees)
+    start, step = rng.integers(0, leaves, n), rng.integers(1, 9, n)
+    v = n + (start[u] + j * step[u]) % leaves
+    w = np.ones(len(u)) if unit else 0.25 - np.log((u * 7919 + v * 104729) % 65521 / 65521.0 + 2.0 ** -32)
+    rows, cols = np.concatenate([u, v]), np.concatenate([v, u])
+    o = np.lexsort((cols, rows))
+    rp = np.zeros(n + leaves + 1, np.int32)
+    np.cumsum(np.bincount(rows, minlength=n + leaves), out=rp[1:])
+    return lvb.Graph(rp, cols[o].astype(np.int32), np.concatenate([w, w])[o].astype(np.float32))
+
+
+@pytest.mark.parametrize("unit", [True, False], ids=["unit", "fine"])
+@pytest.mark.parametrize("over", [0, 1])
+@pytest.mark.parametrize("lo,hi,per_sm", [(33, 84, 192), (85, 319, 56), (320, 600, 10)])
+def test_buckets_of_few_rows_match_oracle(lvb, orc, lo, hi, per_sm, over, unit):
+    """Sweeps with as many rows in a bucket as still get a mapping of their own,
+    and with one more, at the bounds of each table (rows of more than 4096
+    entries leave the list of the last bucket, one is beyond the giant degree)."""
+    import torch
+
+    n = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + over
+    deg = np.random.default_rng(n).integers(lo, hi + 1, n)
+    deg[:2] = lo, hi
+    if hi == 600:
+        deg[2:9] = 512, 513, 4095, 4096, 4097, 9000, 20000
+        deg = np.append(deg, 70001)
+    g = _rows_of(lvb, deg, unit)
+    assert int((np.diff(g.rowptr) > 32).sum()) == len(deg)
+    o = orc.Oracle(g.rowptr, g.col, g.w)
+    with lvb.Louvain(g) as e:
+        for _ in range(3):
+            assert e.sweep() == o.sweep()
+            assert np.array_equal(e.communities(), o.communities())
+    o.close()
