@@ -735,13 +735,47 @@ __global__ void __launch_bounds__(256) move_warp_narrow_kernel(GraphView<WT> g, 
     if (lane == 0 && delta_acc) atomicAdd(dE, delta_acc);
 }
 
+// The queues' CTAs are bound by the latency of one row's steps (issue slots
+// 36 % busy): item -> vertex -> row bounds -> columns -> communities -> sums ->
+// reduction.  An item is therefore fetched by thread 0 in three steps that lie
+// between the phases of the item before it, each load being used only a phase
+// later, and the registers are held to what 48 warps per SM leave (40 and 32
+// warps: 0.3 and 0.7 ms more, 56 and 64: 1.3 and 2.7 ms more; the largest
+// tables leave room for one CTA of 1024 threads, and two of 512 measured the
+// same).  Degree > 319 class, before and after, ms per run: R-MAT scale 21 with
+// fine weights 18.1 -> 16.9, scale 20 9.66 -> 9.1, scale 24 89.9 -> 87.0.
+__host__ __device__ constexpr int queue_ctas(int threads) { return threads >= 1024 ? 1 : 1536 / threads; }
+
+struct QueueItem {
+    int32_t item, v, r0, r1;
+    int32_t p, P, first, src;   // of the large queue
+};
+__device__ __forceinline__ void take_item(const Fallback &fb, QueueItem &q) { q.item = atomicAdd(fb.next, 1); }
+template <bool PART>
+__device__ __forceinline__ void load_item(const Fallback &fb, int32_t count, QueueItem &q) {
+    if (q.item >= count) return;
+    q.v = fb.v[q.item];
+    if (PART) {
+        q.p = fb.p[q.item];
+        q.P = fb.P[q.item];
+        q.first = fb.first[q.item];
+        q.src = fb.src[q.item];
+    }
+}
+template <typename WT>
+__device__ __forceinline__ void load_item_row(const GraphView<WT> &g, int32_t count, QueueItem &q) {
+    if (q.item >= count) return;
+    q.r0 = g.rowptr[q.v];
+    q.r1 = g.rowend[q.v];
+}
+
 // Fallback CTAs.  PART = false: items are whole rows of degree <= CAP / 2
 // (small and medium queues).  PART = true: key-space partitions of a row or
 // of a giant's staged pairs (large queue).  The occupied list holds CAP / 2
 // slots; a partition with more distinct communities than that reports
 // DEVERR_HASH_FULL.
 template <typename WT, int THREADS, int CAP, bool PART>
-__global__ void __launch_bounds__(THREADS) move_fallback_kernel(GraphView<WT> g, StateView st,
+__global__ void __launch_bounds__(THREADS, queue_ctas(THREADS)) move_fallback_kernel(GraphView<WT> g, StateView st,
                                                                 Fallback fb, HubGlobal hg,
                                                                 uint8_t *hint, int32_t hint_set, u64 *dE,
                                                                 Fallback large) {
@@ -752,26 +786,39 @@ __global__ void __launch_bounds__(THREADS) move_fallback_kernel(GraphView<WT> g,
     u64 *vals = reinterpret_cast<u64 *>(smem_raw);
     int32_t *keys = reinterpret_cast<int32_t *>(vals + CAP);
     int32_t *occ = keys + CAP;
-    __shared__ int32_t nocc, item_sh;
+    __shared__ int32_t nocc;
+    __shared__ QueueItem cur;
     for (int s = threadIdx.x; s < CAP; s += THREADS) { keys[s] = -1; vals[s] = 0; }
-    if (threadIdx.x == 0) nocc = 0;
+    QueueItem nx;   // thread 0's: the next item
+    if (threadIdx.x == 0) {
+        nocc = 0;
+        take_item(fb, nx);
+        load_item<PART>(fb, count, nx);
+        load_item_row(g, count, nx);
+        cur = nx;
+    }
     __syncthreads();
     u64 delta_acc = 0;
     for (;;) {
-        if (threadIdx.x == 0) item_sh = atomicAdd(fb.next, 1);
-        __syncthreads();
-        const int32_t item = item_sh;
+        const int32_t item = cur.item;
         if (item >= count) break;
-        const int32_t v = fb.v[item];
+        const int32_t v = cur.v;
+        const int32_t r0 = cur.r0, r1 = cur.r1;
         int32_t p = 0, P = 1, first = item, src = -1;
-        if (PART) { p = fb.p[item]; P = fb.P[item]; first = fb.first[item]; src = fb.src[item]; }
+        if (PART) { p = cur.p; P = cur.P; first = cur.first; src = cur.src; }
+        if (threadIdx.x == 0) take_item(fb, nx);
         const int32_t own = __ldg(st.comm + v);
         u64 e_own = 0;
         if (src < 0) {
             // the vertex's row
-            const int32_t r0 = g.rowptr[v], r1 = g.rowend[v];
             if (!PART && r1 - r0 > OCC_CAP) {   // only in a direct list
-                if (threadIdx.x == 0) enqueue_large(large, v, r1 - r0, st.err);
+                __syncthreads();   // cur was read
+                if (threadIdx.x == 0) {
+                    enqueue_large(large, v, r1 - r0, st.err);
+                    load_item<PART>(fb, count, nx);
+                    load_item_row(g, count, nx);
+                    cur = nx;
+                }
                 __syncthreads();
                 continue;
             }
@@ -841,14 +888,17 @@ __global__ void __launch_bounds__(THREADS) move_fallback_kernel(GraphView<WT> g,
             if (p == 0 && threadIdx.x == 0) e_own = hg.eown[src];
         }
         __syncthreads();
+        if (threadIdx.x == 0) load_item<PART>(fb, count, nx);
         const int32_t nd = min(nocc, OCC_CAP);
         const MoveCtx m = move_ctx(own, __ldg(st.size + own) == 1, st.T, __ldg(st.k + v), __ldg(st.S + own));
         Best b = best_init(own);
         b.eo = e_own;
         eval_slots<1, true, true>(keys, vals, occ, nd, threadIdx.x, THREADS, m, st.S, st.size, b);
+        if (threadIdx.x == 0) load_item_row(g, count, nx);
         cta_reduce_best<THREADS>(m, b);
         if (threadIdx.x == 0) {
             nocc = 0;
+            cur = nx;
             bool decide = P == 1;
             int32_t distinct = nd;
             Best t = b;
@@ -902,7 +952,7 @@ __global__ void __launch_bounds__(THREADS) move_fallback_kernel(GraphView<WT> g,
 // <= CAP / 2 in a piece table (fire-and-forget adds), evaluated over the
 // claimed-slot list.
 template <typename WT, int THREADS, int CAP>
-__global__ void __launch_bounds__(THREADS) move_rowq_narrow_kernel(GraphView<WT> g, StateView st, Fallback fb,
+__global__ void __launch_bounds__(THREADS, queue_ctas(THREADS)) move_rowq_narrow_kernel(GraphView<WT> g, StateView st, Fallback fb,
                                                                    uint8_t *hint, int32_t hint_set, u64 *dE,
                                                                    Fallback large) {
     constexpr int OCC_CAP = CAP / 2;
@@ -915,21 +965,33 @@ __global__ void __launch_bounds__(THREADS) move_rowq_narrow_kernel(GraphView<WT>
     t.hi = t.lo + CAP;
     t.keys = reinterpret_cast<int32_t *>(t.hi + CAP);
     int32_t *occ = t.keys + CAP;
-    __shared__ int32_t nocc, item_sh;
+    __shared__ int32_t nocc;
+    __shared__ QueueItem cur;
     for (int s = threadIdx.x; s < CAP; s += THREADS) { t.keys[s] = -1; t.lo[s] = 0; t.hi[s] = 0; }
-    if (threadIdx.x == 0) nocc = 0;
+    QueueItem nx;   // thread 0's: the next item
+    if (threadIdx.x == 0) {
+        nocc = 0;
+        take_item(fb, nx);
+        load_item<false>(fb, count, nx);
+        load_item_row(g, count, nx);
+        cur = nx;
+    }
     __syncthreads();
     u64 delta_acc = 0;
     for (;;) {
-        if (threadIdx.x == 0) item_sh = atomicAdd(fb.next, 1);
-        __syncthreads();
-        const int32_t item = item_sh;
-        if (item >= count) break;
-        const int32_t v = fb.v[item];
+        if (cur.item >= count) break;
+        const int32_t v = cur.v;
+        const int32_t r0 = cur.r0, r1 = cur.r1;
+        if (threadIdx.x == 0) take_item(fb, nx);
         const int32_t own = __ldg(st.comm + v);
-        const int32_t r0 = g.rowptr[v], r1 = g.rowend[v];
         if (r1 - r0 > OCC_CAP) {   // only in a direct list
-            if (threadIdx.x == 0) enqueue_large(large, v, r1 - r0, st.err);
+            __syncthreads();   // cur was read
+            if (threadIdx.x == 0) {
+                enqueue_large(large, v, r1 - r0, st.err);
+                load_item<false>(fb, count, nx);
+                load_item_row(g, count, nx);
+                cur = nx;
+            }
             __syncthreads();
             continue;
         }
@@ -939,6 +1001,7 @@ __global__ void __launch_bounds__(THREADS) move_rowq_narrow_kernel(GraphView<WT>
         insert_row_piece<LV_U_FB, true>(g, st.comm, v, own, r0, r1, threadIdx.x, THREADS, t, lg, st.err, occ,
                                         &nocc, OCC_CAP, e_own, (LV_DEDUP && st.dedup != 0));
         __syncthreads();
+        if (threadIdx.x == 0) load_item<false>(fb, count, nx);
         const int32_t nd = min(nocc, OCC_CAP);
         const MoveCtx m = move_ctx(own, __ldg(st.size + own) == 1, st.T, __ldg(st.k + v), __ldg(st.S + own));
         Best b = best_init(own);
@@ -955,9 +1018,11 @@ __global__ void __launch_bounds__(THREADS) move_rowq_narrow_kernel(GraphView<WT>
             const int32_t szc = (cand && guard_needs_size(m, c)) ? __ldg(st.size + c) : 0;
             eval_loaded(c, ec, Sc, szc, m, b);
         }
+        if (threadIdx.x == 0) load_item_row(g, count, nx);
         cta_reduce_best<THREADS>(m, b);
         if (threadIdx.x == 0) {
             nocc = 0;
+            cur = nx;
             u64 delta = 0;
             st.newc[v] = move_decision(m, b, &delta);
             record_features(st, v, m, b);
