@@ -330,10 +330,13 @@ struct StateView {
     const uint8_t *wrow;   // rows with a weight of 2^32 or more (nullptr: none); such a
                            // vertex is decided by the large fallback queue (64-bit sums)
     // the sub-round's movers: mv_cnt holds their count (low half) and their row
-    // units of 32 entries (high half), mv_off[i] the units before mover i
+    // units of 32 entries (high half); mv_list has four arrays of mv_stride
+    // words: the movers, the units before each, and, by vertex, the community
+    // a mover leaves and the number of the last sub-round that moved it
     u64 *mv_cnt;
     int32_t *mv_list;
-    uint32_t *mv_off;
+    int32_t mv_stride;
+    uint32_t mv_round;     // this sub-round's number, never used twice
     // table sweeps: NctView::lg and the number of vertices without tables (the
     // giant kernels take only giants without tables)
     const uint8_t *tlg;
@@ -342,6 +345,13 @@ struct StateView {
                            // equal keys before their shared atomics (key_peers)
 };
 
+__device__ __forceinline__ uint32_t *mover_offsets(const StateView &st) {
+    return reinterpret_cast<uint32_t *>(st.mv_list + st.mv_stride);
+}
+__device__ __forceinline__ int32_t *mover_left(const StateView &st) { return st.mv_list + 2 * (size_t)st.mv_stride; }
+__device__ __forceinline__ uint32_t *mover_round(const StateView &st) {
+    return reinterpret_cast<uint32_t *>(st.mv_list + 3 * (size_t)st.mv_stride);
+}
 __device__ __forceinline__ uint32_t mover_units(int32_t d) { return (uint32_t)(d + 31) >> 5; }
 
 // Exact 64-bit add to a table value.  In shared memory a 64-bit atomicAdd

@@ -154,8 +154,8 @@ struct lv_handle {
     int cur_buf = -1;
 
     int32_t *comm = nullptr, *newc = nullptr, *size = nullptr, *orig2comm = nullptr;
-    int32_t *mv_list = nullptr;    // movers of a sub-round
-    uint32_t *mv_off = nullptr;
+    int32_t *mv_list = nullptr;    // movers of a sub-round (StateView::mv_list)
+    uint32_t mv_round = 0;         // sub-rounds launched so far
     u64 *k = nullptr, *S = nullptr;
     int32_t *list = nullptr;
     int32_t *cls_scratch = nullptr;   // class counts, cursors, then V0 entries of scratch
@@ -395,8 +395,17 @@ bool narrow_weights(const lv_handle *h) {
 StateView state_of(lv_handle *h) {
     return StateView{h->comm, h->newc, h->size, h->k, h->S, h->T, &h->tot_d->err, h->feat,
                      (LV_NARROW_ESCAPES == 1 && h->cur_w32 && h->wrows_any) ? h->wrow : nullptr,
-                     h->blk_d->movers, h->mv_list, h->mv_off, nullptr, nullptr,
+                     h->blk_d->movers, h->mv_list, h->V0 + 1, 0, nullptr, nullptr,
                      (LV_DEDUP == 2 || (LV_DEDUP == 1 && h->level > 0)) ? 1 : 0};
+}
+
+// Numbers a sub-round.  When the numbers run out, the old ones are forgotten.
+void next_round(lv_handle *h, StateView &st) {
+    if (++h->mv_round == 0) {
+        cudaMemsetAsync(h->mv_list + 3 * ((size_t)h->V0 + 1), 0, sizeof(int32_t) * ((size_t)h->V0 + 1), h->stream);
+        h->mv_round = 1;
+    }
+    st.mv_round = h->mv_round;
 }
 
 // ---------------------------------------------------------------------------
@@ -724,6 +733,7 @@ void enqueue_sweep(lv_handle *h) {
         const int32_t hg0 = (b == 6) ? h->cls_off[CLS_HG] : hi;   // bucket 6: giants after
         const FallbackSet fs = queues_on(h, b >= 4 ? b - 4 : 3);
         st.mv_cnt = h->blk_d->movers + b;
+        next_round(h, st);
         int64_t edges = 0;
         for (int c = c0; c < c1; ++c)
             if (c != CLS_HG) edges += h->cls_edges[c];
@@ -787,6 +797,7 @@ void enqueue_sweep_tables(lv_handle *h) {
         if (hi == lo) continue;
         const FallbackSet fs = queues_on(h, b >= 4 ? b - 4 : 3);
         st.mv_cnt = h->blk_d->movers + b;
+        next_round(h, st);
         if (b < 4) {
             launch_move_class<WT>(b, g, st, h->list + lo, hi - lo, h->di, dE, h->stream, narrow_weights<WT>(h), fs);
         } else {
@@ -1140,6 +1151,7 @@ void enqueue_sweep_active(lv_handle *h, const int32_t *cnt) {
         for (int c = c0; c < c1; ++c) any += cnt[c];
         if (!any) continue;
         st.mv_cnt = h->blk_d->movers + b;
+        next_round(h, st);
         if (b < 4) {
             launch_move_class<WT>(b, g, st, h->alist + h->cls_off[b], cnt[b], h->di, dE, h->stream,
                                   narrow_weights<WT>(h), queues_on(h, 3));
@@ -1572,8 +1584,9 @@ int ensure_move(lv_handle *h) {
     if (h->move_ready) return LV_OK;
     const size_t V = (size_t)h->V0;
     LV_TRY(dalloc(h, &h->list, V + 1));
-    LV_TRY(dalloc(h, &h->mv_list, V + 1));
-    LV_TRY(dalloc(h, &h->mv_off, V + 1));
+    LV_TRY(dalloc(h, &h->mv_list, 4 * (V + 1)));
+    LV_CUDA(h, cudaMemsetAsync(h->mv_list + 3 * (V + 1), 0, sizeof(int32_t) * (V + 1), h->stream));
+    h->mv_round = 0;
     LV_TRY(dalloc(h, &h->sort_buf, 3 * V + 16));
     h->sort_temp_bytes = sort_by_degree_temp_bytes((int32_t)V, HG_MIN_DEG_HI) + 256;
     {

@@ -68,7 +68,9 @@ __device__ __forceinline__ void block_note_movers(const StateView &st, int32_t v
     if (v >= 0) {
         const u64 at = at0 + pre + inc - own;
         st.mv_list[(uint32_t)at] = v;
-        st.mv_off[(uint32_t)at] = (uint32_t)(at >> 32);
+        mover_offsets(st)[(uint32_t)at] = (uint32_t)(at >> 32);
+        mover_left(st)[v] = st.comm[v];
+        mover_round(st)[v] = st.mv_round;
     }
 }
 
@@ -1452,9 +1454,7 @@ __global__ void __launch_bounds__(THREADS) giant_merge_kernel(StateView st, HubG
 // per-vertex updates 2(e_best - e_own) assumed j static; the exact change of
 // the pair's two CSR entries differs by
 //   w_uj ([n_u = n_j] - [n_u = c_j] - [c_u = n_j] + [c_u = c_j])
-// from each side (c = community before, n = after the sub-round).  Vertices
-// outside the sub-round's bucket have newc == comm, so "j moved" is newc[j] !=
-// comm[j].  Sums wrap in uint64; the final total is exact.
+// from each side (c = community before, n = after the sub-round).  Sums wrap in uint64; the final total is exact.
 __device__ __forceinline__ u64 pair_correction(int32_t cu, int32_t nu, int32_t cj, int32_t nj, u64 w) {
     const int t = (int)(nu == nj) - (int)(nu == cj) - (int)(cu == nj) + (int)(cu == cj);
     return (u64)(i64)t * w;
@@ -1490,13 +1490,37 @@ __global__ void __launch_bounds__(256) collect_movers_kernel(GraphView<WT> g, St
     block_note_movers<256>(st, v, units);
 }
 
+// The end of a sub-round (updateVertexCommunity, the Sigma_tot update and the
+// correction): the listed movers take their communities, the communities'
+// totals follow, and the pairs of neighbours that moved together are corrected.
+// The correction reads neither comm nor what the commit writes (a neighbour
+// moved in this sub-round if it carries its number; what it left and took lie
+// beside), so one kernel does both in any order, and an entry costs one
+// gather instead of two.  Runs against two kernels that compared comm with
+// newc, ms: R-MAT scale 14 3.59 -> 3.33, 16 5.20 -> 4.89, 18 15.1 -> 14.4, 20
+// 26.7 -> 26.3, 24 225.1 -> 222.7, LFR graph of 300,007 vertices 5.26 -> 5.09.
+// Summing the changes per community in a shared table first measured no faster
+// (R-MAT-20 28.2 against 27.9 ms).
 // TABLES: the neighbours' tables follow the moves as well (lv_nct.cuh).
 template <typename WT, bool TABLES>
-__global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, StateView st, u64 *dE, NctView t) {
+__global__ void __launch_bounds__(256) apply_movers_kernel(GraphView<WT> g, StateView st, u64 *dE, u64 *moves, NctView t) {
     pdl_trigger();
     pdl_wait();
     const u64 cu64 = *st.mv_cnt;
     const uint32_t n = (uint32_t)cu64, units = (uint32_t)(cu64 >> 32);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(moves, (u64)n);
+    const int32_t *left = mover_left(st);
+    const uint32_t *offs = mover_offsets(st), *round = mover_round(st);
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        const int32_t v = st.mv_list[i];
+        const int32_t nc = st.newc[v], oc = left[v];
+        const u64 kv = st.k[v];
+        st.comm[v] = nc;
+        atomicAdd(st.size + nc, 1);
+        atomicSub(st.size + oc, 1);
+        atomicAdd(st.S + nc, kv);
+        atomicAdd(st.S + oc, (u64)0 - kv);
+    }
     const int lane = threadIdx.x & 31;
     const uint32_t nw = gridDim.x * 8, w = blockIdx.x * 8 + (threadIdx.x >> 5);
     const uint32_t per = (units + nw - 1) / nw;
@@ -1510,7 +1534,7 @@ __global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, State
         while (hi - lo > 1) {
             const uint32_t step = (hi - lo + 31) >> 5;
             const u64 p = (u64)lo + (u64)lane * step;
-            const bool le = p < hi && st.mv_off[p] <= (uint32_t)u0;
+            const bool le = p < hi && offs[p] <= (uint32_t)u0;
             const int k = __popc(__ballot_sync(FULL, le)) - 1;   // lane 0 always holds
             lo += (uint32_t)k * step;
             hi = (u64)lo + step < hi ? lo + step : hi;
@@ -1523,8 +1547,8 @@ __global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, State
             uint32_t lo_u = 0;
             if (i0 + lane < n) {
                 lv = st.mv_list[i0 + lane];
-                lo_u = st.mv_off[i0 + lane];
-                lc = st.comm[lv];
+                lo_u = offs[i0 + lane];
+                lc = left[lv];
                 ln = st.newc[lv];
                 lr0 = g.rowptr[lv];
                 lr1 = g.rowend[lv];
@@ -1543,18 +1567,15 @@ __global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, State
                         const int32_t e = e0 + 32 * q;
                         jj[q] = e < e1 ? __ldg(g.col + e) : v;
                     }
-                    int32_t cj[CORR_U], nj[CORR_U];
+                    uint32_t rj[CORR_U];   // the sub-round that moved the neighbour last
 #pragma unroll
                     for (int q = 0; q < CORR_U; ++q) {
-                        cj[q] = nj[q] = 0;
-                        if (jj[q] != v) {
-                            cj[q] = __ldg(st.comm + jj[q]);
-                            nj[q] = __ldg(st.newc + jj[q]);
-                        }
+                        rj[q] = jj[q] != v ? round[jj[q]] : 0;
                     }
 #pragma unroll
                     for (int q = 0; q < CORR_U; ++q) {
-                        if (cj[q] != nj[q]) acc += pair_correction(cu, nu, cj[q], nj[q], gw(g, e0 + 32 * q));
+                        if (rj[q] == st.mv_round)
+                            acc += pair_correction(cu, nu, left[jj[q]], st.newc[jj[q]], gw(g, e0 + 32 * q));
                         if (TABLES && jj[q] != v) nct_move(t, jj[q], cu, nu, gw(g, e0 + 32 * q));
                     }
                 }
@@ -1563,29 +1584,6 @@ __global__ void __launch_bounds__(256) corr_movers_kernel(GraphView<WT> g, State
         }
     }
     block_add_total<256>(acc, dE);
-}
-
-// ------------------------------------------------------------------------
-// commit of one sub-round (updateVertexCommunity + Sigma_tot update)
-// ------------------------------------------------------------------------
-// Over the listed movers only (grid-stride; the count is on the device).
-// Summing the changes per community in a shared table first measured no
-// faster (R-MAT-20 28.2 against 27.9 ms).
-__global__ void __launch_bounds__(256) commit_kernel(StateView st, u64 *moves) {
-    pdl_trigger();
-    pdl_wait();
-    const uint32_t n = (uint32_t)*st.mv_cnt;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(moves, (u64)n);
-    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
-        const int32_t v = st.mv_list[i];
-        const int32_t nc = st.newc[v], oc = st.comm[v];
-        const u64 kv = st.k[v];
-        st.comm[v] = nc;
-        atomicAdd(st.size + nc, 1);
-        atomicSub(st.size + oc, 1);
-        atomicAdd(st.S + nc, kv);
-        atomicAdd(st.S + oc, (u64)0 - kv);
-    }
 }
 
 template <int G, int MODE, typename WT>
@@ -2016,10 +2014,9 @@ void launch_movers(const GraphView<WT> &g, const StateView &st, int32_t n, const
                    cudaStream_t s, const NctView *t) {
     if (n <= 0) return;
     const unsigned grid = (unsigned)imin64(nblocks(n, 8), (int64_t)di.sms * 8);
-    if (t) launch_pdl((corr_movers_kernel<WT, true>), grid, 256, 0, s, g, st, dE, *t);
-    else launch_pdl((corr_movers_kernel<WT, false>), grid, 256, 0, s, g, st, dE, NctView());
-    launch_pdl(commit_kernel, (unsigned)imin64(nblocks(n, 256), (int64_t)di.sms * 8), 256, 0, s, st, moves);
-    note_launches(2);
+    if (t) launch_pdl((apply_movers_kernel<WT, true>), grid, 256, 0, s, g, st, dE, moves, *t);
+    else launch_pdl((apply_movers_kernel<WT, false>), grid, 256, 0, s, g, st, dE, moves, NctView());
+    note_launches(1);
 }
 
 template <typename WT>

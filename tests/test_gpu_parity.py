@@ -538,3 +538,35 @@ def test_buckets_of_few_rows_match_oracle(lvb, orc, lo, hi, per_sm, over, unit):
             assert e.sweep() == o.sweep()
             assert np.array_equal(e.communities(), o.communities())
     o.close()
+
+
+@pytest.mark.parametrize("half", [1, 15, 16, 17, 63, 64, 65, 160])
+def test_neighbours_that_move_together_match_oracle(lvb, orc, half):
+    """Sweeps over a ring whose vertices are joined to the next `half` on either
+    side, some to themselves too (rows around the units that the end of a
+    sub-round works in; most neighbours move together): communities, moves and
+    the modularity kept up to date by the corrections."""
+    V = 3001
+    rng = np.random.default_rng(half)
+    src = np.repeat(np.arange(V, dtype=np.int64), half)
+    dst = (src + np.tile(np.arange(1, half + 1), V)) % V
+    w = rng.integers(1, 5, len(src)).astype(np.float32)
+    loops = np.arange(0, V, 3)
+    rows, cols = np.concatenate([src, dst, loops]), np.concatenate([dst, src, loops])
+    ww = np.concatenate([w, w, np.ones(len(loops), np.float32)])
+    o = np.lexsort((cols, rows))
+    rp = np.zeros(V + 1, np.int32)
+    np.cumsum(np.bincount(rows, minlength=V), out=rp[1:])
+    g = lvb.Graph(rp, cols[o].astype(np.int32), ww[o])
+    ref = orc.Oracle(g.rowptr, g.col, g.w)
+    with lvb.Louvain(g) as e:
+        for _ in range(4):
+            assert e.sweep() == ref.sweep()
+            assert np.array_equal(e.communities(), ref.communities())
+    with lvb.Louvain(g, max_sweeps=4) as e:
+        e.optimise_modularity(0.0)
+        kept = e.calculate_modularity()
+    with lvb.Louvain(g, max_sweeps=4, sweep_graph=False, verify=True) as e:
+        e.optimise_modularity(0.0)
+        assert e.calculate_modularity() == kept
+    ref.close()
