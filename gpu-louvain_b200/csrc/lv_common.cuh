@@ -346,7 +346,7 @@ struct StateView {
 };
 
 __device__ __forceinline__ uint32_t *mover_offsets(const StateView &st) {
-    return reinterpret_cast<uint32_t *>(st.mv_list + st.mv_stride);
+    return reinterpret_cast<uint32_t *>(st.mv_list + (size_t)st.mv_stride);
 }
 __device__ __forceinline__ int32_t *mover_left(const StateView &st) { return st.mv_list + 2 * (size_t)st.mv_stride; }
 __device__ __forceinline__ uint32_t *mover_round(const StateView &st) {

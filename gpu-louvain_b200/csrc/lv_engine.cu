@@ -395,14 +395,14 @@ bool narrow_weights(const lv_handle *h) {
 StateView state_of(lv_handle *h) {
     return StateView{h->comm, h->newc, h->size, h->k, h->S, h->T, &h->tot_d->err, h->feat,
                      (LV_NARROW_ESCAPES == 1 && h->cur_w32 && h->wrows_any) ? h->wrow : nullptr,
-                     h->blk_d->movers, h->mv_list, h->V0 + 1, 0, nullptr, nullptr,
+                     h->blk_d->movers, h->mv_list, h->V0, 0, nullptr, nullptr,
                      (LV_DEDUP == 2 || (LV_DEDUP == 1 && h->level > 0)) ? 1 : 0};
 }
 
 // Numbers a sub-round.  When the numbers run out, the old ones are forgotten.
 void next_round(lv_handle *h, StateView &st) {
     if (++h->mv_round == 0) {
-        cudaMemsetAsync(h->mv_list + 3 * ((size_t)h->V0 + 1), 0, sizeof(int32_t) * ((size_t)h->V0 + 1), h->stream);
+        cudaMemsetAsync(h->mv_list + 3 * (size_t)h->V0, 0, sizeof(int32_t) * (size_t)h->V0, h->stream);
         h->mv_round = 1;
     }
     st.mv_round = h->mv_round;
@@ -1584,8 +1584,8 @@ int ensure_move(lv_handle *h) {
     if (h->move_ready) return LV_OK;
     const size_t V = (size_t)h->V0;
     LV_TRY(dalloc(h, &h->list, V + 1));
-    LV_TRY(dalloc(h, &h->mv_list, 4 * (V + 1)));
-    LV_CUDA(h, cudaMemsetAsync(h->mv_list + 3 * (V + 1), 0, sizeof(int32_t) * (V + 1), h->stream));
+    LV_TRY(dalloc(h, &h->mv_list, 4 * V + 1));
+    LV_CUDA(h, cudaMemsetAsync(h->mv_list + 3 * V, 0, sizeof(int32_t) * V, h->stream));
     h->mv_round = 0;
     LV_TRY(dalloc(h, &h->sort_buf, 3 * V + 16));
     h->sort_temp_bytes = sort_by_degree_temp_bytes((int32_t)V, HG_MIN_DEG_HI) + 256;
