@@ -6,8 +6,8 @@ singleton communities on the seeded R-MAT-24 graph (a=.57 b=.19 c=.19,
 edge factor 16, float32 weights uniform in [0.5, 1.5)).
 
   value : edge-sweeps/s with the graph resident in HBM (lv_create_device once,
-          lv_reset + lv_run per step, default options: each level's sweep loop
-          runs as one CUDA graph), timed with CUDA events between barriers,
+          lv_reset + lv_run per step, default options: the sweep loop's stop
+          rule is decided on the device), timed with CUDA events between barriers,
           max over ranks; whole-job value = sum of all ranks' edge-sweeps.
   e2e   : the same metric through the public C ABI with host buffers: each
           step creates the engine from pinned host CSR (host->device copies
@@ -235,11 +235,13 @@ def ncu_class_split(csv_path: str) -> dict:
     dram__bytes_read.sum,dram__bytes_write.sum --csv``, every launch).
 
     Launches are attributed the way the engine issues a sweep: each degree
-    bucket's move kernels, then its correction kernels, then commit_kernel;
-    a bucket is named by its move kernel (move_group_*<G,...>: G = 4/8/16/32
-    -> buckets 0-3) or, for the warp buckets, by its correction kernel
-    (corr_group_kernel<32> -> bucket 4, corr_cta_kernel<128> -> bucket 5,
-    corr_cta_kernel<256|512> -> bucket 6).  In bucket 6 the giant kernels
+    bucket's move kernels, then (buckets 4 to 6) collect_movers_kernel, then
+    apply_movers_kernel; a bucket is named by its move kernel
+    (move_group_*<G,2G>: G = 4/8/16/32 -> buckets 0-3, <32,256> -> bucket 4)
+    or, for the warp buckets, by the one before it in the sweep, so every
+    bucket from 3 on must hold vertices.  Lists recorded with separate
+    corr_*_kernel and commit_kernel launches name buckets 4 to 6 by the former
+    (corr_group_kernel<32>, corr_cta_kernel<128>, <256|512>).  In bucket 6 the giant kernels
     (giant_stage_*, giant_merge_* and the large queue after them) form the
     b6_giants class, as the engine's class events bracket them."""
     import csv
@@ -282,24 +284,31 @@ def ncu_class_split(csv_path: str) -> dict:
            for c in CLASS_NAMES[:8]}
     seg = []
 
+    MOVERS = ("collect_movers", "apply_movers", "corr_", "commit_kernel")
+    last = 3   # bucket of the sub-round before
+
     def close(seg):
+        nonlocal last
         names = [short(launches[i]["name"]) for i in seg]
-        moves = [i for i, n in zip(seg, names) if not n.startswith(("corr_", "commit_kernel"))]
+        moves = [i for i, n in zip(seg, names) if not n.startswith(MOVERS)]
         corr = [n for n in names if n.startswith("corr_")]
-        grp = [re.match(r"move_group\w*<(\d+),", n) for n in names]
-        grp = [int(m.group(1)) for m in grp if m]
+        grp = [re.match(r"move_group\w*<(\d+),(?: *(256)\b)?", n) for n in names]
+        grp = [m for m in grp if m]
         if grp:
-            b = {4: 0, 8: 1, 16: 2, 32: 3}.get(grp[0])
+            b = 4 if grp[0].group(2) else {4: 0, 8: 1, 16: 2, 32: 3}.get(int(grp[0].group(1)))
         elif any(n.startswith("corr_group_kernel<32") for n in corr):
             b = 4
         elif any(n.startswith("corr_cta_kernel<128") for n in corr):
             b = 5
-        elif corr:
+        elif corr or any(n.startswith("giant_") for n in names):
             b = 6
+        elif moves:
+            b = last + 1 if 3 <= last < 6 else 4
         else:
             return
         if b is None:
             return
+        last = b
         parts = {CLASS_NAMES[b]: []}
         if b == 6:
             parts["b6_giants"] = []
@@ -326,7 +335,7 @@ def ncu_class_split(csv_path: str) -> dict:
             in_sweep = True
         if in_sweep:
             seg.append(lid)
-        if n.startswith("commit_kernel"):
+        if n.startswith(("apply_movers_kernel", "commit_kernel")):
             close(seg)
             seg, in_sweep = [], False
     for c, o in out.items():
@@ -812,9 +821,12 @@ def batch_summary(args, ranks: Ranks):
                 "sweeps": int(gs["sweeps"][i]), "ms": round(float(gs["latency_ms"][i]), 2)} for i in slow]
     lat = np.concatenate(lat)
     # the launch against its load: the summed per-graph latencies spread over
-    # the CTAs (the launch time with perfect balancing) and the longest graph
+    # the CTAs that run at a time, two per SM (a lower bound of the launch time
+    # with perfect balancing: a graph that several CTAs share counts once), and
+    # the longest graph
     ctas = int(st.get("ctas", 0) or 0)
-    busy = float(lat.sum()) / 2 / ctas if ctas else None
+    resident = min(ctas, 2 * torch.cuda.get_device_properties(0).multi_processor_count)
+    busy = float(lat.sum()) / 2 / resident if resident else None
     return {"workload": f"batch{G}_planted", "graphs_per_s": 2 * G / (dev_ms * 1e-3),
             "ms_per_launch": dev_ms / 2, "edge_sweeps_per_s": es / (dev_ms * 1e-3),
             "latency_ms": {"p50": float(np.percentile(lat, 50)), "p99": float(np.percentile(lat, 99)),
