@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "lv_sym.h"
+
 // Tuning knobs (compile-time): edges per lane in flight in the insert loops
 // of the group kernels (LV_U_GROUP), the warp kernel (LV_U_WARP), the small
 // and medium fallback CTAs (LV_U_FB) and the giant staging CTAs
@@ -1032,20 +1034,6 @@ __device__ __forceinline__ u128 warp_sum_u128(u128 x) {
         x += ((u128)hi << 64) | (u128)lo;
     }
     return x;
-}
-
-// One entry's share of the symmetry check: the sum over all entries of
-// mix(row, col, w) - mix(col, row, w) is zero when the entries and their
-// mirror images are the same multiset (and otherwise zero by a chance of
-// 2^-64 only).
-__device__ __forceinline__ u64 sym_mix(uint32_t a, uint32_t b, u64 w) {
-    u64 x = ((u64)a << 32 | b) * 0x9E3779B97F4A7C15ull + (w ^ (w >> 32) * 0x85EBCA6Bull);
-    x ^= x >> 29;
-    x *= 0xD6E8FEB86659FD93ull;
-    return x ^ (x >> 32);
-}
-__device__ __forceinline__ u64 sym_share(int32_t v, int32_t j, u64 w) {
-    return sym_mix((uint32_t)v, (uint32_t)j, w) - sym_mix((uint32_t)j, (uint32_t)v, w);
 }
 
 // 128-bit accumulate into two device words with an exact carry.
