@@ -305,6 +305,26 @@ constexpr uint32_t MBAR_MAX_POLLS = 1u << 22;   // each try_wait may itself susp
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Loads of what the sub-rounds change (comm, newc, size, S).  __ldg promises
+// data that nothing writes while the kernel lives; a kernel launched with
+// launch_pdl lives while the one before it still writes, so it reads them with
+// ordinary loads, which stay behind its pdl_wait (CO).  Both measured the same.
+__device__ __forceinline__ int32_t ld_coherent(const int32_t *p) {
+    int32_t x;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(x) : "l"(p));
+    return x;
+}
+__device__ __forceinline__ u64 ld_coherent(const u64 *p) {
+    u64 x;
+    asm volatile("ld.global.b64 %0, [%1];" : "=l"(x) : "l"(p));
+    return x;
+}
+template <bool CO, typename T>
+__device__ __forceinline__ T ld_state(const T *p) {
+    if constexpr (CO) return ld_coherent(p);
+    else return __ldg(p);
+}
+
 template <typename... K, typename... A>
 inline void launch_pdl(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchConfig_t cfg = {};
@@ -609,9 +629,9 @@ __device__ __forceinline__ void table_insert_occ_capped(int32_t *keys, u64 *vals
 // into a table, U edges per lane at a time so that U column loads and then U
 // community gathers are in flight together.  Self-loops are skipped; the
 // weight to the own community is summed into *e_own instead of the table.
-// OCC: record newly claimed slots in occ[] / *nocc.
-template <int U, bool OCC, typename WT>
-__device__ __forceinline__ void insert_row(const GraphView<WT> &g, const int32_t *__restrict__ comm,
+// OCC: record newly claimed slots in occ[] / *nocc.  CO: as in ld_state.
+template <int U, bool OCC, bool CO = false, typename WT>
+__device__ __forceinline__ void insert_row(const GraphView<WT> &g, const int32_t *comm,
                                            int32_t v, int32_t own, int32_t r0, int32_t r1, int lane,
                                            int stride, int32_t *keys, u64 *vals, int lg, int *err,
                                            int32_t *occ, int32_t *nocc, u64 &e_own, bool dedup = false) {
@@ -632,7 +652,7 @@ __device__ __forceinline__ void insert_row(const GraphView<WT> &g, const int32_t
                 ww[u] = gw(g, e);
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) cc[u] = jj[u] != v ? __ldg(comm + jj[u]) : -1;
+            for (int u = 0; u < U; ++u) cc[u] = jj[u] != v ? ld_state<CO>(comm + jj[u]) : -1;
         } else {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -645,7 +665,7 @@ __device__ __forceinline__ void insert_row(const GraphView<WT> &g, const int32_t
                 }
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) cc[u] = (jj[u] >= 0 && jj[u] != v) ? __ldg(comm + jj[u]) : -1;
+            for (int u = 0; u < U; ++u) cc[u] = (jj[u] >= 0 && jj[u] != v) ? ld_state<CO>(comm + jj[u]) : -1;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -672,8 +692,8 @@ __device__ __forceinline__ void insert_row(const GraphView<WT> &g, const int32_t
 // insert_row for piece tables (weights below 2^32, at most PIECE_MAX_ADDS
 // entries): OCC records every newly claimed slot in occ[] (the first occ_cap
 // of them; *nocc counts them all).
-template <int U, bool OCC, typename WT>
-__device__ __forceinline__ void insert_row_piece(const GraphView<WT> &g, const int32_t *__restrict__ comm,
+template <int U, bool OCC, bool CO = false, typename WT>
+__device__ __forceinline__ void insert_row_piece(const GraphView<WT> &g, const int32_t *comm,
                                                  int32_t v, int32_t own, int32_t r0, int32_t r1, int lane,
                                                  int stride, const PieceTable &t, int lg, int *err,
                                                  int32_t *occ, int32_t *nocc, int32_t occ_cap, u64 &e_own,
@@ -695,7 +715,7 @@ __device__ __forceinline__ void insert_row_piece(const GraphView<WT> &g, const i
                 ww[u] = gw(g, e);
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) cc[u] = jj[u] != v ? __ldg(comm + jj[u]) : -1;
+            for (int u = 0; u < U; ++u) cc[u] = jj[u] != v ? ld_state<CO>(comm + jj[u]) : -1;
         } else {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -708,7 +728,7 @@ __device__ __forceinline__ void insert_row_piece(const GraphView<WT> &g, const i
                 }
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) cc[u] = (jj[u] >= 0 && jj[u] != v) ? __ldg(comm + jj[u]) : -1;
+            for (int u = 0; u < U; ++u) cc[u] = (jj[u] >= 0 && jj[u] != v) ? ld_state<CO>(comm + jj[u]) : -1;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -868,11 +888,11 @@ __device__ __forceinline__ void eval_candidate(int32_t c, u64 ec, const MoveCtx 
 // U Sigma_tot (and guard size) gathers, then the comparisons.  Entries come
 // from slot indices (OCC: occ[i], else i itself, i < n); each visited slot is
 // cleared when CLEAR is set.
-template <int U, bool OCC, bool CLEAR>
+template <int U, bool OCC, bool CLEAR, bool CO = false>
 __device__ __forceinline__ void eval_slots(int32_t *keys, u64 *vals, const int32_t *occ, int32_t n,
                                            int lane, int stride, const MoveCtx &m,
-                                           const u64 *__restrict__ S,
-                                           const int32_t *__restrict__ size, Best &b) {
+                                           const u64 *S,
+                                           const int32_t *size, Best &b) {
     for (int32_t i0 = lane; i0 < n; i0 += U * stride) {
         int32_t cc[U];
         u64 ee[U];
@@ -898,8 +918,8 @@ __device__ __forceinline__ void eval_slots(int32_t *keys, u64 *vals, const int32
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const bool cand = cc[u] >= 0 && cc[u] != m.own;
-            SS[u] = cand ? __ldg(S + cc[u]) : 0;
-            zz[u] = (cand && guard_needs_size(m, cc[u])) ? __ldg(size + cc[u]) : 0;
+            SS[u] = cand ? ld_state<CO>(S + cc[u]) : 0;
+            zz[u] = (cand && guard_needs_size(m, cc[u])) ? ld_state<CO>(size + cc[u]) : 0;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)

@@ -120,16 +120,16 @@ __global__ void __launch_bounds__(256) move_group_kernel(GraphView<WT> g, StateV
     u64 e_own = 0;   // weight to the own community: kept out of the table
     if (active) {
         v = list[idx];
-        own = __ldg(st.comm + v);
-        insert_row<(CAP > 32 ? LV_U_CTA : LV_U_GROUP), false>(g, st.comm, v, own, g.rowptr[v], g.rowend[v], lane, G,
+        own = ld_coherent(st.comm + v);
+        insert_row<(CAP > 32 ? LV_U_CTA : LV_U_GROUP), false, true>(g, st.comm, v, own, g.rowptr[v], g.rowend[v], lane, G,
                                                keys, vals, LG, st.err, nullptr, nullptr, e_own);
     }
     __syncwarp();
-    const MoveCtx m = move_ctx(own, active ? __ldg(st.size + own) == 1 : false, st.T,
-                               active ? __ldg(st.k + v) : 0, active ? __ldg(st.S + own) : 0);
+    const MoveCtx m = move_ctx(own, active ? ld_coherent(st.size + own) == 1 : false, st.T,
+                               active ? __ldg(st.k + v) : 0, active ? ld_coherent(st.S + own) : 0);
     Best b = best_init(own);
     b.eo = e_own;
-    if (active) eval_slots<(CAP / G > 1 ? (LV_U_EVAL < 2 ? LV_U_EVAL : 2) : 1), false, false>(keys, vals, nullptr, CAP, lane, G, m, st.S, st.size, b);
+    if (active) eval_slots<(CAP / G > 1 ? (LV_U_EVAL < 2 ? LV_U_EVAL : 2) : 1), false, false, true>(keys, vals, nullptr, CAP, lane, G, m, st.S, st.size, b);
     group_reduce_best(m, b, G);
     u64 delta = 0;
     int32_t mover = -1;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256) move_group_narrow_kernel(GraphView<WT> g,
         v = list[idx];
         r0 = g.rowptr[v];
         r1 = g.rowend[v];
-        own = __ldg(st.comm + v);
+        own = ld_coherent(st.comm + v);
         if (st.wrow && st.wrow[v]) {
             // a row with a sum of 2^32 or more: decided by the large queue
             if (lane == 0) enqueue_large(fbl, v, r1 - r0, st.err);
@@ -183,11 +183,11 @@ __global__ void __launch_bounds__(256) move_group_narrow_kernel(GraphView<WT> g,
         }
     }
     if (active)
-        insert_row_piece<(CAP > 32 ? LV_U_CTA : LV_U_GROUP), false>(g, st.comm, v, own, r0, r1, lane, G, t, LG,
+        insert_row_piece<(CAP > 32 ? LV_U_CTA : LV_U_GROUP), false, true>(g, st.comm, v, own, r0, r1, lane, G, t, LG,
                                                                      st.err, nullptr, nullptr, 0, e_own);
     __syncwarp();
-    const MoveCtx m = move_ctx(own, active ? __ldg(st.size + own) == 1 : false, st.T,
-                               active ? __ldg(st.k + v) : 0, active ? __ldg(st.S + own) : 0);
+    const MoveCtx m = move_ctx(own, active ? ld_coherent(st.size + own) == 1 : false, st.T,
+                               active ? __ldg(st.k + v) : 0, active ? ld_coherent(st.S + own) : 0);
     Best b = best_init(own);
     b.eo = e_own;
     if (active) {
@@ -196,8 +196,8 @@ __global__ void __launch_bounds__(256) move_group_narrow_kernel(GraphView<WT> g,
             const int32_t c = t.keys[s];
             if (c < 0) continue;
             const bool cand = c != own;
-            const u64 Sc = cand ? __ldg(st.S + c) : 0;
-            const int32_t szc = (cand && guard_needs_size(m, c)) ? __ldg(st.size + c) : 0;
+            const u64 Sc = cand ? ld_coherent(st.S + c) : 0;
+            const int32_t szc = (cand && guard_needs_size(m, c)) ? ld_coherent(st.size + c) : 0;
             eval_loaded(c, piece_value(t, (uint32_t)s), Sc, szc, m, b);
         }
     }
@@ -1666,7 +1666,7 @@ __global__ void __launch_bounds__(THREADS) row_reduce_cta_kernel(GraphView<WT> g
     if (MODE == 2) block_add_total<THREADS>(zeros, total + 1);
 }
 
-__global__ void __launch_bounds__(256) s2_kernel(const u64 *__restrict__ S, int32_t V,
+__global__ void __launch_bounds__(256) s2_kernel(const u64 *S, int32_t V,
                                                  u64 *total_hi_lo) {
     pdl_trigger();
     pdl_wait();
