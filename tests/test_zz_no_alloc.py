@@ -73,3 +73,59 @@ def test_noalloc_rejects_bad_sizes(lvb):
     # entries without vertices: malformed, as for lv_create_device
     rc, _, msg = _noalloc(lvb, d.data_ptr(), d.data_ptr(), d.data_ptr(), 0, 4, d.data_ptr())
     assert rc == lvb.LV_ERR_INVALID, msg
+
+
+def _csr(rows, V):
+    """CSR of the given rows' entries (lists of columns), unit weights."""
+    rp = np.zeros(V + 1, np.int32)
+    np.cumsum([len(r) for r in rows], out=rp[1:])
+    cl = np.concatenate([np.asarray(r, np.int32) for r in rows]) if rp[-1] else np.zeros(0, np.int32)
+    return rp, cl.astype(np.int32)
+
+
+def _skewed(name):
+    rng = np.random.default_rng(11)
+    V = 3000
+    pick = lambda n: rng.integers(0, V, n)
+    if name == "one_vertex":
+        return _csr([[0] * 700], 1)
+    if name == "no_entries":
+        return _csr([[] for _ in range(V)], V)
+    if name == "hub_first":
+        return _csr([pick(100000)] + [pick(i % 5) for i in range(V - 1)], V)
+    if name == "hub_last_after_empty_rows":
+        return _csr([pick(3)] + [[] for _ in range(V - 2)] + [pick(70001)], V)
+    if name == "hubs_between_empty_rows":
+        return _csr([pick(9000) if i in (7, 1500, 1501) else [] for i in range(V)], V)
+    if name == "rows_around_the_long_limit":   # 128 entries, and around 8 and 32 lanes times 4
+        return _csr([pick(n) for n in np.resize([0, 1, 7, 8, 31, 32, 33, 127, 128, 129, 160, 255, 257], V)], V)
+    if name == "every_row_one_entry":
+        return _csr([pick(1) for _ in range(V)], V)
+
+
+@pytest.mark.parametrize("name", ["one_vertex", "no_entries", "hub_first", "hub_last_after_empty_rows",
+                                  "hubs_between_empty_rows", "rows_around_the_long_limit", "every_row_one_entry"])
+def test_noalloc_rows_shared_by_warps(lvb, name):
+    """Rows cut anywhere, empty and one-entry rows, hubs: the handle path's
+    value exactly, and a community id outside [0, V) of any vertex is found,
+    with entries or without."""
+    import torch
+    rp, cl = _skewed(name)
+    V, E = len(rp) - 1, len(cl)
+    rng = np.random.default_rng(4)
+    w = rng.uniform(0.5, 1.5, E).astype(np.float32)
+    d_rp, d_cl, d_w = (torch.from_numpy(x).cuda() for x in (rp, cl, w))
+    csr = (d_rp.data_ptr(), d_cl.data_ptr() if E else 0, d_w.data_ptr() if E else 0, V, E)
+    with lvb.Louvain(device_csr=csr) as e:
+        for comm in (rng.integers(0, min(V, 40), V), np.arange(V), rng.integers(0, V, V)):
+            comm = comm.astype(np.int32)
+            e.set_communities(comm)
+            want = e.calculate_modularity()
+            rc, q, msg = _noalloc(lvb, *csr, torch.from_numpy(comm).cuda().data_ptr())
+            assert rc == lvb.LV_OK, msg
+            assert q == want or (E == 0 and np.isnan(q) and np.isnan(want))
+    for at in (0, V // 2, V - 1):
+        bad = np.zeros(V, np.int32)
+        bad[at] = V
+        rc, _, msg = _noalloc(lvb, *csr, torch.from_numpy(bad).cuda().data_ptr())
+        assert rc == lvb.LV_ERR_INVALID and "community id" in msg
