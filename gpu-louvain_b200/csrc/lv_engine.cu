@@ -269,6 +269,15 @@ int dalloc(lv_handle *h, T **p, size_t n) {
     return LV_OK;
 }
 
+// dalloc of a buffer that a run can do without: false when it cannot be had.
+template <typename T>
+bool dalloc_optional(lv_handle *h, T **p, size_t n) {
+    void *q = nullptr;
+    const bool ok = h->mem.alloc(&q, n * sizeof(T), h->stream) == cudaSuccess;
+    *p = (T *)q;
+    return ok;
+}
+
 // Stream-ordered free (after the handle's queued work).
 template <typename T>
 void dfree(lv_handle *h, T *&p) {
@@ -986,7 +995,8 @@ constexpr double NCT_MAX_SLOTS = LV_NCT_MAX_SLOTS;
 constexpr int32_t NCT_SAMPLES = 4096;
 
 // Prepares table sweeps of the current level; *ok = 0 when its rows do not
-// allow them (an entry without its mirror entry, or of weight zero).
+// allow them (an entry without its mirror entry, or of weight zero) or there is
+// no memory for the tables.
 int nct_begin(lv_handle *h, int *ok) {
     *ok = 0;
     LV_TRY(reset_totals(h));
@@ -1005,19 +1015,19 @@ int nct_begin(lv_handle *h, int *ok) {
     else check(view_of<float>(h));
     LV_TRY(read_totals(h));
     if (h->tot_h->s2[0] || h->tot_h->s2[1]) return LV_OK;
-    if (!h->nct.lg) {
-        LV_TRY(dalloc(h, &h->nct.lg, (size_t)h->V0 + 1));
-        LV_TRY(dalloc(h, &h->nct.off, (size_t)h->V0 + 1));
-        LV_TRY(dalloc(h, &h->nct.queue, (size_t)h->V0 + 1));
-        LV_TRY(dalloc(h, &h->nct.cursor, 2));
-    }
+    // without memory for tables the sweeps go on from the rows
+    NctView &t = h->nct;
+    const size_t V = (size_t)h->V0 + 1;
+    if ((!t.lg && !dalloc_optional(h, &t.lg, V)) || (!t.off && !dalloc_optional(h, &t.off, V)) ||
+        (!t.queue && !dalloc_optional(h, &t.queue, V)) || (!t.cursor && !dalloc_optional(h, &t.cursor, 2)))
+        return LV_OK;
     // half a slot per entry of the level: rows with many communities that do
     // not fit go on being summed from the row
     const u64 want = (u64)h->E / 2 + 1024;
     if (want > h->nct_alloc) {
-        dfree(h, h->nct.slots);
+        dfree(h, t.slots);
         h->nct_alloc = 0;
-        LV_TRY(dalloc(h, &h->nct.slots, (size_t)want));
+        if (!dalloc_optional(h, &t.slots, (size_t)want)) return LV_OK;
         h->nct_alloc = want;
     }
     h->nct.cap = want;
@@ -1922,6 +1932,12 @@ int lv_set_communities(lv_handle *h, const int32_t *comm) {
     launch_set_communities(tmp, h->comm, h->newc, h->size, h->k, h->S, h->V, &h->tot_d->err, h->stream);
     h->e_own_valid = false;
     LV_TRY(read_totals(h));
+    return LV_OK;
+}
+
+int lv_set_test_limits(lv_handle *h, int32_t fail_alloc) {
+    if (!h || fail_alloc < 0) return LV_ERR_INVALID;
+    h->mem.fail_at = fail_alloc;
     return LV_OK;
 }
 

@@ -107,6 +107,7 @@ struct MemSet {
     std::vector<MemBlock> blocks, slabs;
     unsigned char *slab = nullptr;
     size_t slab_at = 0, slab_end = 0;
+    int fail_at = 0;   // test hook: the fail_at-th alloc from now on fails (0: none)
     cudaError_t alloc(void **p, size_t bytes, cudaStream_t s);
     cudaError_t alloc_own(void **p, size_t bytes, cudaStream_t s);   // a block of its own
     // Frees p after the work queued on s (a slab's part stays with the owner).

@@ -206,6 +206,7 @@ bool mem_pooled(int dev) {
 
 cudaError_t MemSet::alloc(void **p, size_t bytes, cudaStream_t s) {
     *p = nullptr;
+    if (fail_at > 0 && --fail_at == 0) return cudaErrorMemoryAllocation;
     if (bytes == 0) bytes = 1;
     if (bytes < LARGE_BYTES) {
         const size_t at = (slab_at + 255) / 256 * 256;

@@ -176,6 +176,9 @@ int lv_get_communities(lv_handle *h, int32_t *out);
 /* Test hook: set the current level's communities (Sigma_tot and sizes are
  * recomputed), e.g. to drive lv_aggregate from a given community vector. */
 int lv_set_communities(lv_handle *h, const int32_t *comm);
+/* Test hook: the handle's fail_alloc-th device allocation from now on fails
+ * as if the device had no memory left (0: none). */
+int lv_set_test_limits(lv_handle *h, int32_t fail_alloc);
 int lv_get_level_info(lv_handle *h, int32_t *V, int64_t *E, int32_t *level);
 /* The current level's work classes (LV_NUM_CLASSES entries each): vertices
  * and CSR entries per class (degree (0,4], (4,8], (8,16], (16,32], (32,84],

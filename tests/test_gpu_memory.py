@@ -1,0 +1,48 @@
+"""Device memory that runs out at any allocation of a handle: a call either
+fails with LV_ERR_NOMEM or, where the buffer only makes later sweeps faster,
+gives the usual result; the handle, reset, then runs as if nothing had been.
+The failures are made on the host (lv_set_test_limits)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GAIN = 1e-7
+
+
+def _graph(lvb, name):
+    if name == "small":      # one launch
+        return lvb.gen_planted(2000, 16, 12.0, 2.0, 1, "uniform"), {}
+    if name == "levels":
+        return lvb.gen_planted(10007, 64, 14.0, 3.0, 2, "uniform"), {}
+    if name == "giants":     # rows beyond the giant degree
+        return lvb.gen_rmat(15, 16, 3), {"giant_degree": 1024}
+    if name == "tables":     # late sweeps from tables
+        return lvb.gen_planted(10000, 24, 300.0, 15.0, 3, "uniform"), {}
+
+
+def _result(e):
+    q = e.run(GAIN)
+    m, n = e.original_to_community()
+    return q, n, m
+
+
+@pytest.mark.parametrize("name", ["small", "levels", "giants", "tables"])
+def test_failing_allocations(lvb, name):
+    g, kw = _graph(lvb, name)
+    with lvb.Louvain(g, **kw) as e:
+        want = _result(e)
+    refused = 0
+    for n in range(1, 80):
+        with lvb.Louvain(g, **kw) as e:
+            e.set_test_limits(n)
+            for again in (False, True):   # the second time with the hook off
+                try:
+                    got = _result(e)
+                    assert got[:2] == want[:2] and np.array_equal(got[2], want[2]), n
+                except lvb.LouvainError as x:
+                    assert x.status == lvb.LV_ERR_NOMEM and not again, (n, x)
+                    refused += 1
+                e.set_test_limits(0)
+                e.reset()
+    assert 0 < refused < 79   # the last failures lie past the last allocation
