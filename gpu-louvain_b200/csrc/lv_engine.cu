@@ -217,6 +217,7 @@ struct lv_handle {
     std::vector<Pending> pend;
 
     // learned active set and move traces
+    bool active_ready = false;      // every buffer below allocated
     float *feat = nullptr;          // [2 V0] features recorded by the move kernels
     uint8_t *moved = nullptr;       // [V0] moved in the previous sweep
     int32_t *nmoved = nullptr;      // [V0] row entries whose vertex moved in the previous sweep
@@ -1123,7 +1124,7 @@ bool learned_mode(const lv_handle *h) {
 }
 
 int ensure_active(lv_handle *h) {
-    if (h->feat) return LV_OK;
+    if (h->active_ready) return LV_OK;
     const size_t V = (size_t)h->V0 + 1;
     LV_TRY(dalloc(h, &h->feat, 2 * V));
     LV_TRY(dalloc(h, &h->moved, V));
@@ -1143,6 +1144,7 @@ int ensure_active(lv_handle *h) {
         LV_TRY(dalloc(h, &h->tr_v, (size_t)h->tr_cap));
         LV_TRY(dalloc(h, &h->tr_y, (size_t)h->tr_cap));
     }
+    h->active_ready = true;
     return LV_OK;
 }
 

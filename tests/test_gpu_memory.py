@@ -19,6 +19,17 @@ def _graph(lvb, name):
         return lvb.gen_rmat(15, 16, 3), {"giant_degree": 1024}
     if name == "tables":     # late sweeps from tables
         return lvb.gen_planted(10000, 24, 300.0, 15.0, 3, "uniform"), {}
+    if name == "learned":    # the proposals' buffers
+        return lvb.gen_lfr(70000, 0.4, 5)[0], {"active_set": True, "active_start": 0.2, "active_min_recall": 0.5}
+    if name == "traced":
+        return lvb.gen_planted(3000, 24, 14.0, 3.0, 5, "uniform"), {"trace_sample": 0.5}
+
+
+def _engine(lvb, g, kw):
+    e = lvb.Louvain(g, **kw)
+    if kw.get("active_set"):
+        e.set_active_model(*lvb.load_active_model())
+    return e
 
 
 def _result(e):
@@ -27,14 +38,14 @@ def _result(e):
     return q, n, m
 
 
-@pytest.mark.parametrize("name", ["small", "levels", "giants", "tables"])
+@pytest.mark.parametrize("name", ["small", "levels", "giants", "tables", "learned", "traced"])
 def test_failing_allocations(lvb, name):
     g, kw = _graph(lvb, name)
-    with lvb.Louvain(g, **kw) as e:
+    with _engine(lvb, g, kw) as e:
         want = _result(e)
     refused = 0
     for n in range(1, 80):
-        with lvb.Louvain(g, **kw) as e:
+        with _engine(lvb, g, kw) as e:
             e.set_test_limits(n)
             for again in (False, True):   # the second time with the hook off
                 try:
