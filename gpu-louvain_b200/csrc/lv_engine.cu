@@ -1484,7 +1484,11 @@ int aggregate_t(lv_handle *h) {
 int aggregate(lv_handle *h) {
     LV_TRY(ensure_setup(h));
     LV_TRY(ensure_agg(h));
-    return h->cur_w ? aggregate_t<u64>(h) : aggregate_t<float>(h);
+    const int rc = h->cur_w ? aggregate_t<u64>(h) : aggregate_t<float>(h);
+    // the level stays, but its giants' layout may point to staging buffers that
+    // the aggregation outgrew before it failed
+    if (rc && !h->setup_due) h->setup_due = SETUP_LISTS;
+    return rc;
 }
 
 // ---------------------------------------------------------------------------

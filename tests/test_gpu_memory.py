@@ -57,3 +57,39 @@ def test_failing_allocations(lvb, name):
                 e.set_test_limits(0)
                 e.reset()
     assert 0 < refused < 79   # the last failures lie past the last allocation
+
+
+@pytest.mark.parametrize("name", ["levels", "giants", "tables"])
+def test_level_goes_on_after_a_failed_aggregation(lvb, name):
+    """An aggregation that ran out of memory leaves its level as it was: swept
+    again and aggregated, it gives what a handle gives whose aggregation never
+    failed."""
+    g, kw = _graph(lvb, name)
+
+    def operators(fail):
+        out, failed = [], 0
+        with lvb.Louvain(g, **kw) as e:
+            while e.optimise_modularity(GAIN):
+                if fail:
+                    e.set_test_limits(fail)
+                    try:
+                        e.aggregate_communities()
+                        e.set_test_limits(0)
+                        return None, 0   # past the level's last allocation
+                    except lvb.LouvainError as x:
+                        assert x.status == lvb.LV_ERR_NOMEM
+                        failed += 1
+                    e.set_test_limits(0)
+                    fail = 0
+                out.append((e.sweep(), e.calculate_modularity()))
+                e.aggregate_communities()
+                out.append(e.level_info())
+            return out + [e.original_to_community()[0].tobytes()], failed
+
+    want, _ = operators(0)
+    for n in range(1, 60):
+        got, failed = operators(n)
+        if got is None:
+            break
+        assert failed == 1 and got == want, n
+    assert 20 < n < 59
