@@ -7,6 +7,7 @@
 // host reads back one small totals record per sweep (the sweep's modularity
 // parts, its move count and the device error word) and a few counts per
 // level.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -469,21 +470,36 @@ int ensure_tables(lv_handle *h, size_t slots) {
     return LV_OK;
 }
 
+// The staging buffers for n entries of giants.
+constexpr size_t STAGING_BYTES = 28;   // per entry
+int alloc_staging(lv_handle *h, size_t n) {
+    dfree(h, h->occ_buf);
+    dfree(h, h->stage_key);
+    dfree(h, h->stage_val);
+    dfree(h, h->stage2_key);
+    dfree(h, h->stage2_val);
+    h->occ_cap = 0;
+    LV_TRY(dalloc(h, &h->occ_buf, n));
+    LV_TRY(dalloc(h, &h->stage_key, n));
+    LV_TRY(dalloc(h, &h->stage_val, n));
+    LV_TRY(dalloc(h, &h->stage2_key, n));
+    LV_TRY(dalloc(h, &h->stage2_val, n));
+    h->occ_cap = n;
+    return LV_OK;
+}
+
 int ensure_occ(lv_handle *h, size_t entries, size_t hubs) {
     if (entries > h->occ_cap) {
-        dfree(h, h->occ_buf);
-        dfree(h, h->stage_key);
-        dfree(h, h->stage_val);
-        dfree(h, h->stage2_key);
-        dfree(h, h->stage2_val);
-        h->occ_cap = 0;
-        size_t want = entries + entries / 4 + 1;
-        LV_TRY(dalloc(h, &h->occ_buf, want));
-        LV_TRY(dalloc(h, &h->stage_key, want));
-        LV_TRY(dalloc(h, &h->stage_val, want));
-        LV_TRY(dalloc(h, &h->stage2_key, want));
-        LV_TRY(dalloc(h, &h->stage2_val, want));
-        h->occ_cap = want;
+        // never more entries than the level 0 has.  A run that outgrows its
+        // first buffers mostly goes on to about that many, so it takes them at
+        // once where that is a small part of the device's memory: fewer
+        // outgrown buffers for the next run to ask for again
+        const size_t all = (size_t)h->E0, want = std::max(entries, std::min(entries + entries / 4 + 1, all));
+        const size_t more = std::min(4 * entries, all);
+        size_t avail = 0, total = 0;
+        const bool grown = h->occ_cap > 0 && more > want && cudaMemGetInfo(&avail, &total) == cudaSuccess &&
+                           more * STAGING_BYTES <= total / 8 && alloc_staging(h, more) == LV_OK;
+        if (!grown) LV_TRY(alloc_staging(h, want));
     }
     if (hubs > h->nocc_cap) {
         dfree(h, h->nocc_buf);

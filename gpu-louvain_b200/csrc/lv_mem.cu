@@ -11,8 +11,14 @@
 //     next request of about that size (at most 1/4 larger than asked for);
 //   - smaller buffers are cut from 4 MB slabs, which are such blocks;
 //   - streams are kept likewise, a few per device.
-// The kept blocks never exceed the largest amount that was in use at one time;
-// beyond that the oldest go back to the stream-ordered pool they come from.
+// Blocks in use and kept together never exceed the largest amount that was in
+// use at one time by more than an eighth (blocks outgrown during a run, and
+// those of a small graph between two large ones, find room there); beyond that
+// the oldest go back to the stream-ordered pool they come from.  A buffer that
+// a run outgrows is kept too: given to the pool, it was asked of the pool again
+// by the next run, which now and then mapped it anew (the first four of twelve
+// like runs of R-MAT-24 from host arrays took 753, 451, 345 and 323 ms; now
+// 691, 325, 323 and 322).
 // lv_trim_device_memory returns everything unused to the system.  All of it is
 // safe with several threads: a block belongs to one owner from take to give,
 // and is given only when no queued work uses it.
@@ -21,7 +27,7 @@
 #include <unordered_map>
 #include <vector>
 
-#include "lv_internal.h"
+#include "lv_mem.h"
 
 namespace lv {
 namespace {
@@ -72,6 +78,19 @@ cudaMemPool_t pool_of(int dev) {
     return d.pool;
 }
 
+// Takes the oldest blocks off the list until what is kept fits beside `live`
+// bytes in use.  Under g_mu.
+void evict(DeviceMemory &d, size_t live, std::vector<MemBlock> *out) {
+    const size_t most = std::max(d.peak_bytes, live), limit = most + most / 8;
+    size_t n = 0;
+    while (n < d.kept.size() && live + d.kept_bytes > limit) {
+        out->push_back(d.kept[n]);
+        d.kept_bytes -= d.kept[n].bytes;
+        ++n;
+    }
+    d.kept.erase(d.kept.begin(), d.kept.begin() + (long)n);
+}
+
 size_t rounded(size_t bytes) {
     size_t p = LARGE_BYTES;
     while (p * 2 <= bytes) p *= 2;
@@ -94,13 +113,14 @@ cudaError_t mem_take(int dev, size_t bytes, cudaStream_t s, MemBlock *out) {
     out->p = nullptr;
     if (dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
     const size_t want = rounded(bytes);
+    std::vector<MemBlock> old;
     cudaMemPool_t pool = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_mu);
         DeviceMemory &d = g_dev[dev];
         size_t best = d.kept.size();
         for (size_t i = 0; i < d.kept.size(); ++i)
-            if (d.kept[i].bytes >= want && d.kept[i].bytes <= want + want / 4 &&
+            if (d.kept[i].bytes >= bytes && d.kept[i].bytes <= want + want / 4 &&
                 (best == d.kept.size() || d.kept[i].bytes < d.kept[best].bytes))
                 best = i;
         if (best < d.kept.size()) {
@@ -108,15 +128,17 @@ cudaError_t mem_take(int dev, size_t bytes, cudaStream_t s, MemBlock *out) {
             d.kept.erase(d.kept.begin() + (long)best);
             d.kept_bytes -= out->bytes;
             d.live_bytes += out->bytes;
-            d.peak_bytes = std::max(d.peak_bytes, d.live_bytes);
             return cudaSuccess;
         }
         pool = pool_of(dev);
+        evict(d, d.live_bytes + want, &old);
     }
+    for (const MemBlock &b : old) free_raw(pool, b.p, s);
     out->bytes = want;
     cudaError_t e = alloc_raw(pool, &out->p, want, s);
     if (e != cudaSuccess) {
-        // everything kept goes back first, and the pool gives up what it holds unused
+        // everything kept goes back first, and the pool gives up what it holds
+        // unused; then the size asked for has to do
         cudaGetLastError();
         std::vector<MemBlock> kept;
         {
@@ -129,6 +151,11 @@ cudaError_t mem_take(int dev, size_t bytes, cudaStream_t s, MemBlock *out) {
         if (pool) cudaMemPoolTrimTo(pool, 0);
         cudaGetLastError();
         e = alloc_raw(pool, &out->p, want, s);
+        if (e != cudaSuccess && bytes < want) {
+            cudaGetLastError();
+            out->bytes = bytes;
+            e = alloc_raw(pool, &out->p, bytes, s);
+        }
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -137,14 +164,14 @@ cudaError_t mem_take(int dev, size_t bytes, cudaStream_t s, MemBlock *out) {
     }
     std::lock_guard<std::mutex> lock(g_mu);
     DeviceMemory &d = g_dev[dev];
-    d.live_bytes += want;
+    d.live_bytes += out->bytes;
     d.peak_bytes = std::max(d.peak_bytes, d.live_bytes);
     return cudaSuccess;
 }
 
 void mem_give(int dev, const MemBlock &b, cudaStream_t s) {
     if (!b.p) return;
-    std::vector<MemBlock> out;
+    std::vector<MemBlock> old;
     cudaMemPool_t pool = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_mu);
@@ -152,27 +179,10 @@ void mem_give(int dev, const MemBlock &b, cudaStream_t s) {
         d.live_bytes -= b.bytes;
         d.kept.push_back(b);
         d.kept_bytes += b.bytes;
-        size_t n = 0;
-        while (d.kept_bytes > d.peak_bytes) {
-            out.push_back(d.kept[n]);
-            d.kept_bytes -= d.kept[n].bytes;
-            ++n;
-        }
-        d.kept.erase(d.kept.begin(), d.kept.begin() + (long)n);
+        evict(d, d.live_bytes, &old);
         pool = d.pool;
     }
-    for (const MemBlock &x : out) free_raw(pool, x.p, s);
-}
-
-void mem_drop(int dev, const MemBlock &b, cudaStream_t s) {
-    if (!b.p) return;
-    cudaMemPool_t pool = nullptr;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        g_dev[dev].live_bytes -= b.bytes;
-        pool = g_dev[dev].pool;
-    }
-    free_raw(pool, b.p, s);
+    for (const MemBlock &x : old) free_raw(pool, x.p, s);
 }
 
 cudaError_t mem_trim(int dev) {
@@ -240,7 +250,8 @@ cudaError_t MemSet::alloc_own(void **p, size_t bytes, cudaStream_t s) {
 void MemSet::free(void *p, cudaStream_t s) {
     for (size_t i = 0; i < blocks.size(); ++i)
         if (blocks[i].p == p) {
-            mem_drop(dev, blocks[i], s);
+            cudaStreamSynchronize(s);
+            mem_give(dev, blocks[i], s);
             blocks[i] = blocks.back();
             blocks.pop_back();
             return;
