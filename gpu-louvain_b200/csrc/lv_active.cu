@@ -380,19 +380,17 @@ uint64_t gcd_u64(uint64_t a, uint64_t b) {
     return a;
 }
 
+// The device buffers of one call, from the library's blocks (which give way
+// when the device is full); the call's work is done when it ends.
 struct DevBuf {
-    std::vector<void *> p;
-    ~DevBuf() {
-        for (void *q : p) cudaFree(q);
-    }
+    MemSet m;
+    cudaStream_t s;   // the stream they are used on
+    DevBuf(int device, cudaStream_t stream) : s(stream) { m.dev = device; }
+    ~DevBuf() { m.give_all(s); }
     template <typename T>
     bool get(T **out, size_t n) {
         void *q = nullptr;
-        if (cudaMalloc(&q, sizeof(T) * (n ? n : 1)) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        p.push_back(q);
+        if (m.alloc(&q, sizeof(T) * (n ? n : 1), s) != cudaSuccess) return false;
         *out = (T *)q;
         return true;
     }
@@ -432,15 +430,23 @@ int lv_active_train(const float *x, const uint8_t *y, int64_t n, int32_t epochs,
     for (int i = 0; i < NP; ++i) wq_h[i] = host_bf16(master[i]);
     const int64_t steps_per_epoch = (n + batch - 1) / batch;
     const int64_t steps = steps_per_epoch * epochs;
-    DevBuf B;
+    struct Stream {
+        int dev;
+        cudaStream_t s = nullptr;
+        ~Stream() { stream_give(dev, s); }
+    } own{device};
+    if (stream_take(device, &own.s) != cudaSuccess) {
+        cudaGetLastError();
+        return LV_ERR_CUDA;
+    }
+    const cudaStream_t s = own.s;
+    DevBuf B(device, s);
     float *dx = nullptr, *part = nullptr, *dm = nullptr, *m1 = nullptr, *m2 = nullptr, *loss = nullptr;
     uint8_t *dy = nullptr;
     uint16_t *wq = nullptr;
     if (!B.get(&dx, (size_t)n * NF) || !B.get(&dy, (size_t)n) || !B.get(&part, (size_t)TR_BLOCKS * NG) ||
         !B.get(&dm, NP) || !B.get(&m1, NP) || !B.get(&m2, NP) || !B.get(&wq, NP) || !B.get(&loss, (size_t)steps))
         return LV_ERR_NOMEM;
-    cudaStream_t s = nullptr;
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return LV_ERR_CUDA;
     cudaMemcpyAsync(dx, x, sizeof(float) * (size_t)n * NF, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dy, y, (size_t)n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dm, master.data(), sizeof(float) * NP, cudaMemcpyHostToDevice, s);
@@ -469,7 +475,6 @@ int lv_active_train(const float *x, const uint8_t *y, int64_t n, int32_t epochs,
     cudaMemcpyAsync(wq_h.data(), wq, sizeof(uint16_t) * NP, cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(lh.data(), loss, sizeof(float) * (size_t)steps, cudaMemcpyDeviceToHost, s);
     const cudaError_t e = cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
     if (e != cudaSuccess || cudaGetLastError() != cudaSuccess) return LV_ERR_CUDA;
     std::memcpy(model_out, wq_h.data(), sizeof(uint16_t) * NP);
     if (epoch_loss) {
@@ -495,7 +500,7 @@ int lv_active_predict(const uint16_t *model, const float *x, int64_t n, int32_t 
     }
     if (device < 0 || device >= ndev) return LV_ERR_INVALID;
     cudaSetDevice(device);
-    DevBuf B;
+    DevBuf B(device, 0);
     uint16_t *wq = nullptr;
     float *dx = nullptr, *dz = nullptr;
     if (!B.get(&wq, NP) || !B.get(&dx, (size_t)n * NF) || !B.get(&dz, (size_t)n)) return LV_ERR_NOMEM;
