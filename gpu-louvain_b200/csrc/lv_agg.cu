@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(256) merge_group_kernel(const int32_t *__restr
                                                           const int32_t *__restrict__ newid,
                                                           int32_t *vkey, u64 *vw, uint32_t *vw32,
                                                           int32_t *newdeg, int32_t *epos_new, int *err,
-                                                          int *hiflag, uint8_t *wrow) {
+                                                          int *hiflag) {
     constexpr int GPB = 256 / G;
     constexpr int LG = (CAP == 64) ? 6 : (CAP == 128) ? 7 : 8;
     static_assert((1 << LG) == CAP, "CAP");
@@ -233,10 +233,7 @@ __global__ void __launch_bounds__(256) merge_group_kernel(const int32_t *__restr
         }
         cnt += __popc(bal);
     }
-    if (hi) {
-        atomicOr(hiflag, 1);
-        wrow[self] = 1;
-    }
+    if (hi) atomicOr(hiflag, 1);
     if (active && lane == 0) {
         const int32_t nid = newid[c];
         newdeg[nid] = cnt;
@@ -251,7 +248,7 @@ __global__ void __launch_bounds__(T) merge_cta_kernel(const int32_t *__restrict_
                                                       const int32_t *__restrict__ newid,
                                                       int32_t *vkey, u64 *vw, uint32_t *vw32,
                                                       int32_t *newdeg, int32_t *epos_new, int *err,
-                                                      int *hiflag, uint8_t *wrow) {
+                                                      int *hiflag) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64 *vals = reinterpret_cast<u64 *>(smem_raw);
     int32_t *keys = reinterpret_cast<int32_t *>(vals + CAPMAX);
@@ -283,10 +280,7 @@ __global__ void __launch_bounds__(T) merge_cta_kernel(const int32_t *__restrict_
                 vkey[pos] = key;
                 vw[pos] = x;
                 vw32[pos] = x < W32_ESC ? (uint32_t)x : W32_ESC;
-                if (key != self && x >= W32_ESC) {   // the self-loop is read as uint64 only
-                    atomicOr(hiflag, 1);
-                    wrow[self] = 1;
-                }
+                if (key != self && x >= W32_ESC) atomicOr(hiflag, 1);   // the self-loop is read as uint64 only
                 keys[s] = -1;
                 vals[s] = 0;
             }
@@ -314,7 +308,7 @@ __global__ void __launch_bounds__(T) merge_cta_narrow_kernel(const int32_t *__re
                                                              const int32_t *__restrict__ newid,
                                                              int32_t *vkey, u64 *vw, uint32_t *vw32,
                                                              int32_t *newdeg, int32_t *epos_new, int *err,
-                                                             int *hiflag, uint8_t *wrow) {
+                                                             int *hiflag) {
     static_assert(CAPMAX / 2 <= PIECE_MAX_ADDS, "a community's entries fit the piece counters");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PieceTable t;
@@ -350,10 +344,7 @@ __global__ void __launch_bounds__(T) merge_cta_narrow_kernel(const int32_t *__re
                 vkey[pos] = key;
                 vw[pos] = x;
                 vw32[pos] = x < W32_ESC ? (uint32_t)x : W32_ESC;
-                if (x >= W32_ESC) {
-                    atomicOr(hiflag, 1);
-                    wrow[self] = 1;
-                }
+                if (x >= W32_ESC) atomicOr(hiflag, 1);
                 t.keys[s] = -1;
                 t.lo[s] = 0;
                 t.hi[s] = 0;
@@ -530,7 +521,7 @@ __global__ void __launch_bounds__(256) mergeg_emit_kernel(HubGlobal hg,
                                                           const int32_t *__restrict__ P,
                                                           const int32_t *__restrict__ newid,
                                                           int32_t *vkey, u64 *vw, uint32_t *vw32,
-                                                          int *hiflag, uint8_t *wrow) {
+                                                          int *hiflag) {
     const int32_t bidx = blockIdx.x;
     const int32_t h = hg.schunk_hub[bidx];
     const int32_t c = hg.hubs[h];
@@ -552,10 +543,7 @@ __global__ void __launch_bounds__(256) mergeg_emit_kernel(HubGlobal hg,
         if (key != self && x >= W32_ESC) hi = 1;   // the self-loop is read as uint64 only
         tbl[sl] = GSlot{0u, 0u, 0};
     }
-    if (hi) {
-        atomicOr(hiflag, 1);
-        wrow[self] = 1;
-    }
+    if (hi) atomicOr(hiflag, 1);
 }
 
 __global__ void mergeg_finish_kernel(HubGlobal hg, const int32_t *__restrict__ mstart,
@@ -674,38 +662,38 @@ void agg_new_vertices(const int32_t *size, const u64 *S, int32_t V, const AggBuf
 }
 
 void agg_merge_class(int acls, const AggBuffers &ab, const int32_t *P, const int32_t *list,
-                     int32_t n, int32_t *vkey, u64 *vw, uint32_t *vw32, int *err, int *hiflag, uint8_t *wrow,
+                     int32_t n, int32_t *vkey, u64 *vw, uint32_t *vw32, int *err, int *hiflag,
                      int sms, cudaStream_t s, bool narrow) {
     if (n <= 0) return;
     switch (acls) {
     case AC1:
         merge_group_kernel<8, 64><<<nblocks(n, 32), 256, 0, s>>>(list, n, ab.mstart, P, ab.flag, vkey,
-                                                                  vw, vw32, ab.newdeg, ab.epos_new, err, hiflag, wrow); note_launches(1);
+                                                                  vw, vw32, ab.newdeg, ab.epos_new, err, hiflag); note_launches(1);
         break;
     case AC2:
         merge_group_kernel<32, 256><<<nblocks(n, 8), 256, 0, s>>>(list, n, ab.mstart, P, ab.flag, vkey,
-                                                                   vw, vw32, ab.newdeg, ab.epos_new, err, hiflag, wrow); note_launches(1);
+                                                                   vw, vw32, ab.newdeg, ab.epos_new, err, hiflag); note_launches(1);
         break;
     case AC3:
         if (narrow)
             merge_cta_narrow_kernel<A3_T, A3_CAP><<<(unsigned)imin64(n, (int64_t)sms * g_occ_a3), A3_T, A3_CAP * 12,
                                                     s>>>(list, n, ab.mstart, P, ab.flag, vkey, vw, vw32, ab.newdeg,
-                                                         ab.epos_new, err, hiflag, wrow);
+                                                         ab.epos_new, err, hiflag);
         else
             merge_cta_kernel<A3_T, A3_CAP><<<(unsigned)imin64(n, (int64_t)sms * g_occ_a3), A3_T,
                                              A3_CAP * 12, s>>>(list, n, ab.mstart, P, ab.flag, vkey, vw, vw32,
-                                                               ab.newdeg, ab.epos_new, err, hiflag, wrow);
+                                                               ab.newdeg, ab.epos_new, err, hiflag);
         note_launches(1);
         break;
     case AC4:
         if (narrow)
             merge_cta_narrow_kernel<A4_T, A4_CAP><<<(unsigned)imin64(n, (int64_t)sms * g_occ_a4), A4_T, A4_CAP * 12,
                                                     s>>>(list, n, ab.mstart, P, ab.flag, vkey, vw, vw32, ab.newdeg,
-                                                         ab.epos_new, err, hiflag, wrow);
+                                                         ab.epos_new, err, hiflag);
         else
             merge_cta_kernel<A4_T, A4_CAP><<<(unsigned)imin64(n, (int64_t)sms * g_occ_a4), A4_T,
                                              A4_CAP * 12, s>>>(list, n, ab.mstart, P, ab.flag, vkey, vw, vw32,
-                                                               ab.newdeg, ab.epos_new, err, hiflag, wrow);
+                                                               ab.newdeg, ab.epos_new, err, hiflag);
         note_launches(1);
         break;
     default: break;
@@ -713,7 +701,7 @@ void agg_merge_class(int acls, const AggBuffers &ab, const int32_t *P, const int
 }
 
 void agg_merge_global(const HubGlobal &hg, const AggBuffers &ab, const int32_t *P, int32_t *vkey,
-                      u64 *vw, uint32_t *vw32, int *err, int *hiflag, uint8_t *wrow, cudaStream_t s,
+                      u64 *vw, uint32_t *vw32, int *err, int *hiflag, cudaStream_t s,
                       bool narrow) {
     if (hg.nhubs <= 0) return;
     // the per-community list lengths are zero between uses; cleared here too
@@ -726,7 +714,7 @@ void agg_merge_global(const HubGlobal &hg, const AggBuffers &ab, const int32_t *
         mergeg_insert_kernel<<<hg.n_echunks, HG_INSERT_THREADS, HG_INSERT_SMEM, s>>>(hg, ab.mstart, P, ab.flag, vkey,
                                                                                      vw, err);
     note_launches(1);
-    mergeg_emit_kernel<<<hg.n_schunks, 256, 0, s>>>(hg, ab.mstart, P, ab.flag, vkey, vw, vw32, hiflag, wrow); note_launches(1);
+    mergeg_emit_kernel<<<hg.n_schunks, 256, 0, s>>>(hg, ab.mstart, P, ab.flag, vkey, vw, vw32, hiflag); note_launches(1);
     mergeg_finish_kernel<<<grid_for(hg.nhubs), 256, 0, s>>>(hg, ab.mstart, P, ab.flag, ab.newdeg, ab.epos_new); note_launches(1);
 }
 

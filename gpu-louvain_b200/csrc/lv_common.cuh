@@ -207,9 +207,9 @@ struct GraphView {
 
 // The 32-bit copy of an aggregated level holds each sum below W32_ESC as it
 // is and W32_ESC (an escape) for larger ones, whose exact value is read from
-// the uint64 sums.  A row with an escaped entry other than its self-loop is
-// marked (lv_handle::wrow) and decided by the 64-bit kernels, so the
-// piece-counter tables only ever see weights below 2^32.
+// the uint64 sums.  The move phase reads the copy only when no entry but
+// self-loops, which it skips, is escaped, so the piece-counter tables only ever
+// see weights below 2^32.
 constexpr uint32_t W32_ESC = 0xFFFFFFFFu;
 
 // Exact weight of entry e of a level's row.
@@ -349,8 +349,6 @@ struct StateView {
     u64 T;
     int *err;
     float *feat;   // learned active set: 2 features per vertex, written when set
-    const uint8_t *wrow;   // rows with a weight of 2^32 or more (nullptr: none); such a
-                           // vertex is decided by the large fallback queue (64-bit sums)
     // the sub-round's movers: mv_cnt holds their count (low half) and their row
     // units of 32 entries (high half); mv_list has four arrays of mv_stride
     // words: the movers, the units before each, and, by vertex, the community

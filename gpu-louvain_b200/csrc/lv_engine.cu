@@ -33,10 +33,10 @@ void agg_permute(int cls, const GraphView<WT> &g, const AggBuffers &ab, const in
 void agg_new_vertices(const int32_t *size, const u64 *S, int32_t V, const AggBuffers &ab,
                       const int32_t *P, u64 *knew, cudaStream_t s);
 void agg_merge_class(int acls, const AggBuffers &ab, const int32_t *P, const int32_t *list,
-                     int32_t n, int32_t *vkey, u64 *vw, uint32_t *vw32, int *err, int *hiflag, uint8_t *wrow,
+                     int32_t n, int32_t *vkey, u64 *vw, uint32_t *vw32, int *err, int *hiflag,
                      int sms, cudaStream_t s, bool narrow);
 void agg_merge_global(const HubGlobal &hg, const AggBuffers &ab, const int32_t *P, int32_t *vkey,
-                      u64 *vw, uint32_t *vw32, int *err, int *hiflag, uint8_t *wrow, cudaStream_t s,
+                      u64 *vw, uint32_t *vw32, int *err, int *hiflag, cudaStream_t s,
                       bool narrow);
 void agg_row_bounds(const AggBuffers &ab, int32_t Vn, int32_t *start, int32_t *end, cudaStream_t s);
 void launch_gather_degrees(const int32_t *rowptr, const int32_t *rowend, const int32_t *list,
@@ -47,15 +47,6 @@ void launch_gather_cdeg(const int32_t *mstart, const int32_t *P, const int32_t *
 
 using namespace lv;
 
-// Aggregated levels holding a sum of 2^32 or more: swept with the 64-bit
-// kernels on the uint64 sums (0), through the 32-bit view with the narrow
-// (piece-table) kernels and those rows sent to the large queue (1), or
-// through the 32-bit view with the 64-bit-table kernels, escaped sums read
-// from the uint64 copy (2).  0 is the default: on R-MAT-24 the move phase of
-// a run took 241 ms in mode 0, 262 ms in mode 1 (the piece tables' two
-// atomics per add serialise where many lanes add to one community) and
-// 256 ms in mode 2 (the escape test per entry costs more than the 4 bytes
-// per entry it saves).
 // Table sweeps (lv_nct.cuh), see where they are used below; settable so that
 // small graphs can be run through them.
 #ifndef LV_NCT_MIN_ENTRIES
@@ -66,9 +57,6 @@ using namespace lv;
 #endif
 #ifndef LV_NCT_MAX_SLOTS
 #define LV_NCT_MAX_SLOTS 0.3
-#endif
-#ifndef LV_NARROW_ESCAPES
-#define LV_NARROW_ESCAPES 0
 #endif
 
 namespace {
@@ -140,11 +128,16 @@ struct lv_handle {
     // current level: row v = cur_col/cur_w[cur_rowptr[v] .. cur_rowend[v])
     int32_t *cur_rowptr = nullptr, *cur_rowend = nullptr, *cur_col = nullptr;
     u64 *cur_w = nullptr;   // nullptr at level 0 (float input weights)
-    uint32_t *cur_w32 = nullptr;   // 32-bit copy of cur_w (sums of 2^32 or more escaped to
-                                   // cur_w); the move kernels read it, the modularity
-                                   // pass and the aggregation read cur_w
-    uint8_t *wrow = nullptr;       // [V0] current level: row holds a non-self-loop sum >= 2^32
-    bool wrows_any = false;
+    // 32-bit copy of cur_w: the move kernels read it, the modularity pass and
+    // the aggregation read cur_w.  nullptr when the level holds a sum of 2^32 or
+    // more outside the self-loops: it is swept with the 64-bit kernels on the
+    // uint64 sums.  Both other ways were slower (move phase of an R-MAT-24 run
+    // 241 ms): the 32-bit copy with those rows in the large queue 262 ms (the
+    // piece tables' two atomics per add serialise where many lanes add to one
+    // community), the 32-bit copy with 64-bit tables and the escaped sums read
+    // from the uint64 ones 256 ms (the escape test per entry costs more than the
+    // 4 bytes that it saves).
+    uint32_t *cur_w32 = nullptr;
 
     // aggregated levels, ping-pong: rows stay where the merge wrote them
     int32_t *lvl_start[2] = {nullptr, nullptr};
@@ -396,16 +389,13 @@ GraphView<uint32_t> view_of<uint32_t>(lv_handle *h) {
 template <typename WT>
 bool narrow_weights(const lv_handle *h) {
     if (h->opts.wide_weights) return false;
-    // the 32-bit view of a level holding escaped sums: narrow kernels (with
-    // the marked rows sent to the large queue) only in mode 1
-    if (std::is_same<WT, uint32_t>::value) return LV_NARROW_ESCAPES == 1 || !h->wrows_any;
+    if (std::is_same<WT, uint32_t>::value) return true;
     if (std::is_same<WT, float>::value) return h->w0_narrow;
     return false;
 }
 
 StateView state_of(lv_handle *h) {
     return StateView{h->comm, h->newc, h->size, h->k, h->S, h->T, &h->tot_d->err, h->feat,
-                     (LV_NARROW_ESCAPES == 1 && h->cur_w32 && h->wrows_any) ? h->wrow : nullptr,
                      h->blk_d->movers, h->mv_list, h->V0, 0, nullptr, nullptr,
                      (LV_DEDUP == 2 || (LV_DEDUP == 1 && h->level > 0)) ? 1 : 0};
 }
@@ -772,8 +762,7 @@ void enqueue_sweep(lv_handle *h) {
             tc->sbytes = (8.0 + wbytes) * (double)edges + 20.0 * (double)(hg0 - lo);
         }
         if (b < 4)
-            launch_move_class<WT>(b, g, st, h->list + lo, hi - lo, h->di, dE, h->stream, narrow_weights<WT>(h),
-                                  fs);
+            launch_move_class<WT>(b, g, st, h->list + lo, hi - lo, dE, h->stream, narrow_weights<WT>(h));
         else if (hg0 > lo)
             launch_move_wide<WT>(g, st, h->list + lo, hg0 - lo, fs, h->di, dE, h->stream,
                                  b == 6 ? h->giant_degree : (b == 4 ? 84 : 319), narrow_weights<WT>(h),
@@ -825,7 +814,7 @@ void enqueue_sweep_tables(lv_handle *h) {
         st.mv_cnt = h->blk_d->movers + b;
         next_round(h, st);
         if (b < 4) {
-            launch_move_class<WT>(b, g, st, h->list + lo, hi - lo, h->di, dE, h->stream, narrow_weights<WT>(h), fs);
+            launch_move_class<WT>(b, g, st, h->list + lo, hi - lo, dE, h->stream, narrow_weights<WT>(h));
         } else {
             // rows of bucket 4 never hold more communities than a warp builds
             NctView t = h->nct;
@@ -1181,8 +1170,8 @@ void enqueue_sweep_active(lv_handle *h, const int32_t *cnt) {
         st.mv_cnt = h->blk_d->movers + b;
         next_round(h, st);
         if (b < 4) {
-            launch_move_class<WT>(b, g, st, h->alist + h->cls_off[b], cnt[b], h->di, dE, h->stream,
-                                  narrow_weights<WT>(h), queues_on(h, 3));
+            launch_move_class<WT>(b, g, st, h->alist + h->cls_off[b], cnt[b], dE, h->stream,
+                                  narrow_weights<WT>(h));
         } else {
             for (int c = c0; c < c1; ++c) {
                 if (c == CLS_HG || !cnt[c]) continue;
@@ -1412,7 +1401,6 @@ int ensure_agg(lv_handle *h) {
         LV_TRY(dalloc(h, &h->lvl_w[b], E));
         LV_TRY(dalloc(h, &h->lvl_w32[b], E));
     }
-    LV_TRY(dalloc(h, &h->wrow, V + 1));
     h->agg_ready = true;
     return LV_OK;
 }
@@ -1430,7 +1418,7 @@ int aggregate_t(lv_handle *h) {
     int32_t *hiflag = ab.scalars + 12;   // set when a merged sum is 2^32 or more
     // the permuted inter-community weights are the current level's
     // non-self-loop weights: below 2^32 when the move phase reads them narrow
-    const bool narrow = h->cur_w32 ? !h->wrows_any : narrow_weights<WT>(h);
+    const bool narrow = h->cur_w32 || narrow_weights<WT>(h);
     agg_prepare(h->cur_rowptr, h->cur_rowend, h->comm, h->size, V, ab, h->mslot, h->degm, h->P,
                 h->stream);
     LV_CUDA(h, cudaMemcpyAsync(h->small_h, ab.scalars, sizeof(int32_t) * (2 + NAC),
@@ -1458,11 +1446,10 @@ int aggregate_t(lv_handle *h) {
                         h->cls_off[c + 1] - h->cls_off[c], vkey, vw, h->di.sms, h->stream);
     agg_new_vertices(h->size, h->S, V, ab, h->P, h->k, h->stream);
     LV_CUDA(h, cudaMemsetAsync(hiflag, 0, sizeof(int32_t), h->stream));
-    LV_CUDA(h, cudaMemsetAsync(h->wrow, 0, (size_t)newV + 1, h->stream));
     for (int c = 0; c < NAC - 1; ++c)
         agg_merge_class(c, ab, h->P, ab.clist + aoff[c], aoff[c + 1] - aoff[c], vkey, vw, vw32,
-                        &h->tot_d->err, hiflag, h->wrow, h->di.sms, h->stream, narrow);
-    agg_merge_global(h->hub_agg.view, ab, h->P, vkey, vw, vw32, &h->tot_d->err, hiflag, h->wrow, h->stream,
+                        &h->tot_d->err, hiflag, h->di.sms, h->stream, narrow);
+    agg_merge_global(h->hub_agg.view, ab, h->P, vkey, vw, vw32, &h->tot_d->err, hiflag, h->stream,
                      narrow);
     agg_row_bounds(ab, newV, h->lvl_start[nb], h->lvl_end[nb], h->stream);
     // E' = number of stored entries (P is free again after the merges)
@@ -1479,14 +1466,12 @@ int aggregate_t(lv_handle *h) {
                      h->st.aggregate_ms);
     LV_TRY(check_device_error(h, h->tot_h->err));
     const int64_t newE = h->small_h[0];
-    h->wrows_any = h->small_h[1] != 0;
     h->cur_buf = nb;
     h->cur_rowptr = h->lvl_start[nb];
     h->cur_rowend = h->lvl_end[nb];
     h->cur_col = h->lvl_col[nb];
     h->cur_w = h->lvl_w[nb];
-    // mode 0: a level with escaped sums is swept on its uint64 sums
-    h->cur_w32 = (h->opts.wide_weights || (LV_NARROW_ESCAPES == 0 && h->wrows_any)) ? nullptr : h->lvl_w32[nb];
+    h->cur_w32 = h->opts.wide_weights || h->small_h[1] ? nullptr : h->lvl_w32[nb];
     h->V = newV;
     h->E = newE;
     h->level += 1;
@@ -1578,7 +1563,6 @@ int team_finish(lv_handle *h, double min_gain, double *q, int *done) {
         h->cur_col = rows.col[r->cur];
         h->cur_w = rows.w64[r->cur];
         h->cur_w32 = nullptr;
-        h->wrows_any = false;
         h->cur_buf = -1;
     }
     h->e_own_valid = false;
@@ -1601,7 +1585,6 @@ int to_level0(lv_handle *h) {
     h->cur_col = h->in_col;
     h->cur_w = nullptr;
     h->cur_w32 = nullptr;
-    h->wrows_any = false;
     h->cur_buf = -1;
     h->e_own_valid = false;
     launch_iota_i32(h->orig2comm, h->V0, h->stream);

@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(256) move_group_kernel(GraphView<WT> g, StateV
 template <int G, int CAP, typename WT>
 __global__ void __launch_bounds__(256) move_group_narrow_kernel(GraphView<WT> g, StateView st,
                                                                 const int32_t *__restrict__ list,
-                                                                int32_t n, u64 *dE, Fallback fbl) {
+                                                                int32_t n, u64 *dE) {
     pdl_trigger();
     constexpr int GPB = 256 / G;
     constexpr int LG = ilog2_c(CAP);
@@ -166,21 +166,16 @@ __global__ void __launch_bounds__(256) move_group_narrow_kernel(GraphView<WT> g,
     for (int s = lane; s < CAP; s += G) { t.keys[s] = -1; t.lo[s] = 0; t.hi[s] = 0; }
     __syncwarp();
     pdl_wait();
-    bool active = idx < n;
+    const bool active = idx < n;
     int32_t v = 0, own = 0, r0 = 0, r1 = 0;
     u64 e_own = 0;
     if (active) {
-        // the row bounds, the community and the wide-row flag are loaded
-        // together (none depends on another)
+        // the row bounds and the community are loaded together (none depends
+        // on another)
         v = list[idx];
         r0 = g.rowptr[v];
         r1 = g.rowend[v];
         own = ld_coherent(st.comm + v);
-        if (st.wrow && st.wrow[v]) {
-            // a row with a sum of 2^32 or more: decided by the large queue
-            if (lane == 0) enqueue_large(fbl, v, r1 - r0, st.err);
-            active = false;
-        }
     }
     if (active)
         insert_row_piece<(CAP > 32 ? LV_U_CTA : LV_U_GROUP), false, true>(g, st.comm, v, own, r0, r1, lane, G, t, LG,
@@ -540,17 +535,14 @@ __global__ void __launch_bounds__(256) move_warp_narrow_kernel(GraphView<WT> g, 
     if (lane == 0) idx = atomicAdd(fs.warp_next, 1);
     idx = __shfl_sync(FULL, idx, 0);
     int32_t nv = 0, nr0 = 0, nr1 = 0, nown = 0;
-    bool nwide = false;
     if (idx < n) {
         nv = list[idx];
         nr0 = g.rowptr[nv];
         nr1 = g.rowend[nv];
         nown = __ldg(st.comm + nv);
-        nwide = st.wrow && st.wrow[nv];
     }
     while (idx < n) {
         const int32_t v = nv, r0 = nr0, r1 = nr1, own = nown;
-        const bool wide = nwide;
         int32_t nidx = 0;
         if (lane == 0) nidx = atomicAdd(fs.warp_next, 1);
         nidx = __shfl_sync(FULL, nidx, 0);
@@ -559,14 +551,9 @@ __global__ void __launch_bounds__(256) move_warp_narrow_kernel(GraphView<WT> g, 
             nr0 = g.rowptr[nv];
             nr1 = g.rowend[nv];
             nown = __ldg(st.comm + nv);
-            nwide = st.wrow && st.wrow[nv];
         }
         idx = nidx;
         const int32_t d = r1 - r0;
-        if (wide) {   // a sum of 2^32 or more: 64-bit sums in the large queue
-            if (lane == 0) enqueue_large(fs.q[NFBQ], v, d, st.err);
-            continue;
-        }
         if (d > fs.warp_limit && fs.hint[v]) {
             if (lane == 0) enqueue_fallback(fs, v, d, st.err);
             continue;
@@ -1248,7 +1235,6 @@ __global__ void __launch_bounds__(STAGE_THREADS) giant_stage_narrow_kernel(Graph
     for (int32_t ch = blockIdx.x; ch < hg.n_echunks; ch += gridDim.x) {
         const int32_t h = hg.echunk_hub[ch];
         const int32_t v = hg.hubs[h];
-        if (st.wrow && st.wrow[v]) continue;   // staged by giant_stage_kernel (64-bit sums)
         if (st.tlg && st.tlg[v] != NCT_NEVER) continue;   // decided from its table
         const int32_t r1 = g.rowend[v];
         const int32_t e0 = g.rowptr[v] + hg.echunk_e0[ch];
@@ -1279,11 +1265,9 @@ __global__ void __launch_bounds__(STAGE_THREADS) giant_stage_narrow_kernel(Graph
 
 template <typename WT>
 __global__ void __launch_bounds__(STAGE_THREADS) giant_stage_kernel(GraphView<WT> g, StateView st,
-                                                                    HubGlobal hg, const uint8_t *only) {
-    // only != nullptr: just the giants marked there (the rest are staged by
-    // the narrow kernel).  Persistent over the chunks, as the narrow kernel:
-    // the table is initialised once and after each chunk only its claimed
-    // slots are cleared.
+                                                                    HubGlobal hg) {
+    // Persistent over the chunks, as the narrow kernel: the table is initialised
+    // once and after each chunk only its claimed slots are cleared.
     if (st.tnever && *st.tnever == 0) return;   // every giant has its table
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int LCAP = 2 * STAGE_CHUNK;
@@ -1298,7 +1282,6 @@ __global__ void __launch_bounds__(STAGE_THREADS) giant_stage_kernel(GraphView<WT
     for (int32_t ch = blockIdx.x; ch < hg.n_echunks; ch += gridDim.x) {
         const int32_t h = hg.echunk_hub[ch];
         const int32_t v = hg.hubs[h];
-        if (only && !only[v]) continue;
         if (st.tlg && st.tlg[v] != NCT_NEVER) continue;   // decided from its table
         const int32_t r1 = g.rowend[v];
         const int32_t e0 = g.rowptr[v] + hg.echunk_e0[ch];
@@ -1835,20 +1818,13 @@ static void launch_fallback_large(const GraphView<WT> &g, const StateView &st, c
 
 template <typename WT>
 void launch_move_class(int cls, const GraphView<WT> &g, const StateView &st, const int32_t *list,
-                       int32_t n, const DeviceInfo &di, u64 *dE, cudaStream_t s, bool narrow,
-                       const FallbackSet &fs) {
+                       int32_t n, u64 *dE, cudaStream_t s, bool narrow) {
     if (n <= 0) return;
-    // rows marked in st.wrow go to the large queue, decided right after
-    const bool large = narrow && st.wrow;
-    if (large) {
-        cudaMemsetAsync(fs.q[NFBQ].count, 0, 2 * sizeof(int32_t), s);   // count, next
-        cudaMemsetAsync(fs.q[NFBQ].done, 0, sizeof(int32_t) * (size_t)fs.q[NFBQ].cap, s);
-    }
 #define LV_GROUP(G, CAP)                                                                              \
     do {                                                                                              \
         if (narrow)                                                                                   \
             launch_pdl((move_group_narrow_kernel<G, CAP, WT>), nblocks(n, 256 / G), 256, 0, s, g, st, list, n, \
-                       dE, fs.q[NFBQ]);                                                               \
+                       dE);                                                                           \
         else                                                                                          \
             launch_pdl((move_group_kernel<G, CAP, WT>), nblocks(n, 256 / G), 256, 0, s, g, st, list, n, dE); \
         note_launches(1);                                                                             \
@@ -1861,7 +1837,6 @@ void launch_move_class(int cls, const GraphView<WT> &g, const StateView &st, con
     default: break;
     }
 #undef LV_GROUP
-    if (large) launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
 }
 
 template <typename WT>
@@ -1880,14 +1855,9 @@ void launch_move_giants(const GraphView<WT> &g, const StateView &st, const HubGl
         giant_stage_narrow_kernel<WT><<<(unsigned)imin64(hg.n_echunks, (int64_t)di.sms * di.occ_stage_narrow),
                                         STAGE_THREADS, STAGE_SMEM, s>>>(g, st, hg);
         note_launches(1);
-        if (st.wrow) {
-            giant_stage_kernel<WT><<<(unsigned)imin64(hg.n_echunks, (int64_t)di.sms * di.occ_stage), STAGE_THREADS,
-                                     STAGE_SMEM, s>>>(g, st, hg, st.wrow);
-            note_launches(1);
-        }
     } else {
         giant_stage_kernel<WT><<<(unsigned)imin64(hg.n_echunks, (int64_t)di.sms * di.occ_stage), STAGE_THREADS,
-                                 STAGE_SMEM, s>>>(g, st, hg, nullptr);
+                                 STAGE_SMEM, s>>>(g, st, hg);
         note_launches(1);
     }
     if (LV_GIANT_REGROUP && hg.poff) {
@@ -1931,29 +1901,26 @@ void launch_move_wide(const GraphView<WT> &g, const StateView &st, const int32_t
                       const FallbackSet &fs, const DeviceInfo &di, u64 *dE, cudaStream_t s,
                       int32_t max_degree, bool narrow, bool large_later) {
     if (n <= 0) return;
-    if (!st.wrow) {
-        // Few rows: a warp per row leaves the GPU to the longest rows' latency
-        // (LFR graph of 300,007 vertices, 655 rows of 320 to 2000 entries: 67
-        // us).  So rows of up to 84 entries go to groups of 32 lanes with a
-        // table of 256 slots (no queue), longer ones to a CTA each.
-        if (max_degree <= 84 && n <= di.sms * SMALL_B4_PER_SM) {
-            if (narrow)
-                launch_pdl((move_group_narrow_kernel<32, 256, WT>), nblocks(n, 8), 256, 0, s, g, st, list, n, dE,
-                           fs.q[NFBQ]);
-            else
-                launch_pdl((move_group_kernel<32, 256, WT>), nblocks(n, 8), 256, 0, s, g, st, list, n, dE);
-            note_launches(1);
-            return;
-        }
-        if (max_degree > 84 && max_degree <= FBQ_MAXDEG(0) && n <= di.sms * SMALL_B5_PER_SM) {
-            launch_row_queue<WT, 0>(g, st, fs, di, dE, s, narrow, list, n);
-            return;
-        }
-        if (max_degree > FBQ_MAXDEG(0) && n <= di.sms * SMALL_B6_PER_SM) {
-            launch_row_queue<WT, NFBQ - 1>(g, st, fs, di, dE, s, narrow, list, n);
-            if (!large_later) launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
-            return;
-        }
+    // Few rows: a warp per row leaves the GPU to the longest rows' latency
+    // (LFR graph of 300,007 vertices, 655 rows of 320 to 2000 entries: 67
+    // us).  So rows of up to 84 entries go to groups of 32 lanes with a
+    // table of 256 slots (no queue), longer ones to a CTA each.
+    if (max_degree <= 84 && n <= di.sms * SMALL_B4_PER_SM) {
+        if (narrow)
+            launch_pdl((move_group_narrow_kernel<32, 256, WT>), nblocks(n, 8), 256, 0, s, g, st, list, n, dE);
+        else
+            launch_pdl((move_group_kernel<32, 256, WT>), nblocks(n, 8), 256, 0, s, g, st, list, n, dE);
+        note_launches(1);
+        return;
+    }
+    if (max_degree > 84 && max_degree <= FBQ_MAXDEG(0) && n <= di.sms * SMALL_B5_PER_SM) {
+        launch_row_queue<WT, 0>(g, st, fs, di, dE, s, narrow, list, n);
+        return;
+    }
+    if (max_degree > FBQ_MAXDEG(0) && n <= di.sms * SMALL_B6_PER_SM) {
+        launch_row_queue<WT, NFBQ - 1>(g, st, fs, di, dE, s, narrow, list, n);
+        if (!large_later) launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
+        return;
     }
     if (narrow) {
         const unsigned grid = (unsigned)imin64((n + 7) / 8, (int64_t)di.sms * di.occ_warp_narrow);
@@ -1964,7 +1931,6 @@ void launch_move_wide(const GraphView<WT> &g, const StateView &st, const int32_t
     }
     note_launches(1);
     if (max_degree <= fs.warp_limit) {   // no vertex can overflow its warp table
-        if (narrow && st.wrow) launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
         return;
     }
     if (!large_later) launch_fallback_large<WT>(g, st, HubGlobal(), fs, di, dE, s);
@@ -2066,12 +2032,10 @@ void launch_s2(const u64 *S, int32_t V, u64 *total_hi_lo, cudaStream_t s) {
     note_launches(1);
 }
 
-template void launch_move_class<float>(int, const GraphView<float> &, const StateView &,
-                                       const int32_t *, int32_t, const DeviceInfo &, u64 *,
-                                       cudaStream_t, bool, const FallbackSet &);
-template void launch_move_class<u64>(int, const GraphView<u64> &, const StateView &,
-                                     const int32_t *, int32_t, const DeviceInfo &, u64 *,
-                                     cudaStream_t, bool, const FallbackSet &);
+template void launch_move_class<float>(int, const GraphView<float> &, const StateView &, const int32_t *, int32_t, u64 *,
+                                       cudaStream_t, bool);
+template void launch_move_class<u64>(int, const GraphView<u64> &, const StateView &, const int32_t *, int32_t, u64 *,
+                                       cudaStream_t, bool);
 template void launch_move_wide<float>(const GraphView<float> &, const StateView &, const int32_t *,
                                       int32_t, const FallbackSet &, const DeviceInfo &, u64 *,
                                       cudaStream_t, int32_t, bool, bool);
@@ -2106,9 +2070,8 @@ template void launch_row_reduce<u64>(int, int, const GraphView<u64> &, const int
                                      u64 *, const int32_t *, int32_t, const DeviceInfo &,
                                      cudaStream_t);
 
-template void launch_move_class<uint32_t>(int, const GraphView<uint32_t> &, const StateView &,
-                                     const int32_t *, int32_t, const DeviceInfo &, u64 *,
-                                     cudaStream_t, bool, const FallbackSet &);
+template void launch_move_class<uint32_t>(int, const GraphView<uint32_t> &, const StateView &, const int32_t *, int32_t, u64 *,
+                                       cudaStream_t, bool);
 template void launch_move_wide<uint32_t>(const GraphView<uint32_t> &, const StateView &, const int32_t *,
                                     int32_t, const FallbackSet &, const DeviceInfo &, u64 *,
                                     cudaStream_t, int32_t, bool, bool);
