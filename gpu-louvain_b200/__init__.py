@@ -91,7 +91,7 @@ EXPORTED = [
     "lv_gen_lfr", "lv_set_active_model", "lv_get_traces", "lv_get_active_stats", "lv_active_train",
     "lv_active_predict", "lv_write_csr", "lv_read_csr", "lv_write_csr_stamped", "lv_read_csr_stamp", "lv_gen_planted_batch", "lv_read_mtx_device",
     "lv_csr_from_entries_device", "lv_read_mtx_entries", "lv_get_level_classes", "lv_get_device_name",
-    "lv_read_active_model", "lv_set_test_limits",
+    "lv_read_active_model", "lv_set_test_limits", "lv_get_table_stats",
 ]
 
 _lib = None
@@ -136,7 +136,8 @@ def lib() -> C.CDLL:
     L.lv_get_communities.argtypes = [C.c_void_p, P32]
     L.lv_set_communities.argtypes = [C.c_void_p, P32]
     L.lv_get_level_info.argtypes = [C.c_void_p, P32, P64, P32]
-    L.lv_set_test_limits.argtypes = [C.c_void_p, C.c_int32]
+    L.lv_set_test_limits.argtypes = [C.c_void_p, C.c_int32, C.c_int64]
+    L.lv_get_table_stats.argtypes = [C.c_void_p, P64, P64, P64, P32, P32]
     L.lv_get_csr.argtypes = [C.c_void_p, P32, P32, P64]
     L.lv_get_scale.argtypes = [C.c_void_p, P32, C.POINTER(C.c_uint64), P32]
     L.lv_get_stats.argtypes = [C.c_void_p, C.POINTER(_Stats)]
@@ -517,9 +518,17 @@ class Louvain:
         self._c(lib().lv_sweep(self._h, C.byref(m)))
         return m.value
 
-    def set_test_limits(self, fail_alloc: int = 0) -> None:
-        """Test hook: the fail_alloc-th device allocation from now on fails."""
-        self._c(lib().lv_set_test_limits(self._h, fail_alloc))
+    def set_test_limits(self, fail_alloc: int = 0, table_slots: int = 0) -> None:
+        """Test hook: the fail_alloc-th device allocation from now on fails; at
+        most table_slots slots for the tables of late sweeps."""
+        self._c(lib().lv_set_test_limits(self._h, fail_alloc, table_slots))
+
+    def table_stats(self) -> dict:
+        """Late sweeps from neighbour-community tables (lv_get_table_stats)."""
+        sw, sl, wo, fu, st = C.c_int64(), C.c_int64(), C.c_int64(), C.c_int32(), C.c_int32()
+        self._c(lib().lv_get_table_stats(self._h, C.byref(sw), C.byref(sl), C.byref(wo), C.byref(fu), C.byref(st)))
+        return {"sweeps": sw.value, "slots": sl.value, "without": wo.value, "pool_full": bool(fu.value),
+                "stale": bool(st.value)}
 
     # -- state access --
     def level_info(self):

@@ -179,6 +179,9 @@ struct lv_handle {
     void *loop_d = nullptr;        // device state of the sweep loop
     NctView nct;                   // neighbour-community tables (late sweeps)
     u64 nct_alloc = 0;             // slots allocated in the pool
+    int64_t table_limit = 0;       // test hook: most slots of the pool (0: the default)
+    int64_t table_sweeps = 0, table_slots = 0, table_without = 0;   // lv_get_table_stats
+    int32_t table_full = 0, table_stale = 0;
 
     // level_setup not run yet for the current level: the state arrays are
     // unset (SETUP_ALL) or a team run set them and only the class lists are
@@ -803,10 +806,7 @@ void enqueue_sweep_tables(lv_handle *h) {
     StateView st = state_of(h);
     st.tlg = h->nct.lg;
     st.tnever = h->nct.cursor + 1;
-    const double wbytes = sizeof(WT) == 4 ? 4.0 : 8.0;
     u64 *dE = &h->tot_d->dE;
-    Timer tm(h, 100);
-    int64_t sweep_verts = 0;
     for (int b = 0; b < NBUCKETS; ++b) {
         const int32_t lo = h->cls_off[b], hi = b < 6 ? h->cls_off[b + 1] : h->cls_off[NCLS];
         if (hi == lo) continue;
@@ -829,12 +829,7 @@ void enqueue_sweep_tables(lv_handle *h) {
             launch_collect_movers<WT>(g, st, h->list + lo, hi - lo, h->stream);
         }
         launch_movers<WT>(g, st, hi - lo, h->di, dE, &h->tot_d->moves, h->stream, &h->nct);
-        sweep_verts += hi - lo;
     }
-    tm.bytes = 12.0 * (double)h->E + 20.0 * (double)sweep_verts;
-    tm.sbytes = (8.0 + wbytes) * (double)h->E + 20.0 * (double)sweep_verts;
-    tm.stop();
-    h->st.move_bytes += tm.bytes;
 }
 
 template <typename WT>
@@ -1025,11 +1020,12 @@ int nct_begin(lv_handle *h, int *ok) {
     NctView &t = h->nct;
     const size_t V = (size_t)h->V0 + 1;
     if ((!t.lg && !dalloc_optional(h, &t.lg, V)) || (!t.off && !dalloc_optional(h, &t.off, V)) ||
-        (!t.queue && !dalloc_optional(h, &t.queue, V)) || (!t.cursor && !dalloc_optional(h, &t.cursor, 2)))
+        (!t.queue && !dalloc_optional(h, &t.queue, V)) || (!t.cursor && !dalloc_optional(h, &t.cursor, 4)))
         return LV_OK;
     // half a slot per entry of the level: rows with many communities that do
     // not fit go on being summed from the row
-    const u64 want = (u64)h->E / 2 + 1024;
+    u64 want = (u64)h->E / 2 + 1024;
+    if (h->table_limit > 0 && want > (u64)h->table_limit) want = (u64)h->table_limit;
     if (want > h->nct_alloc) {
         dfree(h, t.slots);
         h->nct_alloc = 0;
@@ -1038,7 +1034,7 @@ int nct_begin(lv_handle *h, int *ok) {
     }
     h->nct.cap = want;
     LV_CUDA(h, cudaMemsetAsync(h->nct.lg, 0, (size_t)h->V, h->stream));
-    LV_CUDA(h, cudaMemsetAsync(h->nct.cursor, 0, 2 * sizeof(u64), h->stream));
+    LV_CUDA(h, cudaMemsetAsync(h->nct.cursor, 0, 4 * sizeof(u64), h->stream));
     *ok = 1;
     return LV_OK;
 }
@@ -1079,9 +1075,25 @@ int run_sweeps(lv_handle *h, bool tables, LoopState *ls) {
     LV_TRY(rc);
     LV_CUDA(h, cudaMemcpyAsync(ls, ld, sizeof(*ls), cudaMemcpyDeviceToHost, h->stream));
     LV_CUDA(h, cudaMemcpyAsync(h->tot_h, h->tot_d, sizeof(Totals), cudaMemcpyDeviceToHost, h->stream));
+    u64 *cur = reinterpret_cast<u64 *>(h->small_h);
+    if (tables)
+        LV_CUDA(h, cudaMemcpyAsync(cur, h->nct.cursor, 4 * sizeof(u64), cudaMemcpyDeviceToHost, h->stream));
     LV_TRY(sync(h));
     LV_TRY(check_device_error(h, h->tot_h->err));
     const int32_t ran = ls->sweeps - sweeps0;
+    if (tables) {
+        h->table_sweeps += ran;
+        cur[0] = std::min(cur[0], h->nct.cap);   // refused requests count as well
+        h->table_slots += (int64_t)cur[0];
+        h->table_without += (int64_t)cur[1];
+        if (cur[2]) h->table_full = 1;
+        if (cur[3]) h->table_stale = 1;
+        // rows of up to 32 entries every time, the others once and then their tables
+        double wide = 0;
+        for (int c = CLS_B4; c < NCLS; ++c) wide += (double)h->cls_edges[c];
+        h->st.move_bytes += ran * (12.0 * ((double)h->E - wide) + 20.0 * (double)h->V) + 12.0 * wide +
+                            (ran - 1) * sizeof(GSlot) * (double)cur[0];
+    }
     h->e_own_cur = ls->e_own;
     h->st.sweeps += ran;
     h->st.edge_sweeps += h->E * (int64_t)ran;
@@ -1940,9 +1952,21 @@ int lv_set_communities(lv_handle *h, const int32_t *comm) {
     return LV_OK;
 }
 
-int lv_set_test_limits(lv_handle *h, int32_t fail_alloc) {
-    if (!h || fail_alloc < 0) return LV_ERR_INVALID;
+int lv_set_test_limits(lv_handle *h, int32_t fail_alloc, int64_t table_slots) {
+    if (!h || fail_alloc < 0 || table_slots < 0) return LV_ERR_INVALID;
     h->mem.fail_at = fail_alloc;
+    h->table_limit = table_slots;
+    return LV_OK;
+}
+
+int lv_get_table_stats(lv_handle *h, int64_t *sweeps, int64_t *slots, int64_t *without, int32_t *pool_full,
+                       int32_t *stale) {
+    if (!h) return LV_ERR_INVALID;
+    if (sweeps) *sweeps = h->table_sweeps;
+    if (slots) *slots = h->table_slots;
+    if (without) *without = h->table_without;
+    if (pool_full) *pool_full = h->table_full;
+    if (stale) *stale = h->table_stale;
     return LV_OK;
 }
 
@@ -2101,6 +2125,8 @@ int lv_clear_stats(lv_handle *h) {
     h->act_evaluated = h->act_full = h->act_active = 0;
     h->act_recall = -1.0;
     h->act_fell_back = 0;
+    h->table_sweeps = h->table_slots = h->table_without = 0;
+    h->table_full = h->table_stale = 0;
     return LV_OK;
 }
 

@@ -148,7 +148,9 @@ struct NctView {
     uint8_t *lg = nullptr;      // [V] log2 of the vertex's slots; 0 = no valid table, NCT_NEVER = none ever
     uint32_t *off = nullptr;    // [V] first slot
     GSlot *slots = nullptr;     // the pool: cap slots, *cursor of them taken
-    u64 *cursor = nullptr;      // [0] slots taken, [1] vertices marked NCT_NEVER
+    // [0] slots taken, [1] vertices marked NCT_NEVER; [2], [3]: 1 when some table
+    // found the pool used up / went stale
+    u64 *cursor = nullptr;
     u64 cap = 0;
     int32_t *queue = nullptr;   // [V] vertices for the CTA build
     int32_t *qctr = nullptr;    // its count, next

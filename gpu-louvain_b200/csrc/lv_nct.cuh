@@ -45,6 +45,11 @@ __device__ __forceinline__ bool nct_add(GSlot *tb, int lg, int32_t c, u64 w, uin
     return false;
 }
 
+// Sets a word to 1 (a store only the first time).
+__device__ __forceinline__ void nct_flag(u64 *p) {
+    if (*(volatile u64 *)p == 0) *(volatile u64 *)p = 1;
+}
+
 // A neighbour of j, over an entry of weight w, moves between communities.
 __device__ __forceinline__ void nct_move(const NctView &t, int32_t j, int32_t from, int32_t to, u64 w) {
     const int lg = ((volatile uint8_t *)t.lg)[j];
@@ -64,7 +69,10 @@ __device__ __forceinline__ void nct_move(const NctView &t, int32_t j, int32_t fr
         s = (s + 1u) & mask;
     }
     if (ok) ok = nct_add(tb, lg, to, w, NCT_PROBES);
-    if (!ok) t.lg[j] = 0;   // stale: the next evaluation reads the row again
+    if (!ok) {
+        t.lg[j] = 0;   // stale: the next evaluation reads the row again
+        nct_flag(t.cursor + 3);
+    }
 }
 
 // Would tables be small?  A warp per sampled vertex (n of them, evenly spaced in
@@ -116,10 +124,13 @@ __global__ void __launch_bounds__(256) nct_sample_kernel(const int32_t *__restri
 __device__ __forceinline__ bool nct_alloc(const NctView &t, int32_t d, int *lg, uint32_t *off) {
     *lg = max(5, ceil_log2_i(2 * (int64_t)d));
     const u64 cap = 1ull << *lg;
-    if (*((volatile u64 *)t.cursor) + cap > t.cap) return false;
-    const u64 at = atomicAdd(t.cursor, cap);
-    *off = (uint32_t)at;
-    return at + cap <= t.cap;
+    if (*((volatile u64 *)t.cursor) + cap <= t.cap) {
+        const u64 at = atomicAdd(t.cursor, cap);
+        *off = (uint32_t)at;
+        if (at + cap <= t.cap) return true;
+    }
+    nct_flag(t.cursor + 2);
+    return false;
 }
 
 // A warp per vertex of list[0 .. n) (one update bucket, degree > 32), 32

@@ -102,7 +102,10 @@ typedef struct lv_stats {
     double modularity_ms;      /* modularity reductions                      */
     double aggregate_ms;       /* aggregation                                */
     double setup_ms;           /* level set-up (k_i, classes, hub tables)    */
-    double move_bytes;         /* algorithmic bytes of the move sweeps       */
+    double move_bytes;         /* algorithmic bytes of the move sweeps: 12
+                                  per entry and 20 per vertex, 16 per slot
+                                  where a sweep reads tables; runs in one
+                                  launch count skipped vertices too          */
     int64_t kernel_launches;   /* engine kernels launched since the handle's
                                   creation or last lv_clear_stats (counted
                                   process-wide)                              */
@@ -177,8 +180,16 @@ int lv_get_communities(lv_handle *h, int32_t *out);
  * recomputed), e.g. to drive lv_aggregate from a given community vector. */
 int lv_set_communities(lv_handle *h, const int32_t *comm);
 /* Test hook: the handle's fail_alloc-th device allocation from now on fails
- * as if the device had no memory left (0: none). */
-int lv_set_test_limits(lv_handle *h, int32_t fail_alloc);
+ * as if the device had no memory left (0: none), and the tables of late sweeps
+ * take at most table_slots slots (0: the default, half the level's entries). */
+int lv_set_test_limits(lv_handle *h, int32_t fail_alloc, int64_t table_slots);
+/* Late sweeps of large levels, since the handle's creation or lv_clear_stats:
+ * sweeps that read neighbour-community tables instead of rows, table slots
+ * taken, vertices that got no table for having too many neighbour communities,
+ * and whether some table found no slots left (and its row was summed instead)
+ * or went stale and was built again.  Any pointer may be NULL. */
+int lv_get_table_stats(lv_handle *h, int64_t *sweeps, int64_t *slots, int64_t *without, int32_t *pool_full,
+                       int32_t *stale);
 int lv_get_level_info(lv_handle *h, int32_t *V, int64_t *E, int32_t *level);
 /* The current level's work classes (LV_NUM_CLASSES entries each): vertices
  * and CSR entries per class (degree (0,4], (4,8], (8,16], (16,32], (32,84],
