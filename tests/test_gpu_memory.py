@@ -93,3 +93,60 @@ def test_level_goes_on_after_a_failed_aggregation(lvb, name):
             break
         assert failed == 1 and got == want, n
     assert 20 < n < 59
+
+
+def test_threads_share_the_device_memory(lvb):
+    """Engines, batches and CSR builds of several sizes in four threads, each
+    from create to destroy, give what they give alone: blocks and streams pass
+    from one owner to the next through the library's per-device lists."""
+    import threading
+
+    def engine(g, **kw):
+        def f():
+            with _engine(lvb, g, kw) as e:
+                q, n, m = _result(e)
+            return q, n, m.tobytes()
+        return f
+
+    def batch(graphs):
+        def f():
+            with lvb.Batch(graphs) as b:
+                b.run(GAIN)
+                r = b.results()
+            return r["communities"].tobytes(), r["modularity"].tobytes()
+        return f
+
+    def entries(g):
+        u, v, w = g.edges()
+
+        def f():
+            d = lvb.csr_from_entries_device(g.V, u, v, w)
+            with lvb.Louvain(device_csr=(d.rowptr, d.col, d.w, d.V, d.E)) as e:
+                q, n, m = _result(e)
+            d.free()
+            return q, n, m.tobytes()
+        return f
+
+    graphs = [lvb.gen_planted(300 + 900 * i, 8 + i, 12.0, 2.0, i, "uniform") for i in range(6)]
+    jobs = [engine(graphs[2]), engine(lvb.gen_rmat(14, 16, 1)), engine(lvb.gen_rmat(15, 16, 2), giant_degree=1024),
+            engine(lvb.gen_planted(10000, 24, 300.0, 15.0, 3, "uniform")),
+            engine(lvb.gen_lfr(70000, 0.4, 5)[0], active_set=True, active_start=0.2, active_min_recall=0.5),
+            batch(graphs), batch([lvb.gen_planted(20000, 40, 14.0, 3.0, 9, "uniform")] + graphs[:3]),
+            entries(lvb.gen_rmat(13, 16, 4))]
+    alone = [f() for f in jobs]
+    bad = []
+
+    def work(t):
+        try:
+            for i in np.random.default_rng(t).permutation(np.repeat(np.arange(len(jobs)), 3)):
+                if jobs[i]() != alone[i]:
+                    bad.append((t, int(i), "differs"))
+        except Exception as x:   # noqa: BLE001 -- reported below
+            bad.append((t, int(i), x))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
