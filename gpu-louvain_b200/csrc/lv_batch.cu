@@ -54,11 +54,22 @@ constexpr int CTAB = BW * WTAB;     // slots of the CTA table (the warp tables t
 constexpr int WIDE_CLAIMS = 160;    // distinct communities a warp accepts in a longer row
 // Work split of a launch (plan_launch): a team's CTA takes TEAM_PART of the
 // entries that one resident CTA would have if the batch were spread evenly
-// over the GPU.  256 planted graphs of 100 to 50,000 vertices took 27.0 /
-// 25.9 / 24.8 / 25.4 / 34.3 ms with 0.3 / 0.5 / 0.7 / 1 / 2 (152 ms with one
-// CTA per graph, the largest graph's time), 2048 of 100 to 1500 vertices 7.1 /
-// 6.0 / 5.8 / 5.8 / 5.8 ms.  A lone graph is split down to 2048 entries per CTA.
-constexpr double TEAM_PART = 0.7, TEAM_MIN_PART = 2048.0;
+// over the GPU, BATCH_MIN_PART at least.  256 planted graphs of 100 to 50,000
+// vertices took 27.0 / 25.9 / 24.8 / 25.4 / 34.3 ms with 0.3 / 0.5 / 0.7 / 1 /
+// 2 (152 ms with one CTA per graph, the largest graph's time), 2048 of 100 to
+// 1500 vertices 7.1 / 6.0 / 5.8 / 5.8 / 5.8 ms.  296 graphs of 300 vertices
+// (3600 entries) took 1.78 ms split in two and 0.93 whole.  A lone graph of
+// lv_run is split down to TEAM_MIN_PART entries per CTA.
+constexpr double TEAM_PART = 0.7, BATCH_MIN_PART = 4096.0, TEAM_MIN_PART = 2048.0;
+// Teams of many graphs of about one size do not all fit on the GPU and run in
+// waves, which costs more than they save when the parts are small.  So the
+// parts grow until the CTAs of the graphs that are not small (more than half
+// the even share) fit, up to this many entries.  148 / 200 / 296 planted graphs
+// of 2000 vertices took 2.79 / 3.24 / 3.30 ms without this, 1.69 / 2.21 / 2.42
+// with it (1.87 / 2.21 / 2.43 with one CTA each), of 10,000 vertices 10.6 / 12.3 /
+// 15.1 ms both ways (11.4 / 13.7 / 14.7); 128 of 1000 to 20,000 vertices 7.7 and
+// 8.0 ms, 8.5 with a limit of 65,536.
+constexpr double TEAM_FIT_PART = 49152.0;
 // Iteration caps that keep a launch bounded; a graph that reaches one stops
 // with LV_ERR_DEVICE (the rule itself has no cap: with min_gain <= 0 a sweep
 // loop that keeps moving at zero gain would not end).
@@ -1645,8 +1656,8 @@ int batch_begin(const int32_t *graph_ptr, int32_t G, int32_t V, int64_t E, const
 }
 
 // Launches by graph size (the order is by decreasing entries): the larger the
-// graph, the more CTAs run it, entries / (TEAM_PART * even share) of them,
-// rounded up to a power of two and at most 16 (the largest cluster).
+// graph, the more CTAs run it, one per part of its entries, rounded up to a
+// power of two and at most 16 (the largest cluster).
 int plan_launch(lv_batch *b, const std::vector<int32_t> &order) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
@@ -1654,12 +1665,23 @@ int plan_launch(lv_batch *b, const std::vector<int32_t> &order) {
     if (!widest) return bfail(b, LV_ERR_CUDA, "batch kernel attributes");
     int64_t total = 0;
     for (int64_t e : b->entries_h) total += e;
-    const double part = std::max(TEAM_MIN_PART, TEAM_PART * (double)total / (2.0 * (sms > 0 ? sms : 148)));
-    b->tiers.clear();
-    for (int32_t i = 0; i < b->G; ++i) {
+    const int resident = 2 * (sms > 0 ? sms : 148);
+    const double share = (double)total / resident;
+    double part = std::max(BATCH_MIN_PART, TEAM_PART * share);
+    auto team_of = [&](int32_t i) {
         const double e = (double)b->entries_h[order[i]];
         int nc = 1;
         while (nc < widest && e > part * nc) nc *= 2;
+        return nc;
+    };
+    for (; part < TEAM_FIT_PART; part *= 1.2) {
+        int64_t ctas = 0;
+        for (int32_t i = 0; i < b->G && (double)b->entries_h[order[i]] > 0.5 * share; ++i) ctas += team_of(i);
+        if (ctas <= resident) break;
+    }
+    b->tiers.clear();
+    for (int32_t i = 0; i < b->G; ++i) {
+        const int nc = team_of(i);
         if (b->tiers.empty() || b->tiers.back().nc != nc) b->tiers.push_back({nc, i, i});
         b->tiers.back().hi = i + 1;
     }

@@ -301,3 +301,26 @@ def test_run_batch_sharded_two_ranks(lvb):
     graphs = [lvb.gen_planted(200 + 97 * i, 4 + i % 5, 10.0, 2.0, seed=i) for i in range(9)]
     ref = _oracle_runner(graphs, 1e-6, 0, 0)
     assert [(r["modularity"], r["communities"].tolist(), r["levels"]) for r in ref] == got[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,V", [(40, 2000), (148, 2000), (200, 2000), (296, 2000), (296, 300), (16, 2000), (1, 30000)])
+def test_teams_of_like_graphs_run_at_a_time(lvb, G, V):
+    """Graphs of about one size whose parts would be small: the CTAs of their
+    teams fit on the GPU together (two per SM) instead of running in waves, few
+    or large graphs still get teams, and the results are lv_run's."""
+    import torch
+    resident = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    graphs = [lvb.gen_planted(V, max(4, V // 60), 13.0, 2.0, i, "uniform") for i in range(G)]
+    with lvb.Batch(graphs) as b:
+        ctas = b.stats()["ctas"]
+        b.run(1e-6)
+        r = b.results()
+        parts = b.split(r["communities"])
+    assert G <= ctas <= resident
+    if 16 * G <= resident:
+        assert ctas >= 4 * G
+    for i in (0, G // 2, G - 1):
+        with lvb.Louvain(graphs[i]) as e:
+            assert e.run(1e-6) == r["modularity"][i]
+            assert np.array_equal(e.original_to_community()[0], parts[i])
