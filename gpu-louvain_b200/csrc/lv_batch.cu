@@ -52,6 +52,7 @@ constexpr int WTAB = 256;           // slots of one warp's table
 constexpr int DW = WTAB / 2;        // degree / merged-row bound served by a warp table
 constexpr int CTAB = BW * WTAB;     // slots of the CTA table (the warp tables together)
 constexpr int WIDE_CLAIMS = 160;    // distinct communities a warp accepts in a longer row
+constexpr int FEW_WIDE = 2;         // longer rows per CTA that are not tried by a warp first
 // Work split of a launch (plan_launch): a team's CTA takes TEAM_PART of the
 // entries that one resident CTA would have if the batch were spread evenly
 // over the GPU, BATCH_MIN_PART at least.  256 planted graphs of 100 to 50,000
@@ -647,7 +648,11 @@ static __device__ void decide_cta(const Rows &L, const BatchParams &P, const GSt
 // while the row shows at most WIDE_CLAIMS distinct communities (most rows of
 // an aggregated level after its first sweeps), else a whole CTA afterwards
 // (the vertices are listed in members, free during sweeps).  A vertex whose
-// table needs the graph's one global table is left to the first CTA.
+// table needs the graph's one global table is left to the first CTA.  When a
+// CTA has no more than FEW_WIDE of them, they go to whole CTAs at once: a warp
+// alone reads a long row slowly and its attempt is often in vain (512 R-MAT-10
+// graphs 8.73 ms, with 2 / 4 rows 8.16 / 8.39; 200 stars of 500 vertices 1.00 ->
+// 0.94; 2048 planted graphs of 100 to 1500 vertices 5.59 both ways).
 static __device__ void decide_wide(const Rows &L, const BatchParams &P, const GState &gs, const Team &t,
                             const int32_t *list, int32_t n, u64 drift, BatchSmem &sm) {
     constexpr int U = 2;
@@ -662,6 +667,10 @@ static __device__ void decide_wide(const Rows &L, const BatchParams &P, const GS
     for (int32_t i = t.warp(); i < n; i += t.warps()) {
         const int32_t v = list[i];
         if (drift < P.lim[v]) continue;
+        if (n <= FEW_WIDE * t.nc) {
+            if (lane == 0) ovf[atomicAdd(novf, 1)] = v;
+            continue;
+        }
         const int32_t r0 = L.r0(v), r1 = L.r1(v);
         const int32_t own = P.comm[v];
         const u64 kv = P.k[v], sown = P.S[own];

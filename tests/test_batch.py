@@ -324,3 +324,36 @@ def test_teams_of_like_graphs_run_at_a_time(lvb, G, V):
         with lvb.Louvain(graphs[i]) as e:
             assert e.run(1e-6) == r["modularity"][i]
             assert np.array_equal(e.original_to_community()[0], parts[i])
+
+
+@pytest.mark.gpu
+def test_few_and_many_long_rows(lvb, orc):
+    """Graphs around the limits at which long rows go to whole CTAs at once (two
+    per CTA of the team), with rows that a warp could and could not hold."""
+    def graph(V, hubs, degree, seed):
+        rng = np.random.default_rng(seed)
+        base = lvb.gen_planted(V, max(4, V // 50), 6.0, 1.0, seed, "uniform")
+        u, v, w = base.edges()
+        hu = np.repeat(np.arange(hubs), degree)
+        hv = np.concatenate([rng.choice(np.arange(hubs, V), degree, False) for _ in range(hubs)])
+        u, v = np.concatenate([u, hu]), np.concatenate([v, hv])
+        w = np.concatenate([w, rng.integers(1, 9, len(hu)) / 8.0]).astype(np.float32)
+        n = u != v
+        rows, cols, ww = np.concatenate([u, v[n]]), np.concatenate([v, u[n]]), np.concatenate([w, w[n]])
+        o = np.lexsort((cols, rows))
+        rp = np.zeros(V + 1, np.int32)
+        np.cumsum(np.bincount(rows, minlength=V), out=rp[1:])
+        return lvb.Graph(rp, cols[o].astype(np.int32), ww[o])
+
+    graphs = [graph(600, k, d, 10 * k + d) for k in (1, 2, 3, 5) for d in (140, 400)]
+    graphs += [graph(9000, k, 700, k) for k in (2, 4, 5, 16, 31, 32, 33, 40)]
+    with lvb.Batch(graphs) as b:
+        b.run(1e-6)
+        r = b.results()
+        parts = b.split(r["communities"])
+        for i, g in enumerate(graphs):
+            o = orc.Oracle(g.rowptr, g.col, g.w, 1)
+            q, _ = o.run(1e-6, 0)
+            assert r["modularity"][i] == q, i
+            assert np.array_equal(parts[i], o.original_to_community()), i
+            o.close()
