@@ -236,12 +236,14 @@ def ncu_class_split(csv_path: str) -> dict:
 
     Launches are attributed the way the engine issues a sweep: each degree
     bucket's move kernels, then (buckets 4 to 6) collect_movers_kernel, then
-    apply_movers_kernel; a bucket is named by its move kernel
-    (move_group_*<G,2G>: G = 4/8/16/32 -> buckets 0-3, <32,256> -> bucket 4)
-    or, for the warp buckets, by the one before it in the sweep, so every
-    bucket from 3 on must hold vertices.  Lists recorded with separate
-    corr_*_kernel and commit_kernel launches name buckets 4 to 6 by the former
-    (corr_group_kernel<32>, corr_cta_kernel<128>, <256|512>).  In bucket 6 the giant kernels
+    apply_movers_kernel, and s2_kernel after the last bucket.  Buckets 0 to 3
+    and a short bucket 4 are named by their move kernel (move_group_*<G,2G>: G =
+    4/8/16/32, or <32,256>), bucket 6 by its giants or by the large queue
+    (move_fallback_kernel<..., 1>), the others by their order among buckets 4 to
+    6; a lone bucket 4 or 5, which launch the same warp kernel, goes to
+    "unnamed".  Lists recorded with separate corr_*_kernel and commit_kernel
+    launches name buckets 4 to 6 by the former (corr_group_kernel<32>,
+    corr_cta_kernel<128>, <256|512>).  In bucket 6 the giant kernels
     (giant_stage_*, giant_merge_* and the large queue after them) form the
     b6_giants class, as the engine's class events bracket them."""
     import csv
@@ -282,33 +284,50 @@ def ncu_class_split(csv_path: str) -> dict:
 
     out = {c: {"class_launches": 0, "kernel_launches": 0, "ms": 0.0, "dram_bytes": 0.0}
            for c in CLASS_NAMES[:8]}
-    seg = []
-
+    out["unnamed"] = dict(out[CLASS_NAMES[0]])
     MOVERS = ("collect_movers", "apply_movers", "corr_", "commit_kernel")
-    last = 3   # bucket of the sub-round before
 
-    def close(seg):
-        nonlocal last
+    def named(seg):
+        """Bucket of a sub-round's launches by their names: 0 to 6, None when
+        the order has to tell, with whether it may be bucket 6."""
         names = [short(launches[i]["name"]) for i in seg]
-        moves = [i for i, n in zip(seg, names) if not n.startswith(MOVERS)]
         corr = [n for n in names if n.startswith("corr_")]
-        grp = [re.match(r"move_group\w*<(\d+),(?: *(256)\b)?", n) for n in names]
-        grp = [m for m in grp if m]
+        grp = [m for m in (re.match(r"move_group\w*<(\d+),(?: *(256)\b)?", n) for n in names) if m]
         if grp:
-            b = 4 if grp[0].group(2) else {4: 0, 8: 1, 16: 2, 32: 3}.get(int(grp[0].group(1)))
-        elif any(n.startswith("corr_group_kernel<32") for n in corr):
-            b = 4
-        elif any(n.startswith("corr_cta_kernel<128") for n in corr):
-            b = 5
-        elif corr or any(n.startswith("giant_") for n in names):
-            b = 6
-        elif moves:
-            b = last + 1 if 3 <= last < 6 else 4
-        else:
-            return
+            return (4 if grp[0].group(2) else {4: 0, 8: 1, 16: 2, 32: 3}.get(int(grp[0].group(1)))), False
+        if any(n.startswith("corr_group_kernel<32") for n in corr):
+            return 4, False
+        if any(n.startswith("corr_cta_kernel<128") for n in corr):
+            return 5, False
+        if corr or any(n.startswith("giant_") for n in names):
+            return 6, True
+        return None, any(re.match(r"move_fallback_kernel<.*, 1>", n) for n in names)
+
+    def close(sweep):
+        """Books a sweep's sub-rounds."""
+        marks = [named(seg) for seg in sweep]
+        lo = 1 + max([b for b, _ in marks if b is not None and b <= 4], default=3)   # buckets left: max(lo, 4) .. hi
+        hi = 5 if any(b == 6 for b, _ in marks) else 6
+        left = list(range(max(lo, 4), hi + 1))
+        for b, _ in marks:
+            if b in left:
+                left.remove(b)
+        todo = [i for i, (b, _) in enumerate(marks) if b is None]
+        if len(todo) < len(left) and todo and marks[todo[-1]][1] and 6 in left:
+            marks[todo.pop()] = (6, True)
+            left.remove(6)
+        elif len(todo) < len(left) and 6 in left:
+            left.remove(6)
+        for i, b in zip(todo, left if len(todo) == len(left) else [None] * len(todo)):
+            marks[i] = (b, False)
+        for seg, (b, _) in zip(sweep, marks):
+            book(seg, b)
+
+    def book(seg, b):
+        moves = [i for i in seg if not short(launches[i]["name"]).startswith(MOVERS)]
         if b is None:
+            add({"unnamed": moves})
             return
-        last = b
         parts = {CLASS_NAMES[b]: []}
         if b == 6:
             parts["b6_giants"] = []
@@ -319,6 +338,9 @@ def ncu_class_split(csv_path: str) -> dict:
                 parts[cur].append(i)
         else:
             parts[CLASS_NAMES[b]] = moves
+        add(parts)
+
+    def add(parts):
         for c, ids in parts.items():
             if not ids:
                 continue
@@ -328,16 +350,19 @@ def ncu_class_split(csv_path: str) -> dict:
             o["ms"] += 1e3 * sum(launches[i]["s"] for i in ids)
             o["dram_bytes"] += sum(launches[i]["bytes"] for i in ids)
 
-    in_sweep = False
+    sweep, seg = [], []
     for lid in order:
         n = short(launches[lid]["name"])
-        if n.startswith(("move_", "giant_", "corr_")):
-            in_sweep = True
-        if in_sweep:
+        if seg or n.startswith(("move_", "giant_", "corr_")):
             seg.append(lid)
         if n.startswith(("apply_movers_kernel", "commit_kernel")):
-            close(seg)
-            seg, in_sweep = [], False
+            if seg:
+                sweep.append(seg)
+            seg = []
+        elif n.startswith("s2_kernel"):
+            close(sweep)
+            sweep, seg = [], []
+    close(sweep)
     for c, o in out.items():
         k = max(o["class_launches"], 1)
         o["dram_bytes_per_launch"] = o["dram_bytes"] / k

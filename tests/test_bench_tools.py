@@ -95,6 +95,48 @@ def test_ncu_class_split(tmp_path):
     assert c["b1_deg8"]["class_launches"] == 0
 
 
+def _sub_round(*names):
+    k = lambda n: "void lv::<unnamed>::" + n + "(lv::GraphView<T1>, lv::StateView)"   # noqa: E731
+    out = [(k(n), 10.0, 100) for n in names]
+    if not names[0].startswith("move_group") or "256" in names[0]:
+        out.append((k("collect_movers_kernel<float>"), 1.0, 1))
+    return out + [(k("apply_movers_kernel<float, (bool)0>"), 2.0, 1)]
+
+
+@pytest.mark.parametrize("buckets", [
+    [0, 3, 4, 5, 6], [0, 5, 6], [4, 5], [3, 4, 6], [2, 4], ["4s", 5, 6], [3, "4s", 5], ["4s", "6g"], [4, 5, "6g"],
+    ["6s"], ["5s", "6s"], [4, "6g"], [0], [6]])
+def test_ncu_class_split_names_buckets_by_order(tmp_path, buckets):
+    """Sub-rounds as the engine launches them now (s: short bucket, g: giants
+    alone), with buckets left out: none is booked under another's name, and a
+    lone one of two that launch the same kernel is not named at all."""
+    b = load_bench()
+    warp = "move_warp_narrow_kernel<float>"
+    large = "move_fallback_kernel<float, (int)1024, (int)16384, (bool)1>"
+    kernels = {0: ["move_group_narrow_kernel<(int)4, (int)8, float>"],
+               2: ["move_group_narrow_kernel<(int)16, (int)32, float>"],
+               3: ["move_group_narrow_kernel<(int)32, (int)64, float>"], 4: [warp], 5: [warp],
+               "4s": ["move_group_narrow_kernel<(int)32, (int)256, float>"],
+               "5s": ["move_rowq_narrow_kernel<float, (int)256, (int)704>"],
+               "6s": ["move_rowq_narrow_kernel<float, (int)1024, (int)8192>", large],
+               6: [warp, large, "move_rowq_narrow_kernel<float, (int)256, (int)2048>"],
+               "6g": ["giant_stage_narrow_kernel<float>", "giant_merge_kernel<(int)1024, (int)16384>", large]}
+    sweep = [r for x in buckets for r in _sub_round(*kernels[x])]
+    sweep.append(("void <unnamed>::s2_kernel(const unsigned long long *, int, unsigned long long *)", 3.0, 300))
+    path = str(tmp_path / "launches.csv")
+    write_list(path, sweep + sweep)
+    c = b.ncu_class_split(path)["classes"]
+    num = [int(str(x)[0]) for x in buckets]
+    alone = [x for x in buckets if x in (4, 5, "5s")]
+    # the order tells when both of 4 and 5 are there or a short bucket 4 is
+    ambiguous = len(alone) == 1 and "4s" not in buckets
+    for i, name in enumerate(b.CLASS_NAMES[:7]):
+        want = 2 if i in num and not (ambiguous and i in (4, 5)) and not (i == 6 and "6g" in buckets) else 0
+        assert c[name]["class_launches"] == want, (name, buckets)
+    assert c["b6_giants"]["class_launches"] == (2 if "6g" in buckets else 0)
+    assert c["unnamed"]["class_launches"] == (2 if ambiguous else 0)
+
+
 def test_committed_traffic_is_keyed_by_threshold():
     """The committed traffic file holds the dominant class for the default
     giant threshold and for the one the tuner picks on some boxes."""
