@@ -122,7 +122,8 @@ def mem(tmp_path):
     so = str(tmp_path / "shim.so")
     nvcc = subprocess.run(["which", "nvcc"], capture_output=True, text=True).stdout.strip()
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc))) if nvcc else "/usr/local/cuda"
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-I", os.path.join(cuda, "include"),
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread",
+                    "-Wl,-Bsymbolic", "-I", os.path.join(cuda, "include"),
                     "-I", os.path.join(PKG_DIR, "csrc"), str(tmp_path / "shim.cpp"), "-o", so], check=True)
     L = C.CDLL(so)
     for n in ("fake_used", "most", "in_use", "kept"):
