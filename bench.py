@@ -41,7 +41,7 @@ data path; the only collectives are the timing barrier and max/sum).
 Other workloads (not the default line):
   --workload batch : 4096 seeded planted-partition graphs (V log-uniform in
           [100, 50000], 4-256 blocks, intra degree 8-24, inter 1-4) run by
-          lv_batch_run in one persistent launch; value = graphs/s, with
+          lv_batch_run (one call, a launch per team size); value = graphs/s, with
           per-graph latency p50/p99, edge-sweeps/s, the single-graph engine
           run graph by graph on a sample (sequential launches) and the CPU
           oracle on the same sample.  Under torchrun the graphs are sharded
@@ -798,7 +798,7 @@ def run_batch(args, ranks: Ranks):
         "edge_sweeps_per_s": es_value, "edge_sweeps_per_run": es_tot // max(args.steps, 1),
         "latency_ms": {"p50": float(np.percentile(lat, 50)), "p99": float(np.percentile(lat, 99)),
                        "max": float(lat.max()), "note": "device time from a graph's start to its end "
-                                                        "inside the persistent launch"},
+                                                        "inside the launches"},
         "sequential": {"graphs_per_s": (1.0 / seq_lat) if seq_lat else None, "sample": len(pick),
                        "mean_latency_ms": seq_lat * 1e3,
                        "note": "lv_create + lv_run + map per graph (host buffers), graphs spread "
@@ -816,7 +816,7 @@ def run_batch(args, ranks: Ranks):
 
 def batch_summary(args, ranks: Ranks):
     """Compact driver-visible summary of the batched workload (the 4096-graph
-    batch in one persistent launch, device-timed, 1 warm-up + 2 timed runs)."""
+    batch in one call, device-timed, 1 warm-up + 2 timed runs)."""
     import numpy as np
     import torch
     lvb = load_pkg()
@@ -859,7 +859,7 @@ def batch_summary(args, ranks: Ranks):
             "ctas": ctas, "balanced_ms_per_launch": busy,
             "all_ok": ok, "V_total": len(rp) - 1, "E_csr_total": len(cl), "generation_s": round(t_gen, 1),
             "slowest": slowest,
-            "note": "lv_batch_run, one persistent launch per run, device time (1 warm-up + 2 timed runs); "
+            "note": "lv_batch_run, one call per run (a launch per team size), device time (1 warm-up + 2 timed runs); "
                     "bench.py --workload batch gives the full line"}
 
 

@@ -707,7 +707,7 @@ def concat_graphs(graphs):
 
 class Batch:
     """Many independent graphs, each run through the level loop of lv_run in
-    one persistent launch (lv_batch_run).  Build it from a list of Graphs or
+    a CTA or cluster per graph (lv_batch_run).  Build it from a list of Graphs or
     from a block-diagonal CSR plus graph_ptr (vertex offsets of the graphs);
     device_csr=(rowptr, col, w) device pointers borrows a resident CSR."""
 

@@ -1,5 +1,5 @@
-// lv_batch.cu -- many independent graphs in one persistent launch
-// (lv_batch_create / lv_batch_run).
+// lv_batch.cu -- many independent graphs, each run by one CTA or one
+// thread-block cluster from start to finish (lv_batch_create / lv_batch_run).
 //
 // Every graph of a batch goes through the level loop of gpulouvain.cu:30-37
 // with the rule of lv_run: sweeps of the seven degree-bucket sub-rounds
@@ -18,8 +18,9 @@
 // level-L vertices of a graph whose first vertex is v0 are v0 .. v0 + V_L - 1.
 //
 // Tables.  A vertex of degree <= DW (or a merged row of at most DW entries)
-// is handled by a lane group or a warp with a table in shared memory; a larger
-// one by the whole CTA, with the CTA's shared table when 2 * min(degree, V)
+// is handled by a lane group or a warp with a table in shared memory; a longer
+// row by a warp while it shows few communities, else (as larger merged rows) by
+// the whole CTA, with the CTA's shared table when 2 * min(degree, V)
 // slots fit, else with the graph's own global table of 2^ceil(log2(2 V0))
 // slots.  Every table is empty between uses.
 //

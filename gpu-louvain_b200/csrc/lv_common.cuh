@@ -929,7 +929,7 @@ __device__ __forceinline__ void eval_slots(int32_t *keys, u64 *vals, const int32
 // i.e. G_best - T * e_own > 0.  *delta receives the mover's contribution to
 // sum_i e_{i->C(i)} when none of its neighbours moves in the same sub-round,
 // 2 (e_best - e_own) as a wrapping uint64 (corrected for co-moving neighbours
-// by the correction kernel).
+// by apply_movers_kernel).
 __device__ __forceinline__ int32_t move_decision(const MoveCtx &m, const Best &b, u64 *delta) {
     *delta = 0;
     if (b.c == m.own) return m.own;

@@ -4,9 +4,9 @@
 // loop, gpulouvain.cu:30-37, optimiseModularity,
 // modularity_optimisation.cu:284-363, and aggregateCommunities,
 // community_aggregation.cu:248-347).  All state lives in device memory; the
-// host reads back one small totals record per sweep (the sweep's modularity
-// parts, its move count and the device error word) and a few counts per
-// level.
+// host waits for one word per sweep (whether another follows; in host-loop mode
+// it reads the sweep's modularity parts, move count and error word) and reads a
+// few counts per level.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -422,7 +422,7 @@ void next_round(lv_handle *h, StateView &st) {
 struct PinnedBlock {
     Totals tot;
     int32_t small[128];
-    volatile int32_t flag[2];   // written by sweep_end_flag_kernel: go on, sweep number
+    volatile int32_t flag[2];   // written by sweep_end_kernel: go on, sweep number
 };
 std::mutex g_pinned_mu;
 std::vector<PinnedBlock *> g_pinned_free;
@@ -877,7 +877,7 @@ int modularity(lv_handle *h, double *q) {
 
 // One sweep followed by the modularity of the resulting state.  The edge
 // pass of calculateModularity is replaced by the exact update of
-// sum_i e_{i->C(i)} accumulated by the move and correction kernels; only the
+// sum_i e_{i->C(i)} accumulated by the move and mover kernels; only the
 // sum of Sigma_tot^2 is recomputed (a pass over V).
 int sweep_and_q(lv_handle *h, int64_t *moves, double *q) {
     h->singletons = false;

@@ -1,6 +1,6 @@
 // lv_mem.cu -- device memory and streams of the library's objects.
 //
-// Handles, batches and the CSR builders ask for dozens of buffers, up to 20 GB
+// Handles, batches and the CSR builders ask for dozens of buffers, 55 GB in all
 // for an R-MAT-24 run, and a program that runs one graph after another asks
 // for nearly the same sizes again.  Mapping that memory anew cost 150 of 370
 // ms of such a run when each graph's entry count differed a little from the

@@ -144,12 +144,14 @@ int lv_create_device(const int32_t *d_rowptr, const int32_t *d_col, const float 
 /* Return to level 0 with singleton communities (no reallocation). */
 int lv_reset(lv_handle *h);
 /* deleteStructures (utils.cu:108-141).  The handle's device memory goes back
- * to the library's per-device memory pool, which keeps it mapped so that the
- * next handle on that device reuses it instead of allocating again; call
- * lv_trim_device_memory to return it to the system. */
+ * to the library's per-device blocks, kept for the next handle on that device
+ * (kept and used blocks together exceed the most that was in use at one time
+ * by an eighth at most); call lv_trim_device_memory to return them to the
+ * system. */
 int lv_destroy(lv_handle *h);
-/* Release the device memory that destroyed handles left in the library's pool
- * for `device` (memory of live handles is untouched).  No counterpart in the
+/* Release the device memory that the library keeps for `device`: blocks of
+ * destroyed handles and batches, of CSR builds and of arrays given to
+ * lv_free_device (memory of live objects is untouched).  No counterpart in the
  * reference, which allocates and frees per call. */
 int lv_trim_device_memory(int32_t device);
 const char *lv_last_error(const lv_handle *h);
@@ -298,6 +300,9 @@ int lv_gen_lfr(int32_t V, double tau1, double mean_degree, int32_t kmax, double 
 int lv_gen_rmat_device(int32_t scale, int32_t edge_factor, uint64_t seed, double a, double b,
                        double c, int32_t weight_mode, int32_t device, int32_t *V, int64_t *E,
                        int32_t **d_rowptr, int32_t **d_col, float **d_w);
+/* Gives back an array that the library allocated on the device (waits for the
+ * device, as cudaFree does).  The memory stays with the library for its next
+ * allocation until lv_trim_device_memory. */
 void lv_free_device(void *p);
 
 /* ---- allocation-free modularity of a given partition ----
@@ -381,8 +386,9 @@ int lv_active_predict(const uint16_t *model, const float *features, int64_t n, i
  * graph_ptr[g] .. graph_ptr[g+1]-1 (graph_ptr is a HOST array of num_graphs+1
  * nondecreasing offsets, graph_ptr[0] = 0, graph_ptr[num_graphs] = V) and its
  * rows reference only its own vertices.  lv_batch_run runs the level loop of
- * lv_run on every graph in one persistent launch (one CTA per graph at a time,
- * largest graphs first); each graph's communities, modularity, level and sweep
+ * lv_run on every graph on the device: one launch per team size, side by side,
+ * a team being the one CTA or the thread-block cluster of up to 16 that runs a
+ * graph (larger graphs get larger teams and start first); each graph's communities, modularity, level and sweep
  * counts equal those of lv_create + lv_run on that graph alone.  Each graph
  * gets its own fixed-point scale, as lv_create would choose it.  Whole-CSR
  * errors (offsets, column range, weights, a graph of more than
@@ -412,7 +418,7 @@ int lv_batch_get_results(lv_batch *b, int32_t *communities, double *modularity, 
  * launch (ms).  Any pointer may be NULL. */
 int lv_batch_get_graph_stats(lv_batch *b, int32_t *levels, int64_t *sweeps, int64_t *edge_sweeps,
                              double *latency_ms);
-/* Last run: device time of the launch (ms, CUDA events), total edge-sweeps
+/* Last run: device time of its launches (ms, CUDA events), total edge-sweeps
  * and vertex-sweeps (sums over sweeps of the level's entries / vertices), and
  * the number of CTAs launched.  Any pointer may be NULL. */
 int lv_batch_get_stats(lv_batch *b, double *device_ms, int64_t *edge_sweeps, int64_t *vertex_sweeps,
