@@ -489,9 +489,8 @@ int ensure_occ(lv_handle *h, size_t entries, size_t hubs) {
         // outgrown buffers for the next run to ask for again
         const size_t all = (size_t)h->E0, want = std::max(entries, std::min(entries + entries / 4 + 1, all));
         const size_t more = std::min(4 * entries, all);
-        size_t avail = 0, total = 0;
-        const bool grown = h->occ_cap > 0 && more > want && cudaMemGetInfo(&avail, &total) == cudaSuccess &&
-                           more * STAGING_BYTES <= total / 8 && alloc_staging(h, more) == LV_OK;
+        const bool grown = h->occ_cap > 0 && more > want && more * STAGING_BYTES <= mem_total(h->device) / 8 &&
+                           alloc_staging(h, more) == LV_OK;
         if (!grown) LV_TRY(alloc_staging(h, want));
     }
     if (hubs > h->nocc_cap) {
@@ -982,7 +981,13 @@ __global__ void sweep_end_kernel(const SweepBlock *blk, LoopState *ls, volatile 
 }
 
 // Tables pay off on levels whose sweeps are bound by their rows: below this many
-// entries the tables save less than their checks cost.
+// entries the tables save less than their checks and builds cost.  Runs without
+// tables / from 2^21 / from 2^18 entries, ms: R-MAT scale 16 (1.8 million
+// entries) 8.59 / 8.58 / 8.80, 17 (with edge factor 16, 3.7 million) 15.54 / 13.45
+// / 13.46, 18 (7.6 million) 16.55 / 14.45 / 14.35, planted graph of 3000 vertices and
+// 0.8 million entries 0.56 / 0.56 / 0.62.  Where one sweep is left after the switch
+// they cost a little (20,000 vertices, 5.6 million entries 1.14 / 1.35), and the
+// checks alone up to 2 % (LFR graph of 300,007 vertices 4.89 / 5.01).
 constexpr int64_t NCT_MIN_ENTRIES = LV_NCT_MIN_ENTRIES;
 // ... once the movers' rows, which the table updates visit with random
 // accesses, are a small part of the entries: lv_run of R-MAT-24 takes 240 / 236

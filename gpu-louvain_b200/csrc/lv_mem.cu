@@ -38,7 +38,7 @@ constexpr size_t MAX_STREAMS = 16;
 struct DeviceMemory {
     cudaMemPool_t pool = nullptr;
     std::vector<MemBlock> kept;      // oldest first
-    size_t kept_bytes = 0, live_bytes = 0, peak_bytes = 0;
+    size_t kept_bytes = 0, live_bytes = 0, peak_bytes = 0, total_bytes = 0;
     std::vector<cudaStream_t> streams;
 };
 
@@ -212,6 +212,18 @@ cudaError_t mem_trim(int dev) {
 bool mem_pooled(int dev) {
     std::lock_guard<std::mutex> lock(g_mu);
     return dev >= 0 && dev < MAX_DEVICES && pool_of(dev) != nullptr;
+}
+
+size_t mem_total(int dev) {
+    if (dev < 0 || dev >= MAX_DEVICES) return 0;
+    std::lock_guard<std::mutex> lock(g_mu);
+    size_t avail = 0, &total = g_dev[dev].total_bytes;
+    // asked once: the call takes tens of milliseconds at times
+    if (!total && cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+        cudaGetLastError();
+        total = 0;
+    }
+    return total;
 }
 
 cudaError_t MemSet::alloc(void **p, size_t bytes, cudaStream_t s) {

@@ -20,6 +20,7 @@ cudaError_t mem_take(int dev, size_t bytes, cudaStream_t s, MemBlock *out);
 void mem_give(int dev, const MemBlock &b, cudaStream_t s);
 cudaError_t mem_trim(int dev);
 bool mem_pooled(int dev);   // the device has a stream-ordered pool
+size_t mem_total(int dev);  // bytes of the current device dev; 0: unknown
 // The buffers of one owner.
 struct MemSet {
     int dev = 0;

@@ -1886,6 +1886,11 @@ void launch_move_giants(const GraphView<WT> &g, const StateView &st, const HubGl
 // 14.78 / 14.78 / 15.6, R-MAT scale 14 4.74 / 3.47 / 3.5, scale 16 5.90 /
 // 5.08 / 5.1, scale 18 15.0 / 14.8 / 16.3, scale 20 27.3 / 27.2 / 27.3:
 // where every warp has several rows anyway, the warp per row is the cheaper.
+// One limit at a time, off / as it is / four times as high: bucket 4 R-MAT-16
+// 8.79 / 8.58 / 8.58 and LFR 1,000,003 18.4 / 18.4 / 18.8; bucket 5 R-MAT-14 3.57 /
+// 3.33 / 3.34 and LFR 1,000,003 18.4 / 18.4 / 19.1; bucket 6 R-MAT-14 4.28 / 3.33 /
+// 3.33, LFR 300,007 6.08 / 5.01 / 5.02 and R-MAT-18 14.4 / 14.4 / 15.7 (runs on a
+// kept handle).
 constexpr int32_t SMALL_B4_PER_SM = 192, SMALL_B5_PER_SM = 56, SMALL_B6_PER_SM = 10;
 
 void clear_move_state(const FallbackSet &fs, const HubGlobal &hg, cudaStream_t s) {

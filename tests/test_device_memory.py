@@ -53,6 +53,7 @@ cudaError_t cudaFree(void *p) {
     return cudaSuccess;
 }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }
+cudaError_t cudaMemGetInfo(size_t *a, size_t *t) { *t = f_room; *a = f_room - f_used; return cudaSuccess; }
 
 void fake_room(size_t n) { f_room = n; }
 size_t fake_used() { return f_used; }
