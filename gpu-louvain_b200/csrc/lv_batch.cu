@@ -53,6 +53,11 @@ constexpr int WTAB = 256;           // slots of one warp's table
 constexpr int DW = WTAB / 2;        // degree / merged-row bound served by a warp table
 constexpr int CTAB = BW * WTAB;     // slots of the CTA table (the warp tables together)
 constexpr int WIDE_CLAIMS = 160;    // distinct communities a warp accepts in a longer row
+// Graphs with fewer entries evaluate every vertex: their few sweeps skip less
+// than the limits cost to keep (ms with / without skipping: 8192 planted graphs
+// of 60 to 160 vertices 12.0 / 11.4, 592 R-MAT-8 graphs 2.48 / 2.36, 592 planted
+// graphs of 200 vertices 1.36 / 1.35, of 400 (about 5400 entries) 1.57 / 1.63).
+constexpr int64_t SKIP_MIN_ENTRIES = 4608;
 constexpr int FEW_WIDE = 2;         // longer rows per CTA that are not tried by a warp first
 // Work split of a launch (plan_launch): a team's CTA takes TEAM_PART of the
 // entries that one resident CTA would have if the batch were spread evenly
@@ -140,14 +145,13 @@ struct GState {
     int dsh;        // drift is counted in units of 2^dsh
     float dunit;    // 2^-dsh
     bool narrow;    // level-0 weights fit 32 bits
-    bool sym;       // every entry has its mirror entry (same weight): vertices may be skipped
+    bool sym;       // every entry has its mirror entry (same weight)
+    bool skip;      // vertices may be skipped: sym, and the graph is not too small
     // what one move of a vertex of weight k adds to the drift: an upper bound of 2 k
     __device__ __forceinline__ u64 drift_of(u64 k) const { return ((2 * k) >> dsh) + 1; }
 };
 
 struct Acc {
-    int status;
-    int32_t levels;
     int64_t sweeps, edge_sweeps, vertex_sweeps, moves;
     double q;
 };
@@ -290,6 +294,17 @@ struct BatchSmem {
     int32_t err, nbig, cnt;
     uint8_t ord[BW][32];       // a warp's chunk: lanes holding vertices to decide, in order
     uint8_t occ[BW][DW];       // claimed slots of the warp's group tables
+    // State that is the same in every thread.  In registers it was spilled in
+    // the sub-rounds' loops, and the local memory of 1024 threads pushed the
+    // graph's state out of L1 (stack frame 248 -> 120 bytes; 2048 planted graphs
+    // of 100 to 1500 vertices 5.52 -> 5.07 ms, 592 of 1600 4.35 -> 4.09, 200 stars of
+    // 500 vertices 0.89 -> 0.79).  gs, rows: every thread writes the same values
+    // before it reads them; the others are thread 0's.
+    GState gs;
+    Rows rows;
+    Acc acc;
+    double q_before;           // modularity before the current sweep
+    u64 e_own;                 // sum of e_{i->C(i)}
 };
 
 // The CTAs that run one graph together: this CTA alone (nc == 1), or every
@@ -495,7 +510,7 @@ static __device__ void decide_groups(const Rows &L, const BatchParams &P, const 
         bool need = false, lsingle = false;
         if (lane < cs && idx < n) {
             lv = list[idx];
-            need = drift >= P.lim[lv];
+            need = !gs.skip || drift >= P.lim[lv];
         }
         const unsigned mask = __ballot_sync(FULL, need);
         if (!mask) continue;
@@ -573,7 +588,7 @@ static __device__ void decide_groups(const Rows &L, const BatchParams &P, const 
                 u64 d;
                 const int32_t nc = move_decision(m, b, &d);
                 P.newc[v] = nc;
-                P.lim[v] = (nc == own && gs.sym && !single) ? skip_limit(m, b, drift, gs.dunit) : 0;
+                if (gs.skip) P.lim[v] = (nc == own && !single) ? skip_limit(m, b, drift, gs.dunit) : 0;
             }
         }
         __syncwarp();
@@ -639,7 +654,7 @@ static __device__ void decide_cta(const Rows &L, const BatchParams &P, const GSt
             u64 d;
             const int32_t nc = move_decision(m, x, &d);
             P.newc[v] = nc;
-            P.lim[v] = (nc == own && gs.sym && !single) ? skip_limit(m, x, drift, gs.dunit) : 0;
+            if (gs.skip) P.lim[v] = (nc == own && !single) ? skip_limit(m, x, drift, gs.dunit) : 0;
         }
     }
     __syncthreads();
@@ -667,7 +682,7 @@ static __device__ void decide_wide(const Rows &L, const BatchParams &P, const GS
     __syncwarp();
     for (int32_t i = t.warp(); i < n; i += t.warps()) {
         const int32_t v = list[i];
-        if (drift < P.lim[v]) continue;
+        if (gs.skip && drift < P.lim[v]) continue;
         if (n <= FEW_WIDE * t.nc) {
             if (lane == 0) ovf[atomicAdd(novf, 1)] = v;
             continue;
@@ -732,7 +747,7 @@ static __device__ void decide_wide(const Rows &L, const BatchParams &P, const GS
             u64 d;
             const int32_t nc = move_decision(m, b, &d);
             P.newc[v] = nc;
-            P.lim[v] = (nc == own && gs.sym && !single) ? skip_limit(m, b, drift, gs.dunit) : 0;
+            if (gs.skip) P.lim[v] = (nc == own && !single) ? skip_limit(m, b, drift, gs.dunit) : 0;
         }
     }
     t.sync();
@@ -758,8 +773,8 @@ static __device__ void decide_wide(const Rows &L, const BatchParams &P, const GS
 // of this sub-round.  The neighbours need a new evaluation (lim = 0).  A warp
 // takes chunks of the list as in decide_groups and spreads the movers of a
 // chunk over lane groups of 8; wrapping uint64 sum.
-static __device__ __forceinline__ u64 commit_delta(const Rows &L, const BatchParams &P, const Team &t,
-                                            const int32_t *list, int32_t n, BatchSmem &sm) {
+static __device__ __forceinline__ u64 commit_delta(const Rows &L, const BatchParams &P, const GState &gs,
+                                            const Team &t, const int32_t *list, int32_t n, BatchSmem &sm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int grp = lane >> 3, gl = lane & 7;
     uint8_t *ord = sm.ord[warp];
@@ -795,7 +810,7 @@ static __device__ __forceinline__ u64 commit_delta(const Rows &L, const BatchPar
                 if (x == v) continue;
                 const u64 w = L.x(e);
                 const int32_t cx = P.comm[x], nx = P.newc[x];
-                P.lim[x] = 0;
+                if (gs.skip) P.lim[x] = 0;
                 if (nx != cx) {
                     if (nv == nx) d += w;
                     if (ov == cx) d -= w;
@@ -854,12 +869,12 @@ static __device__ u64 sweep(const Rows &L, const BatchParams &P, const GState &g
         if (nb) decide_wide(L, P, gs, t, bl + o + ns, nb, drift, sm);
         t.sync();
         if (nb && t.tid() == 0) *(t.nc == 1 ? &sm.nbig : &t.scr->nbig) = 0;   // used again after the barriers below
-        d += commit_delta(L, P, t, bl + o, ns + nb, sm);
+        d += commit_delta(L, P, gs, t, bl + o, ns + nb, sm);
         t.sync();
         u64 dd = 0;
         const int32_t mv = commit_list(P, gs, t, bl + o, ns + nb, &dd);
         moved += (u64)mv;
-        if (__any_sync(FULL, mv != 0)) {
+        if (gs.skip && __any_sync(FULL, mv != 0)) {
             dd = warp_sum_u64(dd);
             if ((threadIdx.x & 31) == 0) atomicAdd((u64 *)drift_at, dd);
         }
@@ -926,6 +941,7 @@ static __device__ void level_setup(const Rows &L, const BatchParams &P, GState &
         tt = team_totals(tt, t, sm);
         gs.T = tt.a;
         gs.sym = tt.b == 0;
+        gs.skip = gs.sym && gs.E >= SKIP_MIN_ENTRIES;
         // T in at most 2^40 drift units: the drift of a level stays far below 2^62
         gs.dsh = max(0, 64 - __clzll((long long)gs.T) - 40);
         gs.dunit = ldexpf(1.0f, -gs.dsh);
@@ -994,19 +1010,24 @@ static __device__ void level_setup(const Rows &L, const BatchParams &P, GState &
 // without moves; changed = some sweep gained (> 0).  Then
 // originalToCommunity <- C(originalToCommunity) (:251-257, :361).
 static __device__ int optimise_level(const Rows &L, const BatchParams &P, const GState &gs, Team &t, BatchSmem &sm,
-                              Acc &acc) {
+                              int *status) {
     Totals5 tt{};
     tt.a = own_weight(L, P, gs, t);
     tt.s2 = s2_part(P, gs, t);
     tt = team_totals(tt, t, sm);
-    u64 e_own = tt.a;
-    double q_before = modularity_from(gs, e_own, tt.s2);
+    u64 &e_own = sm.e_own;
+    double &q_before = sm.q_before;
+    if (threadIdx.x == 0) {
+        e_own = tt.a;
+        q_before = modularity_from(gs, tt.a, tt.s2);
+    }
+    __syncthreads();
     double gain = P.min_gain;
     int changed = 0, sw = 0;
     while (gain >= P.min_gain) {
         if (P.max_sweeps > 0 && sw >= P.max_sweeps) break;
         if (sw >= P.sweep_cap) {
-            acc.status = LV_ERR_DEVICE;
+            *status = LV_ERR_DEVICE;
             break;
         }
         tt = Totals5{};
@@ -1016,22 +1037,29 @@ static __device__ int optimise_level(const Rows &L, const BatchParams &P, const 
         tt = team_totals(tt, t, sm);
         const int64_t moves = (int64_t)tt.b;
         ++sw;
-        acc.moves += moves;
+        if (threadIdx.x == 0) sm.acc.moves += moves;
         if (tt.err) {
-            acc.status = LV_ERR_DEVICE;
+            *status = LV_ERR_DEVICE;
             break;
         }
-        e_own += tt.a;
-        const double q_after = modularity_from(gs, e_own, tt.s2);
+        const u64 e_now = e_own + tt.a;
+        const double q_after = modularity_from(gs, e_now, tt.s2);
         gain = __dsub_rn(q_after, q_before);
         if (gain > 0) changed = 1;
-        q_before = q_after;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            e_own = e_now;
+            q_before = q_after;
+        }
         if (moves == 0) break;
     }
-    acc.sweeps += sw;
-    acc.edge_sweeps += (int64_t)sw * gs.E;
-    acc.vertex_sweeps += (int64_t)sw * gs.V;
-    acc.q = q_before;
+    if (threadIdx.x == 0) {
+        Acc &acc = sm.acc;
+        acc.sweeps += sw;
+        acc.edge_sweeps += (int64_t)sw * gs.E;
+        acc.vertex_sweeps += (int64_t)sw * gs.V;
+        acc.q = q_before;
+    }
     for (int32_t u = t.tid(); u < gs.V0; u += t.threads()) {
         const int32_t x = P.o2c[gs.v0 + u];
         P.o2c[gs.v0 + u] = P.comm[x];
@@ -1275,7 +1303,7 @@ static __device__ int graph_scale(const BatchParams &P, GState &gs, Team &t, Bat
 
 // The whole level loop of one graph (gpulouvain.cu:30-37).
 static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, BatchSmem &sm) {
-    GState gs;
+    GState &gs = sm.gs;
     gs.g = g;
     gs.v0 = P.job ? 0 : P.gptr[g];
     gs.V0 = P.job ? P.job_V : P.gptr[g + 1] - gs.v0;
@@ -1290,15 +1318,17 @@ static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, Batch
     gs.dunit = 1.0f;
     gs.narrow = P.job_narrow != 0;
     gs.sym = false;
+    gs.skip = false;
     if (threadIdx.x == 0) sm.err = 0;
     for (int s = threadIdx.x; s < CTAB; s += BT) {
         sm.keys[s] = -1;
         sm.vals[s] = 0;
         sm.hi[s] = 0;
     }
-    Acc acc{};
-    acc.status = LV_OK;
-    acc.q = 0.0;
+    Acc &acc = sm.acc;
+    if (threadIdx.x == 0) acc = Acc{};
+    int status = LV_OK;
+    int32_t levels = 0;
     if (P.job) {
         // the scratch area and the graph's table are this launch's own
         if (t.tid() == 0) {
@@ -1313,12 +1343,13 @@ static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, Batch
         t.sync();
     } else {
         if (t.tid() == 0) P.t_start[g] = globaltimer();
-        acc.status = graph_scale(P, gs, t, sm);
+        status = graph_scale(P, gs, t, sm);
     }
-    if (acc.status == LV_OK) {
+    if (status == LV_OK) {
         for (int32_t u = t.tid(); u < gs.V0; u += t.threads()) P.o2c[gs.v0 + u] = gs.v0 + u;
         for (;;) {
-            Rows L;
+            Rows &L = sm.rows;
+            __syncthreads();
             if (gs.cur < 0) {
                 // level 0's fixed-point weights use the graph's part of the second
                 // weight buffer, which the first aggregation does not write
@@ -1335,11 +1366,11 @@ static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, Batch
                 L.w32 = nullptr;
             }
             level_setup(L, P, gs, t, sm);
-            const int changed = optimise_level(L, P, gs, t, sm, acc);
-            acc.levels += 1;
-            if (!changed || acc.status != LV_OK) break;
-            if (aggregate(L, P, gs, t, sm) || acc.levels >= P.level_cap) {
-                acc.status = LV_ERR_DEVICE;
+            const int changed = optimise_level(L, P, gs, t, sm, &status);
+            ++levels;
+            if (!changed || status != LV_OK) break;
+            if (aggregate(L, P, gs, t, sm) || levels >= P.level_cap) {
+                status = LV_ERR_DEVICE;
                 break;
             }
         }
@@ -1347,9 +1378,9 @@ static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, Batch
     if (P.job) {
         if (t.tid() == 0) {
             P.job->q = acc.q;
-            P.job->status = acc.status;
+            P.job->status = status;
             P.job->V = gs.V;
-            P.job->levels = acc.levels;
+            P.job->levels = levels;
             P.job->cur = gs.cur;
             P.job->E = gs.E;
             P.job->sweeps = acc.sweeps;
@@ -1359,7 +1390,7 @@ static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, Batch
         }
         return;
     }
-    if (acc.status != LV_OK) {
+    if (status != LV_OK) {
         // leave the graph's global table empty for the next run
         const int64_t n = P.tbl_off[g + 1] - gs.tbl;
         for (int64_t s = t.tid(); s < n; s += t.threads()) {
@@ -1368,12 +1399,12 @@ static __device__ void run_graph(const BatchParams &P, int32_t g, Team &t, Batch
         }
     }
     for (int32_t u = t.tid(); u < gs.V0; u += t.threads())
-        P.out_comm[gs.v0 + u] = acc.status == LV_OK ? P.o2c[gs.v0 + u] - gs.v0 : -1;
+        P.out_comm[gs.v0 + u] = status == LV_OK ? P.o2c[gs.v0 + u] - gs.v0 : -1;
     if (t.tid() == 0) {
         P.q[g] = acc.q;
-        P.nc[g] = acc.status == LV_OK ? gs.V : 0;
-        P.status[g] = acc.status;
-        P.levels[g] = acc.levels;
+        P.nc[g] = status == LV_OK ? gs.V : 0;
+        P.status[g] = status;
+        P.levels[g] = levels;
         P.sweeps[g] = acc.sweeps;
         P.edge_sweeps[g] = acc.edge_sweeps;
         P.vertex_sweeps[g] = acc.vertex_sweeps;

@@ -357,3 +357,36 @@ def test_few_and_many_long_rows(lvb, orc):
             assert r["modularity"][i] == q, i
             assert np.array_equal(parts[i], o.original_to_community()), i
             o.close()
+
+
+@pytest.mark.gpu
+def test_graphs_around_the_size_from_which_vertices_are_skipped(lvb, orc):
+    """2303 to 2305 edges (4608 entries is the line) in several shapes, each as
+    one of a batch and alone in one launch: the oracle's result."""
+    rng = np.random.default_rng(8)
+    graphs = []
+    for m in (2303, 2304, 2305):
+        for V in (80, 400, 2000):
+            u, v = rng.integers(0, V, 20 * m), rng.integers(0, V, 20 * m)
+            same = (u % 8 == v % 8) | (rng.random(20 * m) < 0.1)   # eight loose blocks
+            keep = np.flatnonzero((u != v) & same)[:m]
+            u, v, w = u[keep], v[keep], rng.integers(1, 9, m) / 8.0
+            rows, cols, ww = np.concatenate([u, v]), np.concatenate([v, u]), np.concatenate([w, w])
+            o = np.lexsort((cols, rows))
+            rp = np.zeros(V + 1, np.int32)
+            np.cumsum(np.bincount(rows, minlength=V), out=rp[1:])
+            graphs.append(lvb.Graph(rp, cols[o].astype(np.int32), ww[o].astype(np.float32)))
+    with lvb.Batch(graphs) as b:
+        b.run(1e-6)
+        r = b.results()
+        parts = b.split(r["communities"])
+    for i, g in enumerate(graphs):
+        assert g.E in (4606, 4608, 4610)
+        o = orc.Oracle(g.rowptr, g.col, g.w, 1)
+        q, _ = o.run(1e-6, 0)
+        assert r["modularity"][i] == q, i
+        assert np.array_equal(parts[i], o.original_to_community()), i
+        o.close()
+        with lvb.Louvain(g) as e:
+            assert e.run(1e-6) == q
+            assert np.array_equal(e.original_to_community()[0], parts[i])
